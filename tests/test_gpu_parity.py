@@ -419,6 +419,54 @@ def test_node_width_changes_nothing(rt, kind):
         assert np.array_equal(res[8][1], res[4][1])
 
 
+@pytest.mark.parametrize("isect", [gbsp.ISECT_REFERENCE_MT, gbsp.ISECT_WATERTIGHT])
+@pytest.mark.parametrize("n_rays", [1, 31, 33, 65536 + 7])
+def test_axis_parallel_and_ragged_rays_at_both_widths(rt, n_rays, isect):
+    """Rays with zero direction components (infinite inverses) take another
+    slab form at 8-wide nodes than the rest; queue tails leave part of a warp
+    without a ray.  Both node widths (4-wide: the general visit) and both
+    kernels (per warp below 65,536 rays, per lane from there on) give the same
+    bits; small batches also agree with the oracle."""
+    import torch
+
+    s = scenes.config3_scene(width=0, height=0, n_spheres=40, level=2, seed=23)
+    r = np.random.default_rng(n_rays)
+    o = r.uniform([-9, 0.2, -9], [9, 6, 9], (n_rays, 3)).astype(np.float32)
+    d = r.standard_normal((n_rays, 3))
+    d[np.arange(n_rays) % 3 == 0, r.integers(0, 3)] = 0.0
+    d[np.arange(n_rays) % 7 == 0] = np.eye(3)[r.integers(0, 3)] * r.choice([-1.0, 1.0])
+    d = (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32)
+    rays = np.concatenate([o, d], axis=1)
+    res = {}
+    for width in (8, 4):
+        scene, ms, _ = gbsp.upload_scene(rt, s)
+        scene.set_intersection(isect)
+        scene.set_node_width(width)
+        packed = np.zeros((n_rays, 8), np.float32)
+        packed[:, 0:3], packed[:, 4:7] = rays[:, 0:3], rays[:, 3:6]
+        dr = torch.from_numpy(packed).cuda()
+        t = torch.empty(n_rays, dtype=torch.float32, device="cuda")
+        tri = torch.empty(n_rays, dtype=torch.int32, device="cuda")
+        obj = torch.empty(n_rays, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        scene.intersect_closest_device(n_rays, dr.data_ptr(), t.data_ptr(), tri.data_ptr(),
+                                       obj.data_ptr())
+        rt.synchronize()
+        res[width] = (t.cpu().numpy(), tri.cpu().numpy(), obj.cpu().numpy())
+        if n_rays > 65536:  # the same rays through the per-warp kernel
+            scene.intersect_closest_device(65535, dr.data_ptr(), t.data_ptr(), tri.data_ptr(),
+                                           obj.data_ptr())
+            rt.synchronize()
+            assert np.array_equal(bits(t.cpu().numpy()), bits(res[width][0]))
+            assert np.array_equal(tri.cpu().numpy(), res[width][1])
+    for a, b in zip(res[8], res[4]):
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+    if isect == gbsp.ISECT_REFERENCE_MT and n_rays < 100:
+        w = build_world("port", s)
+        rt_, robj, rtri, rtied = w.closest(rays, ties=True)
+        check_closest(res[8][0], res[8][1], rt_, rtri, rtied, f"{n_rays} rays")
+
+
 def test_tile_list_matches_tile_renders(rt):
     """gbsp_path_trace_tile_list renders the listed tiles in one pass exactly
     as gbsp_path_trace_tile renders each one (bit-identical pixels, the same

@@ -42,6 +42,7 @@ struct BatchItemDev {
 // single-scene render: images are bit-identical.
 // ---------------------------------------------------------------------------
 struct ManyScenes {
+    static constexpr bool kManyScenes = true;
     const BatchItemDev *items;
     const uint32_t *pathItem;
     __device__ __forceinline__ const SceneView &scene(uint32_t p) const
@@ -414,9 +415,7 @@ __global__ void __launch_bounds__(128) k_batch_sm(const BatchItemDev *__restrict
             if (tmode == 2 && sp == base) {
                 if (lPrim >= 0) {
                     const Instance &in = sv.instances[inst];
-                    Affine model;
-#pragma unroll
-                    for (int k = 0; k < 12; k++) model.r[k] = __ldg(&in.model.r[k]);
+                    const Affine model = load_affine(&in.model);
                     V3 worldHit = transform_point(model, add(lo, mul(ld, lBestT)));
                     float tw = dot(sub(worldHit, o), d);
                     if (tw < bestT || (tw == bestT && (int32_t)inst < bestInst)) {
@@ -454,9 +453,7 @@ __global__ void __launch_bounds__(128) k_batch_sm(const BatchItemDev *__restrict
             if (tmode == 1) {
                 inst = leaf_first(ref);
                 const Instance &in = sv.instances[inst];
-                Affine inv;
-#pragma unroll
-                for (int k = 0; k < 12; k++) inv.r[k] = __ldg(&in.inv.r[k]);
+                const Affine inv = load_affine(&in.inv);
                 lo = transform_point(inv, o);
                 ld = normalize(transform_vector(inv, d), &llen);
                 linvd = inverse(ld);
@@ -645,6 +642,9 @@ static void enqueue_wavefront(gbsp_batch *b)
     const bool resident = b->cfg.blocksPerSm == 0;
     const int grid = rt->smCount * (int)b->cfg.blocksPerSm;
     const int shadeGrid = resident ? shade_grid<ManyScenes>(rt->smCount) : grid;
+    uint32_t quads = b->hostItems[0].sv.nodeQuads;  // 0: the items' node widths differ
+    for (const BatchItemDev &d : b->hostItems)
+        if (d.sv.nodeQuads != quads) quads = 0;
     for (const BatchWave &w : b->waves) {
         k_reset_ctl<<<1, 32, 0, s>>>(ctl, w.paths);
         if (w.maxBounces == 0) {
@@ -660,8 +660,8 @@ static void enqueue_wavefront(gbsp_batch *b)
             const float4 *qD = wb.rayD + ((bn & 1) ? wb.cap : 0);
             k_reset_stage<<<1, 1, 0, s>>>(ctl, outQ);
             // primary rays per warp, bounce rays per lane (the frame renderer's default)
-            launch_trace_stage(bn > 0, b->watertight,
-                resident ? trace_grid<ManyScenes>(bn > 0, b->watertight, rt->smCount) : grid, s,
+            launch_trace_stage(bn > 0, b->watertight, quads,
+                resident ? trace_grid<ManyScenes>(bn > 0, b->watertight, quads, rt->smCount) : grid, s,
                 src, qO, qD, ctl + inQ, wb.hitA, wb.hitInst, ctl, counters, rt->dStatus);
             k_shade<<<shadeGrid, 128, 0, s>>>(src, wb, bn, inQ, ctl, counters);
         }

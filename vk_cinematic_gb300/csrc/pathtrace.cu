@@ -367,8 +367,8 @@ static int render_waves(gbsp_runtime *rt, const SceneView &sv, const MaterialVie
                 int e0 = timing ? rt->stage_event(s) : -1;
                 bool perLane = (opt.flags & GBSP_FLAG_TRACE_PER_LANE) ||
                     (!(opt.flags & GBSP_FLAG_TRACE_PER_WARP) && b > 0);
-                launch_trace_stage(perLane, sv.watertight != 0,
-                    trace_grid<OneScene>(perLane, sv.watertight != 0, rt->smCount), s, one, qO, qD,
+                launch_trace_stage(perLane, sv.watertight != 0, sv.nodeQuads,
+                    trace_grid<OneScene>(perLane, sv.watertight != 0, sv.nodeQuads, rt->smCount), s, one, qO, qD,
                     ctl + inQ, wb.hitA, wb.hitInst, ctl, counters, rt->dStatus);
                 int e1 = timing ? rt->stage_event(s) : -1;
                 k_shade<<<shadeGrid, 128, 0, s>>>(one, wb, b, inQ, ctl, counters);
@@ -606,7 +606,7 @@ extern "C" int gbsp_path_trace_tile_noalloc(const gbsp_context *ctx, gbsp_tile t
                 // (it changes the order of work, not the results)
                 bool perLane = (opt.flags & GBSP_FLAG_TRACE_PER_LANE) ||
                     (!(opt.flags & GBSP_FLAG_TRACE_PER_WARP) && b > 0);
-                launch_trace_stage(perLane, one.sv.watertight != 0, grid, s, one,
+                launch_trace_stage(perLane, one.sv.watertight != 0, one.sv.nodeQuads, grid, s, one,
                     wb.rayO + ((b & 1) ? wb.cap : 0), wb.rayD + ((b & 1) ? wb.cap : 0), ctl + inQ,
                     wb.hitA, wb.hitInst, ctl, counters, status);
                 k_shade<<<shade_grid<OneScene>(rt->smCount), 128, 0, s>>>(one, wb, b, inQ, ctl,

@@ -155,7 +155,8 @@ static int launch_intersect_per_lane(cudaStream_t s, const SceneView &sv, uint32
     const int blocks = (int)((n + 255) / 256);
     k_split_rays<<<blocks, 256, 0, s>>>(rays, count, o, d);
     k_reset_ctl<<<1, 32, 0, s>>>(ctl, count);
-    launch_trace_stage(true, sv.watertight != 0, smCount * 8, s, one, o, d, ctl + kCtlQueue0, hitA,
+    launch_trace_stage(true, sv.watertight != 0, sv.nodeQuads,
+        trace_grid<OneScene>(true, sv.watertight != 0, sv.nodeQuads, smCount), s, one, o, d, ctl + kCtlQueue0, hitA,
         hitInst, ctl, counters, dStatus);
     k_intersect_outputs<<<blocks, 256, 0, s>>>(sv, hitA, hitInst, count, tOut, triOut, objOut,
         attrOut, matOut);

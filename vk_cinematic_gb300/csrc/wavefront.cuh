@@ -68,6 +68,7 @@ struct WaveParams {
 // Scene source of the wave kernels: everything a path needs from its scene.
 // OneScene: one scene for the whole launch (a frame or a tile).
 struct OneScene {
+    static constexpr bool kManyScenes = false;
     SceneView sv;
     MaterialView mv;
     uint32_t maxBounces;
@@ -276,10 +277,12 @@ static __global__ void __launch_bounds__(256) k_generate(WaveParams wp, WaveBuff
     wb.rayD[p] = make_float4(d.x, d.y, d.z, __uint_as_float(rng));
 }
 
-// Closest hit, 32 queued rays per warp (primary rays by default).  7 blocks of
-// 128 per SM (72 registers): 1,521 Msamples/s on the 1080p benchmark frame
-// against 1,516 at 6 blocks and 1,521 at 8 (which spills more).
-template <class Src, bool kWT>
+// Closest hit, 32 queued rays per warp (primary rays by default: they are
+// coherent, 27.7 lanes active per instruction, and the per-lane kernel's vote
+// then only costs: a 1080p frame took 72.4 ms with it for the primary rays too,
+// 69.5 ms with this one).  7 blocks of 128 per SM (72 registers); 6 measured
+// the same.
+template <class Src, bool kWT, int kQ>
 __global__ void __launch_bounds__(128, 7) k_trace(Src src, const float4 *__restrict__ rayO,
     const float4 *__restrict__ rayD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
     unsigned int *ctl, unsigned long long *counters, uint32_t *status)
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(128, 7) k_trace(Src src, const float4 *__restr
         if (i < count) {
             float4 o4 = rayO[i], d4 = rayD[i];
             const SceneView &sv = src.scene((uint32_t)__float_as_int(o4.w));
-            RayHit h = trace_closest<true, kWT>(sv, v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z),
+            RayHit h = trace_closest<true, kWT, kQ>(sv, v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z),
                 status, cnt);
             hitA[i] = make_int4(__float_as_int(h.t), __float_as_int(h.u), __float_as_int(h.v),
                 h.prim);
@@ -324,44 +327,64 @@ __global__ void __launch_bounds__(128, 7) k_trace(Src src, const float4 *__restr
 }
 
 // Per-lane variant of k_trace (bounce rays by default).  Every lane keeps
-// its own ray and stack and advances by single steps (one stack pop: an
-// object- or mesh-level node visit, entering an object, one triangle leaf,
-// leaving an object); a lane whose ray is done takes the next queue index
-// straight away, so short rays no longer wait for the warp's longest one.
-// The fetch is a warp-aggregated atomic over the lanes that are idle at that
-// moment (__activemask), and a lane leaves the loop as soon as the queue is
-// exhausted: there is no whole-warp vote or shuffle inside the loop.  Same
+// its own ray and stack; a lane whose ray is done takes the next queue index,
+// so short rays do not wait for the warp's longest one.
+//
+// Bound: issue slots and load latency on diverged lanes, not memory (DRAM
+// under 2%, L1 55-60% busy).  A walk is a sequence of steps of five kinds (a
+// node visit, a triangle leaf, entering an object, leaving it, storing a
+// finished ray and fetching the next); when every iteration runs each lane's
+// next step, the warp issues all five kinds for a few lanes each (9.6 of 32
+// lanes active per instruction).  Here an iteration runs ONE kind, the one
+// most lanes want, and the other lanes wait for theirs to win: 17.3 lanes
+// active, and one load latency per iteration instead of up to five.  The
+// vote is one __reduce_add_sync over 6-bit counters (32 lanes fit in 6 bits).
+// Some lane always advances, and a waiting kind gains lanes until it wins.
+// 1080p benchmark frame (64 spp, 5 bounces): 85.3 ms before; 76.3 ms with the
+// 256-bit node visits (visit_node8) and 128-bit transform loads; 68.4 ms with
+// the vote; 67.8 ms with the weights below (steps that cost less than a node
+// visit win with fewer lanes).  2^20 incoherent rays against 2^18 triangles:
+// 2,366, 1,865, 1,737 and 1,768 us.
+//
+// Every full-mask intrinsic stands at the loop head or in a branch taken on
+// the vote's (warp-uniform) result; the only exit is the vote's zero.  Same
 // candidate sets, arithmetic and tie rules as trace_closest, hence the same
-// hit records.  8 blocks of 128 per SM (64 registers): on the 1080p benchmark
-// frame 8 blocks gave 1,516 Msamples/s against 1,468 at 7 (72 registers) and
-// 1,461 at 9 (56 registers, which spill).
+// hit records.
+//
+// Blocks per SM: 7 of 128 threads (72 registers): 69.5 ms against 71.0 at 8
+// (64 registers, spills) and 71.4 at 6 on the frame above.  The watertight
+// test and the per-path scenes of a batch need more registers: 6 (a
+// 641 x 359 x 7 watertight frame 1.20 against 1.22 ms at 7; an uneven batch
+// 3.27 against 3.28).
 constexpr uint32_t kMaxLaneRaySteps = 1u << 22;
 constexpr int kLaneThreads = 128;  // block size of k_trace_lane
 constexpr uint32_t kMaxLaneIterations = 1u << 28;
+enum LaneStep : int { kStepNode = 0, kStepLeaf, kStepEnter, kStepLeave, kStepRay };
+constexpr int kWeightNode = 3, kWeightLeaf = 3, kWeightEnter = 4, kWeightLeave = 5, kWeightRay = 3;
 
-template <class Src, bool kWT>
-__global__ void __launch_bounds__(kLaneThreads, 8) k_trace_lane(Src src, const float4 *__restrict__ rayO,
+template <class Src, bool kWT, int kQ>
+__global__ void __launch_bounds__(kLaneThreads, kWT || Src::kManyScenes ? 6 : 7) k_trace_lane(Src src, const float4 *__restrict__ rayO,
     const float4 *__restrict__ rayD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
     unsigned int *ctl, unsigned long long *counters, uint32_t *status)
 {
     const int lane = threadIdx.x & 31;
-    const uint32_t laneMaskLt = (1u << lane) - 1u;
     const uint32_t count = *queueCount;
     unsigned int *work = &ctl[kCtlTraceWork];
     TraceCounters cnt = {0, 0, 0, 0, 0};
     uint32_t done = 0, hits = 0;
     StackEntry stack[kStackSize];
     // State a lane touches only when it fetches a ray, enters or leaves an
-    // object, or stores a hit, kept in shared memory on purpose: the walk
-    // itself then holds just the current level's ray, bounds and stack
-    // pointer in registers.  (In a local array its stores were written
+    // object, tests a leaf or stores a hit, kept in shared memory on purpose:
+    // the walk itself then holds just the current level's ray, bound and
+    // stack pointer in registers.  (In a local array its stores were written
     // through to L2; shared memory keeps them on the SM: 1,556 against
     // 1,552 Msamples/s on the 1080p benchmark frame.)  Word w of the lane
     // is column threadIdx.x of row w, so a warp's accesses to one word are
     // contiguous.  Words: world origin 0-2, direction 3-5, inverse direction
     // 6-8; best hit over objects u 9, v 10, triangle 11, object 12; queue
-    // slot 13; object being walked 14; its best triangle's u 15, v 16.
-    __shared__ uint32_t coldWords[17 * kLaneThreads];
+    // slot 13; object being walked 14; its best triangle's u 15, v 16; the
+    // object-space direction 17-19.
+    __shared__ uint32_t coldWords[20 * kLaneThreads];
     struct ColdWords {
         volatile uint32_t *p;
         __device__ __forceinline__ volatile uint32_t &operator[](int w) const
@@ -370,16 +393,16 @@ __global__ void __launch_bounds__(kLaneThreads, 8) k_trace_lane(Src src, const f
         }
     };
     const ColdWords cold{coldWords + threadIdx.x};
-    // next: the entry to visit next (the nearest child of the last node
-    // visit, or a root), kept out of the stack; ref kEmptyChild when none
-    StackEntry next = StackEntry{kEmptyChild, 0.0f};
-    int sp = 0, base = 0;
-    int mode = 0;  // 0 needs a ray, 1 object level, 2 mesh level
+    // the node or leaf to visit next; kEmptyChild when none
+    uint32_t ref = kEmptyChild;
+    // base: stack height at which the object being walked is done, -1 at
+    // object level, -2 without a ray, -3 when the queue is drained
+    int sp = 0, base = -2;
     uint32_t steps = 0;
-    // the ray of the level being walked: world (mode 1) or object space (mode 2)
-    V3 ro = v3(0, 0, 0), rinvd = v3(0, 0, 0), ld = v3(0, 0, 0);
-    float bestT = kInf;
-    float len = 0.0f, lBestT = kInf;
+    // the ray of the level being walked (world or object space); `bound` is the
+    // largest entry distance still worth a visit at that level
+    V3 ro = v3(0, 0, 0), rinvd = v3(0, 0, 0);
+    float bestT = kInf, bound = kInf, lBestT = kInf;
     int32_t lPrim = -1;
     uint32_t pathId = 0;
     bool drained = false;
@@ -393,120 +416,152 @@ __global__ void __launch_bounds__(kLaneThreads, 8) k_trace_lane(Src src, const f
             __uint_as_float(cold[w + 2]));
     };
     for (uint32_t it = 0; it < kMaxLaneIterations; it++) {
-        if (mode == 0) {
-            unsigned int m = __activemask();
-            int leader = __ffs(m) - 1;
-            uint32_t first = 0;
-            if (lane == leader) first = atomicAdd(work, (unsigned int)__popc(m));
-            first = __shfl_sync(m, first, leader);
-            uint32_t idx = first + __popc(m & laneMaskLt);
-            if (idx >= count) {
-                drained = true;
-                break;
-            }
-            steps = 0;
-            float4 o4 = rayO[idx], d4 = rayD[idx];
-            ro = v3(o4.x, o4.y, o4.z);
-            const V3 d = v3(d4.x, d4.y, d4.z);
-            pathId = (uint32_t)__float_as_int(o4.w);
-            rinvd = inverse(d);
-            put3(0, ro);
-            put3(3, d);
-            put3(6, rinvd);
-            cold[9] = 0u;
-            cold[10] = 0u;
-            cold[11] = 0xFFFFFFFFu;
-            cold[12] = 0xFFFFFFFFu;
-            cold[13] = idx;
-            bestT = kInf;
-            sp = 0;
-            next = StackEntry{src.scene(pathId).tlasRoot, 0.0f};
-            mode = 1;
-        }
-        if (++steps > kMaxLaneRaySteps) {
-            atomicOr(status, kStatusRayStepLimit);
-            mode = 1;
-            sp = 0;  // store the best hit found so far
-            next.ref = kEmptyChild;
-        }
-        const bool levelDone = sp == (mode == 2 ? base : 0) && next.ref == kEmptyChild;
-        if (mode == 2 && levelDone) {
-            // leaving an object: its closest triangle goes back to world space
-            const V3 o = get3(0);
-            if (lPrim >= 0) {
-                const uint32_t inst = cold[14];
-                const Instance &in = src.scene(pathId).instances[inst];
-                Affine model;
-#pragma unroll
-                for (int k = 0; k < 12; k++) model.r[k] = __ldg(&in.model.r[k]);
-                V3 worldHit = transform_point(model, add(ro, mul(ld, lBestT)));
-                float tw = dot(sub(worldHit, o), get3(3));
-                if (tw < bestT || (tw == bestT && (int32_t)inst < (int32_t)cold[12])) {
-                    bestT = tw;
-                    cold[9] = cold[15];
-                    cold[10] = cold[16];
-                    cold[11] = (uint32_t)lPrim;
-                    cold[12] = inst;
+        // ---- what each lane needs next
+        if (ref == kEmptyChild) {
+            const int floor = max(base, 0);
+            while (sp > floor) {
+                sp--;
+                steps++;
+                const StackEntry top = stack[sp];
+                if (!(top.t > bound)) {
+                    ref = top.ref;
+                    break;
                 }
             }
-            ro = o;
-            rinvd = get3(6);
-            mode = 1;
-        } else if (mode == 1 && levelDone) {
-            const int32_t bestPrim = (int32_t)cold[11];
-            const uint32_t slot = cold[13];
-            hitA[slot] = make_int4(__float_as_int(bestT), (int)cold[9], (int)cold[10], bestPrim);
-            hitInst[slot] = (int)cold[12];
-            done++;
-            hits += (bestPrim >= 0 && bestT > 0.0f) ? 1u : 0u;
-            mode = 0;
-        } else {
-            StackEntry top;
-            if (next.ref != kEmptyChild) {
-                top = next;
-                next.ref = kEmptyChild;
-            } else {
-                sp--;
-                top = stack[sp];
-            }
-            uint32_t ref = top.ref;
-            float te = top.t;
-            float bound = mode == 1 ? prune_bound(bestT) : prune_bound(rmin(lBestT, bestT * len));
-            if (te > bound) {
-                // pruned
-            } else if (!child_is_leaf(ref)) {
-                if (mode == 1)
+        }
+        // children that are nodes have bit 31 clear; leaves and "none" have it set
+        int cls = base >= 0 ? kStepLeave : kStepRay;
+        if (!child_is_leaf(ref))
+            cls = kStepNode;
+        else if (ref != kEmptyChild)
+            cls = base >= 0 ? kStepLeaf : kStepEnter;
+        const uint32_t sums = __reduce_add_sync(0xFFFFFFFFu, base == -3 ? 0u : 1u << (6 * cls));
+        if (sums == 0) {
+            drained = true;
+            break;
+        }
+        // the kind with the most lanes, weighted; its number rides in the low bits
+        const int k0 = (int)(sums & 63u) * (8 * kWeightNode) + kStepNode,
+                  k1 = (int)(sums >> 6 & 63u) * (8 * kWeightLeaf) + kStepLeaf,
+                  k2 = (int)(sums >> 12 & 63u) * (8 * kWeightEnter) + kStepEnter,
+                  k3 = (int)(sums >> 18 & 63u) * (8 * kWeightLeave) + kStepLeave,
+                  k4 = (int)(sums >> 24) * (8 * kWeightRay) + kStepRay;
+        const int best = __vimax3_s32(__vimax3_s32(k0, k1, k2), k3, k4) & 7;
+        const bool mine = cls == best && base != -3;
+        if (best == kStepNode) {
+            if (mine) {
+                if (base < 0)
                     cnt.topNodes++;
                 else
                     cnt.meshNodes++;
-                next = visit_node<true, kWT, true>(src.scene(pathId).nodes,
-                    src.scene(pathId).nodeQuads, ref, ro, rinvd, bound, stack, sp, status, cnt);
-            } else if (mode == 1) {
-                // an object whose world box passed: enter its mesh
-                const uint32_t inst = leaf_first(ref);
-                cold[14] = inst;
-                const Instance &in = src.scene(pathId).instances[inst];
-                Affine inv;
-#pragma unroll
-                for (int k = 0; k < 12; k++) inv.r[k] = __ldg(&in.inv.r[k]);
-                const V3 d = get3(3);
-                ro = transform_point(inv, ro);
-                ld = normalize(transform_vector(inv, d), &len);
-                rinvd = inverse(ld);
-                cnt.meshTests++;
-                lBestT = kInf;
-                lPrim = -1;
-                base = sp;
-                next = StackEntry{__ldg(&in.blasRoot), 0.0f};
-                mode = 2;
-            } else {
-                visit_leaf_uv<true, kWT>(src.scene(pathId), ref, ro, ld, rinvd, lBestT, lPrim,
+                ref = visit_nearest<kWT, kQ>(src.scene(pathId).nodes, src.scene(pathId).nodeQuads,
+                    ref, ro, rinvd, bound, stack, sp, status, cnt.boxTests);
+            }
+        } else if (best == kStepLeaf) {
+            if (mine) {
+                visit_leaf_uv<true, kWT>(src.scene(pathId), ref, ro, get3(17), rinvd, lBestT, lPrim,
                     [&](float u, float v) {
                         cold[15] = __float_as_uint(u);
                         cold[16] = __float_as_uint(v);
                     },
                     cnt);
+                bound = rmin(prune_bound(lBestT), bound);
+                ref = kEmptyChild;
             }
+        } else if (best == kStepEnter) {
+            if (mine) {
+                // an object whose world box passed: enter its mesh
+                const uint32_t inst = leaf_first(ref);
+                cold[14] = inst;
+                const Instance &in = src.scene(pathId).instances[inst];
+                const Affine inv = load_affine(&in.inv);
+                const V3 d = get3(3);
+                ro = transform_point(inv, ro);
+                float len;
+                const V3 ld = normalize(transform_vector(inv, d), &len);
+                put3(17, ld);
+                rinvd = inverse(ld);
+                cnt.meshTests++;
+                lBestT = kInf;
+                lPrim = -1;
+                bound = prune_bound(bestT * len);
+                base = sp;
+                ref = __ldg(&in.blasRoot);
+            }
+        } else if (best == kStepLeave) {
+            if (mine) {
+                // leaving an object: its closest triangle goes back to world space
+                const V3 o = get3(0);
+                if (lPrim >= 0) {
+                    const uint32_t inst = cold[14];
+                    const Instance &in = src.scene(pathId).instances[inst];
+                    const Affine model = load_affine(&in.model);
+                    V3 worldHit = transform_point(model, add(ro, mul(get3(17), lBestT)));
+                    float tw = dot(sub(worldHit, o), get3(3));
+                    if (tw < bestT || (tw == bestT && (int32_t)inst < (int32_t)cold[12])) {
+                        bestT = tw;
+                        cold[9] = cold[15];
+                        cold[10] = cold[16];
+                        cold[11] = (uint32_t)lPrim;
+                        cold[12] = inst;
+                    }
+                }
+                ro = o;
+                rinvd = get3(6);
+                bound = prune_bound(bestT);
+                base = -1;
+            }
+        } else {
+            // a finished ray is stored and the next one fetched: one atomic for
+            // the lanes that need a ray
+            const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine);
+            const int leader = __ffs(m) - 1;
+            uint32_t first = 0;
+            if (lane == leader) first = atomicAdd(work, (unsigned int)__popc(m));
+            first = __shfl_sync(0xFFFFFFFFu, first, leader);
+            if (mine) {
+                if (base == -1) {
+                    const int32_t bestPrim = (int32_t)cold[11];
+                    const uint32_t slot = cold[13];
+                    hitA[slot] = make_int4(__float_as_int(bestT), (int)cold[9], (int)cold[10],
+                        bestPrim);
+                    hitInst[slot] = (int)cold[12];
+                    done++;
+                    hits += (bestPrim >= 0 && bestT > 0.0f) ? 1u : 0u;
+                }
+                const uint32_t idx = first + __popc(m & ((1u << lane) - 1u));
+                if (idx < count) {
+                    float4 o4 = rayO[idx], d4 = rayD[idx];
+                    ro = v3(o4.x, o4.y, o4.z);
+                    const V3 d = v3(d4.x, d4.y, d4.z);
+                    pathId = (uint32_t)__float_as_int(o4.w);
+                    rinvd = inverse(d);
+                    put3(0, ro);
+                    put3(3, d);
+                    put3(6, rinvd);
+                    cold[9] = 0u;
+                    cold[10] = 0u;
+                    cold[11] = 0xFFFFFFFFu;
+                    cold[12] = 0xFFFFFFFFu;
+                    cold[13] = idx;
+                    bestT = kInf;
+                    bound = kInf;
+                    sp = 0;
+                    steps = 0;
+                    ref = src.scene(pathId).tlasRoot;
+                    base = -1;
+                } else {
+                    base = -3;
+                }
+            }
+        }
+        if (steps > kMaxLaneRaySteps) {
+            // store the best hit found so far
+            atomicOr(status, kStatusRayStepLimit);
+            steps = 0;
+            base = -1;
+            sp = 0;
+            ref = kEmptyChild;
         }
     }
     if (!drained) atomicOr(status, kStatusQueueOverflow);
@@ -721,39 +776,51 @@ int resident_blocks_per_sm(K kernel)
     return n;
 }
 
-template <class Src>
-int trace_grid(bool perLane, bool watertight, int smCount)
+template <class Src, int kQ>
+int trace_grid_of(bool perLane, bool watertight, int smCount)
 {
-    static const int lane[2] = {resident_blocks_per_sm(k_trace_lane<Src, false>),
-        resident_blocks_per_sm(k_trace_lane<Src, true>)};
-    static const int warp[2] = {resident_blocks_per_sm(k_trace<Src, false>),
-        resident_blocks_per_sm(k_trace<Src, true>)};
+    static const int lane[2] = {resident_blocks_per_sm(k_trace_lane<Src, false, kQ>),
+        resident_blocks_per_sm(k_trace_lane<Src, true, kQ>)};
+    static const int warp[2] = {resident_blocks_per_sm(k_trace<Src, false, kQ>),
+        resident_blocks_per_sm(k_trace<Src, true, kQ>)};
     return smCount * (perLane ? lane[watertight ? 1 : 0] : warp[watertight ? 1 : 0]);
 }
 
-// Launches the closest-hit kernel of one bounce: per-warp or per-lane
-// scheduling, reference MT or watertight triangle test (template arguments,
-// so neither choice costs the other anything).
+// quads: the node width every scene of the launch uses (2: 8-wide, 1: 4-wide), 0: mixed
 template <class Src>
-void launch_trace_stage(bool perLane, bool watertight, int grid, cudaStream_t s, const Src &src,
-    const float4 *qO, const float4 *qD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
-    unsigned int *ctl, unsigned long long *counters, uint32_t *status)
+int trace_grid(bool perLane, bool watertight, uint32_t quads, int smCount)
 {
-    if (perLane) {
-        if (watertight)
-            k_trace_lane<Src, true><<<grid, kLaneThreads, 0, s>>>(src, qO, qD, queueCount, hitA, hitInst,
-                ctl, counters, status);
-        else
-            k_trace_lane<Src, false><<<grid, kLaneThreads, 0, s>>>(src, qO, qD, queueCount, hitA, hitInst,
-                ctl, counters, status);
-    } else {
-        if (watertight)
-            k_trace<Src, true><<<grid, 128, 0, s>>>(src, qO, qD, queueCount, hitA, hitInst, ctl,
-                counters, status);
-        else
-            k_trace<Src, false><<<grid, 128, 0, s>>>(src, qO, qD, queueCount, hitA, hitInst, ctl,
-                counters, status);
-    }
+    return quads == 2 ? trace_grid_of<Src, 2>(perLane, watertight, smCount)
+                      : trace_grid_of<Src, 0>(perLane, watertight, smCount);
+}
+
+template <class Src, bool kWT, int kQ>
+void launch_trace_kernel(bool perLane, int grid, cudaStream_t s, const Src &src, const float4 *qO,
+    const float4 *qD, const unsigned int *queueCount, int4 *hitA, int *hitInst, unsigned int *ctl,
+    unsigned long long *counters, uint32_t *status)
+{
+    if (perLane)
+        k_trace_lane<Src, kWT, kQ><<<grid, kLaneThreads, 0, s>>>(src, qO, qD, queueCount, hitA,
+            hitInst, ctl, counters, status);
+    else
+        k_trace<Src, kWT, kQ><<<grid, 128, 0, s>>>(src, qO, qD, queueCount, hitA, hitInst, ctl,
+            counters, status);
+}
+
+// Launches the closest-hit kernel of one bounce: per-warp or per-lane
+// scheduling, reference MT or watertight triangle test, 8-wide nodes or a
+// width read from the scene (template arguments, so no choice costs another
+// anything).
+template <class Src>
+void launch_trace_stage(bool perLane, bool watertight, uint32_t quads, int grid, cudaStream_t s,
+    const Src &src, const float4 *qO, const float4 *qD, const unsigned int *queueCount, int4 *hitA,
+    int *hitInst, unsigned int *ctl, unsigned long long *counters, uint32_t *status)
+{
+    auto launch = quads == 2 ? (watertight ? launch_trace_kernel<Src, true, 2>
+                                           : launch_trace_kernel<Src, false, 2>)
+                             : (watertight ? launch_trace_kernel<Src, true, 0>
+                                           : launch_trace_kernel<Src, false, 0>);
+    launch(perLane, grid, s, src, qO, qD, queueCount, hitA, hitInst, ctl, counters, status);
 }
 
 }  // namespace gbsp
