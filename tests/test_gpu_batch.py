@@ -99,3 +99,47 @@ def test_batch_rejects_tile_sequential(gpu_lib):
     img = torch.zeros((s.height, s.width, 4), dtype=torch.float32, device="cuda")
     with pytest.raises(gbsp.GbspError, match="hash-per-sample"):
         gbsp.Batch(rt, [rend], [img.data_ptr()])
+
+
+@pytest.mark.parametrize("clamp,nan_policy", [(10.0, gbsp.NAN_ZERO), (0.0, gbsp.NAN_PROPAGATE),
+                                              (-1.0, gbsp.NAN_PROPAGATE)])
+@pytest.mark.parametrize("bounces", [1, 2, 8])
+def test_shading_shortcuts_match_the_general_path(gpu_lib, bounces, clamp, nan_policy):
+    """The wavefront's shading skips what a path's last vertex cannot change;
+    the thread-per-pixel kernel evaluates every vertex in full.  Both give the
+    same bits for materials at the edges of the skip: roughness 0, in and out
+    of the covered range and negative, infinite and NaN albedos (constant and
+    textured), smooth and flat meshes, textured and missing backgrounds, and
+    clamps that do not keep zero.  Odd sizes leave ragged batches."""
+    import torch
+
+    s = scenes.config3_scene(width=67, height=45, spp=3, max_bounces=bounces, n_spheres=24, level=2,
+                             seed=31)
+    s.meshes[0] = (s.meshes[0][0], s.meshes[0][1], True)
+    s.textures = {9: np.random.default_rng(1).random((8, 8, 4)).astype(np.float32)}
+    s.textures[9][2, 3] = np.inf
+    s.textures[9][5, 5] = np.nan
+    edge = [dict(roughness=0.3), dict(roughness=4.0), dict(roughness=4.1), dict(roughness=-1.0),
+            dict(albedo=(np.inf, 0.1, 0.1)), dict(albedo=(np.nan, 0.1, 0.1)),
+            dict(albedo_texture=9, roughness=0.5), dict(albedo_texture=9), dict(emission_texture=9),
+            dict(roughness=np.nan), dict(roughness=1e-3), dict(emission=(np.inf, 1, 1))]
+    for k, e in enumerate(edge):
+        s.materials[2 + k] = scenes.material(**{**dict(albedo=(0.5, 0.6, 0.7)), **e})
+    rt = gbsp.Runtime()
+    for background in (0, 2 + 5, 2 + 7, 999):
+        s.background = background
+        opt = gbsp.default_options(spp=s.spp, max_bounces=bounces, seed=4, radiance_clamp=clamp,
+                                   nan_policy=nan_policy)
+        scene, ms, rend = gbsp.upload_scene(rt, s, opt)
+        img, m = rend.frame()
+        out = torch.zeros((s.height, s.width, 4), device="cuda")
+        b = gbsp.Batch(rt, [rend], [out.data_ptr()])
+        b.set_config(kernel=gbsp.BATCH_THREAD_PER_PIXEL)
+        mb = b.launch()
+        same = (img.view(np.uint32) == out.cpu().numpy().view(np.uint32))
+        nan = np.isnan(img) & np.isnan(out.cpu().numpy())
+        assert np.all(same | nan), (background, int((~(same | nan)).sum()))
+        assert m.as_dict()["nan_samples"] == mb.as_dict()["nan_samples"]
+        assert m.as_dict()["paths_traced"] == mb.as_dict()["paths_traced"]
+        b.close()
+    rt.close()

@@ -289,8 +289,7 @@ static void runtime_teardown(gbsp_runtime *rt)
     rt->rayD.release();
     rt->hitA.release();
     rt->hitInst.release();
-    rt->vertE.release();
-    rt->vertA.release();
+    rt->vert.release();
     rt->pathRad.release();
     rt->queueCounts.release();
     rt->frame.release();

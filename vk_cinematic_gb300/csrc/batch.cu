@@ -517,7 +517,7 @@ struct gbsp_batch {
     std::vector<BatchItemDev> hostItems;
     std::vector<BatchWave> waves;
     uint32_t waveCap = 0, waveBounces = 0;
-    DeviceBuffer<float4> rayO, rayD, vertE, vertA, pathRad;
+    DeviceBuffer<float4> rayO, rayD, vert, pathRad;
     DeviceBuffer<int4> hitA;
     DeviceBuffer<int> hitInst;
     DeviceBuffer<uint32_t> pathItem;
@@ -614,8 +614,8 @@ static int plan_waves(gbsp_batch *b)
     int rc;
     if ((rc = b->rayO.reserve(2 * c, s)) || (rc = b->rayD.reserve(2 * c, s)) ||
         (rc = b->hitA.reserve(c, s)) || (rc = b->hitInst.reserve(c, s)) ||
-        (rc = b->pathItem.reserve(c, s)) || (rc = b->vertE.reserve((size_t)maxB * c, s)) ||
-        (rc = b->vertA.reserve((size_t)maxB * c, s)) || (rc = b->pathRad.reserve(c, s)))
+        (rc = b->pathItem.reserve(c, s)) || (rc = b->vert.reserve(2 * (size_t)(maxB - 1) * c, s)) ||
+        (rc = b->pathRad.reserve(c, s)))
         return rc;
     return GBSP_OK;
 }
@@ -631,8 +631,7 @@ static void enqueue_wavefront(gbsp_batch *b)
     wb.rayD = b->rayD.ptr;
     wb.hitA = b->hitA.ptr;
     wb.hitInst = b->hitInst.ptr;
-    wb.vertE = b->vertE.ptr;
-    wb.vertA = b->vertA.ptr;
+    wb.vert = b->vert.ptr;
     wb.pathRad = b->pathRad.ptr;
     wb.pathAov = nullptr;
     wb.cap = b->waveCap;

@@ -110,8 +110,7 @@ struct gbsp_runtime {
     gbsp::DeviceBuffer<int4> hitA;                 // t, u, v, prim
     gbsp::DeviceBuffer<int> hitInst;
     gbsp::DeviceBuffer<uint32_t> sortHist;       // octant histograms of the ray sort
-    gbsp::DeviceBuffer<float4> vertE;              // emission xyz, cosine
-    gbsp::DeviceBuffer<float4> vertA;              // response xyz
+    gbsp::DeviceBuffer<float4> vert;               // stored path vertices, two float4 each
     gbsp::DeviceBuffer<float4> pathRad;            // radiance per path
     gbsp::DeviceBuffer<unsigned int> queueCounts;  // small control block
     gbsp::DeviceBuffer<float4> frame;              // last frame, RGBA32F

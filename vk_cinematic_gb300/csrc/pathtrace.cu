@@ -4,10 +4,10 @@
 //   generate   one thread per (pixel, sample): seed, jitter, camera ray
 //   trace      persistent closest-hit kernel pulling 32 rays per warp from a
 //              global atomic counter
-//   shade      persistent: surface attributes, hemisphere sample, material
-//              and BRDF terms of the path vertex; continuing rays are
-//              compacted into the next queue with one atomic per warp
-//              (ballot + popc); finished paths are evaluated at once
+//   shade      surface attributes, hemisphere sample, material and BRDF
+//              terms of the path vertex; continuing rays are compacted into
+//              the next queue with one reservation per batch of queue
+//              entries; finished paths are evaluated at once
 //   accumulate one thread per pixel: Neumaier sum of sample * (1/spp)
 //
 // A wave holds a run of whole pixels with all their samples, so the
@@ -108,8 +108,7 @@ static int ensure_wave_buffers(gbsp_runtime *rt, uint32_t cap, uint32_t maxBounc
     int rc;
     if ((rc = rt->rayO.reserve(2 * (size_t)cap, s)) || (rc = rt->rayD.reserve(2 * (size_t)cap, s)) ||
         (rc = rt->hitA.reserve(cap, s)) || (rc = rt->hitInst.reserve(cap, s)) ||
-        (rc = rt->vertE.reserve((size_t)maxBounces * cap, s)) ||
-        (rc = rt->vertA.reserve((size_t)maxBounces * cap, s)) ||
+        (rc = rt->vert.reserve(2 * (size_t)(maxBounces - 1) * cap, s)) ||
         (rc = rt->pathRad.reserve(cap, s)))
         return rc;
     return GBSP_OK;
@@ -322,8 +321,7 @@ static int render_waves(gbsp_runtime *rt, const SceneView &sv, const MaterialVie
     wb.rayD = rt->rayD.ptr;
     wb.hitA = rt->hitA.ptr;
     wb.hitInst = rt->hitInst.ptr;
-    wb.vertE = rt->vertE.ptr;
-    wb.vertA = rt->vertA.ptr;
+    wb.vert = rt->vert.ptr;
     wb.pathRad = rt->pathRad.ptr;
     wb.pathAov = nullptr;
     if (dAov) {
@@ -416,9 +414,8 @@ constexpr size_t kNaRayO = na_align(kNaSlots + 4 * (size_t)kNoAllocMaxObjects);
 constexpr size_t kNaRayD = na_align(kNaRayO + 2 * 16 * (size_t)kNoAllocMaxPaths);
 constexpr size_t kNaHitA = na_align(kNaRayD + 2 * 16 * (size_t)kNoAllocMaxPaths);
 constexpr size_t kNaHitInst = na_align(kNaHitA + 16 * (size_t)kNoAllocMaxPaths);
-constexpr size_t kNaVertE = na_align(kNaHitInst + 4 * (size_t)kNoAllocMaxPaths);
-constexpr size_t kNaVertA = na_align(kNaVertE + 16 * (size_t)kNoAllocMaxBounces * kNoAllocMaxPaths);
-constexpr size_t kNaRad = na_align(kNaVertA + 16 * (size_t)kNoAllocMaxBounces * kNoAllocMaxPaths);
+constexpr size_t kNaVert = na_align(kNaHitInst + 4 * (size_t)kNoAllocMaxPaths);
+constexpr size_t kNaRad = na_align(kNaVert + 32 * (size_t)(kNoAllocMaxBounces - 1) * kNoAllocMaxPaths);
 constexpr size_t kNoAllocBytes = na_align(kNaRad + 16 * (size_t)kNoAllocMaxPaths);
 
 static __device__ __align__(256) unsigned char g_noallocScratch[kNoAllocBytes];
@@ -554,8 +551,7 @@ extern "C" int gbsp_path_trace_tile_noalloc(const gbsp_context *ctx, gbsp_tile t
     wb.rayD = reinterpret_cast<float4 *>(base + kNaRayD);
     wb.hitA = reinterpret_cast<int4 *>(base + kNaHitA);
     wb.hitInst = reinterpret_cast<int *>(base + kNaHitInst);
-    wb.vertE = reinterpret_cast<float4 *>(base + kNaVertE);
-    wb.vertA = reinterpret_cast<float4 *>(base + kNaVertA);
+    wb.vert = reinterpret_cast<float4 *>(base + kNaVert);
     wb.pathRad = reinterpret_cast<float4 *>(base + kNaRad);
     wb.pathAov = nullptr;
     uint32_t pixelsPerWave = kNoAllocMaxPaths / spp;

@@ -48,35 +48,67 @@ __device__ __forceinline__ V3 material_albedo(const MaterialView &mv, int slot, 
                             : v3(m.albedo[0], m.albedo[1], m.albedo[2]);
 }
 
-// Per-vertex terms of ComputeRadianceForPath for the material in `slot`.
-__device__ __forceinline__ void vertex_terms(const MaterialView &mv, int slot, V3 N, V3 L, V3 V,
-    float uvx, float uvy, float4 &ec, float4 &aa)
+// What a path vertex needs of its material: sp_EvaluateMaterial's outputs.
+struct SurfaceMaterial {
+    V3 albedo, emission;
+    float roughness;
+};
+
+// Emission of material m seen along direction dir (textures are
+// equirectangular, src/math_lib.h:849-884).
+__device__ __forceinline__ V3 material_emission(const MaterialView &mv, const DeviceMaterial &m, V3 dir)
 {
-    V3 albedo = v3(0.0f, 0.0f, 0.0f), emission;
-    float roughness = 0.0f;
-    if (slot < 0) {
-        emission = v3(1.0f, 0.0f, 1.0f);  // missing material: magenta
-    } else {
-        const DeviceMaterial &m = mv.materials[slot];
-        albedo = m.albedoTex >= 0 ? texel_nearest(mv, m.albedoTex, uvx, uvy)
-                                  : v3(m.albedo[0], m.albedo[1], m.albedo[2]);
-        if (m.emissionTex == -2) {
-            emission = sky_radiance(mv.sky, neg(V));
-        } else if (m.emissionTex >= 0) {
-            V3 dir = neg(V);  // src/math_lib.h:849-884
-            float inc = atan2f(sqrtf(dir.x * dir.x + dir.z * dir.z), dir.y);
-            float az = atan2f(dir.z, dir.x);
-            if (az < 0.0f) az += 2.0f * kPi;
-            float eu = az / (2.0f * kPi);
-            float ev = cosf(inc) * 0.5f + 0.5f;
-            ev = 1.0f - ev;
-            emission = mul(texel_nearest(mv, m.emissionTex, eu, ev), 1.0f);
-        } else {
-            emission = v3(m.emission[0], m.emission[1], m.emission[2]);
-        }
-        roughness = m.roughness;
+    if (m.emissionTex == -2) return sky_radiance(mv.sky, dir);
+    if (m.emissionTex >= 0) {
+        float inc = atan2f(sqrtf(dir.x * dir.x + dir.z * dir.z), dir.y);
+        float az = atan2f(dir.z, dir.x);
+        if (az < 0.0f) az += 2.0f * kPi;
+        float eu = az / (2.0f * kPi);
+        float ev = cosf(inc) * 0.5f + 0.5f;
+        ev = 1.0f - ev;
+        return mul(texel_nearest(mv, m.emissionTex, eu, ev), 1.0f);
     }
-    float cosine = rmax(0.0f, dot(N, L));
+    return v3(m.emission[0], m.emission[1], m.emission[2]);
+}
+
+// The material in `slot` seen from V; uv(u, v) gives the surface's texture
+// coordinates and is asked only when the albedo is textured.
+template <class UV>
+__device__ __forceinline__ SurfaceMaterial surface_material(const MaterialView &mv, int slot, V3 V,
+    UV uv)
+{
+    if (slot < 0)  // missing material: magenta
+        return SurfaceMaterial{v3(0.0f, 0.0f, 0.0f), v3(1.0f, 0.0f, 1.0f), 0.0f};
+    const DeviceMaterial &m = mv.materials[slot];
+    SurfaceMaterial r;
+    if (m.albedoTex >= 0) {
+        float ux, uy;
+        uv(ux, uy);
+        r.albedo = texel_nearest(mv, m.albedoTex, ux, uy);
+    } else {
+        r.albedo = v3(m.albedo[0], m.albedo[1], m.albedo[2]);
+    }
+    r.emission = material_emission(mv, m, neg(V));
+    r.roughness = m.roughness;
+    return r;
+}
+
+// DistributionGGX (src/simd_path_tracer.cpp:72-84): its numerator and denominator.
+__device__ __forceinline__ void ggx_terms(float roughness, V3 N, V3 H, float &a2, float &denom)
+{
+    float a = roughness * roughness;
+    a2 = a * a;
+    float NdotH = rmax(dot(N, H), 0.0f);
+    float NdotH2 = NdotH * NdotH;
+    denom = (NdotH2 * (a2 - 1.0f) + 1.0f);
+    denom = kPi * denom * denom;
+}
+
+// Response A of ComputeRadianceForPath at a vertex, and the cosine.
+__device__ __forceinline__ void brdf_terms(const SurfaceMaterial &sm, V3 N, V3 L, V3 V, V3 &A,
+    float &cosine)
+{
+    cosine = rmax(0.0f, dot(N, L));
     V3 H = normalize(add(L, V));
     // FresnelSchlick(max(H.V, 0), 0.04) (src/simd_path_tracer.cpp:65-70)
     float p5 = powf(1.0f - rmax(dot(H, V), 0.0f), 5.0f);
@@ -84,29 +116,61 @@ __device__ __forceinline__ void vertex_terms(const MaterialView &mv, int slot, V
     float Fs = F0 + (1.0f - F0) * p5;
     V3 F = v3(Fs, Fs, Fs);
     V3 kD = sub(v3(1.0f, 1.0f, 1.0f), F);
-    // DistributionGGX (:72-84)
-    float a = roughness * roughness;
-    float a2 = a * a;
-    float NdotH = rmax(dot(N, H), 0.0f);
-    float NdotH2 = NdotH * NdotH;
-    float denom = (NdotH2 * (a2 - 1.0f) + 1.0f);
-    denom = kPi * denom * denom;
-    float NDF = a2 / denom;
-    // GeometrySmith (:86-105)
+    float a2, denom;
+    ggx_terms(sm.roughness, N, H, a2, denom);
     float NdotV = rmax(dot(N, V), 0.0f);
     float NdotL = rmax(dot(N, L), 0.0f);
-    float r1 = roughness + 1.0f;
-    float k = (r1 * r1) / 8.0f;
-    float ggx2 = NdotV / (NdotV * (1.0f - k) + k);
-    float ggx1 = NdotL / (NdotL * (1.0f - k) + k);
-    float G = ggx1 * ggx2;
-    V3 numerator = mul(F, NDF * G);
-    float denominator = 4.0f * rmax(dot(N, V), 0.0f) * rmax(dot(N, L), 0.0f) + 0.0001f;
-    V3 specular = mul(numerator, 1.0f / denominator);
+    V3 specular = v3(0.0f, 0.0f, 0.0f);
+    // roughness 0: the distribution is 0 / denom, so the specular term is
+    // exactly zero unless denom is zero too (N.H = 1: 0 / 0, the reference's
+    // NaN) or a cosine is out of range; G is finite in [0, 1.01]^2
+    if (!(sm.roughness == 0.0f && denom > 0.0f && NdotV <= 1.01f && NdotL <= 1.01f)) {
+        float NDF = a2 / denom;
+        // GeometrySmith (:86-105)
+        float r1 = sm.roughness + 1.0f;
+        float k = (r1 * r1) / 8.0f;
+        float ggx2 = NdotV / (NdotV * (1.0f - k) + k);
+        float ggx1 = NdotL / (NdotL * (1.0f - k) + k);
+        float G = ggx1 * ggx2;
+        V3 numerator = mul(F, NDF * G);
+        float denominator = 4.0f * rmax(dot(N, V), 0.0f) * rmax(dot(N, L), 0.0f) + 0.0001f;
+        specular = mul(numerator, 1.0f / denominator);
+    }
     float oneOverPi = 1.0f / kPi;
-    V3 A = add(mul(hadamard(kD, albedo), oneOverPi), specular);
-    ec = make_float4(emission.x, emission.y, emission.z, cosine);
+    A = add(mul(hadamard(kD, sm.albedo), oneOverPi), specular);
+}
+
+// Per-vertex terms of ComputeRadianceForPath for the material in `slot`.
+__device__ __forceinline__ void vertex_terms(const MaterialView &mv, int slot, V3 N, V3 L, V3 V,
+    float uvx, float uvy, float4 &ec, float4 &aa)
+{
+    const SurfaceMaterial sm = surface_material(mv, slot, V, [&](float &u, float &v) {
+        u = uvx;
+        v = uvy;
+    });
+    V3 A;
+    float cosine;
+    brdf_terms(sm, N, L, V, A, cosine);
+    ec = make_float4(sm.emission.x, sm.emission.y, sm.emission.z, cosine);
     aa = make_float4(A.x, A.y, A.z, 0.0f);
+}
+
+// Whether the last vertex of a path adds nothing but its emission: its
+// radiance is E + (A * clamp(0)) * cosine, which is E + 0 when A and the
+// cosine are finite and the clamp keeps 0.  True only where that is certain:
+// finite albedo, a roughness whose geometry terms stay finite, cosines in
+// range and a finite distribution term.  (F lies in [0.04, 1.01].)
+__device__ __forceinline__ bool last_vertex_is_emission(const SurfaceMaterial &sm, V3 N, V3 L, V3 V,
+    float clampValue)
+{
+    const float big = 1.0e30f;
+    if (!(clampValue >= 0.0f && sm.roughness >= 0.0f && sm.roughness <= 4.0f &&
+            fabsf(sm.albedo.x) <= big && fabsf(sm.albedo.y) <= big && fabsf(sm.albedo.z) <= big))
+        return false;
+    if (!(dot(V, V) <= 1.01f && dot(L, L) <= 1.01f && dot(N, N) <= 1.01f)) return false;
+    float a2, denom;
+    ggx_terms(sm.roughness, N, normalize(add(L, V)), a2, denom);
+    return a2 <= denom * big && denom > 0.0f;
 }
 
 // One step of the reverse pass: radiance = E + (A * clamp(radiance)) * cosine.
@@ -130,15 +194,34 @@ __device__ __forceinline__ V3 path_radiance(const float4 *vertE, const float4 *v
     return radiance;
 }
 
-// The same with the last vertex's terms given (not stored) and the len - 1
-// before it read from memory.
-__device__ __forceinline__ V3 path_radiance_last(const float4 *vertE, const float4 *vertA,
-    size_t stride, uint32_t p, uint32_t len, float4 lastE, float4 lastA, float clampValue)
+// A path's stored vertices, two float4 (one 32-byte sector) each: (emission,
+// cosine) and (response, 0).
+__device__ __forceinline__ void store_vertex(float4 *vert, size_t at, float4 ec, float4 aa)
 {
-    V3 radiance = radiance_step(v3(0.0f, 0.0f, 0.0f), lastE, lastA, clampValue);
-    for (int i = (int)len - 2; i >= 0; i--)
-        radiance = radiance_step(radiance, vertE[(size_t)i * stride + p],
-            vertA[(size_t)i * stride + p], clampValue);
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(vert + 2 * at),
+        "f"(ec.x), "f"(ec.y), "f"(ec.z), "f"(ec.w), "f"(aa.x), "f"(aa.y), "f"(aa.z), "f"(aa.w)
+        : "memory");
+}
+
+__device__ __forceinline__ void load_vertex(const float4 *vert, size_t at, float4 &ec, float4 &aa)
+{
+    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=f"(ec.x), "=f"(ec.y), "=f"(ec.z), "=f"(ec.w), "=f"(aa.x), "=f"(aa.y), "=f"(aa.z),
+          "=f"(aa.w)
+        : "l"(vert + 2 * at)
+        : "memory");
+}
+
+// Reverse pass from the radiance of vertex `len` over the `len` stored
+// vertices before it; vertex i of path p is record i * stride + p.
+__device__ __forceinline__ V3 path_radiance_from(V3 radiance, const float4 *vert, size_t stride,
+    uint32_t p, uint32_t len, float clampValue)
+{
+    for (int i = (int)len - 1; i >= 0; i--) {
+        float4 ec, aa;
+        load_vertex(vert, (size_t)i * stride + p, ec, aa);
+        radiance = radiance_step(radiance, ec, aa, clampValue);
+    }
     return radiance;
 }
 

@@ -494,26 +494,44 @@ __device__ RayHit trace_closest(const SceneView &sv, V3 o, V3 d, uint32_t *statu
     return best;
 }
 
-// World-space normal and uv of a hit (src/sp_scene.cpp:189-215, 302-312).
-__device__ __forceinline__ void hit_surface(const SceneView &sv, const RayHit &h, V3 &normal,
-    float &uvx, float &uvy)
+// Texture coordinates of a hit (src/sp_scene.cpp:189-215).
+__device__ __forceinline__ void hit_uv(const SceneView &sv, const RayHit &h, float &uvx, float &uvy)
 {
-    const Instance &in = sv.instances[h.inst];
-    const float4 *tp = reinterpret_cast<const float4 *>(sv.tris + h.prim);
-    float4 A = __ldg(tp + 0), B = __ldg(tp + 1), C = __ldg(tp + 2);
     const float4 *ap = reinterpret_cast<const float4 *>(sv.attrs + h.prim);
-    float4 a0 = __ldg(ap + 0), a1 = __ldg(ap + 1), a2 = __ldg(ap + 2), a3 = __ldg(ap + 3);
+    float4 a2 = __ldg(ap + 2), a3 = __ldg(ap + 3);
     float w = 1.0f - h.u - h.v;
     // uv0 = (a2.y, a2.z), uv1 = (a2.w, a3.x), uv2 = (a3.y, a3.z)
     uvx = a2.y * w + a2.w * h.u + a3.y * h.v;
     uvy = a2.z * w + a3.x * h.u + a3.z * h.v;
-    V3 ln = v3(A.w, B.w, C.w);
+}
+
+// World-space normal of a hit (src/sp_scene.cpp:189-215, 302-312): the face
+// normal in the w lanes of the triangle record, or the interpolated vertex
+// normals of a smooth mesh (only those read the attributes).
+__device__ __forceinline__ V3 hit_normal(const SceneView &sv, const RayHit &h)
+{
+    const Instance &in = sv.instances[h.inst];
+    V3 ln;
     if (__ldg(&in.smooth)) {
-        V3 n0 = v3(a0.x, a0.y, a0.z), n1 = v3(a0.w, a1.x, a1.y), n2 = v3(a1.z, a1.w, a2.x);
+        const float4 *ap = reinterpret_cast<const float4 *>(sv.attrs + h.prim);
+        float4 a0 = __ldg(ap + 0), a1 = __ldg(ap + 1);
+        float a2x = __ldg(&ap[2].x);
+        float w = 1.0f - h.u - h.v;
+        V3 n0 = v3(a0.x, a0.y, a0.z), n1 = v3(a0.w, a1.x, a1.y), n2 = v3(a1.z, a1.w, a2x);
         ln = normalize(add(add(mul(n0, w), mul(n1, h.u)), mul(n2, h.v)));
+    } else {
+        const TriRecord *t = sv.tris + h.prim;
+        ln = v3(__ldg(&t->a_nx.w), __ldg(&t->b_ny.w), __ldg(&t->c_nz.w));
     }
-    const Affine model = load_affine(&in.model);
-    normal = normalize(transform_vector(model, ln));
+    return normalize(transform_vector(load_affine(&in.model), ln));
+}
+
+// World-space normal and uv of a hit.
+__device__ __forceinline__ void hit_surface(const SceneView &sv, const RayHit &h, V3 &normal,
+    float &uvx, float &uvy)
+{
+    normal = hit_normal(sv, h);
+    hit_uv(sv, h, uvx, uvy);
 }
 
 }  // namespace gbsp

@@ -13,7 +13,6 @@ namespace gbsp {
 // Work/queue control words (u32) behind the metric counters.
 enum Ctl : int {
     kCtlTraceWork = 0,
-    kCtlShadeWork = 1,
     kCtlQueue0 = 2,
     kCtlQueue1 = 3,
     kCtlCount = 8
@@ -26,8 +25,8 @@ struct WaveBuffers {
     float4 *rayD;      // 2 * cap: (direction, RNG state bits)
     int4 *hitA;        // cap: (t, u, v, prim) bits
     int *hitInst;      // cap
-    float4 *vertE;     // maxBounces * cap: (emission xyz, cosine), vertices of paths that go on
-    float4 *vertA;     // maxBounces * cap: (A xyz, 0)
+    float4 *vert;      // 2 per vertex, (maxBounces - 1) * cap vertices of paths that go on:
+                       // (emission xyz, cosine), (A xyz, 0)
     float4 *pathRad;   // cap
     float4 *pathAov;   // 2 * cap first-hit G-buffer per path, or null
     uint32_t cap;
@@ -92,7 +91,6 @@ static __global__ void k_reset_ctl(unsigned int *ctl, uint32_t queue0)
 static __global__ void k_reset_stage(unsigned int *ctl, int outQueue)
 {
     ctl[kCtlTraceWork] = 0;
-    ctl[kCtlShadeWork] = 0;
     ctl[outQueue] = 0;
 }
 
@@ -515,10 +513,9 @@ __global__ void __launch_bounds__(kLaneThreads, kWT || Src::kManyScenes ? 6 : 7)
             // a finished ray is stored and the next one fetched: one atomic for
             // the lanes that need a ray
             const uint32_t m = __ballot_sync(0xFFFFFFFFu, mine);
-            const int leader = __ffs(m) - 1;
             uint32_t first = 0;
-            if (lane == leader) first = atomicAdd(work, (unsigned int)__popc(m));
-            first = __shfl_sync(0xFFFFFFFFu, first, leader);
+            if (lane == 0) first = atomicAdd(work, (unsigned int)__popc(m));
+            first = __shfl_sync(0xFFFFFFFFu, first, 0);
             if (mine) {
                 if (base == -1) {
                     const int32_t bestPrim = (int32_t)cold[11];
@@ -583,94 +580,166 @@ __global__ void __launch_bounds__(kLaneThreads, kWT || Src::kManyScenes ? 6 : 7)
     }
 }
 
+// Shading of one bounce.  A warp walks batches of up to kShadeRows x 32 queue
+// entries, sorts their indices into hits and misses (order kept, by ballot)
+// and shades each kind with full warps.
+//
+// Bound, before: the one counter every warp took 32 entries from and the one
+// every warp reserved its outputs at.  Atomics on one address complete at
+// about 0.8 ns each, two per 32 rays: 1.2 to 2 ms of the 4.9 ms a wave of 2^25
+// paths spent here.  Batches are now dealt out by index (their cost is even),
+// and a batch reserves its outputs at once (a batch launch, whose items end at
+// different bounces, still does per 32).  Now: the chain of dependent loads of
+// a vertex (ray and hit, instance, triangle, material), so that there are few
+// of them: a flat hit reads 12 bytes of its triangle instead of 112
+// (attributes only for smooth meshes or textured albedo), a stored vertex is
+// one 32-byte sector, and a path's last vertex, which adds only its emission
+// (last_vertex_is_emission), skips the BRDF.  1080p benchmark frame (64 spp, 5
+// bounces) 67.8 -> 54.6 ms with this kernel, uneven batch 3.24 -> 2.45 ms;
+// 1, 2, 4 and 8 rows with an atomic per batch: 67.7, 63.7, 61.1 and 59.3 ms;
+// by index 8 rows 55.3 and 4 rows 55.1 ms, and 4 are the better ones on short
+// queues (641 x 359 x 7: 1.106 and 1.091 ms).  8, 10 and 12 blocks per SM
+// measured the same; unbounded (72 registers, 7 blocks) the batch took 2.78 ms.
+constexpr uint32_t kShadeRows = 4;
+constexpr int kShadeThreads = 128;
+
 template <class Src>
-__global__ void __launch_bounds__(128) k_shade(Src src, WaveBuffers wb, uint32_t bounce, int inQueue,
-    unsigned int *ctl, unsigned long long *counters)
+__global__ void __launch_bounds__(kShadeThreads, 8) k_shade(Src src, WaveBuffers wb, uint32_t bounce,
+    int inQueue, unsigned int *ctl, unsigned long long *counters)
 {
-    int lane = threadIdx.x & 31;
-    uint32_t count = ctl[inQueue];
+    const int lane = threadIdx.x & 31;
+    const uint32_t laneMaskLt = (1u << lane) - 1u;
+    __shared__ uint8_t lists[kShadeThreads / 32][32 * kShadeRows];
+    uint8_t *list = lists[threadIdx.x >> 5];  // hits from the front, misses from the back
+    const uint32_t count = ctl[inQueue];
     int outQueue = inQueue == kCtlQueue0 ? kCtlQueue1 : kCtlQueue0;
     const float4 *inO = wb.rayO + (inQueue == kCtlQueue0 ? 0 : wb.cap);
     const float4 *inD = wb.rayD + (inQueue == kCtlQueue0 ? 0 : wb.cap);
     float4 *outO = wb.rayO + (inQueue == kCtlQueue0 ? wb.cap : 0);
     float4 *outD = wb.rayD + (inQueue == kCtlQueue0 ? wb.cap : 0);
+    // short queues: fewer rows, so that every warp gets some entries
+    const uint32_t warps = gridDim.x * (kShadeThreads / 32);
+    const uint32_t rows = min(kShadeRows, max(1u, count / (32u * warps)));
     uint32_t finished = 0;
-    for (uint32_t guard = 0; guard <= count / 32 + 1; guard++) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&ctl[kCtlShadeWork], 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= count) break;
-        uint32_t i = base + lane;
-        bool active = i < count;
-        bool cont = false;
-        float4 newO = make_float4(0, 0, 0, 0), newD = make_float4(0, 0, 0, 0);
-        uint32_t p = 0;
-        if (active) {
-            float4 o4 = inO[i], d4 = inD[i];
-            p = (uint32_t)__float_as_int(o4.w);
-            const SceneView &sv = src.scene(p);
-            const MaterialView &mv = src.materials(p);
-            bool lastBounce = bounce + 1 >= src.bounces(p);
-            int4 hA = wb.hitA[i];
-            RayHit h;
-            h.t = __int_as_float(hA.x);
-            h.u = __int_as_float(hA.y);
-            h.v = __int_as_float(hA.z);
-            h.prim = hA.w;
-            h.inst = wb.hitInst[i];
-            V3 o = v3(o4.x, o4.y, o4.z), d = v3(d4.x, d4.y, d4.z);
-            // every path in this queue has `bounce` vertices so far
-            const uint32_t len = bounce;
-            float4 ec, aa;
-            if (h.prim >= 0 && h.t > 0.0f) {
-                // hit vertex (src/simd_path_tracer.cpp:268-288)
-                V3 n;
-                float ux, uy;
-                hit_surface(sv, h, n, ux, uy);
-                V3 pos = add(o, mul(d, h.t));
-                uint32_t rng = __float_as_uint(d4.w);
-                V3 dir = random_hemisphere(n, rng);
-                int slot = mv.instanceSlot[h.inst];
-                vertex_terms(mv, slot, n, dir, neg(d), ux, uy, ec, aa);
-                V3 no = add(pos, mul(n, 0.0001f));
-                newO = make_float4(no.x, no.y, no.z, __int_as_float((int)p));
-                newD = make_float4(dir.x, dir.y, dir.z, __uint_as_float(rng));
-                cont = !lastBounce;
+    // counts stay below 2^31, so the index does not wrap
+    for (uint32_t base = (blockIdx.x * (kShadeThreads / 32) + (threadIdx.x >> 5)) * 32u * rows;
+         base < count; base += warps * 32u * rows) {
+        uint32_t hits = 0, misses = 0;
+        for (uint32_t r = 0; r < rows; r++) {
+            const uint32_t i = base + 32u * r + lane;
+            bool hit = false;
+            if (i < count) {
+                const int4 h = wb.hitA[i];
+                hit = h.w >= 0 && __int_as_float(h.x) > 0.0f;
+            }
+            const uint32_t mh = __ballot_sync(0xFFFFFFFFu, hit);
+            const uint32_t mm = __ballot_sync(0xFFFFFFFFu, i < count && !hit);
+            if (hit)
+                list[hits + __popc(mh & laneMaskLt)] = (uint8_t)(32u * r + lane);
+            else if (i < count)
+                list[32u * kShadeRows - 1u - misses - __popc(mm & laneMaskLt)] = (uint8_t)(32u * r + lane);
+            hits += __popc(mh);
+            misses += __popc(mm);
+        }
+        __syncwarp();
+        finished += lane == 0 ? misses : 0u;
+        // a frame's hits all go on or all end: one queue reservation per batch
+        uint32_t outBase = 0;
+        if (!Src::kManyScenes && bounce + 1 < src.bounces(0)) {
+            if (lane == 0 && hits) outBase = atomicAdd(&ctl[outQueue], hits);
+            outBase = __shfl_sync(0xFFFFFFFFu, outBase, 0);
+        }
+        for (uint32_t k0 = 0; k0 < hits; k0 += 32) {
+            // hit vertex (src/simd_path_tracer.cpp:268-288)
+            bool cont = false;
+            float4 newO = make_float4(0, 0, 0, 0), newD = make_float4(0, 0, 0, 0);
+            if (k0 + lane < hits) {
+                const uint32_t i = base + list[k0 + lane];
+                const float4 o4 = inO[i], d4 = inD[i];
+                const int4 hA = wb.hitA[i];
+                RayHit h;
+                h.t = __int_as_float(hA.x);
+                h.u = __int_as_float(hA.y);
+                h.v = __int_as_float(hA.z);
+                h.prim = hA.w;
+                h.inst = wb.hitInst[i];
+                const uint32_t p = (uint32_t)__float_as_int(o4.w);
+                const SceneView &sv = src.scene(p);
+                const MaterialView &mv = src.materials(p);
+                const V3 o = v3(o4.x, o4.y, o4.z), d = v3(d4.x, d4.y, d4.z);
+                const V3 n = hit_normal(sv, h);
+                const SurfaceMaterial sm = surface_material(mv, mv.instanceSlot[h.inst], neg(d),
+                    [&](float &u, float &v) { hit_uv(sv, h, u, v); });
                 if (wb.pathAov && bounce == 0) {
-                    V3 al = material_albedo(mv, slot, ux, uy);
-                    wb.pathAov[2 * (size_t)p] = make_float4(al.x, al.y, al.z, h.t);
+                    wb.pathAov[2 * (size_t)p] = make_float4(sm.albedo.x, sm.albedo.y, sm.albedo.z, h.t);
                     wb.pathAov[2 * (size_t)p + 1] = make_float4(n.x, n.y, n.z, 1.0f);
                 }
-            } else {
-                // miss: background vertex, path ends (:302-314)
-                vertex_terms(mv, mv.backgroundSlot, v3(0, 0, 0), v3(0, 0, 0), neg(d), 0.0f, 0.0f,
-                    ec, aa);
+                uint32_t rng = __float_as_uint(d4.w);
+                const V3 dir = random_hemisphere(n, rng);
+                // every path in this queue has `bounce` vertices so far
+                cont = bounce + 1 < src.bounces(p);
+                V3 r = add(sm.emission, v3(0.0f, 0.0f, 0.0f));
+                if (cont || !last_vertex_is_emission(sm, n, dir, neg(d), src.clamp(p))) {
+                    V3 A;
+                    float cosine;
+                    brdf_terms(sm, n, dir, neg(d), A, cosine);
+                    const float4 ec = make_float4(sm.emission.x, sm.emission.y, sm.emission.z, cosine);
+                    const float4 aa = make_float4(A.x, A.y, A.z, 0.0f);
+                    if (cont) {
+                        store_vertex(wb.vert, (size_t)bounce * wb.cap + p, ec, aa);
+                        const V3 pos = add(o, mul(d, h.t));
+                        const V3 no = add(pos, mul(n, 0.0001f));
+                        newO = make_float4(no.x, no.y, no.z, o4.w);
+                        newD = make_float4(dir.x, dir.y, dir.z, __uint_as_float(rng));
+                    } else {
+                        r = radiance_step(v3(0.0f, 0.0f, 0.0f), ec, aa, src.clamp(p));
+                    }
+                }
+                if (!cont) {
+                    r = path_radiance_from(r, wb.vert, wb.cap, p, bounce, src.clamp(p));
+                    wb.pathRad[p] = make_float4(r.x, r.y, r.z, 0.0f);
+                    finished++;
+                }
+            }
+            // compaction: one atomic per warp for the continuing rays
+            const uint32_t mask = __ballot_sync(0xFFFFFFFFu, cont);
+            if (Src::kManyScenes) {
+                if (lane == 0 && mask) outBase = atomicAdd(&ctl[outQueue], (unsigned)__popc(mask));
+                outBase = __shfl_sync(0xFFFFFFFFu, outBase, 0);
+            }
+            if (cont) {
+                const uint32_t slot = outBase + (Src::kManyScenes ? 0u : k0) + __popc(mask & laneMaskLt);
+                outO[slot] = newO;
+                outD[slot] = newD;
+            }
+        }
+        for (uint32_t k0 = 0; k0 < misses; k0 += 32) {
+            // miss: background vertex, path ends (:302-314)
+            if (k0 + lane < misses) {
+                const uint32_t i = base + list[32u * kShadeRows - 1u - k0 - lane];
+                const float4 d4 = inD[i];
+                const uint32_t p = (uint32_t)__float_as_int(inO[i].w);
+                const MaterialView &mv = src.materials(p);
+                const V3 z = v3(0.0f, 0.0f, 0.0f), V = neg(v3(d4.x, d4.y, d4.z));
+                const SurfaceMaterial sm = surface_material(mv, mv.backgroundSlot, V,
+                    [&](float &u, float &v) { u = v = 0.0f; });
+                V3 r = add(sm.emission, z);
+                if (!last_vertex_is_emission(sm, z, z, V, src.clamp(p))) {
+                    V3 A;
+                    float cosine;
+                    brdf_terms(sm, z, z, V, A, cosine);
+                    r = radiance_step(z, make_float4(sm.emission.x, sm.emission.y, sm.emission.z, cosine),
+                        make_float4(A.x, A.y, A.z, 0.0f), src.clamp(p));
+                }
                 if (wb.pathAov && bounce == 0) {
                     wb.pathAov[2 * (size_t)p] = make_float4(0, 0, 0, 0);
                     wb.pathAov[2 * (size_t)p + 1] = make_float4(0, 0, 0, 0);
                 }
-            }
-            if (cont) {
-                wb.vertE[(size_t)len * wb.cap + p] = ec;
-                wb.vertA[(size_t)len * wb.cap + p] = aa;
-            } else {
-                // the path ends at this vertex: the reverse pass starts from it
-                V3 r = path_radiance_last(wb.vertE, wb.vertA, wb.cap, p, len + 1, ec, aa,
-                    src.clamp(p));
+                r = path_radiance_from(r, wb.vert, wb.cap, p, bounce, src.clamp(p));
                 wb.pathRad[p] = make_float4(r.x, r.y, r.z, 0.0f);
-                finished++;
             }
         }
-        // compaction: one atomic per warp for the continuing rays
-        uint32_t mask = __ballot_sync(0xFFFFFFFFu, cont);
-        uint32_t outBase = 0;
-        if (lane == 0 && mask) outBase = atomicAdd(&ctl[outQueue], (unsigned)__popc(mask));
-        outBase = __shfl_sync(0xFFFFFFFFu, outBase, 0);
-        if (cont) {
-            uint32_t slot = outBase + __popc(mask & ((1u << lane) - 1u));
-            outO[slot] = newO;
-            outD[slot] = newD;
-        }
+        __syncwarp();
     }
     for (int off = 16; off; off >>= 1) finished += __shfl_xor_sync(0xFFFFFFFFu, finished, off);
     if (lane == 0 && finished)
@@ -756,7 +825,7 @@ int shade_grid(int smCount)
     static int perSm = 0;
     if (perSm == 0) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_shade<Src>, 128, 0) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_shade<Src>, kShadeThreads, 0) !=
                 cudaSuccess || n < 1)
             n = 8;
         perSm = n;
