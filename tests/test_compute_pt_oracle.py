@@ -80,3 +80,25 @@ def test_counts_and_determinism(built):
     assert 48 * 32 <= rays <= 3 * 48 * 32 and hits <= rays
     tris_per_ray = sum(int(s["meshes"][m][0]) // 3 for m in s["entities"][:, 0])
     assert tests == rays * tris_per_ray
+
+
+def test_rejected_clusters_hold_no_accepted_triangle(tmp_path):
+    """The cluster rejection of the compute path tracer (csrc/cpt_clusters.h)
+    on the CPU: over spheres, soups, slivers, needles and planes, with rays
+    at random, at triangles, inside triangles' planes and along them, no
+    triangle of a rejected cluster passes the float triangle test."""
+    import os
+    import subprocess
+
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    exe = tmp_path / "test_cpt_clusters"
+    cmd = ["g++", "-std=c++17", "-O2", "-ffp-contract=off", "-I", os.path.join(root, "include"),
+           "-I", os.path.join(root, "vk_cinematic_gb300", "csrc"), "-I", "/usr/local/cuda/include",
+           os.path.join(root, "tests", "cpp", "test_cpt_clusters.cpp"), "-o", str(exe)]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    r = subprocess.run([str(exe), "4000"], capture_output=True, text=True, timeout=300)
+    print(r.stdout)
+    assert r.returncode == 0, r.stdout
+    # the rejection has to reject something where it matters
+    assert "fine sphere" in r.stdout and float(r.stdout.split("fine sphere")[1].split("%")[0].split()[-1]) > 80

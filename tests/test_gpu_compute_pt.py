@@ -66,3 +66,55 @@ def test_rejects_bad_input(gpu_lib):
     with pytest.raises(gbsp.GbspError, match="vertex index"):
         gbsp.ComputePTScene(rt, s["vertices"], idx, s["meshes"], s["model"], s["inv_model"],
                             s["entities"], s["texture"])
+
+
+def soup_mesh(rng, n, sliver):
+    """n triangles around the origin, a share of them slivers, some without area."""
+    p = rng.uniform(-1.5, 1.5, (n, 1, 3)) + rng.uniform(-0.6, 0.6, (n, 3, 3))
+    thin = rng.random(n) < sliver
+    p[thin, 2] = p[thin, 0] + (p[thin, 1] - p[thin, 0]) * rng.random((thin.sum(), 1)) + \
+        rng.uniform(-1e-5, 1e-5, (thin.sum(), 3))
+    flat = rng.random(n) < sliver / 4
+    p[flat, 2] = p[flat, 1]
+    v = np.zeros((3 * n, 8), np.float32)
+    v[:, 0:3] = p.reshape(-1, 3)
+    v[:, 6:8] = rng.random((3 * n, 2))
+    return v, np.arange(3 * n, dtype=np.uint32)
+
+
+@pytest.mark.parametrize("entities,tris,sliver", [(0, 5, 0.0), (1, 1, 0.0), (1, 17, 0.3),
+                                                  (33, 16, 0.1), (70, 3, 0.0), (2, 700, 0.3),
+                                                  (3, 2100, 0.0), (12, 400, 1.0)])
+def test_clusters_lose_no_hit(gpu_lib, entities, tris, sliver):
+    """Triangle clusters against the oracle's brute force, bit for bit: cluster
+    and warp-step remainders (1, 16, 17 triangles; more entities than a warp
+    has lanes; lists that are run in several parts), meshes without triangles,
+    slivers and degenerate triangles, rotated, scaled and mirrored entities."""
+    pyoracle.build_port()
+    rng = np.random.default_rng(100 * entities + tris)
+    sv, si = soup_mesh(rng, tris, sliver)
+    pv, pi = scenes.plane()
+    s = scenes.compute_pt_scene(n_spheres=1, level=0)
+    s["vertices"] = np.concatenate([pv, sv]).astype(np.float32)
+    s["indices"] = np.concatenate([pi, si]).astype(np.uint32)
+    s["meshes"] = np.array([[len(pi), 0, 0], [len(si), len(pi), len(pv)], [0, 0, 0]], np.uint32)
+    model, inv, ents = [], [], []
+    for k in range(entities):
+        m, i = scenes._trs(rng.uniform([-8, 0, -8], [8, 6, 8]), rng.uniform(-3, 3),
+                           rng.uniform(0.3, 2.0, 3) * rng.choice([-1.0, 1.0], 3))
+        model.append(m)
+        inv.append(i)
+        # a ground quad, an empty mesh now and then, the soup otherwise
+        ents.append((0 if k == 1 else 2 if k % 9 == 5 else 1, [0, 2, 5][k % 3], k))
+    s["model"] = np.array(model, np.float32).reshape(-1, 16)
+    s["inv_model"] = np.array(inv, np.float32).reshape(-1, 16)
+    s["entities"] = np.array(ents, np.uint32).reshape(-1, 3)
+    s["texture"] = np.ascontiguousarray(rng.random((7, 13, 4)).astype(np.float32))
+    w, h = 45, 37
+    tiles = np.arange((w // 16) * 3)
+    ref = np.zeros((h, w, 4), np.float32)
+    ref, c = pyoracle.compute_pt_tiles(s, w, h, 16, 0.8, tiles, image=ref)
+    got, m = render_gpu(s, w, h, tiles)
+    same = (got.view(np.uint32) == ref.view(np.uint32)) | (np.isnan(got) & np.isnan(ref))
+    assert same.all(), f"{(~same).sum()} words differ"
+    assert (m["rays_traced"], m["ray_hit_count"], m["triangle_tests"]) == tuple(int(v) for v in c[:3])

@@ -10,16 +10,28 @@
 // and the normalize(N + rand3) bounce.
 //
 // GB300 layout: the tile's RNG chain makes its pixels sequential, so a whole
-// warp works on one tile and splits each ray's triangle loop across its
-// lanes: lane l tests triangles l, l+32, ... (its own strict-< minimum), then
-// a warp reduction on (t, triangle index) gives the sequential loop's answer
-// (smallest t, lowest index among equal t).  The eight warps of a block trace
-// their rays in step so that every chunk of 256 triangles is staged into
-// shared memory once for eight rays.  Triangles are pre-expanded per mesh
-// into structure-of-arrays a, e1 = b - a, e2 = c - a (the same IEEE
-// subtractions the shader performs), so staging is coalesced; texture
-// coordinates are read only for the winner.  All other per-ray work is
-// warp-uniform.
+// block works on one tile and on one ray at a time.  Each mesh's triangles are
+// grouped into clusters of 16 (cpt_clusters.h); per ray
+//   1. warp 0 moves the ray into up to 32 entities' spaces, one lane each;
+//   2. all warps test 32 clusters of one entity per step and list (each warp
+//      for itself) the clusters whose triangles the float test could accept -
+//      the rejected ones provably contain no accepted triangle, so the set of
+//      hits is the brute-force loop's, rounding included;
+//   3. half-warps run the shader's test on the listed clusters; an entity's
+//      answer is the smallest t, lowest triangle index among equal t, kept by
+//      an atomic minimum on (t, index) in shared memory;
+//   4. warp 0 takes each entity's winner to world space, one lane each, and
+//      reduces in entity order (strict <), then shades and makes the next ray.
+// Texture coordinates are read only for the winner.
+//
+// Bound: the serial chain of a tile (two barriers, one pass over the clusters
+// and warp 0's shading per ray, 5.5 us a ray with one tile on an SM; the
+// longest tile has 768 rays).  A ray among 18 spheres of 1,280 triangles costs
+// 1,440 cluster tests and the tests of about 55 listed clusters instead of
+// 23,042 triangle tests.  512 x 384 pixels of that scene: 107.5 ms with a warp
+// per tile and every triangle staged through shared memory, 5.9 ms now.
+// 4 blocks of 8 warps per SM (64 registers) 5.9 ms, unbounded (2 blocks) 7.4,
+// 4 warps 6.6 and 2 warps per tile 9.8 ms.
 //
 // Built-ins are fixed to one IEEE definition shared with the oracle (dot in
 // x, y, z order; normalize = v * (1 / sqrt(dot)); mat4 * vec4 summed over
@@ -28,6 +40,7 @@
 
 #include <vector>
 
+#include "cpt_clusters.h"
 #include "gbsp_internal.h"
 
 namespace gbsp {
@@ -37,18 +50,21 @@ constexpr float kF32Max = 3.402823466e+38f;
 constexpr uint32_t kMaterialRed = 0, kMaterialCheckerBoard = 2, kMaterialWhiteLight = 5,
                    kMaterialBlack = 6;
 constexpr int kMaxBounces = 3;
-constexpr int kWarpsPerBlock = 8;
-constexpr int kChunk = 32 * kWarpsPerBlock;  // triangles staged per step (one per thread)
-
 struct EntityDev {
     float model[16];
     float inv[16];
-    uint32_t triBegin, triCount, material, pad;
+    uint32_t triBegin, triCount, material;
+    uint32_t clusterBegin, clusterCount, pad[3];
 };
 
-struct TriSoA {
-    const float *ax, *ay, *az, *e1x, *e1y, *e1z, *e2x, *e2y, *e2z;
-    const float2 *uv;  // 3 per triangle
+struct Triangles {
+    // cluster c: 9 components (a, e1, e2) of 16 triangles each, from 144 c;
+    // NaN in the places no triangle fills
+    const float *clustered;
+    const uint32_t *index;    // the clusters' triangles, as indices in their mesh
+    const Cluster *clusters;
+    const float *plain;       // 9 floats per triangle, in mesh order
+    const float2 *uv;         // 3 per triangle, in mesh order
 };
 
 struct View {
@@ -61,11 +77,6 @@ struct Counters {
     unsigned long long *rays, *hits, *tests, *paths;
 };
 
-__device__ __forceinline__ float cdot(V3 a, V3 b) { return (a.x * b.x + a.y * b.y) + a.z * b.z; }
-__device__ __forceinline__ V3 ccross(V3 a, V3 b)
-{
-    return v3(a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x);
-}
 __device__ __forceinline__ V3 cnormalize(V3 v)
 {
     float inv = 1.0f / sqrtf(cdot(v, v));
@@ -106,10 +117,17 @@ __device__ __forceinline__ float wrap_coord(float u, uint32_t n, int32_t &i0, in
     }
     float f = floorf(x);
     float a = x - f;
-    long long i = (long long)f;
-    long long m = ((i % (long long)n) + (long long)n) % (long long)n;
-    i0 = (int32_t)m;
-    i1 = (int32_t)((m + 1) % (long long)n);
+    // |f| < 1e9: 32-bit remainders (64-bit ones cost hundreds of instructions)
+    int32_t m;
+    if (n <= 0x7FFFFFFFu) {
+        m = (int32_t)f % (int32_t)n;
+        if (m < 0) m += (int32_t)n;
+    } else {
+        m = (int32_t)f;  // n is larger than any |f|
+        if (m < 0) m = (int32_t)(uint32_t)((long long)m + (long long)n);
+    }
+    i0 = m;
+    i1 = (uint32_t)m + 1u == n ? 0 : m + 1;
     return a;
 }
 
@@ -144,62 +162,70 @@ struct PathVertex {
     float u, v;
 };
 
-// Radiance of a finished path (test_compute.comp.glsl:441-481).
-__device__ __forceinline__ V3 path_radiance_cpt(const PathVertex *path, int len,
+// Radiance of a finished path (test_compute.comp.glsl:441-481): lane i of the
+// warp holds vertex i and evaluates its material, the reverse pass then takes
+// them from the last to the first.
+__device__ __forceinline__ V3 path_radiance_cpt(const PathVertex &vertex, int len, int lane,
     const float4 *__restrict__ tex, uint32_t texW, uint32_t texH)
 {
-    V3 radiance = v3(0.0f, 0.0f, 0.0f);
-    for (int i = len - 1; i >= 0; i--) {
-        V3 emission = v3(0.0f, 0.0f, 0.0f), albedo = v3(0.0f, 0.0f, 0.0f);
-        uint32_t m = path[i].material;
+    V3 emission = v3(0.0f, 0.0f, 0.0f), albedo = v3(0.0f, 0.0f, 0.0f);
+    float cosine = 0.0f;
+    if (lane < len) {
+        const uint32_t m = vertex.material;
         if (m == kMaterialRed)
             albedo = v3(0.18f, 0.1f, 0.1f);
         else if (m == kMaterialCheckerBoard)
-            albedo = sample_bilinear(tex, texW, texH, path[i].u, path[i].v);
+            albedo = sample_bilinear(tex, texW, texH, vertex.u, vertex.v);
         else if (m == kMaterialWhiteLight)
             emission = v3(1.0f, 1.0f, 1.0f);
-        float cosine = glsl_max(0.0f, cdot(path[i].normal, path[i].incoming));
-        radiance = v3(emission.x + (albedo.x * radiance.x) * cosine,
-            emission.y + (albedo.y * radiance.y) * cosine,
-            emission.z + (albedo.z * radiance.z) * cosine);
+        cosine = glsl_max(0.0f, cdot(vertex.normal, vertex.incoming));
+    }
+    V3 radiance = v3(0.0f, 0.0f, 0.0f);
+#pragma unroll
+    for (int i = kMaxBounces - 1; i >= 0; i--) {
+        const V3 e = v3(__shfl_sync(0xFFFFFFFFu, emission.x, i), __shfl_sync(0xFFFFFFFFu, emission.y, i),
+            __shfl_sync(0xFFFFFFFFu, emission.z, i));
+        const V3 a = v3(__shfl_sync(0xFFFFFFFFu, albedo.x, i), __shfl_sync(0xFFFFFFFFu, albedo.y, i),
+            __shfl_sync(0xFFFFFFFFu, albedo.z, i));
+        const float c = __shfl_sync(0xFFFFFFFFu, cosine, i);
+        if (i < len)
+            radiance = v3(e.x + (a.x * radiance.x) * c, e.y + (a.y * radiance.y) * c,
+                e.z + (a.z * radiance.z) * c);
     }
     return radiance;
 }
 
-// Block-lockstep kernel: the kWarpsPerBlock warps of a block own one tile
-// each and trace their current rays together.  The brute-force triangle
-// loop is the same sequence for every ray (entity by entity, triangle by
-// triangle), so the block stages each chunk of kChunk triangles (9 floats
-// each: a, e1, e2) into shared memory once - double-buffered, the next chunk
-// loading while this one is tested - and every warp tests its own ray
-// against it, lane l taking triangles l, l + 32, ...  Per warp the order of
-// triangles, the strict-< minimum and every RNG draw are those of the
-// shader's sequential loops, so results are unchanged; a warp whose tile is
-// done keeps staging chunks for the others until the whole block is done.
-__global__ void __launch_bounds__(32 * kWarpsPerBlock) k_compute_pt(const EntityDev *__restrict__ ents,
-    uint32_t entityCount, TriSoA tri, const float4 *__restrict__ tex, uint32_t texW, uint32_t texH,
-    View view, const uint32_t *__restrict__ tiles, uint32_t tileCount, float4 *__restrict__ image,
-    Counters counters)
+constexpr int kEntChunk = 32;     // entities whose clusters a ray tests together: one lane of warp 0 each
+constexpr int kListCap = 128;     // clusters a warp lists before it runs their triangles
+
+template <int kWarps>
+__global__ void __launch_bounds__(32 * kWarps, kWarps == 8 ? 4 : 1) k_compute_pt(const EntityDev *__restrict__ ents,
+    uint32_t entityCount, uint64_t triangleTests, Triangles tri, const float4 *__restrict__ tex,
+    uint32_t texW, uint32_t texH, View view, const uint32_t *__restrict__ tiles,
+    float4 *__restrict__ image, Counters counters)
 {
-    __shared__ float sTri[2][9][kChunk];
-    const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t item = blockIdx.x * kWarpsPerBlock + (tid >> 5);
-    bool active = item < tileCount;
-    uint32_t minX = 0, minY = 0, maxX = 0, maxY = 0, tileIndex = 0;
-    if (active) {
-        tileIndex = __ldg(&tiles[item]);
-        uint32_t tx = tileIndex % view.tileCountX, ty = tileIndex / view.tileCountX;
-        minX = tx * view.tileW;
-        minY = ty * view.tileH;
-        maxX = min(view.width, (tx + 1) * view.tileW);
-        maxY = min(view.height, (ty + 1) * view.tileH);
-        active = minX < maxX && minY < maxY;
-    }
+    __shared__ float sRay[kEntChunk][6];                // the ray in each entity's space
+    __shared__ unsigned long long sBest[kEntChunk];     // (t bits, triangle) of its closest hit
+    __shared__ uint32_t sUnits[kEntChunk + 1];          // units of 32 clusters before each entity
+    __shared__ uint32_t sBegin[kEntChunk], sClusters[kEntChunk];
+    __shared__ uint32_t sLists[kWarps][kListCap];       // each warp's listed clusters
+    __shared__ uint8_t sEntities[kWarps][kListCap];     // and their entities
+    __shared__ uint32_t sActive, sNone;                 // sNone: entities the ray cannot hit
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t laneMaskLt = (1u << lane) - 1u;
+    uint32_t *sList = sLists[warp];
+    uint8_t *sEntity = sEntities[warp];
+    const uint32_t tileIndex = __ldg(&tiles[blockIdx.x]);
+    const uint32_t tx = tileIndex % view.tileCountX, ty = tileIndex / view.tileCountX;
+    const uint32_t minX = tx * view.tileW, minY = ty * view.tileH;
+    const uint32_t maxX = min(view.width, (tx + 1) * view.tileW);
+    const uint32_t maxY = min(view.height, (ty + 1) * view.tileH);
+    bool active = minX < maxX && minY < maxY;
     Rng rng{(tileIndex + 1u) * 0xF51C0E49u};
-    uint64_t rays = 0, hits = 0, tests = 0, paths = 0;
+    uint64_t rays = 0, hits = 0, paths = 0;
     uint32_t x = minX, y = minY;
     int len = 0, bounce = 0;
-    PathVertex path[kMaxBounces];
+    PathVertex vertex = {kMaterialBlack, v3(0.0f, 0.0f, 0.0f), v3(0.0f, 0.0f, 0.0f), 0.0f, 0.0f};  // lane i: vertex i
     V3 o = v3(0.0f, 0.0f, 0.0f), d = v3(0.0f, 0.0f, 0.0f);
     // camera ray of pixel (x, y): test_compute.comp.glsl:510-540
     auto start_pixel = [&]() {
@@ -222,134 +248,167 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_compute_pt(const Entity
         len = 0;
         bounce = 0;
     };
-    if (active) start_pixel();
-    // stage the triangles [c, c + n) of entity e into buffer buf
-    auto stage = [&](uint32_t e, uint32_t c, int buf) {
-        const EntityDev &ent = ents[e];
-        uint32_t count = __ldg(&ent.triCount);
-        uint32_t n = count - c < (uint32_t)kChunk ? count - c : (uint32_t)kChunk;
-        if ((uint32_t)tid < n) {
-            uint32_t g = __ldg(&ent.triBegin) + c + tid;
-            sTri[buf][0][tid] = __ldg(tri.ax + g);
-            sTri[buf][1][tid] = __ldg(tri.ay + g);
-            sTri[buf][2][tid] = __ldg(tri.az + g);
-            sTri[buf][3][tid] = __ldg(tri.e1x + g);
-            sTri[buf][4][tid] = __ldg(tri.e1y + g);
-            sTri[buf][5][tid] = __ldg(tri.e1z + g);
-            sTri[buf][6][tid] = __ldg(tri.e2x + g);
-            sTri[buf][7][tid] = __ldg(tri.e2y + g);
-            sTri[buf][8][tid] = __ldg(tri.e2z + g);
-        }
-    };
-
+    // the ray's state lives in warp 0 (every lane holds it)
+    if (warp == 0 && active) start_pixel();
+    const uint32_t chunks = (entityCount + kEntChunk - 1) / kEntChunk;
     for (uint32_t guard = 0; guard < (1u << 30); guard++) {
-        if (!__syncthreads_or(active)) break;
-        // ---- trace: test_compute.comp.glsl:320-430, all warps in step
+        // ---- trace: test_compute.comp.glsl:320-430
         SceneHit res;
         res.t = kF32Max;
         res.material = kMaterialBlack;
         res.normal = v3(0.0f, 0.0f, 0.0f);
         res.u = res.v = 0.0f;
-        if (entityCount) {
-            uint32_t e = 0, c = 0;
-            int buf = 0;
-            V3 lo = mat_mul(ents[0].inv, o, 1.0f);
-            V3 ld = cnormalize(mat_mul(ents[0].inv, d, 0.0f));
-            float bestT = kF32Max, bestU = 0.0f, bestV = 0.0f;
-            uint32_t bestK = 0xFFFFFFFFu;
-            stage(0, 0, 0);
-            __syncthreads();
-            while (e < entityCount) {
-                const EntityDev &ent = ents[e];
-                const uint32_t count = __ldg(&ent.triCount);
-                // next chunk: the rest of this entity, else the next entity (an
-                // entity without triangles is one empty chunk)
-                uint32_t ne = e, nc = c + kChunk;
-                if (nc >= count) {
-                    ne = e + 1;
-                    nc = 0;
+        uint32_t chunk = 0;
+        bool done = false;
+        do {
+            const uint32_t e = chunk * kEntChunk + lane;  // warp 0: the lane's entity
+            const bool mine = warp == 0 && e < entityCount;
+            V3 lo = v3(0.0f, 0.0f, 0.0f), ld = lo;
+            if (warp == 0) {
+                if (mine) {
+                    lo = mat_mul(ents[e].inv, o, 1.0f);
+                    ld = cnormalize(mat_mul(ents[e].inv, d, 0.0f));
+                    sRay[lane][0] = lo.x;
+                    sRay[lane][1] = lo.y;
+                    sRay[lane][2] = lo.z;
+                    sRay[lane][3] = ld.x;
+                    sRay[lane][4] = ld.y;
+                    sRay[lane][5] = ld.z;
                 }
-                if (ne < entityCount) stage(ne, nc, buf ^ 1);
-                if (active) {
-                    uint32_t n = count - c < (uint32_t)kChunk ? count - c : (uint32_t)kChunk;
-                    if (c == 0) tests += count;
-                    for (uint32_t j = lane; j < n; j += 32) {
-                        V3 a = v3(sTri[buf][0][j], sTri[buf][1][j], sTri[buf][2][j]);
-                        V3 e1 = v3(sTri[buf][3][j], sTri[buf][4][j], sTri[buf][5][j]);
-                        V3 e2 = v3(sTri[buf][6][j], sTri[buf][7][j], sTri[buf][8][j]);
-                        V3 T = v3(lo.x - a.x, lo.y - a.y, lo.z - a.z);
-                        V3 p = ccross(ld, e2);
-                        V3 q = ccross(T, e1);
-                        float mx = cdot(q, e2), my = cdot(p, T), mz = cdot(q, ld);
-                        float det = 1.0f / cdot(p, e1);
-                        float t = det * mx, u = det * my, v = det * mz;
-                        float w = 1.0f - u - v;
-                        if (u >= 0.0f && u <= 1.0f && v >= 0.0f && v <= 1.0f && w >= 0.0f &&
-                            w <= 1.0f && t >= 0.0f && t < kF32Max && t < bestT) {
-                            bestT = t;
-                            bestU = u;
-                            bestV = v;
-                            bestK = c + j;
-                        }
+                if (guard == 0 || chunks > 1) {  // a single chunk's tables stay
+                    const uint32_t clusters = mine ? __ldg(&ents[e].clusterCount) : 0u;
+                    sBegin[lane] = mine ? __ldg(&ents[e].clusterBegin) : 0u;
+                    sClusters[lane] = clusters;
+                    uint32_t units = (clusters + 31) / 32;
+                    for (int off = 1; off < 32; off <<= 1) {
+                        uint32_t v = __shfl_up_sync(0xFFFFFFFFu, units, off);
+                        if (lane >= off) units += v;
                     }
-                    if (ne != e) {
-                        // entity e done: the sequential loop's answer, then world space
-#pragma unroll
-                        for (int off = 16; off; off >>= 1) {
-                            float ot = __shfl_xor_sync(0xFFFFFFFFu, bestT, off);
-                            uint32_t ok = __shfl_xor_sync(0xFFFFFFFFu, bestK, off);
-                            if (ot < bestT || (ot == bestT && ok < bestK)) {
-                                bestT = ot;
-                                bestK = ok;
-                            }
-                        }
-                        float meshT = kF32Max, meshU = 0.0f, meshV = 0.0f;
-                        V3 localNormal = v3(0.0f, 0.0f, 0.0f);
-                        if (bestK != 0xFFFFFFFFu) {
-                            int src = (int)(bestK & 31u);
-                            float u = __shfl_sync(0xFFFFFFFFu, bestU, src);
-                            float v = __shfl_sync(0xFFFFFFFFu, bestV, src);
-                            uint32_t g = __ldg(&ent.triBegin) + bestK;
-                            V3 e1 = v3(__ldg(tri.e1x + g), __ldg(tri.e1y + g), __ldg(tri.e1z + g));
-                            V3 e2 = v3(__ldg(tri.e2x + g), __ldg(tri.e2y + g), __ldg(tri.e2z + g));
-                            localNormal = cnormalize(ccross(e1, e2));
-                            float w = 1.0f - u - v;
-                            float2 t0 = __ldg(&tri.uv[(size_t)g * 3 + 0]);
-                            float2 t1 = __ldg(&tri.uv[(size_t)g * 3 + 1]);
-                            float2 t2 = __ldg(&tri.uv[(size_t)g * 3 + 2]);
-                            meshT = bestT;
-                            meshU = (t0.x * w + t1.x * u) + t2.x * v;
-                            meshV = (t0.y * w + t1.y * u) + t2.y * v;
-                        }
-                        V3 localHit = v3(lo.x + ld.x * meshT, lo.y + ld.y * meshT,
-                            lo.z + ld.z * meshT);
-                        V3 worldHit = mat_mul(ent.model, localHit, 1.0f);
-                        float t = cdot(v3(worldHit.x - o.x, worldHit.y - o.y, worldHit.z - o.z), d);
-                        V3 worldNormal = cnormalize(mat_mul(ent.model, localNormal, 0.0f));
-                        if (t >= 0.0f && t < res.t) {
-                            res.t = t;
-                            res.material = __ldg(&ent.material);
-                            res.normal = worldNormal;
-                            res.u = meshU;
-                            res.v = meshV;
-                        }
-                        if (ne < entityCount) {
-                            lo = mat_mul(ents[ne].inv, o, 1.0f);
-                            ld = cnormalize(mat_mul(ents[ne].inv, d, 0.0f));
-                            bestT = kF32Max;
-                            bestU = bestV = 0.0f;
-                            bestK = 0xFFFFFFFFu;
-                        }
-                    }
+                    sUnits[lane + 1] = units;
+                    if (lane == 0) sUnits[0] = 0;
                 }
-                __syncthreads();  // chunk consumed, next chunk staged
-                e = ne;
-                c = nc;
-                buf ^= 1;
+                sBest[lane] = ~0ull;
+                // a ray with a NaN is never accepted: every numerator of the test
+                // has it.  (A path that leaves the scene can go on as one: an
+                // entity's miss at t = FLT_MAX may pass the world-space test and
+                // has no normal.)
+                const bool nan = !(lo.x + lo.y + lo.z == lo.x + lo.y + lo.z) ||
+                    !(ld.x + ld.y + ld.z == ld.x + ld.y + ld.z);
+                const uint32_t none = __ballot_sync(0xFFFFFFFFu, !mine || nan);
+                if (lane == 0) {
+                    sActive = active ? 1u : 0u;
+                    sNone = none;
+                }
             }
-        }
-        if (!active) continue;
-        // ---- shade: test_compute.comp.glsl:558-600 (warp-uniform)
+            __syncthreads();
+            if (!sActive) {
+                done = true;
+                break;
+            }
+            const uint32_t none = sNone;
+            const uint32_t before = sUnits[lane], total = none == 0xFFFFFFFFu ? 0u : sUnits[kEntChunk];
+            uint32_t listed = 0;
+            for (uint32_t u = warp; u < total; u += kWarps) {
+                // the entity of unit u: the last one that starts at or before it
+                const int el = __popc(__ballot_sync(0xFFFFFFFFu, before <= u)) - 1;
+                const uint32_t c = 32u * (u - sUnits[el]) + lane;
+                bool may = false;
+                uint32_t cluster = 0;
+                if (c < sClusters[el] && !(none >> el & 1u)) {
+                    cluster = sBegin[el] + c;
+                    const float4 *p = reinterpret_cast<const float4 *>(tri.clusters + cluster);
+                    may = cluster_may_hit(__ldg(p), __ldg(p + 1), __ldg(p + 2),
+                        v3(sRay[el][0], sRay[el][1], sRay[el][2]),
+                        v3(sRay[el][3], sRay[el][4], sRay[el][5]));
+                }
+                const uint32_t m = __ballot_sync(0xFFFFFFFFu, may);
+                if (may) {
+                    const uint32_t at = listed + __popc(m & laneMaskLt);
+                    sList[at] = cluster;
+                    sEntity[at] = (uint8_t)el;
+                }
+                listed += __popc(m);
+                if (u + kWarps < total && listed <= kListCap - 32) continue;
+                // run the listed clusters' triangles, a half-warp each
+                __syncwarp();
+                for (uint32_t k = lane / kClusterTris; k < listed; k += 32 / kClusterTris) {
+                    const uint32_t lc = sList[k], le = sEntity[k], j = lane % kClusterTris;
+                    const float *p = tri.clustered + (size_t)lc * (9 * kClusterTris) + j;
+                    const V3 a = v3(__ldg(p), __ldg(p + kClusterTris), __ldg(p + 2 * kClusterTris));
+                    const V3 e1 = v3(__ldg(p + 3 * kClusterTris), __ldg(p + 4 * kClusterTris),
+                        __ldg(p + 5 * kClusterTris));
+                    const V3 e2 = v3(__ldg(p + 6 * kClusterTris), __ldg(p + 7 * kClusterTris),
+                        __ldg(p + 8 * kClusterTris));
+                    const MtHit h = mt_test(v3(sRay[le][0], sRay[le][1], sRay[le][2]),
+                        v3(sRay[le][3], sRay[le][4], sRay[le][5]), a, e1, e2, kF32Max);
+                    // t >= 0 orders as its bits (+ 0 makes a zero positive)
+                    if (h.ok)
+                        atomicMin(&sBest[le],
+                            (unsigned long long)__float_as_uint(h.t + 0.0f) << 32 |
+                                __ldg(tri.index + (size_t)lc * kClusterTris + j));
+                }
+                listed = 0;
+                __syncwarp();
+            }
+            __syncthreads();
+            if (warp == 0) {
+                // each lane's entity in world space, then the sequential loop's
+                // answer over entities: the smallest t, the first one of equals
+                float t = kF32Max, hu = 0.0f, hv = 0.0f;
+                V3 normal = v3(0.0f, 0.0f, 0.0f);
+                bool cand = false;
+                if (mine) {
+                    const EntityDev &ent = ents[e];
+                    float meshT = kF32Max;
+                    V3 localNormal = v3(0.0f, 0.0f, 0.0f);
+                    if (sBest[lane] != ~0ull) {
+                        const uint32_t g = __ldg(&ent.triBegin) + (uint32_t)sBest[lane];
+                        const float *p = tri.plain + (size_t)g * 9;
+                        const V3 e1 = v3(__ldg(p + 3), __ldg(p + 4), __ldg(p + 5));
+                        const V3 e2 = v3(__ldg(p + 6), __ldg(p + 7), __ldg(p + 8));
+                        const MtHit h = mt_test(lo, ld, v3(__ldg(p), __ldg(p + 1), __ldg(p + 2)), e1, e2,
+                            kF32Max);
+                        localNormal = cnormalize(ccross(e1, e2));
+                        const float w = 1.0f - h.u - h.v;
+                        const float2 t0 = __ldg(&tri.uv[(size_t)g * 3 + 0]);
+                        const float2 t1 = __ldg(&tri.uv[(size_t)g * 3 + 1]);
+                        const float2 t2 = __ldg(&tri.uv[(size_t)g * 3 + 2]);
+                        meshT = h.t;
+                        hu = (t0.x * w + t1.x * h.u) + t2.x * h.v;
+                        hv = (t0.y * w + t1.y * h.u) + t2.y * h.v;
+                    }
+                    const V3 localHit = v3(lo.x + ld.x * meshT, lo.y + ld.y * meshT, lo.z + ld.z * meshT);
+                    const V3 worldHit = mat_mul(ent.model, localHit, 1.0f);
+                    t = cdot(v3(worldHit.x - o.x, worldHit.y - o.y, worldHit.z - o.z), d);
+                    normal = cnormalize(mat_mul(ent.model, localNormal, 0.0f));
+                    cand = t >= 0.0f && t < res.t;
+                }
+                float best = cand ? t : kF32Max;
+                int who = cand ? lane : 32;
+#pragma unroll
+                for (int off = 16; off; off >>= 1) {
+                    const float ot = __shfl_xor_sync(0xFFFFFFFFu, best, off);
+                    const int ow = __shfl_xor_sync(0xFFFFFFFFu, who, off);
+                    if (ow < 32 && (who == 32 || ot < best || (ot == best && ow < who))) {
+                        best = ot;
+                        who = ow;
+                    }
+                }
+                if (who < 32) {
+                    res.t = __shfl_sync(0xFFFFFFFFu, t, who);
+                    res.normal.x = __shfl_sync(0xFFFFFFFFu, normal.x, who);
+                    res.normal.y = __shfl_sync(0xFFFFFFFFu, normal.y, who);
+                    res.normal.z = __shfl_sync(0xFFFFFFFFu, normal.z, who);
+                    res.u = __shfl_sync(0xFFFFFFFFu, hu, who);
+                    res.v = __shfl_sync(0xFFFFFFFFu, hv, who);
+                    res.material = __ldg(&ents[chunk * kEntChunk + who].material);
+                }
+            }
+            chunk++;
+        } while (chunk < chunks);
+        if (done) break;  // the same in every thread
+        if (warp != 0) continue;
+        // ---- shade: test_compute.comp.glsl:558-600 (the same in every lane)
         rays++;
         bool more = false;
         if (res.t > 0.0f && res.t < kF32Max) {
@@ -359,11 +418,7 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_compute_pt(const Entity
             float r2 = rng.bilateral();
             V3 dir = cnormalize(v3(res.normal.x + r0, res.normal.y + r1, res.normal.z + r2));
             if (cdot(dir, res.normal) < 0.0f) dir = v3(-dir.x, -dir.y, -dir.z);
-            path[len].material = res.material;
-            path[len].normal = res.normal;
-            path[len].incoming = dir;
-            path[len].u = res.u;
-            path[len].v = res.v;
+            if (lane == len) vertex = PathVertex{res.material, dir, res.normal, res.u, res.v};
             len++;
             V3 wp = v3(o.x + d.x * res.t, o.y + d.y * res.t, o.z + d.z * res.t);
             o = v3(wp.x + res.normal.x * 0.001f, wp.y + res.normal.y * 0.001f,
@@ -372,32 +427,31 @@ __global__ void __launch_bounds__(32 * kWarpsPerBlock) k_compute_pt(const Entity
             bounce++;
             more = bounce < kMaxBounces;
         } else {
-            path[len].material = kMaterialBlack;
-            path[len].normal = v3(0.0f, 0.0f, 0.0f);
-            path[len].incoming = v3(0.0f, 0.0f, 0.0f);
-            path[len].u = path[len].v = 0.0f;
+            if (lane == len)
+                vertex = PathVertex{kMaterialBlack, v3(0.0f, 0.0f, 0.0f), v3(0.0f, 0.0f, 0.0f), 0.0f, 0.0f};
             len++;
         }
-        if (more) continue;
-        V3 radiance = path_radiance_cpt(path, len, tex, texW, texH);
-        paths++;
-        if (lane == 0)
-            image[(size_t)y * view.width + x] = make_float4(0.0f + radiance.x * 1.0f,
-                0.0f + radiance.y * 1.0f, 0.0f + radiance.z * 1.0f, 1.0f);
-        // next pixel of the tile in scanline order
-        if (++x >= maxX) {
-            x = minX;
-            y++;
+        if (!more) {
+            V3 radiance = path_radiance_cpt(vertex, len, lane, tex, texW, texH);
+            paths++;
+            if (lane == 0)
+                image[(size_t)y * view.width + x] = make_float4(0.0f + radiance.x * 1.0f,
+                    0.0f + radiance.y * 1.0f, 0.0f + radiance.z * 1.0f, 1.0f);
+            // next pixel of the tile in scanline order
+            if (++x >= maxX) {
+                x = minX;
+                y++;
+            }
+            if (y >= maxY)
+                active = false;
+            else
+                start_pixel();
         }
-        if (y >= maxY)
-            active = false;
-        else
-            start_pixel();
     }
-    if (lane == 0) {
+    if (tid == 0) {
         atomicAdd(counters.rays, (unsigned long long)rays);
         atomicAdd(counters.hits, (unsigned long long)hits);
-        atomicAdd(counters.tests, (unsigned long long)tests);
+        atomicAdd(counters.tests, (unsigned long long)(rays * triangleTests));
         atomicAdd(counters.paths, (unsigned long long)paths);
     }
 }
@@ -410,9 +464,11 @@ using namespace gbsp;
 struct gbsp_cpt_scene {
     gbsp_runtime *rt = nullptr;
     uint32_t entityCount = 0, texW = 0, texH = 0;
-    uint64_t triangleCount = 0;
     DeviceBuffer<cpt::EntityDev> entities;
-    DeviceBuffer<float> soa;  // 9 component arrays of triangleCount floats
+    uint64_t triangleTests = 0, units = 0;  // per ray: triangles, and steps of 32 clusters
+    DeviceBuffer<float> plain, clustered;  // cpt::Triangles
+    DeviceBuffer<uint32_t> index;
+    DeviceBuffer<cpt::Cluster> clusters;
     DeviceBuffer<float2> uv;
     DeviceBuffer<float4> tex;
     DeviceBuffer<uint32_t> tiles;
@@ -457,6 +513,7 @@ int gbsp_cpt_scene_create(gbsp_runtime *rt, const gbsp_vertex *vertices, uint32_
         if (en.meshIndex >= meshCount || en.modelMatrixIndex >= matrixCount)
             return set_error(GBSP_ERR_INVALID_ARGUMENT, "entity %u: mesh or matrix out of range", e);
         cpt::EntityDev &d = ents[e];
+        memset(&d, 0, sizeof(d));
         for (int k = 0; k < 16; k++) {
             d.model[k] = modelMatrices[(size_t)en.modelMatrixIndex * 16 + k];
             d.inv[k] = invModelMatrices[(size_t)en.modelMatrixIndex * 16 + k];
@@ -464,36 +521,68 @@ int gbsp_cpt_scene_create(gbsp_runtime *rt, const gbsp_vertex *vertices, uint32_
         d.triBegin = (uint32_t)meshBegin[en.meshIndex];
         d.triCount = (uint32_t)meshTris[en.meshIndex];
         d.material = en.materialId;
-        d.pad = 0;
     }
-    std::vector<float> soa((size_t)total * 9);
+    std::vector<float> plain((size_t)total * 9), clustered;
     std::vector<float2> uv((size_t)total * 3);
+    std::vector<cpt::Cluster> clusters;
+    std::vector<uint32_t> index;
+    std::vector<uint32_t> clusterBegin(meshCount), clusterCount(meshCount);
+    std::vector<V3> ma, me1, me2;
     for (uint32_t m = 0; m < meshCount; m++) {
         const gbsp_cpt_mesh &mesh = meshes[m];
+        ma.resize(meshTris[m]);
+        me1.resize(meshTris[m]);
+        me2.resize(meshTris[m]);
         for (uint64_t k = 0; k < meshTris[m]; k++) {
             uint64_t g = meshBegin[m] + k;
             const gbsp_vertex *v[3];
             for (int j = 0; j < 3; j++)
                 v[j] = &vertices[indices[mesh.indicesOffset + k * 3 + j] + mesh.vertexDataOffset];
             const float *a = v[0]->position, *b = v[1]->position, *c = v[2]->position;
-            float comp[9] = {a[0], a[1], a[2], b[0] - a[0], b[1] - a[1], b[2] - a[2], c[0] - a[0],
-                c[1] - a[1], c[2] - a[2]};
-            for (int j = 0; j < 9; j++) soa[(size_t)j * total + g] = comp[j];
+            ma[k] = v3(a[0], a[1], a[2]);
+            me1[k] = v3(b[0] - a[0], b[1] - a[1], b[2] - a[2]);
+            me2[k] = v3(c[0] - a[0], c[1] - a[1], c[2] - a[2]);
+            const float comp[9] = {ma[k].x, ma[k].y, ma[k].z, me1[k].x, me1[k].y, me1[k].z, me2[k].x,
+                me2[k].y, me2[k].z};
+            memcpy(plain.data() + 9 * g, comp, sizeof(comp));
             for (int j = 0; j < 3; j++) uv[g * 3 + j] = make_float2(v[j]->uv[0], v[j]->uv[1]);
         }
+        const size_t c0 = clusters.size();
+        cpt::build_clusters({ma.data(), me1.data(), me2.data(), (uint32_t)meshTris[m]}, clusters, index);
+        clusterBegin[m] = (uint32_t)c0;
+        clusterCount[m] = (uint32_t)(clusters.size() - c0);
+        clustered.resize(clusters.size() * 9 * cpt::kClusterTris, nanf(""));
+        for (size_t i = c0 * cpt::kClusterTris; i < index.size(); i++) {
+            if (index[i] == 0xFFFFFFFFu) continue;
+            const size_t c = i / cpt::kClusterTris, j = i % cpt::kClusterTris;
+            for (int q = 0; q < 9; q++)
+                clustered[(c * 9 + q) * cpt::kClusterTris + j] = plain[9 * (meshBegin[m] + index[i]) + q];
+        }
+    }
+    uint64_t triangleTests = 0, units = 0;
+    for (uint32_t e = 0; e < entityCount; e++) {
+        const uint32_t m = entities[e].meshIndex;
+        ents[e].clusterBegin = clusterBegin[m];
+        ents[e].clusterCount = clusterCount[m];
+        triangleTests += meshTris[m];
+        units += (clusterCount[m] + 31) / 32;
     }
     int rrc = runtime_retain(rt);
     if (rrc) return rrc;
     gbsp_cpt_scene *s = new gbsp_cpt_scene();
     s->rt = rt;
     s->entityCount = entityCount;
-    s->triangleCount = total;
+    s->triangleTests = triangleTests;
+    s->units = units;
     s->texW = texWidth;
     s->texH = texHeight;
     cudaStream_t st = rt->stream;
     int rc = GBSP_OK;
     if (entityCount) rc = s->entities.upload(ents.data(), ents.size(), st);
-    if (!rc && total) rc = s->soa.upload(soa.data(), soa.size(), st);
+    if (!rc && total) rc = s->plain.upload(plain.data(), plain.size(), st);
+    if (!rc && total) rc = s->clustered.upload(clustered.data(), clustered.size(), st);
+    if (!rc && total) rc = s->index.upload(index.data(), index.size(), st);
+    if (!rc && total) rc = s->clusters.upload(clusters.data(), clusters.size(), st);
     if (!rc && total) rc = s->uv.upload(uv.data(), uv.size(), st);
     if (!rc && texWidth)
         rc = s->tex.upload(reinterpret_cast<const float4 *>(checkerBoard),
@@ -559,12 +648,11 @@ int gbsp_cpt_render_tiles(gbsp_cpt_scene *scene, const gbsp_cpt_view *view,
     v.tileW = view->tileWidth;
     v.tileH = view->tileHeight;
     v.tileCountX = view->width / view->tileWidth;
-    cpt::TriSoA tri;
-    uint64_t n = scene->triangleCount;
-    const float *base = scene->soa.ptr;
-    const float **comp[9] = {&tri.ax, &tri.ay, &tri.az, &tri.e1x, &tri.e1y, &tri.e1z, &tri.e2x,
-        &tri.e2y, &tri.e2z};
-    for (int j = 0; j < 9; j++) *comp[j] = base ? base + (size_t)j * n : nullptr;
+    cpt::Triangles tri;
+    tri.clustered = scene->clustered.ptr;
+    tri.index = scene->index.ptr;
+    tri.clusters = scene->clusters.ptr;
+    tri.plain = scene->plain.ptr;
     tri.uv = scene->uv.ptr;
     cpt::Counters c;
     c.rays = rt->dCounters + GBSP_METRIC_RAYS_TRACED;
@@ -573,10 +661,16 @@ int gbsp_cpt_render_tiles(gbsp_cpt_scene *scene, const gbsp_cpt_view *view,
     c.paths = rt->dCounters + GBSP_METRIC_PATHS_TRACED;
     GBSP_CUDA_TRY(cudaMemsetAsync(rt->dCounters, 0, sizeof(unsigned long long) * GBSP_METRIC_COUNT, s));
     if (metrics) GBSP_CUDA_TRY(cudaEventRecord(rt->ev[0], s));
-    uint32_t grid = (tileCount + cpt::kWarpsPerBlock - 1) / cpt::kWarpsPerBlock;
-    cpt::k_compute_pt<<<grid, 32 * cpt::kWarpsPerBlock, 0, s>>>(scene->entities.ptr,
-        scene->entityCount, tri, scene->tex.ptr, scene->texW, scene->texH, v, scene->tiles.ptr,
-        tileCount, reinterpret_cast<float4 *>(deviceImage), c);
+    // warps per tile: as many as there are steps of 32 clusters to share (57
+    // steps: 8 warps 5.9, 4 warps 6.6, 2 warps 9.8 ms; 10 steps: 4 warps 2.7,
+    // 8 warps 2.9 ms, both at 512 x 384)
+    auto kern = scene->units <= 4 ? cpt::k_compute_pt<2>
+        : scene->units <= 16      ? cpt::k_compute_pt<4>
+                                  : cpt::k_compute_pt<8>;
+    const unsigned threads = scene->units <= 4 ? 64 : scene->units <= 16 ? 128 : 256;
+    kern<<<tileCount, threads, 0, s>>>(scene->entities.ptr, scene->entityCount, scene->triangleTests, tri,
+        scene->tex.ptr, scene->texW, scene->texH, v, scene->tiles.ptr,
+        reinterpret_cast<float4 *>(deviceImage), c);
     GBSP_CUDA_TRY(cudaGetLastError());
     if (!metrics) return GBSP_OK;
     GBSP_CUDA_TRY(cudaEventRecord(rt->ev[1], s));
