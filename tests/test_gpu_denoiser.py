@@ -162,6 +162,42 @@ def test_conv3x3_tcgen05_matches_torch_and_mma(gpu_lib, cin, cout, epi, B, H, W)
     assert ok and ok2
 
 
+@pytest.mark.parametrize("cin,cout,epi", [(16, 48, 0), (48, 48, 2), (32, 48, 2)])
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (3, 6, 1), (2, 3, 127), (1, 9, 129), (1, 2, 130),
+                                   (2, 7, 257)])
+def test_conv3x3_tcgen05_image_borders(gpu_lib, cin, cout, epi, B, H, W):
+    """Row pairs and 130-pixel runs at the image border: one pixel, one column,
+    segments that end on, one and two pixels past a tile, odd row counts (a
+    pair half inside), several images (rows of a neighbour must not leak in).
+    Bounds as in the tests above."""
+    import torch
+
+    from vk_cinematic_gb300.denoiser import _ptr, _stream, from_planar, to_planar
+
+    torch.manual_seed(cin + 7 * H + W)
+    x = torch.randn((B, H, W, cin), device="cuda").to(torch.bfloat16)
+    w = (torch.randn((9, cout, cin), device="cuda") * 0.2).to(torch.bfloat16)
+    bias = torch.randn(cout, device="cuda")
+    L = gbsp.load()
+    out = torch.full((B, H, cout // 8, W, 8), 7.0, device="cuda",
+                     dtype=torch.bfloat16 if epi == 0 else torch.float32)
+    xp = to_planar(x)
+    rc = L.gbsp_dn_conv3x3_forward_tc(_stream(), _ptr(xp), B, H, W, cin, _ptr(w),
+                                      _ptr(bias) if epi == 0 else None, cout, epi,
+                                      _ptr(out) if epi == 0 else None,
+                                      None if epi == 0 else _ptr(out))
+    assert rc == 0, L.gbsp_last_error_string()
+    torch.cuda.synchronize()
+    st = ctypes.c_uint32(0)
+    assert L.gbsp_dn_status(ctypes.byref(st)) == 0, st.value
+    ref, S = ref_conv(x, w, bias if epi == 0 else None)
+    if epi == 0:
+        ref = torch.relu(ref)
+    r, ok = within(from_planar(out), ref, S, bf16=epi == 0)
+    print(f"conv {cin}->{cout} epi {epi} {B}x{H}x{W}: worst error / bound {r:.3f}")
+    assert ok
+
+
 @pytest.mark.parametrize("wgrad,shape", [("mma", (2, 12, 67)), ("simt", (2, 12, 67)),
                                          ("mma", (1, 37, 250)), ("mma", (3, 1, 1)),
                                          ("tcgen05", (2, 12, 67)), ("tcgen05", (1, 37, 250)),

@@ -49,8 +49,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 
 // Activations and their gradients use a channel-group-planar layout,
 // [B][H][C/8][W][8]: each 8-channel group of an image row is a contiguous
-// plane of W x 16 bytes (BF16), so that one TMA box of a row's pixels is one
-// contiguous read.  Element (row = b H + y, x, c):
+// plane of W x 16 bytes (BF16), so that a row segment's pixels are one
+// contiguous read per group.  Element (row = b H + y, x, c):
 __device__ __forceinline__ size_t cg_index(size_t row, int x, int c, int W, int C)
 {
     return ((row * (size_t)(C / 8) + (size_t)(c / 8)) * (size_t)W + (size_t)x) * 8 + (size_t)(c % 8);
@@ -187,23 +187,22 @@ int launch_conv(cudaStream_t s, int smCount, const void *in, int B, int H, int W
 //
 // Shared memory holds the operands in the canonical no-swizzle K-major
 // layout: 8 x 16-byte core matrices (8 rows of 8 BF16 channels), rows
-// contiguous.  Input rows: ring slots of [CIN/8 channel groups][kTcPlane
-// pixels][16 B] (a core matrix = 8 consecutive pixels of one channel group,
-// so a pixel shift moves the start by 16 B); weights: [3 taps][CIN/8
-// groups][3 tap rows x COUT][16 B].  Descriptor strides: leading (K) = next
-// channel group, stride (M or N) = next 8 rows = 128 B.
+// contiguous.  Input rows: ring slots of two rows, each [CIN/8 channel
+// groups][kTcSpx pixels][16 B] (a core matrix = 8 consecutive pixels of one
+// channel group, so a pixel shift moves the start by 16 B); weights: [3
+// taps][CIN/8 groups][3 tap rows x COUT][16 B].  Descriptor strides: leading
+// (K) = next channel group, stride (M or N) = next 8 rows = 128 B.
 //
 // One persistent CTA per SM walks vertical strips (one 128-pixel column
 // segment, a run of rows) with its warps specialised and coupled only by
 // mbarriers:
-//   * lane 0 of warp 1 (producer) loads input rows into a ring of kTcRing
-//     slots with TMA (cp.async.bulk.tensor: one box of 130 pixels x every
-//     channel group per row, which in the channel-group-planar activation
-//     layout is CIN/8 contiguous 2,080-byte runs; zero outside the image),
-//     as many rows in flight as the ring allows; a row lands on its rowFull
-//     barrier by transaction count, and its slot is reused once the MMAs of
-//     the last row group that reads it have completed (rowEmpty, signalled
-//     by tcgen05.commit);
+//   * warp 1 (producer) loads input rows in pairs into a ring of kTcRing slots,
+//     one lane per channel plane of a pair (cp.async.bulk of the plane's 130
+//     pixels, one contiguous run of the planar layout; pixels outside the image
+//     are zeroed by the warp), as many pairs in flight as the ring allows; a
+//     pair lands on its rowFull barrier by transaction count, and its slot is
+//     reused once the MMAs of the last row group that reads it have completed
+//     (rowEmpty, signalled by tcgen05.commit);
 //   * lane 0 of warp 0 issues, per group of kTcGroupRows output rows, the
 //     (kTcGroupRows + 2) x 3 x CIN/16 MMAs reading its input rows into one
 //     TMEM accumulator, then commits to that accumulator's accFull and to the
@@ -215,6 +214,14 @@ int launch_conv(cudaStream_t s, int smCount, const void *in, int B, int H, int W
 //     already works on the next group.
 // Every wait is bounded; a timeout raises a shared abort flag that ends the
 // other roles' waits, and sets g_dnStatus.
+//
+// What bounds it (48 -> 48 at 1080p, 85.9 GFLOP, 398 MB in and out): memory, 79
+// us = 5.0 TB/s, with the MMAs behind it (54 of about 70 cycles per row group,
+// 49 us).  Before, 99 us: the issuing thread waited on six row barriers per
+// group at about 340 cycles each, none of it hidden (without loads, stores and
+// eight ninths of the MMAs 47 us; with one wait per group 29); and TMA boxes of
+// [group][130 pixels][8 channels] move 16 bytes per request (loads alone 60
+// us, 49 as runs).  Two epilogue groups per accumulator: 79 us, the same.
 // ---------------------------------------------------------------------------
 constexpr int kTcTileP = 128;
 // One CTA per SM: warp 0 issues the MMAs, lane 0 of warp 1 loads rows, warps 4-11 are
@@ -223,9 +230,10 @@ constexpr int kTcThreads = 384;
 constexpr int kTcEpiGroups = 2;
 constexpr int kTcAccSlots = 4;  // at most; accumulator a is drained by epilogue group a % 2
 constexpr int kTcSpx = kTcTileP + 2;     // staged pixels per row: x0 - 1 .. x0 + 128
-constexpr int kTcPlane = kTcSpx;         // pixels per channel-group plane of a ring slot
 constexpr int kTcGroupRows = 4;  // output rows per accumulator
-constexpr int kTcRing = 14;  // input row slots: 6 read by a row group's MMAs, the rest in flight
+// Input rows travel in pairs: one full and one empty barrier per two rows.  A row group reads three pairs, two of them new, so its issuing
+// thread waits twice for rows and releases two slots.
+constexpr int kTcRing = 7;  // row pairs in shared memory: 3 read by a group's MMAs, the rest in flight
 constexpr uint32_t kTcWaitLimit = 1u << 26;
 
 __device__ uint32_t g_dnStatus;
@@ -369,30 +377,42 @@ __device__ __forceinline__ void conv_store(const uint32_t (&r)[COUT], size_t row
 
 // Softmax of the 25 kernel logits (accumulators + bias) and the 5x5 filter of
 // the noisy radiance around pixel p = (x, y): the same arithmetic as k_filter
-// on stored logits, so the fused and unfused results are bit-identical.
+// on stored logits, so the fused and unfused results are bit-identical.  The
+// clamped columns and rows are computed once each (25 clamped tap indices had
+// cost more than the filter: 160 -> 117 us at 1080p).  Loading the 25 taps
+// ahead of the accumulators spills and was slower (129 us), as were twice the
+// epilogue warps (129 us).
 template <int COUT>
 __device__ __forceinline__ void conv_filter_store(const uint32_t (&r)[COUT], size_t p, int x, int y,
     int W, int H, const float *__restrict__ bias, const float4 *__restrict__ noisy,
     float4 *__restrict__ out)
 {
     static_assert(COUT >= 25, "kernel logits");
-    float l[25], wk[25];
+    float wk[25];
 #pragma unroll
-    for (int k = 0; k < 25; k++) l[k] = __uint_as_float(r[k]) + bias[k];
-    softmax25(l, wk);
+    for (int k = 0; k < 25; k++) wk[k] = __uint_as_float(r[k]) + bias[k];
+    softmax25(wk, wk);
+    int dx[5];
+#pragma unroll
+    for (int i = 0; i < 5; i++) dx[i] = min(max(x + i - 2, 0), W - 1);
+    const float4 *image = noisy + (p - (size_t)x - (size_t)y * W);
     float3 o = make_float3(0, 0, 0);
 #pragma unroll
-    for (int k = 0; k < 25; k++) {
-        float4 c = __ldg(noisy + tap_pixel(p, x, y, W, H, k));
-        o.x += wk[k] * c.x;
-        o.y += wk[k] * c.y;
-        o.z += wk[k] * c.z;
+    for (int j = 0; j < 5; j++) {
+        const float4 *line = image + (size_t)min(max(y + j - 2, 0), H - 1) * W;
+#pragma unroll
+        for (int i = 0; i < 5; i++) {
+            const float4 c = __ldg(line + dx[i]);
+            o.x += wk[5 * j + i] * c.x;
+            o.y += wk[5 * j + i] * c.y;
+            o.z += wk[5 * j + i] * c.z;
+        }
     }
     out[p] = make_float4(o.x, o.y, o.z, 1.0f);
 }
 
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_constant__ CUtensorMap tmIn,
+__global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat16 *__restrict__ in,
     int B, int H, int W, int rowsPerStrip, int reverseStrips, const __nv_bfloat16 *__restrict__ w,
     const float *__restrict__ bias, __nv_bfloat16 *__restrict__ outB, float *__restrict__ outF,
     const float4 *__restrict__ noisy, float4 *__restrict__ outFilt)
@@ -408,8 +428,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_const
     constexpr int TMEM_COLS = 512;
     extern __shared__ __align__(128) unsigned char smemRaw[];
     uint4 *sW = reinterpret_cast<uint4 *>(smemRaw);  // [3][KG][3 COUT]
-    // ring slots of [KG][kTcPlane] 16-byte pixels, each slot 128-byte aligned for TMA
-    constexpr uint32_t kSlotBytes = (uint32_t)((KG * kTcPlane * 16 + 127) / 128 * 128);
+    // ring slots of [2 rows][KG][kTcSpx] 16-byte pixels, each slot 128-byte aligned for TMA
+    constexpr uint32_t kRowUnits = (uint32_t)(KG * kTcSpx);  // 16-byte units
+    constexpr uint32_t kSlotBytes = (2 * kRowUnits * 16 + 127) / 128 * 128;
     const uint32_t ringAddr = (smem_u32(sW + 9 * KG * COUT) + 127u) & ~127u;
     __shared__ __align__(8) uint64_t rowFull[kTcRing], rowEmpty[kTcRing];
     __shared__ __align__(8) uint64_t accFull[SLOTS], accEmpty[SLOTS], drain;
@@ -478,21 +499,30 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_const
             idesc[1] = instr_desc_bf16<kTcTileP, COUT>();
             idesc[2] = instr_desc_bf16<kTcTileP, 2 * COUT>();
             idesc[3] = instr_desc_bf16<kTcTileP, 3 * COUT>();
-            const uint64_t aDesc0 = smem_desc(ringAddr, kTcPlane * 16, 128);
+            const uint64_t aDesc0 = smem_desc(ringAddr, kTcSpx * 16, 128);
             const uint64_t bDesc0 = smem_desc(smem_u32(sW), 3 * COUT * 16, 128);
             // issue order per (tx, kc): k = 2 and k = G + 1 first (their outputs tile all G
             // rows, so they can start the accumulator), then the rest
             static_assert(G == 4, "issue order below is for groups of 4 rows");
             constexpr int kOrder[G + 2] = {2, 5, 0, 1, 3, 4};
-            uint32_t qBase = 0, groupCount = 0;
+            uint32_t groupCount = 0;
+            uint32_t pos = 0;    // ring slot of the group's first row pair
+            uint32_t phase = 0;  // parity of the next wait on each slot (bit per slot)
             bool ok = true;
+            const auto next_slot = [](uint32_t v) { return v + 1u == (uint32_t)kTcRing ? 0u : v + 1u; };
+            const auto wait_pair = [&](uint32_t slot) {
+                const bool r = tc_wait(smem_u32(&rowFull[slot]), phase >> slot & 1u, &abortFlag);
+                phase ^= 1u << slot;
+                return r;
+            };
             for (int strip = blockIdx.x; strip < numStrips && ok; strip += gridDim.x) {
                 GBSP_STRIP_GEOMETRY(strip);
+                ok = wait_pair(pos);
                 for (int p = 0; p < P && ok; p++) {
-                    const uint32_t q0 = qBase + (uint32_t)(G * p);  // input row y - 1
-                    for (uint32_t q = q0; q < q0 + G + 2 && ok; q++)
-                        ok = tc_wait(smem_u32(&rowFull[q % kTcRing]), (q / kTcRing) & 1u,
-                            &abortFlag);
+                    // input rows y - 1 .. y + G: the pairs in slots pos, pos + 1 and pos + 2
+                    const uint32_t slot1 = next_slot(pos), slot2 = next_slot(slot1);
+                    ok = wait_pair(slot1);
+                    ok = ok && wait_pair(slot2);
                     if (!ok) break;
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     const uint32_t acc = groupCount % SLOTS, use = groupCount / SLOTS;
@@ -502,6 +532,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_const
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;");
                     const uint32_t dAcc = tmem + acc * (uint32_t)ACC_COLS;
+                    // A descriptors of the three pairs: only the low word's address field differs
+                    const uint32_t aHi = (uint32_t)(aDesc0 >> 32);
+                    const uint32_t aLo[3] = {(uint32_t)aDesc0 + pos * (kSlotBytes / 16),
+                        (uint32_t)aDesc0 + slot1 * (kSlotBytes / 16),
+                        (uint32_t)aDesc0 + slot2 * (kSlotBytes / 16)};
 #pragma unroll
                     for (int tx = 0; tx < 3; tx++) {
 #pragma unroll
@@ -510,10 +545,9 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_const
                             for (int o = 0; o < G + 2; o++) {
                                 const int k = kOrder[o];
                                 const int jlo = k - 2 > 0 ? k - 2 : 0, jhi = k < G - 1 ? k : G - 1;
-                                const uint32_t slot = (q0 + (uint32_t)k) % kTcRing;
-                                // 16-byte units: slot row, channel group 2 kc, pixel tx
-                                const uint64_t aDesc = aDesc0 +
-                                    (uint64_t)(slot * (kSlotBytes / 16) + 2 * kc * kTcPlane + tx);
+                                // 16-byte units: row of the pair, channel group 2 kc, pixel tx
+                                const uint64_t aDesc = (uint64_t)aHi << 32 |
+                                    (aLo[k / 2] + (k % 2) * kRowUnits + 2 * kc * kTcSpx + tx);
                                 // weight block (tx, 2 kc), starting at tap row ty = k - jlo
                                 const uint64_t bDesc = bDesc0 +
                                     (uint64_t)((tx * KG + 2 * kc) * 3 * COUT + (2 - k + jlo) * COUT);
@@ -525,16 +559,15 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_const
                     }
                     tc_commit(smem_u32(&accFull[acc]));
                     // input rows y - 1 .. y + G - 2 have no later reader
-                    for (int k = 0; k < G; k++)
-                        tc_commit(smem_u32(&rowEmpty[(q0 + (uint32_t)k) % kTcRing]));
+                    tc_commit(smem_u32(&rowEmpty[pos]));
+                    tc_commit(smem_u32(&rowEmpty[slot1]));
+                    pos = slot2;
                     groupCount++;
                 }
                 if (!ok) break;
-                // the strip's last two input rows are free once its last MMAs finish
-                const uint32_t qLast = qBase + (uint32_t)(G * P) + 1u;
-                tc_commit(smem_u32(&rowEmpty[(qLast - 1u) % kTcRing]));
-                tc_commit(smem_u32(&rowEmpty[qLast % kTcRing]));
-                qBase = qLast + 1u;
+                // the strip's last row pair is free once its last MMAs finish
+                tc_commit(smem_u32(&rowEmpty[pos]));
+                pos = next_slot(pos);
             }
             // every MMA issued has finished before the accumulators are freed
             // (waited for even after an abort: the tensor memory is freed below)
@@ -545,41 +578,78 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __grid_const
         }
         __syncwarp();
     } else if (warp < 4) {
-        // ---- producer (lane 0 of warp 1): input rows y0 - 1 .. y0 + G P of every strip,
-        // one TMA box per row (8 channels x 130 pixels x every channel group, zero outside
-        // the image, landing as [group][pixel][8 channels]), completing the row's rowFull
-        // transaction count
-        if (warp == 1 && lane == 0) {
-            constexpr uint32_t kRowBytes = (uint32_t)(KG * kTcSpx * 16);
-            uint32_t q = 0;
+        // ---- producer (warp 1): row pairs (y0 - 1, y0), ..., (y0 + G P - 1, y0 + G P) of
+        // every strip.  Lane l copies plane l % KG of row l / KG of a pair: its pixels
+        // x0 - 1 .. x0 + 128 are one contiguous run of the planar layout, so the copy is one
+        // cp.async.bulk of up to 2,080 bytes; what lies outside the image is zeroed by the
+        // warp before the pair's barrier is armed.
+        if (warp == 1) {
+            constexpr int kPlanes = 2 * KG;
+            static_assert(kPlanes <= 32, "a lane per plane");
+            uint32_t q = 0, slot = 0, use = 0;  // row pair q goes to slot q % kTcRing for the use-th time
             bool ok = true;
             for (int strip = blockIdx.x; strip < numStrips && ok; strip += gridDim.x) {
                 GBSP_STRIP_GEOMETRY(strip);
-                for (int gy = y0 - 1; gy <= y0 + G * P; gy++, q++) {
-                    const uint32_t slot = q % kTcRing, use = q / kTcRing;
-                    if (use > 0 && !tc_wait(smem_u32(&rowEmpty[slot]), (use - 1u) & 1u, &abortFlag)) {
+                // pixels [first, last) of the 130 lie inside the image
+                const int first = x0 == 0 ? 1 : 0;
+                const int last = min(kTcSpx, W - x0 + 1);
+                for (int gy = y0 - 1; gy <= y0 + G * P; gy += 2, q++) {
+                    if (use > 0)
+                        ok = tc_wait(smem_u32(&rowEmpty[slot]), (use - 1u) & 1u, &abortFlag);
+                    if (!__all_sync(0xFFFFFFFFu, ok)) {
                         ok = false;
                         break;
                     }
-                    const uint32_t bar = smem_u32(&rowFull[slot]);
-                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                                 :: "r"(bar), "r"(kRowBytes) : "memory");
                     const uint32_t dst = ringAddr + slot * kSlotBytes;
-                    asm volatile(
-                        "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes"
-                        " [%0], [%1, {%2, %3, %4, %5, %6}], [%7];"
-                        :: "r"(dst), "l"(reinterpret_cast<uint64_t>(&tmIn)), "r"(0), "r"(x0 - 1),
-                           "r"(0), "r"(gy), "r"(b), "r"(bar)
-                        : "memory");
+                    const bool in0 = gy >= 0 && gy < H, in1 = gy + 1 < H;  // gy + 1 >= 0
+                    const int border = first + kTcSpx - last;  // pixels of a row outside the image
+                    if (!(in0 && in1) || border > 0) {
+                        const auto zero = [&](int plane, int px) {
+                            asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};"
+                                         :: "r"(dst + 16u * (uint32_t)(plane * kTcSpx + px)), "r"(0u) : "memory");
+                        };
+                        for (int i = lane; i < kPlanes * border; i += 32) {
+                            const int px = i / kPlanes;
+                            zero(i % kPlanes, px < first ? px : last + px - first);
+                        }
+                        if (!in0)
+                            for (int i = lane; i < KG * kTcSpx; i += 32) zero(i / kTcSpx, i % kTcSpx);
+                        if (!in1)
+                            for (int i = lane; i < KG * kTcSpx; i += 32) zero(KG + i / kTcSpx, i % kTcSpx);
+                        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    }
+                    __syncwarp();
+                    const uint32_t bar = smem_u32(&rowFull[slot]);
+                    const uint32_t bytes = (uint32_t)(last - first) * 16u;
+                    if (lane == 0)
+                        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                                     :: "r"(bar), "r"(bytes * (uint32_t)(KG * ((in0 ? 1 : 0) + (in1 ? 1 : 0))))
+                                     : "memory");
+                    __syncwarp();
+                    if (lane < kPlanes && (lane < KG ? in0 : in1)) {
+                        const size_t row = (size_t)b * H + (size_t)(gy + lane / KG);
+                        const __nv_bfloat16 *src = in + cg_index(row, x0 - 1 + first, 8 * (lane % KG), W, CIN);
+                        asm volatile(
+                            "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes"
+                            " [%0], [%1], %2, [%3];"
+                            :: "r"(dst + 16u * (uint32_t)(lane * kTcSpx + first)), "l"(src), "r"(bytes), "r"(bar)
+                            : "memory");
+                    }
+                    if (++slot == (uint32_t)kTcRing) {
+                        slot = 0;
+                        use++;
+                    }
                 }
             }
-            // every box issued has landed before the CTA's shared memory is released
-            volatile uint32_t never = 0u;
-            for (uint32_t s0 = 0; s0 < kTcRing && s0 < q; s0++) {
-                const uint32_t lastUse = (q - 1u - ((q - 1u - s0) % kTcRing)) / kTcRing;
-                if (!tc_wait(smem_u32(&rowFull[s0]), lastUse & 1u, &never)) abortFlag = 1u;
+            // every copy issued has landed before the CTA's shared memory is released
+            if (lane == 0) {
+                volatile uint32_t never = 0u;
+                for (uint32_t s0 = 0; s0 < kTcRing && s0 < q; s0++) {
+                    const uint32_t lastUse = (q - 1u - ((q - 1u - s0) % kTcRing)) / kTcRing;
+                    if (!tc_wait(smem_u32(&rowFull[s0]), lastUse & 1u, &never)) abortFlag = 1u;
+                }
+                if (!ok) abortFlag = 1u;
             }
-            if (!ok) abortFlag = 1u;
         }
         __syncwarp();
     } else {
@@ -711,33 +781,10 @@ static PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder()
 }
 
 // TMA map of a channel-group-planar BF16 activation tensor [B][H][cin/8][W][8]
-// (dimension order: 8 channels, pixel, channel group, row, image): one box =
-// 8 channels x boxPixels pixels x every channel group of one row, i.e. cin/8
-// contiguous runs of 16 boxPixels bytes, written to shared memory as
-// [group][pixel][8 channels], zero outside the tensor.  input_tensor_map: the
-// forward convolution's boxes of kTcSpx pixels.
-static int planar_tensor_map(CUtensorMap *map, const void *in, int B, int H, int W, int cin,
-    int boxPixels)
-{
-    PFN_cuTensorMapEncodeTiled_v12000 encode = tensor_map_encoder();
-    if (!encode) return set_error(GBSP_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    const cuuint64_t dims[5] = {8, (cuuint64_t)W, (cuuint64_t)cin / 8, (cuuint64_t)H, (cuuint64_t)B};
-    const cuuint64_t strides[4] = {16, (cuuint64_t)W * 16, (cuuint64_t)W * cin * 2,
-        (cuuint64_t)H * W * cin * 2};
-    const cuuint32_t box[5] = {8, (cuuint32_t)boxPixels, (cuuint32_t)cin / 8, 1, 1};
-    const cuuint32_t elem[5] = {1, 1, 1, 1, 1};
-    CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, const_cast<void *>(in), dims,
-        strides, box, elem, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-        CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (r != CUDA_SUCCESS)
-        return set_error(GBSP_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r);
-    return GBSP_OK;
-}
-
-// The same tensor seen as 32-bit words [B][H][cin/8][W * 4] (dimension order:
+// seen as 32-bit words [B][H][cin/8][W * 4] (dimension order:
 // word, channel group, row, image): one box = boxPixels * 4 words (boxPixels
-// <= 64) of every channel group of one row, landing as the same
-// [group][pixel][8 channels] bytes in one 16 boxPixels-byte run per group.
+// <= 64) of every channel group of one row, landing as [group][pixel][8
+// channels] in one 16 boxPixels-byte run per group, zero outside the tensor.
 // x coordinates are pixel * 4 (16-byte aligned, negative allowed).
 static int planar_words_tensor_map(CUtensorMap *map, const void *in, int B, int H, int W, int cin,
     int boxPixels)
@@ -760,11 +807,6 @@ static int planar_words_tensor_map(CUtensorMap *map, const void *in, int B, int 
     return GBSP_OK;
 }
 
-static int input_tensor_map(CUtensorMap *map, const void *in, int B, int H, int W, int cin)
-{
-    return planar_tensor_map(map, in, B, H, W, cin, kTcSpx);
-}
-
 template <int CIN, int COUT, int EPI>
 int launch_conv_tc(cudaStream_t s, int smCount, const void *in, int B, int H, int W, const void *w,
     const float *bias, void *outB, float *outF, const float4 *noisy = nullptr,
@@ -772,12 +814,9 @@ int launch_conv_tc(cudaStream_t s, int smCount, const void *in, int B, int H, in
 {
     // weights, then the ring (rounded up to a 128-byte boundary inside the kernel)
     size_t smem = (size_t)9 * (CIN / 8) * COUT * 16 +
-        (size_t)kTcRing * (((CIN / 8) * kTcPlane * 16 + 127) / 128 * 128) + 128;
+        (size_t)kTcRing * ((2 * (CIN / 8) * kTcSpx * 16 + 127) / 128 * 128) + 128;
     auto kern = k_conv3x3_tc<CIN, COUT, EPI>;
     GBSP_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CUtensorMap map;
-    int rc = input_tensor_map(&map, in, B, H, W, CIN);
-    if (rc) return rc;
     const int ctas = smCount;  // one CTA per SM (the row ring takes most of shared memory)
     const int cols = B * ((W + kTcTileP - 1) / kTcTileP);
     // rows per strip: about six strips per CTA (strips go round-robin, so
@@ -790,7 +829,7 @@ int launch_conv_tc(cudaStream_t s, int smCount, const void *in, int B, int H, in
     // consecutive convolutions walk the strips in opposite orders, so a layer
     // starts on the rows its predecessor wrote last (still in L2)
     const int reverse = (int)(g_convLaunches.fetch_add(1, std::memory_order_relaxed) & 1u);
-    kern<<<grid, kTcThreads, smem, s>>>(map, B, H, W, rows, reverse,
+    kern<<<grid, kTcThreads, smem, s>>>(reinterpret_cast<const __nv_bfloat16 *>(in), B, H, W, rows, reverse,
         reinterpret_cast<const __nv_bfloat16 *>(w), bias, reinterpret_cast<__nv_bfloat16 *>(outB),
         outF, noisy, outFilt);
     GBSP_CUDA_TRY(cudaGetLastError());
