@@ -555,6 +555,15 @@ int gbsp_dn_tile_merge(void *stream, const float *denoised, const float *plainA,
 /* wt[8-tap][ci][co] = w[tap][co][ci]: weights of the data-gradient conv. */
 int gbsp_dn_flip_transpose(void *stream, const uint16_t *w, uint32_t cout, uint32_t cin,
     uint16_t *wt);
+/* dIn = BF16 of (data gradient of a conv3x3 layer) * (act > 0), one launch:
+ * dOut is the layer's output gradient (cout channels), weights its forward
+ * weights [tap][cout][cin] (BF16), act its input activations after ReLU (cin
+ * channels); the values are those of gbsp_dn_flip_transpose,
+ * gbsp_dn_conv3x3_forward_tc (epilogue 2) and gbsp_dn_relu_backward.
+ * (cin, cout): (48, 48), (48, 32).  Tensors 16-byte aligned. */
+int gbsp_dn_conv3x3_data_grad_relu_tc(void *stream, const uint16_t *dOut, uint32_t B, uint32_t H,
+    uint32_t W, uint32_t cout, const uint16_t *weights, uint32_t cin, const uint16_t *act,
+    uint16_t *dIn);
 /* out = dAct * (act > 0), as BF16. */
 int gbsp_dn_relu_backward(void *stream, const float *dAct, const uint16_t *act, uint64_t n,
     uint16_t *out);
@@ -588,6 +597,16 @@ int gbsp_dn_relmse_backward(void *stream, const float *logits, const float *nois
 /* One Adam step on n parameters (FP32 master copy, optional BF16 mirror). */
 int gbsp_dn_adam(void *stream, float *param, uint16_t *paramBf16, const float *grad, float *m,
     float *v, uint64_t n, float lr, float beta1, float beta2, float eps, uint32_t step);
+/* The same step on several tensors in one launch (paramBf16 may be NULL). */
+typedef struct gbsp_dn_adam_tensor {
+    float *param;
+    uint16_t *paramBf16;
+    const float *grad;
+    float *m, *v;
+    uint64_t n;
+} gbsp_dn_adam_tensor;
+int gbsp_dn_adam_all(void *stream, const gbsp_dn_adam_tensor *tensors, uint32_t count, float lr,
+    float beta1, float beta2, float eps, uint32_t step);
 
 /* ---- procedural meshes (src/mesh_generation.cpp) ------------------------------ */
 /* CreateIcosahedronMesh (src/mesh_generation.cpp:220-337) without its 2048

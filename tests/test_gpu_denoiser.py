@@ -503,3 +503,93 @@ def test_served_output_runs_end_to_end(gpu_lib, check_spp):
     # an untrained network is far from the bound: most tiles fall back
     assert st["flagged"] > 0 and st["fallback_samples"] > 0
     torch.cuda.set_stream(torch.cuda.default_stream())
+
+
+@pytest.mark.parametrize("li", [1, 7])
+@pytest.mark.parametrize("B,H,W", [(1, 1, 3), (2, 5, 129), (3, 33, 64)])
+def test_fused_data_gradient_matches_its_parts(gpu_lib, li, B, H, W):
+    """gbsp_dn_conv3x3_data_grad_relu_tc against data_grad followed by the ReLU
+    mask, bit for bit; zeros, negative zeros and NaNs among the activations."""
+    import torch
+
+    from vk_cinematic_gb300.denoiser import KPCNN, LAYERS, _check, _ptr, _stream
+
+    torch.manual_seed(10 * li + W)
+    net = KPCNN(seed=2)
+    cin, cout = LAYERS[li][0], LAYERS[li][1]
+    d = torch.randn((B, H, cout // 8, W, 8), device="cuda").to(torch.bfloat16)
+    act = torch.randn((B, H, cin // 8, W, 8), device="cuda").to(torch.bfloat16)
+    flat = act.view(-1)
+    flat[0::17], flat[1::23], flat[2::29] = 0.0, -0.0, float("nan")
+    got = net.data_grad_relu(li, d, act)
+    dact = net.data_grad(li, d)
+    ref = torch.empty_like(got)
+    _check(net.L.gbsp_dn_relu_backward(_stream(), _ptr(dact), _ptr(act),
+                                       ctypes.c_uint64(dact.numel()), _ptr(ref)))
+    torch.cuda.synchronize()
+    assert torch.equal(got.view(torch.int16), ref.view(torch.int16))
+
+
+@pytest.mark.parametrize("offset", [0, 1])
+def test_relmse_gradient_at_any_alignment(gpu_lib, offset):
+    """Logits on and off a 16-byte boundary (vector and scalar accesses) give
+    the same gradients, ragged block tails included."""
+    import torch
+
+    from vk_cinematic_gb300.denoiser import _check, _ptr, _stream
+
+    torch.manual_seed(5)
+    B, H, W = 2, 7, 19
+    L = gbsp.load()
+    n = B * H * W
+    store = torch.randn(n * 32 + 4, device="cuda")
+    noisy = torch.rand((B, H, W, 4), device="cuda")
+    target = torch.rand((B, H, W, 4), device="cuda")
+    out = []
+    for off in (0, offset):
+        logits = torch.empty(n * 32 + 4, device="cuda")[off:off + n * 32]
+        logits.copy_(store[:n * 32])
+        d = torch.empty((B, H, 4, W, 8), dtype=torch.bfloat16, device="cuda")
+        loss = torch.zeros(1, device="cuda")
+        _check(L.gbsp_dn_relmse_backward(_stream(), _ptr(logits), _ptr(noisy), _ptr(target), B, H,
+                                         W, _ptr(d), _ptr(loss)))
+        torch.cuda.synchronize()
+        out.append((d, float(loss)))
+    assert torch.equal(out[0][0].view(torch.int16), out[1][0].view(torch.int16))
+    assert abs(out[0][1] - out[1][1]) <= 1e-5 * abs(out[0][1])
+
+
+@pytest.mark.parametrize("sizes", [[1], [256, 257, 48], [7] * 40])
+def test_adam_over_several_tensors_matches_one_by_one(gpu_lib, sizes):
+    """gbsp_dn_adam_all against gbsp_dn_adam per tensor, bit for bit: block
+    remainders, more tensors than one launch takes, with and without mirror."""
+    import torch
+
+    from vk_cinematic_gb300.denoiser import _check, _ptr, _stream
+
+    torch.manual_seed(len(sizes))
+    L = gbsp.load()
+    f = ctypes.c_float
+
+    def make():
+        return [[torch.randn(n, device="cuda") for n in sizes] for _ in range(3)]
+
+    p, g, m = make()
+    v = [x.abs() * 0.1 for x in m]
+    q, mq, vq = ([x.clone() for x in t] for t in (p, m, v))
+    b1 = [torch.zeros(n, dtype=torch.bfloat16, device="cuda") for n in sizes]
+    b2 = [x.clone() for x in b1]
+    rows = [(p[k].data_ptr(), b1[k].data_ptr() if k % 2 == 0 else 0, g[k].data_ptr(), m[k].data_ptr(),
+             v[k].data_ptr(), n) for k, n in enumerate(sizes)]
+    table = np.array(rows, np.uint64)
+    _check(L.gbsp_dn_adam_all(_stream(), table.ctypes.data_as(ctypes.c_void_p), len(sizes), f(1e-3),
+                              f(0.9), f(0.999), f(1e-8), 3))
+    for k, n in enumerate(sizes):
+        _check(L.gbsp_dn_adam(_stream(), _ptr(q[k]), _ptr(b2[k]) if k % 2 == 0 else None, _ptr(g[k]),
+                              _ptr(mq[k]), _ptr(vq[k]), ctypes.c_uint64(n), f(1e-3), f(0.9), f(0.999),
+                              f(1e-8), 3))
+    torch.cuda.synchronize()
+    for a, b in zip(p + m + v, q + mq + vq):
+        assert torch.equal(a, b)
+    for a, b in zip(b1, b2):
+        assert torch.equal(a.view(torch.int16), b.view(torch.int16))

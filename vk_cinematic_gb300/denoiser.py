@@ -35,6 +35,12 @@ def _stream():
     return _vp(torch.cuda.current_stream().cuda_stream)
 
 
+def _stream_handle() -> int:
+    import torch
+
+    return torch.cuda.current_stream().cuda_stream
+
+
 def _ptr(t) -> _vp:
     return _vp(t.data_ptr())
 
@@ -125,18 +131,16 @@ class KPCNN:
         import torch
 
         B, H, W, cin = _dims(x)
-        _, cout, _ = self.wb[li].shape
+        cout = self.wb[li].shape[1]
         epi = LAYERS[li][2]
         if epi == 0:
             out = torch.empty((B, H, cout // 8, W, 8), dtype=torch.bfloat16, device="cuda")
-            _check(self._conv(_stream(), _ptr(x), _u32(B), _u32(H), _u32(W), _u32(cin),
-                              _ptr(self.wb[li]), _ptr(self.b[li]), _u32(cout), _int(0), _ptr(out),
-                              None))
+            outs = (out.data_ptr(), None)
         else:
             out = torch.empty((B, H, W, cout), dtype=torch.float32, device="cuda")
-            _check(self._conv(_stream(), _ptr(x), _u32(B), _u32(H), _u32(W), _u32(cin),
-                              _ptr(self.wb[li]), _ptr(self.b[li]), _u32(cout), _int(1), None,
-                              _ptr(out)))
+            outs = (None, out.data_ptr())
+        _check(self._conv(_stream_handle(), x.data_ptr(), B, H, W, cin, self.wb[li].data_ptr(),
+                          self.b[li].data_ptr(), cout, 1 if epi else 0, *outs))
         return out
 
     def forward(self, feats, keep=False):
@@ -319,11 +323,29 @@ class KPCNN:
                           None, _u32(cin), _int(2), None, _ptr(out)))
         return out
 
+    def data_grad_relu(self, li, d, act):
+        """dIn of layer li from its output gradient d, masked by the ReLU of the
+        layer's input activations act, BF16.  On the tcgen05 path one kernel;
+        the same values as data_grad() and the ReLU mask apart."""
+        import torch
+
+        B, H, W, cout = _dims(d)
+        out = torch.empty(act.shape, dtype=torch.bfloat16, device="cuda")
+        if self.conv_impl == "tcgen05":
+            _check(self.L.gbsp_dn_conv3x3_data_grad_relu_tc(
+                _stream_handle(), d.data_ptr(), B, H, W, cout, self.wb[li].data_ptr(),
+                self.wb[li].shape[2], act.data_ptr(), out.data_ptr()))
+            return out
+        dact = self.data_grad(li, d)
+        _check(self.L.gbsp_dn_relu_backward(_stream(), _ptr(dact), _ptr(act), _u64(dact.numel()),
+                                            _ptr(out)))
+        return out
+
     def weight_grad(self, li, x, d, dw, db):
         B, H, W, cin = _dims(x)
         cout = _dims(d)[3]
-        _check(self._wgrad(_stream(), _ptr(x), _ptr(d), _u32(B), _u32(H), _u32(W), _u32(cin),
-                           _u32(cout), _ptr(dw), _ptr(db)))
+        _check(self._wgrad(_stream_handle(), x.data_ptr(), d.data_ptr(), B, H, W, cin, cout,
+                           dw.data_ptr(), db.data_ptr()))
 
     def gradients(self, feats, noisy, target):
         """Loss and parameter gradients for one batch."""
@@ -335,33 +357,36 @@ class KPCNN:
         loss = torch.zeros(1, dtype=torch.float32, device="cuda")
         _check(self.L.gbsp_dn_relmse_backward(_stream(), _ptr(logits), _ptr(noisy), _ptr(target),
                                               _u32(B), _u32(H), _u32(W), _ptr(dlog), _ptr(loss)))
-        dws = [torch.zeros_like(w) for w in self.w]
-        dbs = [torch.zeros_like(b) for b in self.b]
+        # the weight-gradient kernels add to what they are given: one zeroed
+        # buffer, cut up (every size is a multiple of 16 floats, so views stay aligned)
+        sizes = [w.numel() for w in self.w] + [b.numel() for b in self.b]
+        flat = torch.zeros(sum(sizes), dtype=torch.float32, device="cuda").split(sizes)
+        dws = [f.view(w.shape) for f, w in zip(flat, self.w)]
+        dbs = list(flat[len(self.w):])
         last = len(LAYERS) - 1
         inputs = [feats] + acts
         self.weight_grad(last, inputs[last], dlog, dws[last], dbs[last])
-        dact = self.data_grad(last, dlog)
+        d = dlog
         for li in range(last - 1, -1, -1):
-            dm = torch.empty(acts[li].shape, dtype=torch.bfloat16, device="cuda")
-            _check(self.L.gbsp_dn_relu_backward(_stream(), _ptr(dact), _ptr(acts[li]),
-                                                _u64(dact.numel()), _ptr(dm)))
-            self.weight_grad(li, inputs[li], dm, dws[li], dbs[li])
-            if li > 0:
-                dact = self.data_grad(li, dm)
+            d = self.data_grad_relu(li + 1, d, acts[li])
+            self.weight_grad(li, inputs[li], d, dws[li], dbs[li])
         return loss, dws, dbs
 
     def train_step(self, feats, noisy, target, lr=1e-4):
         loss, dws, dbs = self.gradients(feats, noisy, target)
         self.step += 1
+        # gbsp_dn_adam_tensor rows: param, BF16 mirror, gradient, m, v, count
+        rows = []
         for li in range(len(LAYERS)):
             m, v, mb, vb = self.state[li]
-            _check(self.L.gbsp_dn_adam(_stream(), _ptr(self.w[li]), _ptr(self.wb[li]),
-                                       _ptr(dws[li]), _ptr(m), _ptr(v), _u64(self.w[li].numel()),
+            rows.append((self.w[li].data_ptr(), self.wb[li].data_ptr(), dws[li].data_ptr(),
+                         m.data_ptr(), v.data_ptr(), self.w[li].numel()))
+            rows.append((self.b[li].data_ptr(), 0, dbs[li].data_ptr(), mb.data_ptr(),
+                         vb.data_ptr(), self.b[li].numel()))
+        table = np.array(rows, np.uint64)
+        _check(self.L.gbsp_dn_adam_all(_stream(), table.ctypes.data_as(_vp), _u32(len(rows)),
                                        _f32(lr), _f32(0.9), _f32(0.999), _f32(1e-8),
                                        _u32(self.step)))
-            _check(self.L.gbsp_dn_adam(_stream(), _ptr(self.b[li]), None, _ptr(dbs[li]),
-                                       _ptr(mb), _ptr(vb), _u64(self.b[li].numel()), _f32(lr),
-                                       _f32(0.9), _f32(0.999), _f32(1e-8), _u32(self.step)))
         B, H, W, _ = noisy.shape
         return loss / (3.0 * B * H * W)
 

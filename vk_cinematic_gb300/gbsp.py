@@ -60,6 +60,7 @@ EXPORTS = [
     "gbsp_batch_set_node_widths", "gbsp_batch_get_node_widths", "gbsp_path_trace_tile_list",
     "gbsp_dn_tile_check", "gbsp_dn_tile_merge", "gbsp_dn_conv3x3_weight_grad_tcgen05",
     "gbsp_path_trace_tile_list_spp", "gbsp_path_trace_tile_split",
+    "gbsp_dn_conv3x3_data_grad_relu_tc", "gbsp_dn_adam_all",
 ]
 
 
@@ -113,6 +114,18 @@ class Material(ctypes.Structure):
 assert ctypes.sizeof(Material) == 36
 
 
+# Argument types of the calls a training step makes dozens of: with them plain
+# integers and floats are converted in C (objects of the same types still pass).
+_ARGTYPES = {
+    "gbsp_dn_conv3x3_forward_tc": [_vp, _vp, _u32, _u32, _u32, _u32, _vp, _vp, _u32, _i32, _vp, _vp],
+    "gbsp_dn_conv3x3_forward": [_vp, _vp, _u32, _u32, _u32, _u32, _vp, _vp, _u32, _i32, _vp, _vp],
+    "gbsp_dn_conv3x3_data_grad_relu_tc": [_vp, _vp, _u32, _u32, _u32, _u32, _vp, _u32, _vp, _vp],
+    "gbsp_dn_conv3x3_weight_grad_tcgen05": [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp],
+    "gbsp_dn_conv3x3_weight_grad_tc": [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp],
+    "gbsp_dn_conv3x3_weight_grad": [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp],
+}
+
+
 class GbspError(RuntimeError):
     pass
 
@@ -146,6 +159,8 @@ def load(build_if_missing: bool = True):
     lib.gbsp_scene_node_width.restype = _u32
     for name in EXPORTS:
         getattr(lib, name)  # raises if a declared symbol is not exported
+    for name, types in _ARGTYPES.items():
+        getattr(lib, name).argtypes = types
     _LIB = lib
     return lib
 
