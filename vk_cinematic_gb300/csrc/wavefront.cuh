@@ -343,6 +343,10 @@ __global__ void __launch_bounds__(128, 7) k_trace(Src src, const float4 *__restr
 // the vote; 67.8 ms with the weights below (steps that cost less than a node
 // visit win with fewer lanes).  2^20 incoherent rays against 2^18 triangles:
 // 2,366, 1,865, 1,737 and 1,768 us.
+// Queues shorter than the grid's lanes use as few lanes per warp as spread them
+// over all warps: a 128 x 128 x 4 crop of a dense part of that scene 692 -> 543
+// us, 641 x 359 x 7 watertight 1,183 -> 1,045 us (at least 4, 8 or 16 lanes
+// instead of 1: 560, 595 and 630 us for the crop).
 //
 // Every full-mask intrinsic stands at the loop head or in a branch taken on
 // the vote's (warp-uniform) result; the only exit is the vote's zero.  Same
@@ -393,9 +397,14 @@ __global__ void __launch_bounds__(kLaneThreads, kWT || Src::kManyScenes ? 6 : 7)
     const ColdWords cold{coldWords + threadIdx.x};
     // the node or leaf to visit next; kEmptyChild when none
     uint32_t ref = kEmptyChild;
+    // Short queues are spread over every warp: only this many lanes of a warp
+    // take rays.  Each lane's steps then wait for fewer others (the longest
+    // ray's chain of steps is what a short launch takes).
+    const uint32_t warps = gridDim.x * (kLaneThreads / 32);
+    const uint32_t quota = (count + warps - 1) / warps;
     // base: stack height at which the object being walked is done, -1 at
     // object level, -2 without a ray, -3 when the queue is drained
-    int sp = 0, base = -2;
+    int sp = 0, base = (uint32_t)lane < quota ? -2 : -3;
     uint32_t steps = 0;
     // the ray of the level being walked (world or object space); `bound` is the
     // largest entry distance still worth a visit at that level
