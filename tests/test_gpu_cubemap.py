@@ -38,6 +38,21 @@ def test_cube_map_matches_oracle(gpu_lib, hdri):
     assert np.array_equal(got[..., 3], ref[..., 3])
 
 
+@pytest.mark.parametrize("width,height", [(1, 1), (31, 9), (33, 7), (64, 8), (65, 1)])
+def test_cube_map_ragged_sizes(gpu_lib, hdri, width, height):
+    # blocks of 32 x 8 texels: one texel, a row and a column short, one over, exact;
+    # the source's odd width leaves its rows at every alignment of a texel pair
+    import torch
+
+    src = np.ascontiguousarray(hdri[:255, :509])
+    got = gbsp.create_cube_map(torch.from_numpy(src).cuda(), width, height).cpu().numpy()
+    ref = pyoracle.create_cube_map(src, width, height)
+    e = rel_err(got, ref)
+    assert got.shape == ref.shape
+    assert np.median(e) <= 1e-5
+    assert np.mean(e > 1e-3) <= max(1e-3, 3 / e.size)
+
+
 @pytest.mark.parametrize("mode,size,spp", [(gbsp.IRRADIANCE_UNIFORM, 12, 0),
                                            (gbsp.IRRADIANCE_RANDOM, 16, 32)])
 def test_irradiance_matches_oracle(gpu_lib, hdri, mode, size, spp):

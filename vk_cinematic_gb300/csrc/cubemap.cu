@@ -26,6 +26,7 @@
 // everything else follows the reference's operation order without
 // contraction.
 
+#include <algorithm>
 #include <vector>
 
 #include "gbsp_internal.h"
@@ -35,6 +36,7 @@ namespace cube {
 
 constexpr float kRadianceClamp = 10.0f;  // RADIANCE_CLAMP, src/config.h:37
 constexpr int kMaxGridSamples = 1024;
+constexpr float kGridDelta = 0.1f;
 constexpr int kIrrWarps = 8;
 
 struct Basis {
@@ -108,29 +110,46 @@ __device__ __forceinline__ V3 face_direction(const Basis &b, uint32_t x, uint32_
     return normalize(add(add(b.forward, mul(b.right, fx)), mul(b.up, fy)));
 }
 
-__global__ void k_cube_map(Image im, uint32_t width, uint32_t height, float4 *__restrict__ out)
+// Bound: instructions of the lookup (two atan2f, a cosf, a square root and
+// four divisions per texel), about 40 us of them at 6 x 1024^2 texels; 134 MB
+// of traffic would take 20.  Texel coordinates come from a 3-d grid: three
+// 64-bit divisions of a flat index had cost a fifth of the kernel.  6 x 1024^2
+// from 2048 x 1024: 78 -> 64 us, 90 % of the issue slots busy.
+constexpr int kCubeX = 32, kCubeY = 8;
+
+__global__ void __launch_bounds__(kCubeX * kCubeY) k_cube_map(Image im, uint32_t width, uint32_t height,
+    float4 *__restrict__ out)
 {
-    uint64_t total = 6ull * width * height;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t x = (uint32_t)(i % width);
-        uint32_t y = (uint32_t)((i / width) % height);
-        uint32_t layer = (uint32_t)(i / ((uint64_t)width * height));
-        V3 dir = face_direction(face_basis(layer), x, y, width, height);
+    const uint32_t x = blockIdx.x * kCubeX + threadIdx.x, layer = blockIdx.z;
+    if (x >= width) return;
+    const Basis b = face_basis(layer);
+    for (uint32_t y = blockIdx.y * kCubeY + threadIdx.y; y < height; y += gridDim.y * kCubeY) {
+        V3 dir = face_direction(b, x, y, width, height);
         float u, v;
         direction_uv(dir, u, v);
-        out[i] = sample_bilinear(im, u, v);
+        out[((size_t)layer * height + y) * width + x] = sample_bilinear(im, u, v);
     }
 }
 
-// Uniform grid: table entries (t.x, t.y = cos(theta), t.z, sin(theta)) of
-// MapSphericalToCartesianCoordinates (src/math_lib.h:864-871).
+// Uniform grid of nPhi x nTheta samples, theta fastest: table entries (t.x,
+// t.y = cos(theta), t.z, sin(theta)) of MapSphericalToCartesianCoordinates
+// (src/math_lib.h:864-871) at phi and theta as the reference's loops reach
+// them (additions of 0.1f, src/cubemap.cpp:155-160).
+//
+// Bound: the gathers, four texels per sample that no neighbouring lane shares
+// (L1 86 % busy, issue 63 %): 95 us for 6 x 32^2 texels, with or without 32-byte
+// loads of texel pairs.  Every block fills its own table, so a call needs no
+// allocation and no upload: 2.9 + 13 us of the call before.  Two samples in
+// flight 162 us for a bake of both maps; one 166, four 163.
 __global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_uniform(Image im, uint32_t width,
-    uint32_t height, const float2 *__restrict__ grid, uint32_t gridCount, float4 *__restrict__ out)
+    uint32_t height, uint32_t nPhi, uint32_t nTheta, float4 *__restrict__ out)
 {
     __shared__ float4 table[kMaxGridSamples];
+    const uint32_t gridCount = nPhi * nTheta;
     for (uint32_t k = threadIdx.x; k < gridCount; k += blockDim.x) {
-        float phi = grid[k].x, theta = grid[k].y;
+        float phi = 0.0f, theta = 0.0f;
+        for (uint32_t i = k / nTheta; i; i--) phi += kGridDelta;
+        for (uint32_t i = k % nTheta; i; i--) theta += kGridDelta;
         float st = sinf(theta);
         float4 e;
         e.x = st * cosf(phi);
@@ -141,18 +160,16 @@ __global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_uniform(Image im,
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
-    uint64_t total = 6ull * width * height;
-    uint64_t warpId = blockIdx.x * (uint64_t)kIrrWarps + (threadIdx.x >> 5);
-    uint64_t warps = (uint64_t)gridDim.x * kIrrWarps;
-    for (uint64_t i = warpId; i < total; i += warps) {
-        uint32_t x = (uint32_t)(i % width);
-        uint32_t y = (uint32_t)((i / width) % height);
-        uint32_t layer = (uint32_t)(i / ((uint64_t)width * height));
+    const uint32_t total = 6u * width * height;  // checked to fit
+    const uint32_t warps = gridDim.x * kIrrWarps;
+    for (uint64_t i64 = blockIdx.x * kIrrWarps + (threadIdx.x >> 5); i64 < total; i64 += warps) {
+        const uint32_t i = (uint32_t)i64, x = i % width, y = i / width % height, layer = i / width / height;
         Basis b = face_basis(layer);
         V3 normal = face_direction(b, x, y, width, height);
         V3 tangent = normalize(cross(b.up, normal));
         V3 bitangent = normalize(cross(normal, tangent));
         V3 irr = v3(0.0f, 0.0f, 0.0f);
+#pragma unroll 2
         for (uint32_t k = lane; k < gridCount; k += 32) {
             float4 e = table[k];
             V3 w = add(add(mul(normal, e.y), mul(tangent, e.x)), mul(bitangent, e.z));
@@ -301,8 +318,9 @@ int gbsp_create_cube_map(void *stream, const float *equirect, uint32_t eqWidth, 
     int rc = check_image(equirect, eqWidth, eqHeight, width, height, faces);
     if (rc) return rc;
     cube::Image im{reinterpret_cast<const float4 *>(equirect), eqWidth, eqHeight};
-    uint64_t total = 6ull * width * height;
-    cube::k_cube_map<<<grid_for(total, 256), 256, 0, (cudaStream_t)stream>>>(im, width, height,
+    const dim3 grid((width + cube::kCubeX - 1) / cube::kCubeX,
+        std::min((height + cube::kCubeY - 1) / cube::kCubeY, 65535u), 6);
+    cube::k_cube_map<<<grid, dim3(cube::kCubeX, cube::kCubeY), 0, (cudaStream_t)stream>>>(im, width, height,
         reinterpret_cast<float4 *>(faces));
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
@@ -323,28 +341,17 @@ int gbsp_create_irradiance_cube_map(void *stream, const float *equirect, uint32_
     uint64_t total = 6ull * width * height;
     if (total >> 32) return set_error(GBSP_ERR_CAPACITY, "cube map too large");
     if (mode == GBSP_IRRADIANCE_UNIFORM) {
-        // the reference's loops: phi, theta += 0.1f in float (src/cubemap.cpp:155-160)
-        std::vector<float2> grid;
-        const float delta = 0.1f;
-        for (float phi = 0.0f; phi < 2.0f * kPi; phi += delta)
-            for (float theta = 0.0f; theta < 0.5f * kPi; theta += delta)
-                grid.push_back(make_float2(phi, theta));
-        if (grid.size() > (size_t)cube::kMaxGridSamples)
+        // the lengths of the reference's loops: phi, theta += 0.1f in float (src/cubemap.cpp:155-160)
+        uint32_t nPhi = 0, nTheta = 0;
+        for (float phi = 0.0f; phi < 2.0f * kPi; phi += cube::kGridDelta) nPhi++;
+        for (float theta = 0.0f; theta < 0.5f * kPi; theta += cube::kGridDelta) nTheta++;
+        if (nPhi * nTheta > (uint32_t)cube::kMaxGridSamples)
             return set_error(GBSP_ERR_CAPACITY, "sample grid too large");
-        float2 *dGrid = nullptr;
-        GBSP_CUDA_TRY(cudaMallocAsync((void **)&dGrid, grid.size() * sizeof(float2), s));
-        cudaError_t e = cudaMemcpyAsync(dGrid, grid.data(), grid.size() * sizeof(float2),
-            cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) {
-            int block = 32 * cube::kIrrWarps;
-            uint64_t blocks = (total + cube::kIrrWarps - 1) / cube::kIrrWarps;
-            int gridBlocks = grid_for(blocks * block, block);
-            cube::k_irradiance_uniform<<<gridBlocks, block, 0, s>>>(im, width, height, dGrid,
-                (uint32_t)grid.size(), reinterpret_cast<float4 *>(faces));
-            e = cudaGetLastError();
-        }
-        cudaFreeAsync(dGrid, s);
-        if (e != cudaSuccess) return cuda_error(e, "irradiance (uniform)");
+        int block = 32 * cube::kIrrWarps;
+        uint64_t blocks = (total + cube::kIrrWarps - 1) / cube::kIrrWarps;
+        cube::k_irradiance_uniform<<<grid_for(blocks * block, block), block, 0, s>>>(im, width, height, nPhi,
+            nTheta, reinterpret_cast<float4 *>(faces));
+        GBSP_CUDA_TRY(cudaGetLastError());
         return GBSP_OK;
     }
     // random mode: jump table J^(2^k), J = M^(3 spp); host copy waits for the upload
