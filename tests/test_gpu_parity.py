@@ -652,6 +652,28 @@ def test_per_lane_trace_matches_static(rt, kind):
             assert ma[k] == mb[k], (k, ma[k], mb[k])
 
 
+@pytest.mark.parametrize("bounces", [1, 2, 3, 4, 7])
+def test_chained_waves_match_one_wave(rt, bounces):
+    """The queue lengths of a wave rotate through three control words that the
+    stages themselves clear, and a stage may start while the one before it
+    drains: many short waves, with sorted queues or without, every number of
+    bounces around the rotation, give the pixels and counters of one wave."""
+    s = scenes.config3_scene(width=70, height=37, spp=3, n_spheres=24, level=2, seed=6)
+    scene, ms, rend = gbsp.upload_scene(rt, s)
+    rend.options.max_bounces = bounces
+    out = []
+    for wave, flags in ((0, 0), (100, 0), (0, gbsp.FLAG_SORT_DIRECTIONS), (100, gbsp.FLAG_SORT_DIRECTIONS)):
+        rend.options.wave_paths, rend.options.flags = wave, flags
+        img, _, m = rend.tile((0, 0, s.width, s.height))
+        out.append((img.copy(), m.as_dict()))
+    a, ma = out[0]
+    assert ma["paths_traced"] == 70 * 37 * 3
+    for b, mb in out[1:]:
+        assert np.array_equal(a.view(np.uint32), b.view(np.uint32))
+        for k in ("paths_traced", "rays_traced", "ray_hit_count", "triangle_tests"):
+            assert ma[k] == mb[k], k
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

@@ -47,19 +47,19 @@ struct ManyScenes {
     const uint32_t *pathItem;
     __device__ __forceinline__ const SceneView &scene(uint32_t p) const
     {
-        return items[__ldg(pathItem + p)].sv;
+        return items[pathItem[p]].sv;
     }
     __device__ __forceinline__ const MaterialView &materials(uint32_t p) const
     {
-        return items[__ldg(pathItem + p)].mv;
+        return items[pathItem[p]].mv;
     }
     __device__ __forceinline__ uint32_t bounces(uint32_t p) const
     {
-        return items[__ldg(pathItem + p)].maxBounces;
+        return items[pathItem[p]].maxBounces;
     }
     __device__ __forceinline__ float clamp(uint32_t p) const
     {
-        return items[__ldg(pathItem + p)].clampValue;
+        return items[pathItem[p]].clampValue;
     }
 };
 
@@ -97,9 +97,10 @@ __device__ __forceinline__ uint32_t find_item_by_pixel(const BatchItemDev *items
 }
 
 __global__ void __launch_bounds__(256) k_bgenerate(const BatchItemDev *__restrict__ items,
-    uint32_t itemCount, BatchWave wave, WaveBuffers wb, uint32_t *pathItem)
+    uint32_t itemCount, BatchWave wave, WaveBuffers wb, uint32_t *pathItem, unsigned int *ctl)
 {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) reset_wave_ctl(ctl, wave.paths);
     if (p >= wave.paths) return;
     uint64_t gp = wave.pathBase + p;
     uint32_t k = find_item_by_path(items, itemCount, gp);
@@ -119,6 +120,7 @@ __global__ void __launch_bounds__(256) k_bgenerate(const BatchItemDev *__restric
 __global__ void __launch_bounds__(256) k_baccumulate(const BatchItemDev *__restrict__ items,
     uint32_t itemCount, BatchWave wave, WaveBuffers wb, unsigned long long *counters)
 {
+    stage_begin();
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t nans = 0;
     if (k < wave.pixels) {
@@ -645,26 +647,22 @@ static void enqueue_wavefront(gbsp_batch *b)
     for (const BatchItemDev &d : b->hostItems)
         if (d.sv.nodeQuads != quads) quads = 0;
     for (const BatchWave &w : b->waves) {
-        k_reset_ctl<<<1, 32, 0, s>>>(ctl, w.paths);
         if (w.maxBounces == 0) {
             k_bzero<<<(w.paths + 255) / 256, 256, 0, s>>>(wb, w.paths);
         } else {
             k_bgenerate<<<(w.paths + 255) / 256, 256, 0, s>>>(b->dItems.ptr, n, w, wb,
-                b->pathItem.ptr);
+                b->pathItem.ptr, ctl);
         }
         for (uint32_t bn = 0; bn < w.maxBounces; bn++) {
-            int inQ = (bn & 1) ? kCtlQueue1 : kCtlQueue0;
-            int outQ = (bn & 1) ? kCtlQueue0 : kCtlQueue1;
             const float4 *qO = wb.rayO + ((bn & 1) ? wb.cap : 0);
             const float4 *qD = wb.rayD + ((bn & 1) ? wb.cap : 0);
-            k_reset_stage<<<1, 1, 0, s>>>(ctl, outQ);
             // primary rays per warp, bounce rays per lane (the frame renderer's default)
             launch_trace_stage(bn > 0, b->watertight, quads,
                 resident ? trace_grid<ManyScenes>(bn > 0, b->watertight, quads, rt->smCount) : grid, s,
-                src, qO, qD, ctl + inQ, wb.hitA, wb.hitInst, ctl, counters, rt->dStatus);
-            k_shade<<<shadeGrid, 128, 0, s>>>(src, wb, bn, inQ, ctl, counters);
+                src, qO, qD, ctl + queue_word(bn), wb.hitA, wb.hitInst, ctl, counters, rt->dStatus);
+            launch_next(k_shade<ManyScenes>, shadeGrid, kShadeThreads, s, src, wb, bn, bn & 1u, ctl, counters);
         }
-        k_baccumulate<<<(w.pixels + 255) / 256, 256, 0, s>>>(b->dItems.ptr, n, w, wb, counters);
+        launch_next(k_baccumulate, (w.pixels + 255) / 256, 256, s, b->dItems.ptr, n, w, wb, counters);
     }
 }
 

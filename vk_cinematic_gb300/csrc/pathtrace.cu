@@ -351,31 +351,27 @@ static int render_waves(gbsp_runtime *rt, const SceneView &sv, const MaterialVie
         if (maxBounces == 0) {
             GBSP_CUDA_TRY(cudaMemsetAsync(wb.pathRad, 0, sizeof(float4) * (size_t)paths, s));
         } else {
-            k_reset_ctl<<<1, 32, 0, s>>>(ctl, paths);
-            k_generate<<<(paths + 255) / 256, 256, 0, s>>>(wp, wb);
-            rt->launches += 2;
+            k_generate<<<(paths + 255) / 256, 256, 0, s>>>(wp, wb, ctl);
+            rt->launches += 1;
             for (uint32_t b = 0; b < maxBounces; b++) {
-                // sorted queues: shade always writes queue 1, the sort moves it to queue 0
+                // sorted queues: shade always writes the second queue, the sort moves it to the first
                 const uint32_t side = sortDirs ? 0u : (b & 1u);
-                int inQ = side ? kCtlQueue1 : kCtlQueue0;
-                int outQ = side ? kCtlQueue0 : kCtlQueue1;
                 const float4 *qO = wb.rayO + (side ? cap : 0);
                 const float4 *qD = wb.rayD + (side ? cap : 0);
-                k_reset_stage<<<1, 1, 0, s>>>(ctl, outQ);
                 int e0 = timing ? rt->stage_event(s) : -1;
                 bool perLane = (opt.flags & GBSP_FLAG_TRACE_PER_LANE) ||
                     (!(opt.flags & GBSP_FLAG_TRACE_PER_WARP) && b > 0);
                 launch_trace_stage(perLane, sv.watertight != 0, sv.nodeQuads,
                     trace_grid<OneScene>(perLane, sv.watertight != 0, sv.nodeQuads, rt->smCount), s, one, qO, qD,
-                    ctl + inQ, wb.hitA, wb.hitInst, ctl, counters, rt->dStatus);
+                    ctl + queue_word(b), wb.hitA, wb.hitInst, ctl, counters, rt->dStatus);
                 int e1 = timing ? rt->stage_event(s) : -1;
-                k_shade<<<shadeGrid, 128, 0, s>>>(one, wb, b, inQ, ctl, counters);
+                launch_next(k_shade<OneScene>, shadeGrid, kShadeThreads, s, one, wb, b, side, ctl, counters);
                 if (sortDirs && b + 1 < maxBounces) {
-                    k_octant_count<<<kSortBlocks, 256, 0, s>>>(wb.rayD + cap, ctl, kCtlQueue1,
+                    k_octant_count<<<kSortBlocks, 256, 0, s>>>(wb.rayD + cap, ctl, queue_word(b + 1),
                         rt->sortHist.ptr);
-                    k_octant_scan<<<1, 1024, 0, s>>>(rt->sortHist.ptr, ctl, kCtlQueue1, kCtlQueue0);
+                    k_octant_scan<<<1, 1024, 0, s>>>(rt->sortHist.ptr);
                     k_octant_scatter<<<kSortBlocks, 256, 0, s>>>(wb.rayO + cap, wb.rayD + cap, ctl,
-                        kCtlQueue1, rt->sortHist.ptr, wb.rayO, wb.rayD);
+                        queue_word(b + 1), rt->sortHist.ptr, wb.rayO, wb.rayD);
                     rt->launches += 3;
                 }
                 int e2 = timing ? rt->stage_event(s) : -1;
@@ -383,11 +379,11 @@ static int render_waves(gbsp_runtime *rt, const SceneView &sv, const MaterialVie
                     rt->traceSpans.emplace_back(e0, e1);
                     rt->shadeSpans.emplace_back(e1, e2);
                 }
-                rt->launches += 3;
+                rt->launches += 2;
                 rt->traceLaunches += 1;
             }
         }
-        k_accumulate<<<(wp.pixels + 255) / 256, 256, 0, s>>>(wp, wb, dImage, imageWidth, counters);
+        launch_next(k_accumulate, (wp.pixels + 255) / 256, 256, s, wp, wb, dImage, imageWidth, counters);
         rt->launches += 1;
         GBSP_CUDA_TRY(cudaGetLastError());
     }
@@ -591,27 +587,23 @@ extern "C" int gbsp_path_trace_tile_noalloc(const gbsp_context *ctx, gbsp_tile t
         if (opt.max_bounces == 0) {
             GBSP_CUDA_TRY(cudaMemsetAsync(wb.pathRad, 0, sizeof(float4) * (size_t)paths, s));
         } else {
-            k_reset_ctl<<<1, 32, 0, s>>>(ctl, paths);
-            k_generate<<<(paths + 255) / 256, 256, 0, s>>>(wp, wb);
-            launches += 2;
+            k_generate<<<(paths + 255) / 256, 256, 0, s>>>(wp, wb, ctl);
+            launches += 1;
             for (uint32_t b = 0; b < opt.max_bounces; b++) {
-                int inQ = (b & 1) ? kCtlQueue1 : kCtlQueue0;
-                int outQ = (b & 1) ? kCtlQueue0 : kCtlQueue1;
-                k_reset_stage<<<1, 1, 0, s>>>(ctl, outQ);
                 // the same per-bounce scheduling choice as the regular entry points
                 // (it changes the order of work, not the results)
                 bool perLane = (opt.flags & GBSP_FLAG_TRACE_PER_LANE) ||
                     (!(opt.flags & GBSP_FLAG_TRACE_PER_WARP) && b > 0);
                 launch_trace_stage(perLane, one.sv.watertight != 0, one.sv.nodeQuads, grid, s, one,
-                    wb.rayO + ((b & 1) ? wb.cap : 0), wb.rayD + ((b & 1) ? wb.cap : 0), ctl + inQ,
+                    wb.rayO + ((b & 1) ? wb.cap : 0), wb.rayD + ((b & 1) ? wb.cap : 0), ctl + queue_word(b),
                     wb.hitA, wb.hitInst, ctl, counters, status);
-                k_shade<<<shade_grid<OneScene>(rt->smCount), 128, 0, s>>>(one, wb, b, inQ, ctl,
-                    counters);
-                launches += 3;
+                launch_next(k_shade<OneScene>, shade_grid<OneScene>(rt->smCount), kShadeThreads, s, one, wb,
+                    b, b & 1u, ctl, counters);
+                launches += 2;
                 traceLaunches += 1;
             }
         }
-        k_accumulate<<<(wp.pixels + 255) / 256, 256, 0, s>>>(wp, wb, image, ip->width, counters);
+        launch_next(k_accumulate, (wp.pixels + 255) / 256, 256, s, wp, wb, image, ip->width, counters);
         launches += 1;
         GBSP_CUDA_TRY(cudaGetLastError());
     }

@@ -84,9 +84,10 @@ __global__ void __launch_bounds__(128) k_intersect(SceneView sv, const float4 *_
 
 // Ray pairs -> queue layout (origin with path id 0, direction).
 __global__ void __launch_bounds__(256) k_split_rays(const float4 *__restrict__ rays, uint32_t count,
-    float4 *__restrict__ o, float4 *__restrict__ d)
+    float4 *__restrict__ o, float4 *__restrict__ d, unsigned int *ctl)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) reset_wave_ctl(ctl, count);
     if (i >= count) return;
     float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
     o[i] = make_float4(a.x, a.y, a.z, 0.0f);
@@ -94,10 +95,11 @@ __global__ void __launch_bounds__(256) k_split_rays(const float4 *__restrict__ r
 }
 
 // Queue-ordered hits -> the per-ray outputs of k_intersect (same values).
-__global__ void __launch_bounds__(256) k_intersect_outputs(SceneView sv, const int4 *__restrict__ hitA,
-    const int *__restrict__ hitInst, uint32_t count, float *tOut, int32_t *triOut, int32_t *objOut,
+__global__ void __launch_bounds__(256) k_intersect_outputs(SceneView sv, const int4 *hitA,
+    const int *hitInst, uint32_t count, float *tOut, int32_t *triOut, int32_t *objOut,
     float *attrOut, uint32_t *matOut)
 {
+    stage_begin();
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= count) return;
     int4 hA = hitA[i];
@@ -153,12 +155,11 @@ static int launch_intersect_per_lane(cudaStream_t s, const SceneView &sv, uint32
     OneScene one = {};
     one.sv = sv;
     const int blocks = (int)((n + 255) / 256);
-    k_split_rays<<<blocks, 256, 0, s>>>(rays, count, o, d);
-    k_reset_ctl<<<1, 32, 0, s>>>(ctl, count);
+    k_split_rays<<<blocks, 256, 0, s>>>(rays, count, o, d, ctl);
     launch_trace_stage(true, sv.watertight != 0, sv.nodeQuads,
-        trace_grid<OneScene>(true, sv.watertight != 0, sv.nodeQuads, smCount), s, one, o, d, ctl + kCtlQueue0, hitA,
+        trace_grid<OneScene>(true, sv.watertight != 0, sv.nodeQuads, smCount), s, one, o, d, ctl + queue_word(0), hitA,
         hitInst, ctl, counters, dStatus);
-    k_intersect_outputs<<<blocks, 256, 0, s>>>(sv, hitA, hitInst, count, tOut, triOut, objOut,
+    launch_next(k_intersect_outputs, blocks, 256, s, sv, hitA, hitInst, count, tOut, triOut, objOut,
         attrOut, matOut);
     cudaError_t e = cudaGetLastError();
     cudaFreeAsync(tmp, s);

@@ -10,13 +10,57 @@
 
 namespace gbsp {
 
-// Work/queue control words (u32) behind the metric counters.
+// Work/queue control words (u32) behind the metric counters.  The queue of
+// bounce b has its length in word kCtlQueues + b % 3: while bounce b is shaded
+// (reads word b, fills word b + 1), nothing reads word b + 2, so the shade
+// kernel zeroes it and the trace kernel's work counter for the next bounce.
+// A reset kernel of its own before every bounce and wave had cost a small
+// frame 7 of 180 us on the device and four launches.
 enum Ctl : int {
     kCtlTraceWork = 0,
-    kCtlQueue0 = 2,
-    kCtlQueue1 = 3,
+    kCtlQueues = 2,
     kCtlCount = 8
 };
+__host__ __device__ __forceinline__ int queue_word(uint32_t bounce) { return kCtlQueues + (int)(bounce % 3u); }
+
+// A new wave's control words, by the kernel that fills its first queue.
+__device__ __forceinline__ void reset_wave_ctl(unsigned int *ctl, uint32_t paths)
+{
+    ctl[kCtlTraceWork] = 0;
+    ctl[queue_word(0)] = paths;
+    ctl[queue_word(1)] = ctl[queue_word(2)] = 0;
+}
+
+// Kernels of a wave follow one another through memory.  Launched with
+// launch_next, a kernel may become resident while the one before it drains;
+// stage_begin, its first statement, holds it until that one has completed and
+// its writes are visible, and only then lets the next one in.  The chain is
+// transitive: a kernel completes after its predecessor did.  What one of them
+// writes, the next reads by plain loads: no __ldg and no const __restrict__,
+// which promise data that is constant for the whole life of a kernel.
+// 128 x 128 x 8 frame 227 -> 214 us, 641 x 359 x 7 watertight 929 -> 899 us, a
+// 128 x 128 x 4 crop 248 -> 232 us; long kernels are the same either way.
+__device__ __forceinline__ void stage_begin()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+// For kernels that start with stage_begin only.
+template <class... P, class... A>
+void launch_next(void (*kernel)(P...), int grid, int block, cudaStream_t s, A... args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // the caller reads cudaGetLastError
+}
 
 struct WaveBuffers {
     // a queued ray carries its path's state: the path id and the RNG state ride
@@ -81,20 +125,6 @@ struct OneScene {
 // ---------------------------------------------------------------------------
 // Stage kernels
 // ---------------------------------------------------------------------------
-static __global__ void k_reset_ctl(unsigned int *ctl, uint32_t queue0)
-{
-    if (threadIdx.x < kCtlCount) ctl[threadIdx.x] = 0;
-    __syncthreads();
-    if (threadIdx.x == 0) ctl[kCtlQueue0] = queue0;
-}
-
-static __global__ void k_reset_stage(unsigned int *ctl, int outQueue)
-{
-    ctl[kCtlTraceWork] = 0;
-    ctl[outQueue] = 0;
-}
-
-// ---------------------------------------------------------------------------
 // Stable counting sort of a ray queue by direction octant (sign bits of d),
 // so that the lanes of a warp walk the tree with the same near-to-far child
 // order.  Queue order otherwise follows path order (neighbouring pixels'
@@ -130,10 +160,8 @@ static __global__ void __launch_bounds__(256) k_octant_count(const float4 *__res
     if (threadIdx.x < 8) hist[threadIdx.x * kSortBlocks + blockIdx.x] = sh[threadIdx.x];
 }
 
-// Exclusive scan of hist[8][kSortBlocks] in (octant, block) order; also
-// publishes the count as the destination queue's length.
-static __global__ void __launch_bounds__(1024) k_octant_scan(uint32_t *hist, unsigned int *ctl,
-    int srcQueue, int dstQueue)
+// Exclusive scan of hist[8][kSortBlocks] in (octant, block) order.
+static __global__ void __launch_bounds__(1024) k_octant_scan(uint32_t *hist)
 {
     constexpr int kPer = 8 * kSortBlocks / 1024;
     __shared__ uint32_t warpSum[32];
@@ -166,7 +194,6 @@ static __global__ void __launch_bounds__(1024) k_octant_scan(uint32_t *hist, uns
         hist[t * kPer + k] = run;
         run += v[k];
     }
-    if (t == 0) ctl[dstQueue] = ctl[srcQueue];
 }
 
 static __global__ void __launch_bounds__(256) k_octant_scatter(const float4 *__restrict__ srcO,
@@ -252,9 +279,10 @@ __device__ __forceinline__ void wave_pixel(const WaveParams &wp, uint64_t pix, u
     tile_pixel(wp, t, pix - __ldg(wp.tileStart + t), x, y);
 }
 
-static __global__ void __launch_bounds__(256) k_generate(WaveParams wp, WaveBuffers wb)
+static __global__ void __launch_bounds__(256) k_generate(WaveParams wp, WaveBuffers wb, unsigned int *ctl)
 {
     uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p == 0) reset_wave_ctl(ctl, wp.paths);
     if (p >= wp.paths) return;
     uint32_t x, y, s;
     if (wp.tileSpp) {
@@ -281,10 +309,11 @@ static __global__ void __launch_bounds__(256) k_generate(WaveParams wp, WaveBuff
 // 69.5 ms with this one).  7 blocks of 128 per SM (72 registers); 6 measured
 // the same.
 template <class Src, bool kWT, int kQ>
-__global__ void __launch_bounds__(128, 7) k_trace(Src src, const float4 *__restrict__ rayO,
-    const float4 *__restrict__ rayD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
+__global__ void __launch_bounds__(128, 7) k_trace(Src src, const float4 *rayO,
+    const float4 *rayD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
     unsigned int *ctl, unsigned long long *counters, uint32_t *status)
 {
+    stage_begin();
     int lane = threadIdx.x & 31;
     uint32_t count = *queueCount;
     TraceCounters cnt = {0, 0, 0, 0, 0};
@@ -365,10 +394,11 @@ enum LaneStep : int { kStepNode = 0, kStepLeaf, kStepEnter, kStepLeave, kStepRay
 constexpr int kWeightNode = 3, kWeightLeaf = 3, kWeightEnter = 4, kWeightLeave = 5, kWeightRay = 3;
 
 template <class Src, bool kWT, int kQ>
-__global__ void __launch_bounds__(kLaneThreads, kWT || Src::kManyScenes ? 6 : 7) k_trace_lane(Src src, const float4 *__restrict__ rayO,
-    const float4 *__restrict__ rayD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
+__global__ void __launch_bounds__(kLaneThreads, kWT || Src::kManyScenes ? 6 : 7) k_trace_lane(Src src, const float4 *rayO,
+    const float4 *rayD, const unsigned int *queueCount, int4 *hitA, int *hitInst,
     unsigned int *ctl, unsigned long long *counters, uint32_t *status)
 {
+    stage_begin();
     const int lane = threadIdx.x & 31;
     const uint32_t count = *queueCount;
     unsigned int *work = &ctl[kCtlTraceWork];
@@ -614,18 +644,20 @@ constexpr int kShadeThreads = 128;
 
 template <class Src>
 __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(Src src, WaveBuffers wb, uint32_t bounce,
-    int inQueue, unsigned int *ctl, unsigned long long *counters)
+    uint32_t side, unsigned int *ctl, unsigned long long *counters)
 {
+    stage_begin();
     const int lane = threadIdx.x & 31;
     const uint32_t laneMaskLt = (1u << lane) - 1u;
     __shared__ uint8_t lists[kShadeThreads / 32][32 * kShadeRows];
     uint8_t *list = lists[threadIdx.x >> 5];  // hits from the front, misses from the back
-    const uint32_t count = ctl[inQueue];
-    int outQueue = inQueue == kCtlQueue0 ? kCtlQueue1 : kCtlQueue0;
-    const float4 *inO = wb.rayO + (inQueue == kCtlQueue0 ? 0 : wb.cap);
-    const float4 *inD = wb.rayD + (inQueue == kCtlQueue0 ? 0 : wb.cap);
-    float4 *outO = wb.rayO + (inQueue == kCtlQueue0 ? wb.cap : 0);
-    float4 *outD = wb.rayD + (inQueue == kCtlQueue0 ? wb.cap : 0);
+    const uint32_t count = ctl[queue_word(bounce)];
+    const int outQueue = queue_word(bounce + 1);
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[queue_word(bounce + 2)] = ctl[kCtlTraceWork] = 0;
+    const float4 *inO = wb.rayO + (side ? wb.cap : 0);
+    const float4 *inD = wb.rayD + (side ? wb.cap : 0);
+    float4 *outO = wb.rayO + (side ? 0 : wb.cap);
+    float4 *outD = wb.rayD + (side ? 0 : wb.cap);
     // short queues: fewer rows, so that every warp gets some entries
     const uint32_t warps = gridDim.x * (kShadeThreads / 32);
     const uint32_t rows = min(kShadeRows, max(1u, count / (32u * warps)));
@@ -758,6 +790,7 @@ __global__ void __launch_bounds__(kShadeThreads, 8) k_shade(Src src, WaveBuffers
 static __global__ void __launch_bounds__(256) k_accumulate(WaveParams wp, WaveBuffers wb, float4 *image,
     uint32_t imageWidth, unsigned long long *counters)
 {
+    stage_begin();
     uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t nans = 0;
     if (k < wp.pixels) {
@@ -878,10 +911,10 @@ void launch_trace_kernel(bool perLane, int grid, cudaStream_t s, const Src &src,
     unsigned long long *counters, uint32_t *status)
 {
     if (perLane)
-        k_trace_lane<Src, kWT, kQ><<<grid, kLaneThreads, 0, s>>>(src, qO, qD, queueCount, hitA,
+        launch_next(k_trace_lane<Src, kWT, kQ>, grid, kLaneThreads, s, src, qO, qD, queueCount, hitA,
             hitInst, ctl, counters, status);
     else
-        k_trace<Src, kWT, kQ><<<grid, 128, 0, s>>>(src, qO, qD, queueCount, hitA, hitInst, ctl,
+        launch_next(k_trace<Src, kWT, kQ>, grid, 128, s, src, qO, qD, queueCount, hitA, hitInst, ctl,
             counters, status);
 }
 
