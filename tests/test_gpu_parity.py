@@ -674,6 +674,39 @@ def test_chained_waves_match_one_wave(rt, bounces):
             assert ma[k] == mb[k], k
 
 
+@pytest.mark.parametrize("count", [1, 2, 3, 9, 257, 16384, 16385])
+def test_object_trees_find_every_object(rt, count):
+    """Scene builds around the size up to which one launch collapses the tree,
+    rebuilt twice on one scene at both widths: a ray down on each object of a
+    scattered grid finds that object."""
+    import torch
+
+    n = int(np.ceil(np.sqrt(count)))
+    sc = gbsp.Scene(rt)
+    v, i = gbsp.icosphere(0)[:2]
+    sc.create_mesh(v, i)
+    rng = np.random.default_rng(count)
+    for rebuild in range(2):
+        sc.clear_objects()
+        cells = rng.permutation(n * n)[:count]
+        xy = np.stack([cells % n, cells // n], 1).astype(np.float32) * 3.0
+        for p in xy:
+            sc.add_object(0, 1, (p[0], p[1], 0.0), scenes.IDENTITY_QUAT, (1.0, 1.0, 1.0))
+        rays = np.zeros((count, 8), np.float32)
+        rays[:, :2] = xy + np.float32(0.1)
+        rays[:, 2], rays[:, 6] = 50.0, -1.0
+        rays = torch.from_numpy(rays).cuda()
+        for width in (8, 4):
+            sc.set_node_width(width)
+            sc.build_broadphase()
+            obj = torch.full((count,), -7, dtype=torch.int32, device="cuda")
+            t, tri = torch.empty(count, device="cuda"), torch.empty_like(obj)
+            torch.cuda.synchronize()
+            sc.intersect_closest_device(count, rays.data_ptr(), t.data_ptr(), tri.data_ptr(), obj.data_ptr())
+            rt.synchronize()
+            assert np.array_equal(obj.cpu().numpy(), np.arange(count)), (rebuild, width)
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

@@ -519,10 +519,10 @@ int gbsp_create_mesh(gbsp_scene *scene, const gbsp_vertex *vertices, uint32_t ve
         hlo[t] = make_float4(mn.x, mn.y, mn.z, 0.0f);
         hhi[t] = make_float4(mx.x, mx.y, mx.z, 0.0f);
     }
-    if ((rc = build_wide_bvh(s, lo.ptr, hi.ptr, triCount, kMaxLeafPrims, scene->nodes, nodeBase,
-             trees, &order, rt->dStatus, hlo.data(), hhi.data())))
-        return rc;
     uint64_t triBase = scene->triCount;
+    if ((rc = build_wide_bvh(s, lo.ptr, hi.ptr, triCount, kMaxLeafPrims, (uint32_t)triBase, scene->nodes,
+             nodeBase, trees, &order, rt->dStatus, hlo.data(), hhi.data(), nullptr, nullptr)))
+        return rc;
     if ((rc = append_device(scene->tris, triBase, triCount, s)) ||
         (rc = append_device(scene->attrs, triBase, triCount, s)) ||
         (rc = append_device(scene->triIds, triBase, triCount, s)))
@@ -530,10 +530,6 @@ int gbsp_create_mesh(gbsp_scene *scene, const gbsp_vertex *vertices, uint32_t ve
     if ((rc = mesh_emit(s, dv.ptr, di.ptr, triCount, order.ptr, scene->tris.ptr + triBase,
              scene->attrs.ptr + triBase, scene->triIds.ptr + triBase, (uint32_t)triBase)))
         return rc;
-    for (int w = 0; w < kNodeWidths; w++)
-        if ((rc = offset_nodes(s, scene->nodes[w], trees[w].nodeCount, nodeBase[w],
-                 (uint32_t)triBase)))
-            return rc;
     gbsp_mesh_info mi;
     for (int w = 0; w < kNodeWidths; w++) {
         mi.rootNode[w] = nodeBase[w];
@@ -628,23 +624,16 @@ int gbsp_build_scene_broadphase(gbsp_scene *scene)
         hi[i] = make_float4(in.hi[0], in.hi[1], in.hi[2], 0.0f);
     }
     int rc;
-    DeviceBuffer<float4> dlo, dhi;
-    DeviceBuffer<uint32_t> order;
-    if ((rc = dlo.upload(lo.data(), n, s)) || (rc = dhi.upload(hi.data(), n, s))) return rc;
+    std::vector<uint32_t> ord;
     WideTree trees[kNodeWidths];
-    if ((rc = build_wide_bvh(s, dlo.ptr, dhi.ptr, n, 1, scene->nodes, scene->meshNodeCount, trees,
-             &order, rt->dStatus, lo.data(), hi.data())))
+    bool clean = false;
+    if ((rc = build_wide_bvh(s, nullptr, nullptr, n, 1, 0, scene->nodes, scene->meshNodeCount, trees, nullptr,
+             rt->dStatus, lo.data(), hi.data(), &ord, &clean)))
         return rc;
-    for (int w = 0; w < kNodeWidths; w++)
-        if ((rc = offset_nodes(s, scene->nodes[w], trees[w].nodeCount, scene->meshNodeCount[w], 0)))
-            return rc;
-    std::vector<uint32_t> ord(n);
-    GBSP_CUDA_TRY(cudaMemcpyAsync(ord.data(), order.ptr, 4 * (size_t)n, cudaMemcpyDeviceToHost, s));
-    GBSP_CUDA_TRY(cudaStreamSynchronize(s));
-    std::vector<Instance> inst(n);
-    for (uint32_t j = 0; j < n; j++)
-        if (ord[j] >= n) return set_error(GBSP_ERR_DEVICE_STATUS, "object order out of range");
     for (int w = 0; w < kNodeWidths; w++) {
+        // kept by the scene: the build above waited for the last upload of it
+        std::vector<Instance> &inst = scene->hostInstances[w];
+        inst.resize(n);
         for (uint32_t j = 0; j < n; j++) {
             const gbsp_object_info &o = scene->objects[ord[j]];
             inst[j] = o.inst;
@@ -655,10 +644,9 @@ int gbsp_build_scene_broadphase(gbsp_scene *scene)
         scene->tlasDepth[w] = trees[w].depth;
         scene->totalNodeCount[w] = scene->meshNodeCount[w] + trees[w].nodeCount;
     }
-    scene->leafOrder = ord;
+    scene->leafOrder.swap(ord);
     scene->committed = true;
-    GBSP_CUDA_TRY(cudaStreamSynchronize(s));
-    return check_stream_status(rt);
+    return clean ? GBSP_OK : check_stream_status(rt);
 }
 
 int gbsp_scene_info(const gbsp_scene *scene, uint32_t *objects, uint64_t *triangles,

@@ -5,7 +5,8 @@
 // depend on the tree shape: the reference returns every leaf whose box the
 // ray passes and the closest triangle among those, so any hierarchy of exact
 // box unions plus the per-triangle box test in the traversal gives the same
-// candidate set.  Here the tree is a linear BVH:
+// candidate set.  Here the binary tree is a binned-SAH tree built on the host
+// (sah_build.cpp), or above kSahMaxPrims primitives a linear BVH:
 //   1. per-primitive boxes and centroids, centroid bounds;
 //   2. 30-bit Morton codes, sorted with a stable LSD radix sort (8-bit digits,
 //      per-block ranks from __match_any_sync);
@@ -15,7 +16,7 @@
 //      from the same binary tree: each wide node repeatedly opens its
 //      largest-area child until it has W children; subtrees of at most
 //      leafMax primitives become leaves.  Leaves index the primitives in the
-//      sorted Morton order, which both widths share, so one triangle pool
+//      binary tree's order, which both widths share, so one triangle pool
 //      serves the trees of both widths.
 // Every loop is bounded by the primitive count or log2 of it.
 
@@ -24,9 +25,12 @@
 #include <vector>
 
 #include "gbsp_internal.h"
+#include "sah_build.h"
 
 namespace gbsp {
 namespace {
+
+using BinaryTreeView = BinaryTree<const float4, const uint32_t>;
 
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;  // elements per thread per tile
@@ -194,7 +198,6 @@ __device__ __forceinline__ int delta(const uint32_t *codes, int n, int i, int j)
 }
 
 // Binary child reference: bit 31 set = leaf (sorted position), else internal.
-constexpr uint32_t kBinLeaf = 0x80000000u;
 
 __global__ void karras_hierarchy(const uint32_t *codes, int n, uint32_t *left, uint32_t *right,
     uint32_t *parent, uint32_t *first, uint32_t *last)
@@ -317,16 +320,15 @@ __device__ __forceinline__ uint32_t node_child(const float4 *node, uint32_t quad
     return __float_as_uint(f);
 }
 
+// One wide node from the binary subtree item.bin; its internal children go to
+// the work list `out`.
 template <int W>
-__global__ void collapse_level(const CollapseItem *in, uint32_t inCount, CollapseItem *out,
-    uint32_t *outCount, uint32_t *nodeCounter, uint32_t nodeCapacity, const uint32_t *left,
-    const uint32_t *right, const uint32_t *first, const uint32_t *last, const float4 *nodeLo,
-    const float4 *nodeHi, const float4 *primLo, const float4 *primHi, const uint32_t *order,
-    uint32_t leafMax, float4 *nodes, uint32_t *status)
+__device__ __forceinline__ void collapse_item(CollapseItem item, CollapseItem *out, uint32_t *outCount,
+    uint32_t *nodeCounter, uint32_t nodeCapacity, const BinaryTreeView &t, uint32_t leafMax, float4 *nodes,
+    uint32_t *status)
 {
-    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= inCount) return;
-    CollapseItem item = in[k];
+    const uint32_t *left = t.left, *right = t.right, *first = t.first, *last = t.last, *order = t.order;
+    const float4 *nodeLo = t.nodeLo, *nodeHi = t.nodeHi, *primLo = t.primLo, *primHi = t.primHi;
     uint32_t ch[W];
     float4 clo[W], chi[W];
     int cnt = 2;
@@ -399,16 +401,24 @@ __global__ void collapse_level(const CollapseItem *in, uint32_t inCount, Collaps
     store_node(nodes + node_offset(item.wide, W / 4), W / 4, lo, hi, child);
 }
 
+template <int W>
+__global__ void collapse_level(const CollapseItem *in, uint32_t inCount, CollapseItem *out,
+    uint32_t *outCount, uint32_t *nodeCounter, uint32_t nodeCapacity, BinaryTreeView t, uint32_t leafMax,
+    float4 *nodes, uint32_t *status)
+{
+    uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= inCount) return;
+    collapse_item<W>(in[k], out, outCount, nodeCounter, nodeCapacity, t, leafMax, nodes, status);
+}
+
 // Structural check of a freshly built tree (relative indices): every
 // internal child index is greater than its parent's and below the node
 // count, every leaf range lies inside the primitives.  Children are always
 // allocated after their parent, so this rules out cycles and makes every
 // traversal loop finite.
-__global__ void validate_nodes(const float4 *nodes, uint32_t quads, uint32_t count,
-    uint32_t prims, uint32_t *status)
+__device__ __forceinline__ void validate_node(const float4 *nodes, uint32_t quads, uint32_t i,
+    uint32_t count, uint32_t prims, uint32_t *status)
 {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
     const float4 *n = nodes + node_offset(i, quads);
     for (uint32_t c = 0; c < 4 * quads; c++) {
         uint32_t r = node_child(n, quads, c);
@@ -417,6 +427,99 @@ __global__ void validate_nodes(const float4 *nodes, uint32_t quads, uint32_t cou
                                    : (r > i && r < count);
         if (!ok) atomicOr(status, kStatusBadIndex);
     }
+}
+
+__global__ void validate_nodes(const float4 *nodes, uint32_t quads, uint32_t count,
+    uint32_t prims, uint32_t *status)
+{
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < count) validate_node(nodes, quads, i, count, prims, status);
+}
+
+// Relative to absolute references of node i.
+__device__ __forceinline__ void offset_node(float4 *nodes, uint32_t quads, uint32_t i, uint32_t nodeBase,
+    uint32_t leafBase)
+{
+    float4 *n = nodes + node_offset(i, quads);
+    for (uint32_t q = 0; q < quads; q++) {
+        float4 &v = n[6 * quads + q];
+        float *w = &v.x;
+        for (int k = 0; k < 4; k++) {
+            uint32_t r = __float_as_uint(w[k]);
+            if (r == kEmptyChild) continue;
+            r = child_is_leaf(r) ? make_leaf(leaf_first(r) + leafBase, leaf_count(r)) : r + nodeBase;
+            w[k] = __uint_as_float(r);
+        }
+    }
+}
+
+// The whole collapse of a small tree, both widths in one launch: block w walks
+// the levels of tree w, then checks it and makes its references absolute.
+// result[4 * w ..]: node count, depth, status of the build, status word.
+//
+// Bound: latency.  The level loop on the host has a launch and a wait per level
+// and width; here there is one of each in all.  A scene build of 257 objects:
+// 446 us with the level loop, 195 with this kernel (and one scratch block
+// instead of seventeen); 4,096: 4.28 and 3.75 ms; 16,384: 17.4 and 16.5 ms.
+// Larger trees keep a launch per level (kOneBlockPrims): one block per width
+// works at one SM's rate.
+constexpr int kCollapseThreads = 256;
+
+struct CollapseJob {
+    float4 *nodes;       // the tree's first node in its pool
+    CollapseItem *work;  // 2 * capacity
+    uint32_t nodeBase;
+};
+
+template <int W>
+__device__ __forceinline__ void collapse_tree(const CollapseJob &job, uint32_t prims, uint32_t capacity,
+    const BinaryTreeView &t, uint32_t leafMax, uint32_t leafBase, uint32_t *dStatus, uint32_t *result)
+{
+    __shared__ uint32_t counts[2], nodeCounter, status;
+    if (threadIdx.x == 0) {
+        counts[0] = nodeCounter = 1;
+        counts[1] = status = 0;
+        job.work[0] = CollapseItem{0, 0};
+    }
+    __syncthreads();
+    uint32_t depth = 0;
+    // every level holds at least one node: at most `capacity` levels
+    while (depth < capacity) {
+        const int side = depth & 1;
+        const uint32_t n = counts[side];
+        if (n == 0) break;
+        const CollapseItem *in = job.work + (side ? capacity : 0);
+        CollapseItem *out = job.work + (side ? 0 : capacity);
+        for (uint32_t k = threadIdx.x; k < n; k += blockDim.x)
+            collapse_item<W>(in[k], out, &counts[side ^ 1], &nodeCounter, capacity, t, leafMax, job.nodes,
+                &status);
+        __syncthreads();
+        if (threadIdx.x == 0) counts[side] = 0;
+        __syncthreads();
+        depth++;
+    }
+    const uint32_t used = min(nodeCounter, capacity);
+    for (uint32_t i = threadIdx.x; i < used; i += blockDim.x) {
+        validate_node(job.nodes, W / 4, i, used, prims, &status);
+        offset_node(job.nodes, W / 4, i, job.nodeBase, leafBase);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        result[0] = used;
+        result[1] = depth;
+        result[2] = status;
+        result[3] = status ? atomicOr(dStatus, status) | status : *dStatus;
+    }
+}
+
+__global__ void __launch_bounds__(kCollapseThreads) k_collapse_small(CollapseJob wide8, CollapseJob wide4,
+    uint32_t prims, uint32_t capacity, BinaryTreeView t, uint32_t leafMax, uint32_t leafBase,
+    uint32_t *dStatus, uint32_t *result)
+{
+    if (blockIdx.x == 0)
+        collapse_tree<8>(wide8, prims, capacity, t, leafMax, leafBase, dStatus, result);
+    else
+        collapse_tree<4>(wide4, prims, capacity, t, leafMax, leafBase, dStatus, result + 4);
 }
 
 __global__ void single_leaf_root(const float4 *lo, const float4 *hi, float4 *nodes, uint32_t quads)
@@ -506,21 +609,10 @@ __global__ void k_offset_nodes(float4 *nodes, uint32_t quads, uint32_t count, ui
     uint32_t leafBase)
 {
     uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    float4 *n = nodes + node_offset(i, quads);
-    for (uint32_t q = 0; q < quads; q++) {
-        float4 &v = n[6 * quads + q];
-        float *w = &v.x;
-        for (int k = 0; k < 4; k++) {
-            uint32_t r = __float_as_uint(w[k]);
-            if (r == kEmptyChild) continue;
-            r = child_is_leaf(r) ? make_leaf(leaf_first(r) + leafBase, leaf_count(r)) : r + nodeBase;
-            w[k] = __uint_as_float(r);
-        }
-    }
+    if (i < count) offset_node(nodes, quads, i, nodeBase, leafBase);
 }
 
-int offset_nodes(cudaStream_t s, NodePool &pool, uint32_t nodeCount, uint32_t nodeBase,
+static int offset_nodes(cudaStream_t s, NodePool &pool, uint32_t nodeCount, uint32_t nodeBase,
     uint32_t leafBase)
 {
     if (!nodeCount) return GBSP_OK;
@@ -559,155 +651,26 @@ static int grow_pool(cudaStream_t s, NodePool &pool, size_t nodes)
     return GBSP_OK;
 }
 
-// Binary tree in the form the collapse reads: internal nodes 0 .. n-2 (root
-// 0), child references with kBinLeaf for a primitive (its sorted position),
-// each internal node's range [first, last] of sorted positions and its box,
-// and order[sorted position] = primitive.
-struct HostBinaryTree {
-    std::vector<uint32_t> left, right, first, last, order;
-    std::vector<float4> lo, hi;
-};
-
-// Top-down binned SAH build (Wald, "On fast construction of SAH-based
-// bounding volume hierarchies", 2007) of the binary tree over n >= 2
-// primitive boxes, split down to single primitives: at every node the
-// primitives' centroids are binned into kSahBins slabs along each axis, and
-// the split between bins that minimises area(left) x count(left) +
-// area(right) x count(right) partitions the node's range (a median split
-// when every centroid coincides).  Node boxes are exact unions.
-// 64 bins: on the 1080p benchmark scene 16, 32, 64 and 128 bins gave 6.71,
-// 6.48, 6.45 and 6.44 node visits per ray (1,518, 1,542, 1,547 and 1,550
-// Msamples/s) for a host build time that grows with the bin count.
-constexpr int kSahBins = 64;
 // Above this many primitives the device LBVH (Morton order, Karras tree)
 // is built instead: the host build's time grows as n log n on one core.
 constexpr uint32_t kSahMaxPrims = 1u << 20;
+// Up to this many primitives the collapse is one launch of one block per width.
+constexpr uint32_t kOneBlockPrims = 16384;
+constexpr uint32_t kMaxCollapseLevels = 201;
 
-static float half_area_host(const float4 &lo, const float4 &hi)
+static int build_status(uint32_t st)
 {
-    float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
-    return dx * dy + dy * dz + dz * dx;
-}
-
-static void sah_binary_tree(const float4 *plo, const float4 *phi, uint32_t n, HostBinaryTree &t)
-{
-    t.left.assign(n - 1, 0);
-    t.right.assign(n - 1, 0);
-    t.first.assign(n - 1, 0);
-    t.last.assign(n - 1, 0);
-    t.lo.assign(n - 1, make_float4(0, 0, 0, 0));
-    t.hi.assign(n - 1, make_float4(0, 0, 0, 0));
-    t.order.resize(n);
-    std::vector<float> cen(3 * (size_t)n);
-    for (uint32_t i = 0; i < n; i++) {
-        t.order[i] = i;
-        cen[3 * (size_t)i + 0] = (plo[i].x + phi[i].x) * 0.5f;
-        cen[3 * (size_t)i + 1] = (plo[i].y + phi[i].y) * 0.5f;
-        cen[3 * (size_t)i + 2] = (plo[i].z + phi[i].z) * 0.5f;
-    }
-    struct Job {
-        uint32_t node, begin, end;
-    };
-    std::vector<Job> jobs;
-    jobs.push_back({0, 0, n});
-    uint32_t next = 1;
-    const float inf = 3.0e38f;
-    while (!jobs.empty()) {
-        const Job j = jobs.back();
-        jobs.pop_back();
-        float4 blo = make_float4(inf, inf, inf, 0), bhi = make_float4(-inf, -inf, -inf, 0);
-        float cmin[3] = {inf, inf, inf}, cmax[3] = {-inf, -inf, -inf};
-        for (uint32_t k = j.begin; k < j.end; k++) {
-            const uint32_t p = t.order[k];
-            blo = make_float4(rmin(blo.x, plo[p].x), rmin(blo.y, plo[p].y), rmin(blo.z, plo[p].z), 0);
-            bhi = make_float4(rmax(bhi.x, phi[p].x), rmax(bhi.y, phi[p].y), rmax(bhi.z, phi[p].z), 0);
-            for (int a = 0; a < 3; a++) {
-                cmin[a] = std::min(cmin[a], cen[3 * (size_t)p + a]);
-                cmax[a] = std::max(cmax[a], cen[3 * (size_t)p + a]);
-            }
-        }
-        t.lo[j.node] = blo;
-        t.hi[j.node] = bhi;
-        t.first[j.node] = j.begin;
-        t.last[j.node] = j.end - 1;
-        int bestAxis = -1, bestBin = 0;
-        float bestCost = inf;
-        for (int a = 0; a < 3; a++) {
-            const float ext = cmax[a] - cmin[a];
-            if (!(ext > 0.0f)) continue;
-            const float scale = (float)kSahBins / ext;
-            uint32_t cnt[kSahBins] = {};
-            float4 lo[kSahBins], hi[kSahBins];
-            for (int b = 0; b < kSahBins; b++) {
-                lo[b] = make_float4(inf, inf, inf, 0);
-                hi[b] = make_float4(-inf, -inf, -inf, 0);
-            }
-            for (uint32_t k = j.begin; k < j.end; k++) {
-                const uint32_t p = t.order[k];
-                const int b = std::min(kSahBins - 1, (int)((cen[3 * (size_t)p + a] - cmin[a]) * scale));
-                cnt[b]++;
-                lo[b] = make_float4(std::min(lo[b].x, plo[p].x), std::min(lo[b].y, plo[p].y),
-                    std::min(lo[b].z, plo[p].z), 0);
-                hi[b] = make_float4(std::max(hi[b].x, phi[p].x), std::max(hi[b].y, phi[p].y),
-                    std::max(hi[b].z, phi[p].z), 0);
-            }
-            // suffix areas and counts, then a prefix sweep
-            float rArea[kSahBins];
-            uint32_t rCnt[kSahBins];
-            float4 rl = make_float4(inf, inf, inf, 0), rh = make_float4(-inf, -inf, -inf, 0);
-            uint32_t rc = 0;
-            for (int b = kSahBins - 1; b > 0; b--) {
-                rc += cnt[b];
-                rl = make_float4(std::min(rl.x, lo[b].x), std::min(rl.y, lo[b].y), std::min(rl.z, lo[b].z), 0);
-                rh = make_float4(std::max(rh.x, hi[b].x), std::max(rh.y, hi[b].y), std::max(rh.z, hi[b].z), 0);
-                rCnt[b] = rc;
-                rArea[b] = rc ? half_area_host(rl, rh) : 0.0f;
-            }
-            float4 ll = make_float4(inf, inf, inf, 0), lh = make_float4(-inf, -inf, -inf, 0);
-            uint32_t lc = 0;
-            for (int b = 0; b < kSahBins - 1; b++) {
-                lc += cnt[b];
-                ll = make_float4(std::min(ll.x, lo[b].x), std::min(ll.y, lo[b].y), std::min(ll.z, lo[b].z), 0);
-                lh = make_float4(std::max(lh.x, hi[b].x), std::max(lh.y, hi[b].y), std::max(lh.z, hi[b].z), 0);
-                if (lc == 0 || rCnt[b + 1] == 0) continue;
-                const float cost = half_area_host(ll, lh) * (float)lc + rArea[b + 1] * (float)rCnt[b + 1];
-                if (cost < bestCost) {
-                    bestCost = cost;
-                    bestAxis = a;
-                    bestBin = b;
-                }
-            }
-        }
-        uint32_t mid = j.begin + (j.end - j.begin) / 2;
-        if (bestAxis >= 0) {
-            const float scale = (float)kSahBins / (cmax[bestAxis] - cmin[bestAxis]);
-            const float c0 = cmin[bestAxis];
-            uint32_t *it = std::partition(t.order.data() + j.begin, t.order.data() + j.end,
-                [&](uint32_t p) {
-                    return std::min(kSahBins - 1, (int)((cen[3 * (size_t)p + bestAxis] - c0) * scale)) <=
-                        bestBin;
-                });
-            const uint32_t m = (uint32_t)(it - t.order.data());
-            if (m > j.begin && m < j.end) mid = m;
-        }
-        const uint32_t ranges[2][2] = {{j.begin, mid}, {mid, j.end}};
-        for (int side = 0; side < 2; side++) {
-            const uint32_t b = ranges[side][0], e = ranges[side][1];
-            uint32_t ref;
-            if (e - b == 1) {
-                ref = kBinLeaf | b;
-            } else {
-                ref = next++;
-                jobs.push_back({ref, b, e});
-            }
-            (side ? t.right : t.left)[j.node] = ref;
-        }
-    }
+    if (st & kStatusBuildLoop)
+        return set_error(GBSP_ERR_DEVICE_STATUS, "BVH build exceeded its node capacity");
+    if (st & kStatusBadIndex)
+        return set_error(GBSP_ERR_DEVICE_STATUS, "BVH build produced an invalid child reference");
+    return GBSP_OK;
 }
 
 int build_wide_bvh(cudaStream_t s, const float4 *dLo, const float4 *dHi, uint32_t n,
-    uint32_t leafMax, NodePool *pools, const uint32_t *nodeBase, WideTree *trees,
-    DeviceBuffer<uint32_t> *orderOut, uint32_t *dStatus, const float4 *hLo, const float4 *hHi)
+    uint32_t leafMax, uint32_t leafBase, NodePool *pools, const uint32_t *nodeBase, WideTree *trees,
+    DeviceBuffer<uint32_t> *orderOut, uint32_t *dStatus, const float4 *hLo, const float4 *hHi,
+    std::vector<uint32_t> *hostOrder, bool *statusClean)
 {
     if (n == 0) return set_error(GBSP_ERR_INVALID_ARGUMENT, "BVH over zero primitives");
     if (n >= (1u << 27)) return set_error(GBSP_ERR_CAPACITY, "BVH over %u primitives (max 2^27)", n);
@@ -715,60 +678,51 @@ int build_wide_bvh(cudaStream_t s, const float4 *dLo, const float4 *dHi, uint32_
     uint32_t capacity = n > 1 ? n - 1 : 1;  // wide nodes never exceed binary internal nodes
     for (int w = 0; w < kNodeWidths; w++)
         if ((rc = grow_pool(s, pools[w], (size_t)nodeBase[w] + capacity))) return rc;
-    if ((rc = orderOut->reserve(n, s))) return rc;
+    if (orderOut && (rc = orderOut->reserve(n, s))) return rc;
+    DeviceBuffer<float4> lo, hi;
+    if (!dLo && (n == 1 || n > kSahMaxPrims)) {
+        if ((rc = lo.upload(hLo, n, s)) || (rc = hi.upload(hHi, n, s))) return rc;
+        dLo = lo.ptr;
+        dHi = hi.ptr;
+    }
     if (n == 1) {
         for (int w = 0; w < kNodeWidths; w++) {
             single_leaf_root<<<1, 1, 0, s>>>(dLo, dHi, pools[w].node(nodeBase[w]), pools[w].quads);
             trees[w].nodeCount = 1;
             trees[w].depth = 1;
+            if ((rc = offset_nodes(s, pools[w], 1, nodeBase[w], leafBase))) return rc;
         }
         GBSP_CUDA_TRY(cudaGetLastError());
-        uint32_t zero = 0;
-        GBSP_CUDA_TRY(cudaMemcpyAsync(orderOut->ptr, &zero, 4, cudaMemcpyHostToDevice, s));
+        if (orderOut) GBSP_CUDA_TRY(cudaMemsetAsync(orderOut->ptr, 0, 4, s));
+        if (hostOrder) hostOrder->assign(1, 0u);
         GBSP_CUDA_TRY(cudaStreamSynchronize(s));
         return GBSP_OK;
     }
 
-    DeviceBuffer<uint32_t> codes[2], vals[2], hist, left, right, parent, first, last, arrivals,
-        counters;
+    BinaryTreeView tree;
+    std::vector<float4> hostTree;
+    DeviceBuffer<float4> treeMem;
+    DeviceBuffer<uint32_t> codes[2], vals[2], hist, left, right, parent, first, last, arrivals;
     DeviceBuffer<int> bounds;
     DeviceBuffer<float4> nodeLo, nodeHi;
-    DeviceBuffer<CollapseItem> q[2];
-    uint32_t sortBlocks = (n + kSortTile - 1) / kSortTile;
-    if ((rc = codes[0].reserve(n, s)) || (rc = codes[1].reserve(n, s)) ||
-        (rc = vals[0].reserve(n, s)) || (rc = vals[1].reserve(n, s)) ||
-        (rc = hist.reserve((size_t)256 * sortBlocks, s)) || (rc = left.reserve(n, s)) ||
-        (rc = right.reserve(n, s)) || (rc = parent.reserve(2 * (size_t)n, s)) ||
-        (rc = first.reserve(n, s)) || (rc = last.reserve(n, s)) ||
-        (rc = arrivals.reserve(n, s)) || (rc = counters.reserve(4, s)) ||
-        (rc = bounds.reserve(6, s)) || (rc = nodeLo.reserve(n, s)) ||
-        (rc = nodeHi.reserve(n, s)) || (rc = q[0].reserve(capacity, s)) ||
-        (rc = q[1].reserve(capacity, s)))
-        return rc;
-
-    const uint32_t *order = nullptr;
     if (hLo && hHi && n <= kSahMaxPrims) {
         // binned SAH tree on the host (the host boxes are the device ones)
-        HostBinaryTree ht;
+        hostTree.resize(BinaryTree<float4, uint32_t>::size(n));  // outlives the copy
+        const BinaryTree<float4, uint32_t> ht(hostTree.data(), n);
         sah_binary_tree(hLo, hHi, n, ht);
-        GBSP_CUDA_TRY(cudaMemcpyAsync(left.ptr, ht.left.data(), 4 * (size_t)(n - 1),
-            cudaMemcpyHostToDevice, s));
-        GBSP_CUDA_TRY(cudaMemcpyAsync(right.ptr, ht.right.data(), 4 * (size_t)(n - 1),
-            cudaMemcpyHostToDevice, s));
-        GBSP_CUDA_TRY(cudaMemcpyAsync(first.ptr, ht.first.data(), 4 * (size_t)(n - 1),
-            cudaMemcpyHostToDevice, s));
-        GBSP_CUDA_TRY(cudaMemcpyAsync(last.ptr, ht.last.data(), 4 * (size_t)(n - 1),
-            cudaMemcpyHostToDevice, s));
-        GBSP_CUDA_TRY(cudaMemcpyAsync(nodeLo.ptr, ht.lo.data(), sizeof(float4) * (n - 1),
-            cudaMemcpyHostToDevice, s));
-        GBSP_CUDA_TRY(cudaMemcpyAsync(nodeHi.ptr, ht.hi.data(), sizeof(float4) * (n - 1),
-            cudaMemcpyHostToDevice, s));
-        GBSP_CUDA_TRY(cudaMemcpyAsync(vals[0].ptr, ht.order.data(), 4 * (size_t)n,
-            cudaMemcpyHostToDevice, s));
-        // the host vectors must outlive the copies
-        GBSP_CUDA_TRY(cudaStreamSynchronize(s));
-        order = vals[0].ptr;
+        if ((rc = treeMem.upload(hostTree.data(), hostTree.size(), s))) return rc;
+        tree = BinaryTreeView(treeMem.ptr, n);
+        if (hostOrder) hostOrder->assign(ht.order, ht.order + n);
     } else {
+        const uint32_t sortBlocks = (n + kSortTile - 1) / kSortTile;
+        if ((rc = codes[0].reserve(n, s)) || (rc = codes[1].reserve(n, s)) ||
+            (rc = vals[0].reserve(n, s)) || (rc = vals[1].reserve(n, s)) ||
+            (rc = hist.reserve((size_t)256 * sortBlocks, s)) || (rc = left.reserve(n, s)) ||
+            (rc = right.reserve(n, s)) || (rc = parent.reserve(2 * (size_t)n, s)) ||
+            (rc = first.reserve(n, s)) || (rc = last.reserve(n, s)) ||
+            (rc = arrivals.reserve(n, s)) || (rc = bounds.reserve(6, s)) ||
+            (rc = nodeLo.reserve(n, s)) || (rc = nodeHi.reserve(n, s)))
+            return rc;
         init_bounds<<<1, 32, 0, s>>>(bounds.ptr);
         centroid_bounds<<<min(blocks_for(n, 256), 1024u), 256, 0, s>>>(dLo, dHi, n, bounds.ptr);
         morton_codes<<<blocks_for(n, 256), 256, 0, s>>>(dLo, dHi, n, bounds.ptr, codes[0].ptr,
@@ -784,18 +738,56 @@ int build_wide_bvh(cudaStream_t s, const float4 *dLo, const float4 *dHi, uint32_
             cur ^= 1;
         }
         GBSP_CUDA_TRY(cudaGetLastError());
-        const uint32_t *sorted = codes[cur].ptr;
-        order = vals[cur].ptr;
-        karras_hierarchy<<<blocks_for(n - 1, 256), 256, 0, s>>>(sorted, (int)n, left.ptr,
+        tree.primLo = dLo, tree.primHi = dHi, tree.nodeLo = nodeLo.ptr, tree.nodeHi = nodeHi.ptr;
+        tree.left = left.ptr, tree.right = right.ptr, tree.first = first.ptr, tree.last = last.ptr;
+        tree.order = vals[cur].ptr;
+        karras_hierarchy<<<blocks_for(n - 1, 256), 256, 0, s>>>(codes[cur].ptr, (int)n, left.ptr,
             right.ptr, parent.ptr, first.ptr, last.ptr);
         GBSP_CUDA_TRY(cudaMemsetAsync(arrivals.ptr, 0, 4 * (size_t)n, s));
         refit<<<blocks_for(n, 256), 256, 0, s>>>((int)n, left.ptr, right.ptr, parent.ptr, dLo,
-            dHi, order, nodeLo.ptr, nodeHi.ptr, arrivals.ptr, dStatus);
+            dHi, tree.order, nodeLo.ptr, nodeHi.ptr, arrivals.ptr, dStatus);
         GBSP_CUDA_TRY(cudaGetLastError());
+        if (hostOrder) {
+            hostOrder->resize(n);
+            GBSP_CUDA_TRY(cudaMemcpyAsync(hostOrder->data(), tree.order, 4 * (size_t)n,
+                cudaMemcpyDeviceToHost, s));
+            GBSP_CUDA_TRY(cudaStreamSynchronize(s));
+            for (uint32_t p : *hostOrder)
+                if (p >= n) return set_error(GBSP_ERR_DEVICE_STATUS, "primitive order out of range");
+        }
+    }
+    if (orderOut)
+        GBSP_CUDA_TRY(cudaMemcpyAsync(orderOut->ptr, tree.order, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s));
+
+    if (n <= kOneBlockPrims) {
+        DeviceBuffer<CollapseItem> work;  // two lists per width, then the results
+        if ((rc = work.reserve(4 * (size_t)capacity + 4, s))) return rc;
+        uint32_t *dResult = reinterpret_cast<uint32_t *>(work.ptr + 4 * (size_t)capacity), result[8];
+        CollapseJob jobs[kNodeWidths];
+        for (int w = 0; w < kNodeWidths; w++)
+            jobs[w] = CollapseJob{pools[w].node(nodeBase[w]), work.ptr + 2 * (size_t)capacity * w, nodeBase[w]};
+        k_collapse_small<<<kNodeWidths, kCollapseThreads, 0, s>>>(jobs[0], jobs[1], n, capacity, tree, leafMax,
+            leafBase, dStatus, dResult);
+        GBSP_CUDA_TRY(cudaGetLastError());
+        GBSP_CUDA_TRY(cudaMemcpyAsync(result, dResult, sizeof(result), cudaMemcpyDeviceToHost, s));
+        GBSP_CUDA_TRY(cudaStreamSynchronize(s));
+        for (int w = 0; w < kNodeWidths; w++) {
+            if (result[4 * w + 1] > kMaxCollapseLevels)
+                return set_error(GBSP_ERR_DEVICE_STATUS, "BVH collapse exceeded 200 levels");
+            trees[w].nodeCount = result[4 * w];
+            trees[w].depth = result[4 * w + 1];
+        }
+        const uint32_t st = result[2] | result[3] | result[6] | result[7];
+        if (statusClean) *statusClean = st == 0;
+        return build_status(st);
     }
 
     // collapse the same binary tree once per width, level by level;
     // counters: [0] node counter, [1..2] queue counts
+    DeviceBuffer<uint32_t> counters;
+    DeviceBuffer<CollapseItem> q[2];
+    if ((rc = counters.reserve(4, s)) || (rc = q[0].reserve(capacity, s)) || (rc = q[1].reserve(capacity, s)))
+        return rc;
     for (int w = 0; w < kNodeWidths; w++) {
         float4 *out = pools[w].node(nodeBase[w]);
         uint32_t init[4] = {1, 0, 0, 0};
@@ -806,13 +798,12 @@ int build_wide_bvh(cudaStream_t s, const float4 *dLo, const float4 *dHi, uint32_
         uint32_t inCount = 1, depth = 0;
         int qi = 0;
         while (inCount > 0) {
-            if (depth > 200)
+            if (depth >= kMaxCollapseLevels)
                 return set_error(GBSP_ERR_DEVICE_STATUS, "BVH collapse exceeded 200 levels");
             GBSP_CUDA_TRY(cudaMemsetAsync(counters.ptr + 1 + (qi ^ 1), 0, 4, s));
             auto kern = pools[w].quads == 2 ? collapse_level<8> : collapse_level<4>;
             kern<<<blocks_for(inCount, 128), 128, 0, s>>>(q[qi].ptr, inCount, q[qi ^ 1].ptr,
-                counters.ptr + 1 + (qi ^ 1), counters.ptr, capacity, left.ptr, right.ptr,
-                first.ptr, last.ptr, nodeLo.ptr, nodeHi.ptr, dLo, dHi, order, leafMax, out, dStatus);
+                counters.ptr + 1 + (qi ^ 1), counters.ptr, capacity, tree, leafMax, out, dStatus);
             GBSP_CUDA_TRY(cudaGetLastError());
             GBSP_CUDA_TRY(cudaMemcpyAsync(&inCount, counters.ptr + 1 + (qi ^ 1), 4,
                 cudaMemcpyDeviceToHost, s));
@@ -828,16 +819,12 @@ int build_wide_bvh(cudaStream_t s, const float4 *dLo, const float4 *dHi, uint32_
         GBSP_CUDA_TRY(cudaGetLastError());
         trees[w].nodeCount = used;
         trees[w].depth = depth;
+        if ((rc = offset_nodes(s, pools[w], used, nodeBase[w], leafBase))) return rc;
     }
-    GBSP_CUDA_TRY(cudaMemcpyAsync(orderOut->ptr, order, 4 * (size_t)n, cudaMemcpyDeviceToDevice, s));
     uint32_t st = 0;
     GBSP_CUDA_TRY(cudaMemcpyAsync(&st, dStatus, 4, cudaMemcpyDeviceToHost, s));
     GBSP_CUDA_TRY(cudaStreamSynchronize(s));
-    if (st & kStatusBuildLoop)
-        return set_error(GBSP_ERR_DEVICE_STATUS, "BVH build exceeded its node capacity");
-    if (st & kStatusBadIndex)
-        return set_error(GBSP_ERR_DEVICE_STATUS, "BVH build produced an invalid child reference");
-    return GBSP_OK;
+    return build_status(st);
 }
 
 }  // namespace gbsp

@@ -176,6 +176,7 @@ struct gbsp_scene {
     // instances in object-BVH leaf order, one array per width (they differ
     // only in the mesh root node index)
     gbsp::DeviceBuffer<gbsp::Instance> instances[gbsp::kNodeWidths];
+    std::vector<gbsp::Instance> hostInstances[gbsp::kNodeWidths];  // what was last uploaded
     uint32_t tlasRoot[gbsp::kNodeWidths] = {gbsp::kEmptyChild, gbsp::kEmptyChild};
     uint32_t tlasDepth[gbsp::kNodeWidths] = {0, 0};
     uint32_t maxDepth[gbsp::kNodeWidths] = {0, 0};
@@ -229,23 +230,22 @@ namespace gbsp {
 // tree built on the host when the host copies of the boxes (hLo/hHi) are
 // given and n <= 2^20, else a linear BVH built on the device.  Tree w is
 // appended to pools[w] at nodeBase[w] (growing the pool, keeping its
-// contents), with node indices relative to nodeBase[w]; trees[w] receives
-// its node count and depth.  Returns the primitive order (sorted position
-// -> primitive) both trees' leaves index.
+// contents); trees[w] receives its node count and depth.  The leaves of both
+// trees index the primitive order (sorted position -> primitive, from
+// leafBase on), returned on the device and on the host where asked for.
+// dLo/dHi may be null when the host copies are given.  Waits for the stream;
+// *statusClean becomes true when the status word was read on the way and was
+// zero.
 int build_wide_bvh(cudaStream_t s, const float4 *dLo, const float4 *dHi, uint32_t n,
-    uint32_t leafMax, NodePool *pools, const uint32_t *nodeBase, WideTree *trees,
-    DeviceBuffer<uint32_t> *orderOut, uint32_t *dStatus, const float4 *hLo = nullptr,
-    const float4 *hHi = nullptr);
+    uint32_t leafMax, uint32_t leafBase, NodePool *pools, const uint32_t *nodeBase, WideTree *trees,
+    DeviceBuffer<uint32_t> *orderOut, uint32_t *dStatus, const float4 *hLo, const float4 *hHi,
+    std::vector<uint32_t> *hostOrder, bool *statusClean);
 // Triangle boxes + records for a mesh: positions from VertexPNT, indices.
 int mesh_prepare(cudaStream_t s, const gbsp_vertex *dVerts, const uint32_t *dIdx,
     uint32_t triCount, float4 *dLo, float4 *dHi);
 int mesh_emit(cudaStream_t s, const gbsp_vertex *dVerts, const uint32_t *dIdx,
     uint32_t triCount, const uint32_t *dOrder, TriRecord *dTris, TriAttr *dAttrs,
     uint32_t *dTriIds, uint32_t triBase);
-// Moves nodeCount nodes at nodeBase of a pool from relative to absolute
-// indices (child node indices += nodeBase, leaf first += leafBase).
-int offset_nodes(cudaStream_t s, NodePool &pool, uint32_t nodeCount, uint32_t nodeBase,
-    uint32_t leafBase);
 
 // trace.cu
 // Reference counting of runtimes: scenes, material systems, batches and
