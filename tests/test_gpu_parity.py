@@ -707,6 +707,47 @@ def test_object_trees_find_every_object(rt, count):
             assert np.array_equal(obj.cpu().numpy(), np.arange(count)), (rebuild, width)
 
 
+@pytest.mark.parametrize("wt,width", [(False, 8), (True, 8), (False, 4)])
+def test_query_sizes_match_the_large_batch(rt, wt, width):
+    """Batches of every size class (one ray, ragged warps, more than a ray per
+    lane, the last size of the one-launch path and the first of the per-lane
+    path), from the host's packed rays and from device rays, give the values
+    that the same rays get within a large batch."""
+    import torch
+
+    s = scenes.config3_scene(width=64, height=64, spp=1, n_spheres=12, level=2, seed=3)
+    scene, ms, _ = gbsp.upload_scene(rt, s)
+    scene.set_intersection(gbsp.ISECT_WATERTIGHT if wt else gbsp.ISECT_REFERENCE_MT)
+    scene.set_node_width(width)
+    n = 65536 + 300
+    rng = np.random.default_rng(4)
+    rays = np.concatenate([rng.uniform(-8, 8, (n, 3)), rng.normal(size=(n, 3))], 1).astype(np.float32)
+    packed = np.zeros((n, 8), np.float32)
+    packed[:, 0:3], packed[:, 4:7] = rays[:, :3], rays[:, 3:]
+    dr = torch.from_numpy(packed).cuda()
+
+    def device(k):
+        t = torch.full((k,), -9.0, device="cuda")
+        tri, obj = (torch.full((k,), -9, dtype=torch.int32, device="cuda") for _ in range(2))
+        torch.cuda.synchronize()
+        scene.intersect_closest_device(k, dr.data_ptr(), t.data_ptr(), tri.data_ptr(), obj.data_ptr())
+        rt.synchronize()
+        return [x.cpu().numpy() for x in (t, tri, obj)]
+
+    whole, (attr, mat, m) = device(n), scene.intersect(rays)
+    assert m.as_dict()["rays_traced"] == n
+    assert 0.05 < (whole[1] >= 0).mean() < 0.95
+    assert np.array_equal(attr[:, 0].view(np.uint32), whole[0].view(np.uint32))
+    for k in (1, 31, 33, 1065, 7 * 152 + 1, 65535, 65536):
+        for a, b in zip(device(k), whole):
+            assert np.array_equal(a.view(np.uint32), b[:k].view(np.uint32)), k
+        ak, mk, m = scene.intersect(rays[:k])
+        assert np.array_equal(ak.view(np.uint32), attr[:k].view(np.uint32)), k
+        assert np.array_equal(mk, mat[:k]), k
+        m = m.as_dict()
+        assert m["rays_traced"] == k == m["ray_hit_count"] + m["ray_miss_count"]
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

@@ -65,7 +65,15 @@ struct DeviceBuffer {
     }
 };
 
-struct Counters;  // device metric block
+// Memory of host queries that a runtime keeps: device block, pinned results.
+constexpr size_t kQueryKeep = 64u << 20, kStageBytes = 1u << 20;
+
+// The block of counters, queue words and status as the host reads it.
+constexpr int kStatusSlot = GBSP_METRIC_COUNT + 8;  // u64 index of the status word
+struct Readback {
+    unsigned long long words[kStatusSlot + 1];
+    uint32_t status() const { return (uint32_t)words[kStatusSlot]; }
+};
 
 // Paths per wave of the wavefront renderers when the caller leaves it to the
 // library: 2^25 (about 9 GB of wave state at 5 bounces).  Larger waves have
@@ -102,8 +110,14 @@ struct gbsp_runtime {
     cudaStream_t stream = nullptr;
     bool ownsStream = false;
     int smCount = 0;
-    uint32_t *dStatus = nullptr;        // kernel status word
-    unsigned long long *dCounters = nullptr;  // GBSP_METRIC_COUNT u64 counters
+    // GBSP_METRIC_COUNT u64 counters, queue control words, status word: one
+    // block, so that the end of a call reads all of it in one copy
+    unsigned long long *dCounters = nullptr;
+    uint32_t *dStatus = nullptr;        // kernel status word, in that block
+    gbsp::Readback *readback = nullptr;  // pinned copy of the block
+    gbsp::DeviceBuffer<int32_t> slots;   // material slot per instance of the current render
+    gbsp::DeviceBuffer<float> query;     // rays and results of a host query
+    unsigned char *stage = nullptr;      // pinned results of a host query, kStageBytes
     cudaEvent_t ev[8] = {};
     // wavefront state, grown on demand
     gbsp::DeviceBuffer<float4> rayO, rayD;         // two queues back to back
@@ -112,7 +126,6 @@ struct gbsp_runtime {
     gbsp::DeviceBuffer<uint32_t> sortHist;       // octant histograms of the ray sort
     gbsp::DeviceBuffer<float4> vert;               // stored path vertices, two float4 each
     gbsp::DeviceBuffer<float4> pathRad;            // radiance per path
-    gbsp::DeviceBuffer<unsigned int> queueCounts;  // small control block
     gbsp::DeviceBuffer<float4> frame;              // last frame, RGBA32F
     gbsp::DeviceBuffer<float4> aov;                // 2 per pixel when GBSP_FLAG_AOV
     gbsp::DeviceBuffer<float4> pathAov;            // 2 per path of a wave
@@ -254,9 +267,10 @@ int mesh_emit(cudaStream_t s, const gbsp_vertex *dVerts, const uint32_t *dIdx,
 int runtime_retain(gbsp_runtime *rt);
 void runtime_release(gbsp_runtime *rt);
 
-int launch_intersect(cudaStream_t s, const SceneView &sv, uint32_t count, const float4 *rays,
-    float *tOut, int32_t *triOut, int32_t *objOut, float *attrOut, uint32_t *matOut,
-    const Instance *instHost, int smCount, unsigned long long *counters, uint32_t *dStatus);
+// Closest hits of `count` rays on rt's stream: six packed floats per ray, or
+// 16-byte aligned (origin, pad, direction, pad); outputs may be null.
+int launch_intersect(gbsp_runtime *rt, const SceneView &sv, uint32_t count, const float *rays, bool packed,
+    float *tOut, int32_t *triOut, int32_t *objOut, float *attrOut, uint32_t *matOut);
 
 // pathtrace.cu
 int render_frame(gbsp_runtime *rt, const SceneView &sv, const MaterialView &mv,

@@ -1,13 +1,13 @@
 // Batched closest-hit ray casting (config 2 and sp_RayIntersectScene batches).
 //
-// Small batches: k_intersect, a persistent kernel whose warps take 32 rays at
-// a time from a global atomic counter until the batch is exhausted (the
-// counter only grows, so each warp loops at most count/32 times).  Large
-// batches of (typically incoherent) rays go through the wavefront's per-lane
-// closest-hit kernel instead, where a lane fetches its next ray as soon as
-// its current one is done: the rays are split into the queue layout, traced,
-// and the queue-ordered hits turned into the requested outputs.  Rays are
-// (origin, pad, direction, pad) float4 pairs, read with 128-bit loads.
+// Small batches: k_intersect, one launch that takes the rays, walks them and
+// writes the outputs.  Large batches of (typically incoherent) rays go through
+// the wavefront's per-lane closest-hit kernel instead, where a lane fetches its
+// next ray as soon as its current one is done: the rays are split into the
+// queue layout, traced, and the queue-ordered hits turned into the requested
+// outputs, three chained launches.
+
+#include <algorithm>
 
 #include "gbsp_internal.h"
 #include "traverse.cuh"
@@ -15,107 +15,26 @@
 
 namespace gbsp {
 
-__device__ __forceinline__ void warp_add_counters(unsigned long long *counters,
-    const TraceCounters &c, uint32_t rays, uint32_t hits)
-{
-    uint32_t v[7] = {rays, hits, c.topNodes, c.meshNodes, c.triTests, c.boxTests, c.meshTests};
-#pragma unroll
-    for (int k = 0; k < 7; k++)
-        for (int off = 16; off; off >>= 1) v[k] += __shfl_xor_sync(0xFFFFFFFFu, v[k], off);
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(&counters[GBSP_METRIC_RAYS_TRACED], (unsigned long long)v[0]);
-        atomicAdd(&counters[GBSP_METRIC_RAY_HIT_COUNT], (unsigned long long)v[1]);
-        atomicAdd(&counters[GBSP_METRIC_RAY_MISS_COUNT], (unsigned long long)(v[0] - v[1]));
-        atomicAdd(&counters[GBSP_METRIC_BROADPHASE_NODE_VISITS], (unsigned long long)v[2]);
-        atomicAdd(&counters[GBSP_METRIC_MIDPHASE_NODE_VISITS], (unsigned long long)v[3]);
-        atomicAdd(&counters[GBSP_METRIC_TRIANGLE_TESTS], (unsigned long long)v[4]);
-        atomicAdd(&counters[GBSP_METRIC_MIDPHASE_BOX_TESTS], (unsigned long long)v[5]);
-        atomicAdd(&counters[GBSP_METRIC_MESH_TESTS_PERFORMED], (unsigned long long)v[6]);
-    }
-}
+constexpr int kWarpsPerSm = 7;  // k_intersect, see there
 
-template <bool kWT>
-__global__ void __launch_bounds__(128) k_intersect(SceneView sv, const float4 *__restrict__ rays,
-    uint32_t count, float *tOut, int32_t *triOut, int32_t *objOut, float *attrOut,
-    uint32_t *matOut, unsigned int *work, unsigned long long *counters, uint32_t *status)
-{
-    int lane = threadIdx.x & 31;
-    TraceCounters cnt = {0, 0, 0, 0, 0};
-    uint32_t rays_done = 0, hits = 0;
-    for (uint32_t guard = 0; guard <= count / 32 + 1; guard++) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(work, 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= count) break;
-        uint32_t i = base + lane;
-        if (i < count) {
-            float4 o4 = __ldg(rays + 2 * (size_t)i), d4 = __ldg(rays + 2 * (size_t)i + 1);
-            RayHit h = trace_closest<true, kWT>(sv, v3(o4.x, o4.y, o4.z), v3(d4.x, d4.y, d4.z), status,
-                cnt);
-            bool hit = h.prim >= 0;
-            rays_done++;
-            hits += hit ? 1u : 0u;
-            if (tOut) tOut[i] = hit ? h.t : -1.0f;
-            if (triOut) triOut[i] = hit ? (int32_t)__ldg(sv.triIds + h.prim) : -1;
-            const Instance *in = hit ? sv.instances + h.inst : nullptr;
-            if (objOut) objOut[i] = hit ? (int32_t)__ldg(&in->objectIndex) : -1;
-            if (attrOut) {
-                float *a = attrOut + 6 * (size_t)i;
-                if (hit) {
-                    V3 n;
-                    float ux, uy;
-                    hit_surface(sv, h, n, ux, uy);
-                    a[0] = h.t;
-                    a[1] = n.x;
-                    a[2] = n.y;
-                    a[3] = n.z;
-                    a[4] = ux;
-                    a[5] = uy;
-                } else {
-                    a[0] = -1.0f;
-                    a[1] = a[2] = a[3] = a[4] = a[5] = 0.0f;
-                }
-            }
-            if (matOut) matOut[i] = hit ? __ldg(&in->materialId) : 0u;
-        }
-    }
-    warp_add_counters(counters, cnt, rays_done, hits);
-}
 
-// Ray pairs -> queue layout (origin with path id 0, direction).
-__global__ void __launch_bounds__(256) k_split_rays(const float4 *__restrict__ rays, uint32_t count,
-    float4 *__restrict__ o, float4 *__restrict__ d, unsigned int *ctl)
-{
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0) reset_wave_ctl(ctl, count);
-    if (i >= count) return;
-    float4 a = __ldg(rays + 2 * (size_t)i), b = __ldg(rays + 2 * (size_t)i + 1);
-    o[i] = make_float4(a.x, a.y, a.z, 0.0f);
-    d[i] = make_float4(b.x, b.y, b.z, 0.0f);
-}
+struct QueryOutputs {
+    float *t;
+    int32_t *tri, *obj;
+    float *attr;  // 6 per ray: t, normal, uv
+    uint32_t *mat;
+};
 
-// Queue-ordered hits -> the per-ray outputs of k_intersect (same values).
-__global__ void __launch_bounds__(256) k_intersect_outputs(SceneView sv, const int4 *hitA,
-    const int *hitInst, uint32_t count, float *tOut, int32_t *triOut, int32_t *objOut,
-    float *attrOut, uint32_t *matOut)
+__device__ __forceinline__ void write_outputs(const SceneView &sv, const RayHit &h, uint32_t i,
+    const QueryOutputs &out)
 {
-    stage_begin();
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= count) return;
-    int4 hA = hitA[i];
-    RayHit h;
-    h.t = __int_as_float(hA.x);
-    h.u = __int_as_float(hA.y);
-    h.v = __int_as_float(hA.z);
-    h.prim = hA.w;
-    h.inst = hitInst[i];
-    bool hit = h.prim >= 0;
-    if (tOut) tOut[i] = hit ? h.t : -1.0f;
-    if (triOut) triOut[i] = hit ? (int32_t)__ldg(sv.triIds + h.prim) : -1;
+    const bool hit = h.prim >= 0;
+    if (out.t) out.t[i] = hit ? h.t : -1.0f;
+    if (out.tri) out.tri[i] = hit ? (int32_t)__ldg(sv.triIds + h.prim) : -1;
     const Instance *in = hit ? sv.instances + h.inst : nullptr;
-    if (objOut) objOut[i] = hit ? (int32_t)__ldg(&in->objectIndex) : -1;
-    if (attrOut) {
-        float *a = attrOut + 6 * (size_t)i;
+    if (out.obj) out.obj[i] = hit ? (int32_t)__ldg(&in->objectIndex) : -1;
+    if (out.attr) {
+        float *a = out.attr + 6 * (size_t)i;
         if (hit) {
             V3 n;
             float ux, uy;
@@ -131,59 +50,156 @@ __global__ void __launch_bounds__(256) k_intersect_outputs(SceneView sv, const i
             a[1] = a[2] = a[3] = a[4] = a[5] = 0.0f;
         }
     }
-    if (matOut) matOut[i] = hit ? __ldg(&in->materialId) : 0u;
+    if (out.mat) out.mat[i] = hit ? __ldg(&in->materialId) : 0u;
 }
 
-// Batches from this size on take the per-lane path.
+// Ray i of a batch: (origin, pad, direction, pad) float4 pairs, or six packed
+// floats as the host API takes them (4-byte aligned).
+template <bool kPacked>
+__device__ __forceinline__ void load_ray(const float *rays, size_t i, V3 &o, V3 &d)
+{
+    if (kPacked) {
+        const float *r = rays + 6 * i;
+        o = v3(__ldg(r), __ldg(r + 1), __ldg(r + 2));
+        d = v3(__ldg(r + 3), __ldg(r + 4), __ldg(r + 5));
+    } else {
+        const float4 *r = reinterpret_cast<const float4 *>(rays) + 2 * i;
+        const float4 a = __ldg(r), b = __ldg(r + 1);
+        o = v3(a.x, a.y, a.z);
+        d = v3(b.x, b.y, b.z);
+    }
+}
+
+// One ray per lane, `lanes` lanes of a warp.
+//
+// Bound: the latency of the longest walk, and the host around it.  Up to 7
+// warps per SM share a batch before a warp takes a second ray.  4,096, 20,011
+// and 65,535 rays against 24 spheres of 1,280 triangles: 27.2, 34.9 and 38.9 us
+// on the device (39.2, 40.9 and 43.9 with full warps taken from a counter and
+// general node visits); at 4 warps per SM 30.0, 40.4 and 41.3, at 14 27.1, 35.8
+// and 40.2, at 28 37.4, 44.6 and 45.6 us.  The per-lane path's three launches
+// cost 35 us for one ray where this takes 8.
+template <bool kWT, int kQ, bool kPacked>
+__global__ void __launch_bounds__(128, 7) k_intersect(SceneView sv, const float *__restrict__ rays,
+    uint32_t count, uint32_t lanes, QueryOutputs out, unsigned long long *counters, uint32_t *status)
+{
+    const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t i = warp * lanes + lane;
+    TraceCounters cnt = {0, 0, 0, 0, 0};
+    uint32_t done = 0, hits = 0;
+    if (lane < lanes && i < count) {
+        V3 o, d;
+        load_ray<kPacked>(rays, i, o, d);
+        const RayHit h = trace_closest<true, kWT, kQ>(sv, o, d, status, cnt);
+        write_outputs(sv, h, i, out);
+        done = 1;
+        hits = h.prim >= 0 ? 1u : 0u;
+    }
+    __syncwarp();
+    uint32_t v[7] = {done, hits, cnt.topNodes, cnt.meshNodes, cnt.triTests, cnt.boxTests, cnt.meshTests};
+#pragma unroll
+    for (int k = 0; k < 7; k++) v[k] = __reduce_add_sync(0xFFFFFFFFu, v[k]);
+    if (lane == 0 && v[0]) {
+        atomicAdd(&counters[GBSP_METRIC_RAYS_TRACED], (unsigned long long)v[0]);
+        atomicAdd(&counters[GBSP_METRIC_RAY_HIT_COUNT], (unsigned long long)v[1]);
+        atomicAdd(&counters[GBSP_METRIC_RAY_MISS_COUNT], (unsigned long long)(v[0] - v[1]));
+        atomicAdd(&counters[GBSP_METRIC_BROADPHASE_NODE_VISITS], (unsigned long long)v[2]);
+        atomicAdd(&counters[GBSP_METRIC_MIDPHASE_NODE_VISITS], (unsigned long long)v[3]);
+        atomicAdd(&counters[GBSP_METRIC_TRIANGLE_TESTS], (unsigned long long)v[4]);
+        atomicAdd(&counters[GBSP_METRIC_MIDPHASE_BOX_TESTS], (unsigned long long)v[5]);
+        atomicAdd(&counters[GBSP_METRIC_MESH_TESTS_PERFORMED], (unsigned long long)v[6]);
+    }
+}
+
+// Rays -> queue layout (origin with path id 0, direction).
+template <bool kPacked>
+__global__ void __launch_bounds__(256) k_split_rays(const float *__restrict__ rays, uint32_t count,
+    float4 *__restrict__ qo, float4 *__restrict__ qd, unsigned int *ctl)
+{
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) reset_wave_ctl(ctl, count);
+    if (i >= count) return;
+    V3 o, d;
+    load_ray<kPacked>(rays, i, o, d);
+    qo[i] = make_float4(o.x, o.y, o.z, 0.0f);
+    qd[i] = make_float4(d.x, d.y, d.z, 0.0f);
+}
+
+// Queue-ordered hits -> the per-ray outputs asked for.
+__global__ void __launch_bounds__(256) k_intersect_outputs(SceneView sv, const int4 *hitA,
+    const int *hitInst, uint32_t count, QueryOutputs out)
+{
+    stage_begin();
+    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count) return;
+    int4 hA = hitA[i];
+    RayHit h;
+    h.t = __int_as_float(hA.x);
+    h.u = __int_as_float(hA.y);
+    h.v = __int_as_float(hA.z);
+    h.prim = hA.w;
+    h.inst = hitInst[i];
+    write_outputs(sv, h, i, out);
+}
+
+// Batches from this size on take the per-lane path (which counts as hits those
+// in front of the origin only, as frames do): it is the faster one where many
+// rays per lane differ in length, 2^20 rays against 2^18 triangles, and costs
+// two launches more, 55 against 39 us at this size on the scene above.
 constexpr uint32_t kPerLaneBatch = 1u << 16;
 
-static int launch_intersect_per_lane(cudaStream_t s, const SceneView &sv, uint32_t count,
-    const float4 *rays, float *tOut, int32_t *triOut, int32_t *objOut, float *attrOut,
-    uint32_t *matOut, int smCount, unsigned long long *counters, uint32_t *dStatus)
+template <bool kPacked>
+static int launch_small(cudaStream_t s, const SceneView &sv, uint32_t count, const float *rays,
+    const QueryOutputs &out, int smCount, unsigned long long *counters, uint32_t *status)
 {
-    // one allocation: O, D, hits (16 B each per ray), instance ids, control block
-    const size_t n = count;
-    const size_t bytes = n * (16 + 16 + 16 + 4) + sizeof(unsigned int) * kCtlCount + 64;
-    unsigned char *tmp = nullptr;
-    GBSP_CUDA_TRY(cudaMallocAsync((void **)&tmp, bytes, s));
-    float4 *o = reinterpret_cast<float4 *>(tmp);
-    float4 *d = o + n;
-    int4 *hitA = reinterpret_cast<int4 *>(d + n);
-    int *hitInst = reinterpret_cast<int *>(hitA + n);
-    unsigned int *ctl = reinterpret_cast<unsigned int *>(
-        (reinterpret_cast<uintptr_t>(hitInst + n) + 63) & ~(uintptr_t)63);
-    OneScene one = {};
-    one.sv = sv;
-    const int blocks = (int)((n + 255) / 256);
-    k_split_rays<<<blocks, 256, 0, s>>>(rays, count, o, d, ctl);
-    launch_trace_stage(true, sv.watertight != 0, sv.nodeQuads,
-        trace_grid<OneScene>(true, sv.watertight != 0, sv.nodeQuads, smCount), s, one, o, d, ctl + queue_word(0), hitA,
-        hitInst, ctl, counters, dStatus);
-    launch_next(k_intersect_outputs, blocks, 256, s, sv, hitA, hitInst, count, tOut, triOut, objOut,
-        attrOut, matOut);
-    cudaError_t e = cudaGetLastError();
-    cudaFreeAsync(tmp, s);
-    GBSP_CUDA_TRY(e);
+    auto kern = sv.nodeQuads == 2 ? (sv.watertight ? k_intersect<true, 2, kPacked> : k_intersect<false, 2, kPacked>)
+                                  : (sv.watertight ? k_intersect<true, 0, kPacked> : k_intersect<false, 0, kPacked>);
+    const uint32_t warps = (uint32_t)smCount * kWarpsPerSm;
+    const uint32_t lanes = std::min(32u, (count + warps - 1) / warps);
+    const uint32_t used = (count + lanes - 1) / lanes;
+    kern<<<(used + 3) / 4, 128, 0, s>>>(sv, rays, count, lanes, out, counters, status);
+    GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
 }
 
-int launch_intersect(cudaStream_t s, const SceneView &sv, uint32_t count, const float4 *rays,
-    float *tOut, int32_t *triOut, int32_t *objOut, float *attrOut, uint32_t *matOut,
-    const Instance *, int smCount, unsigned long long *counters, uint32_t *dStatus)
+int launch_intersect(gbsp_runtime *rt, const SceneView &sv, uint32_t count, const float *rays, bool packed,
+    float *tOut, int32_t *triOut, int32_t *objOut, float *attrOut, uint32_t *matOut)
 {
     if (!count) return GBSP_OK;
-    if (count >= kPerLaneBatch)
-        return launch_intersect_per_lane(s, sv, count, rays, tOut, triOut, objOut, attrOut, matOut,
-            smCount, counters, dStatus);
-    // the work counter lives in the last counter slot's neighbour block
-    unsigned int *work = reinterpret_cast<unsigned int *>(counters + GBSP_METRIC_COUNT);
-    GBSP_CUDA_TRY(cudaMemsetAsync(work, 0, sizeof(unsigned int), s));
-    int grid = smCount * 8;
-    uint64_t needed = ((uint64_t)count + 127) / 128;
-    if ((uint64_t)grid > needed) grid = (int)needed;
-    auto kern = sv.watertight ? k_intersect<true> : k_intersect<false>;
-    kern<<<grid, 128, 0, s>>>(sv, rays, count, tOut, triOut, objOut, attrOut, matOut, work,
-        counters, dStatus);
+    cudaStream_t s = rt->stream;
+    const bool watertight = sv.watertight != 0;
+    const QueryOutputs out = {tOut, triOut, objOut, attrOut, matOut};
+    if (count < kPerLaneBatch) {
+        auto launch = packed ? launch_small<true> : launch_small<false>;
+        return launch(s, sv, count, rays, out, rt->smCount, rt->dCounters, rt->dStatus);
+    }
+    const size_t n = count;
+    // The runtime's wave buffers hold the queue.  A call that is being captured
+    // brings its own memory: a graph must not refer to buffers that a later
+    // call may replace.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    GBSP_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+    DeviceBuffer<float4> ownRays;
+    DeviceBuffer<int4> ownHits;
+    DeviceBuffer<int> ownInst;
+    const bool own = capture != cudaStreamCaptureStatusNone;
+    DeviceBuffer<int4> &hits = own ? ownHits : rt->hitA;
+    DeviceBuffer<int> &inst = own ? ownInst : rt->hitInst;
+    int rc;
+    if ((own && (rc = ownRays.reserve(2 * n, s))) ||
+        (!own && ((rc = rt->rayO.reserve(n, s)) || (rc = rt->rayD.reserve(n, s)))) ||
+        (rc = hits.reserve(n, s)) || (rc = inst.reserve(n, s)))
+        return rc;
+    float4 *o = own ? ownRays.ptr : rt->rayO.ptr, *d = own ? ownRays.ptr + n : rt->rayD.ptr;
+    unsigned int *ctl = reinterpret_cast<unsigned int *>(rt->dCounters + GBSP_METRIC_COUNT);
+    OneScene one = {};
+    one.sv = sv;
+    const int blocks = (int)((n + 255) / 256);
+    (packed ? k_split_rays<true> : k_split_rays<false>)<<<blocks, 256, 0, s>>>(rays, count, o, d, ctl);
+    launch_trace_stage(true, watertight, sv.nodeQuads,
+        trace_grid<OneScene>(true, watertight, sv.nodeQuads, rt->smCount), s, one, o, d,
+        ctl + queue_word(0), hits.ptr, inst.ptr, ctl, rt->dCounters, rt->dStatus);
+    launch_next(k_intersect_outputs, blocks, 256, s, sv, hits.ptr, inst.ptr, count, out);
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
 }
