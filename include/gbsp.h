@@ -586,6 +586,20 @@ int gbsp_dn_conv3x3_weight_grad_tc(void *stream, const uint16_t *in, const uint1
  * counterpart. */
 int gbsp_dn_conv3x3_weight_grad_tcgen05(void *stream, const uint16_t *in, const uint16_t *dOut,
     uint32_t B, uint32_t H, uint32_t W, uint32_t cin, uint32_t cout, float *dW, float *dBias);
+/* The same for up to 8 layers over one B x H x W, with their gradients in
+ * distinct tensors: a launch per shape and one reduction.  The sums of a layer
+ * are those of a call of its own.  scratch: device memory of
+ * gbsp_dn_weight_grads_scratch bytes, 16-byte aligned, free again behind the
+ * call's kernels; NULL: allocated for the call. */
+typedef struct gbsp_dn_weight_grad_layer {
+    const uint16_t *in, *dOut;
+    float *dW, *dBias;
+    uint32_t cin, cout;
+} gbsp_dn_weight_grad_layer;
+uint64_t gbsp_dn_weight_grads_scratch(const gbsp_dn_weight_grad_layer *layers, uint32_t count, uint32_t B,
+    uint32_t H, uint32_t W);
+int gbsp_dn_weight_grads_tcgen05(void *stream, const gbsp_dn_weight_grad_layer *layers, uint32_t count,
+    uint32_t B, uint32_t H, uint32_t W, float *scratch);
 /* out[p] = sum_k softmax(logits[p][0..24])_k * noisy[p + off5x5(k)] (edge-clamped);
  * logits have 32 channels per pixel. */
 int gbsp_dn_filter(void *stream, const float *logits, const float *noisy, uint32_t B, uint32_t H,

@@ -593,3 +593,62 @@ def test_adam_over_several_tensors_matches_one_by_one(gpu_lib, sizes):
         assert torch.equal(a, b)
     for a, b in zip(b1, b2):
         assert torch.equal(a.view(torch.int16), b.view(torch.int16))
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (1, 3, 65), (2, 9, 64), (1, 40, 130), (3, 64, 128)])
+def test_weight_gradients_together_match_one_by_one(gpu_lib, B, H, W):
+    # fewer chunks than SMs, one chunk per CTA and several; layers of all three
+    # shapes in one call, and one layer alone: the sums of a call each, bit for bit
+    import torch
+
+    from vk_cinematic_gb300 import denoiser
+
+    net = denoiser.KPCNN(seed=1)
+    g = torch.Generator().manual_seed(B * H * W)
+
+    def tensor(c):
+        t = torch.randn((B, H, c // 8, W, 8), generator=g) * 0.5
+        return t.to(torch.bfloat16).cuda()
+
+    inputs = [tensor(cin) for cin, _, _ in denoiser.LAYERS]
+    todo = [(li, tensor(cout)) for li, (_, cout, _) in enumerate(denoiser.LAYERS)][::-1]
+    one, together = [], []
+    for out in (one, together):
+        for _ in range(2):
+            out.append([torch.full_like(w, 0.25) for w in net.w])
+            out.append([torch.full_like(b, 0.25) for b in net.b])
+    for k in range(2):
+        for li, d in todo:
+            net.weight_grad(li, inputs[li], d, one[2 * k][li], one[2 * k + 1][li])
+    net.weight_grads(todo, inputs, together[0], together[1])
+    for part in (todo[:1], todo[1:4], todo[4:]):
+        net.weight_grads(part, inputs, together[2], together[3])
+    torch.cuda.synchronize()
+    for a, b in zip(one, together):
+        for x, y in zip(a, b):
+            assert torch.equal(x, y)
+    for (li, d) in todo:
+        ref = d.float().sum((0, 1, 3)).reshape(-1).cpu() + 0.25
+        tol = 2e-6 * float(d.float().abs().sum((0, 1, 3)).max()) + 1e-6
+        assert float((together[1][li].cpu() - ref).abs().max()) <= tol
+
+
+def test_kept_output_gradients_are_bounded(gpu_lib, monkeypatch):
+    # gradients taken layer by layer, in twos and all together are the same
+    import torch
+
+    from vk_cinematic_gb300 import denoiser
+
+    torch.manual_seed(9)
+    net = denoiser.KPCNN(seed=3)
+    B, H, W = 2, 8, 70
+    feats = torch.randn((B, H, 2, W, 8), device="cuda").to(torch.bfloat16)
+    rad, target = (torch.rand((B, H, W, 4), device="cuda") for _ in range(2))
+    out = []
+    for keep in (0, 2 * 2 * B * H * W * 48, 4 << 30):
+        monkeypatch.setattr(denoiser, "WGRAD_KEEP", keep)
+        loss, dws, dbs = net.gradients(feats, rad, target)
+        out.append(dws + dbs)
+    torch.cuda.synchronize()
+    for other in out[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(out[0], other))

@@ -1087,34 +1087,51 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(const __nv_bfloat16 *_
     if (tid < COUT) out[9 * COUT * CIN + tid] = bacc;
 }
 
-// dW[i] += sum over CTA slices of partial[slice][i] in a fixed order: thread
-// group g of kReduceGroups adds slices g, g + 8, ... and the groups' sums are
-// added in pairs; the last COUT entries of a slice are the bias gradient.
-// Bound: the latency of the loads (12.6 MB from L2 at 152 slices of 48 x 48
-// weights).  One thread per entry walking all slices took 13 us, 8 groups of
-// threads with 8 loads in flight each 7 us (4 groups 9.6).
+// dW[i] += sum over CTA slices of partial[slice][i] in a fixed order, for one
+// or several layers: thread group g of kReduceGroups adds slices g, g + 8, ...
+// and the groups' sums are added in pairs; the last COUT entries of a slice are
+// the bias gradient.
+// Bound: the latency of the loads (12.6 MB at 152 slices of 48 x 48 weights).
+// One thread per entry walking all slices took 13 us a layer, 8 groups of
+// threads with 8 loads in flight each 7 us (4 groups 9.6); the eight layers of
+// the network in one launch 27 us instead of 54.
 constexpr int kReduceGroups = 8, kReduceEntries = 32;
+constexpr int kWgLayers = 8;  // layers per launch
+
+struct ReduceJobs {
+    struct Layer {
+        const float *partial;
+        float *dW, *dBias;
+        int perSlice, wCount;
+        uint32_t firstBlock;
+    } l[kWgLayers];
+    int count, slices;
+};
 
 __global__ void __launch_bounds__(kReduceGroups * kReduceEntries) k_wgrad_reduce(
-    const float *__restrict__ partial, int slices, int perSlice, int wCount, float *dW, float *dBias)
+    const __grid_constant__ ReduceJobs jobs)
 {
     __shared__ float sums[kReduceGroups][kReduceEntries];
+    int layer = 0;
+    while (layer + 1 < jobs.count && blockIdx.x >= jobs.l[layer + 1].firstBlock) layer++;
+    const ReduceJobs::Layer &l = jobs.l[layer];
     const int e = threadIdx.x % kReduceEntries, g = threadIdx.x / kReduceEntries;
-    const int i = blockIdx.x * kReduceEntries + e;
+    const int i = (int)(blockIdx.x - l.firstBlock) * kReduceEntries + e;
     float sum = 0.0f;
-    if (i < perSlice) {
+    if (i < l.perSlice) {
+        const float *__restrict__ partial = l.partial;
 #pragma unroll 8
-        for (int k = g; k < slices; k += kReduceGroups) sum += __ldg(partial + (size_t)k * perSlice + i);
+        for (int k = g; k < jobs.slices; k += kReduceGroups) sum += __ldg(partial + (size_t)k * l.perSlice + i);
     }
     sums[g][e] = sum;
     __syncthreads();
-    if (g != 0 || i >= perSlice) return;
+    if (g != 0 || i >= l.perSlice) return;
     sum = ((sums[0][e] + sums[1][e]) + (sums[2][e] + sums[3][e])) +
         ((sums[4][e] + sums[5][e]) + (sums[6][e] + sums[7][e]));
-    if (i < wCount)
-        dW[i] += sum;
+    if (i < l.wCount)
+        l.dW[i] += sum;
     else
-        dBias[i - wCount] += sum;
+        l.dBias[i - l.wCount] += sum;
 }
 
 // ---------------------------------------------------------------------------
@@ -1140,19 +1157,32 @@ __global__ void __launch_bounds__(kReduceGroups * kReduceEntries) k_wgrad_reduce
 // accumulator row 3 CIN the sum of d over the chunk: with column block
 // tx = 1, the bias gradient.
 //
-// One persistent CTA per SM walks its chunks (b, y, 64-pixel segment) through
-// a ring of kWtStages stages: lane 0 of warp 0 waits for a free stage (its
-// `empty` barrier, committed by the MMAs that read it) and issues the six
-// loads against the stage's `full` transaction count; lane 0 of warp 1 waits
-// on `full` and issues the MMAs into FP32 accumulators in tensor memory that
-// persist over all of the CTA's chunks.  At the end the warps read the
-// accumulators and write the CTA's partial sums to its slice of a scratch
-// buffer; k_wgrad_reduce adds the slices in a fixed order (deterministic).
-// Every wait is bounded and raises g_dnStatus on timeout.
+// One launch takes up to kWgLayers layers of one shape.  One persistent CTA per
+// SM walks its chunks (b, y, 64-pixel segment), layer after layer, through a
+// ring of kWtStages stages: lane 0 of the producer warp waits for a free stage
+// (its `empty` barrier, committed by the MMAs that read it) and issues the six
+// loads against the stage's `full` transaction count, into the next layer
+// without a stop; lane 0 of the MMA warp waits on `full` and issues the MMAs
+// into FP32 accumulators in tensor memory that persist over all of the CTA's
+// chunks of a layer.  At a layer's end (`done`) the other warps read the
+// accumulators, write the CTA's partial sums to its slice of a scratch buffer
+// and hand the accumulators back (`drained`); k_wgrad_reduce adds the slices in
+// a fixed order (deterministic).  Every wait is bounded and raises g_dnStatus
+// on timeout.
+//
+// Bound: the loads (each input row three times, from L2) and, with a launch, an
+// allocation and a reduction per layer, the host: a training step of 16 crops
+// of 128 x 128 took 585 us around 485 us on the device, with 16 launches for
+// its weight gradients; with four 550 around 490, and 364 us of the host
+// instead of 570.  The six 48 x 48 layers: 99 us together, 112 one by one.
 // ---------------------------------------------------------------------------
 constexpr int kWtPx = 64;
 constexpr int kWtStages = 4;
-constexpr int kWtThreads = 256;
+constexpr int kWtThreads = 320;  // eight epilogue warps, the producer, the MMA issuer
+
+struct WtMaps {
+    CUtensorMap x[kWgLayers], d[kWgLayers];
+};
 
 template <int CIN, int COUT>
 struct WtShape {
@@ -1172,15 +1202,14 @@ struct WtShape {
 
 template <int CIN, int COUT>
 __global__ void __launch_bounds__(kWtThreads, 1) k_conv3x3_wgrad_tma(
-    const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmD, int B, int H,
-    int W, float *__restrict__ partial)
+    const __grid_constant__ WtMaps maps, int layers, int B, int H, int W, float *__restrict__ partial)
 {
     using S = WtShape<CIN, COUT>;
     constexpr int N = S::N, MB = S::MB, MROWS = S::MROWS;
     // the ring starts at the first 1 KB boundary (the launch adds 1 KB of slack)
     extern __shared__ __align__(128) unsigned char smemRaw[];
     const uint32_t base = (smem_u32(smemRaw) + 1023u) & ~1023u;
-    __shared__ __align__(8) uint64_t full[kWtStages], empty[kWtStages], done;
+    __shared__ __align__(8) uint64_t full[kWtStages], empty[kWtStages], done, drained;
     __shared__ uint32_t tmemBase;
     __shared__ volatile uint32_t abortFlag;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -1202,6 +1231,7 @@ __global__ void __launch_bounds__(kWtThreads, 1) k_conv3x3_wgrad_tma(
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&empty[i])));
         }
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&done)));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(&drained)), "r"(4 * MB));
         abortFlag = 0u;
         asm volatile("fence.mbarrier_init.release.cluster;");
     }
@@ -1212,36 +1242,39 @@ __global__ void __launch_bounds__(kWtThreads, 1) k_conv3x3_wgrad_tma(
     const int segs = (W + kWtPx - 1) / kWtPx;
     const int chunks = B * H * segs;
 
-    if (warp == 0) {
+    // the launch sizes the grid so that every CTA has a chunk
+    if (warp == 8) {
         if (lane == 0) {
             uint32_t i = 0;
             bool ok = true;
-            for (int c = blockIdx.x; c < chunks && ok; c += gridDim.x, i++) {
-                const uint32_t st = i % kWtStages, use = i / kWtStages;
-                if (use > 0 && !(ok = tc_wait(smem_u32(&empty[st]), (use - 1u) & 1u, &abortFlag)))
-                    break;
-                const int seg = c % segs, row = c / segs;
-                const int b = row / H, y = row % H, x0 = seg * kWtPx;
-                const uint32_t bar = smem_u32(&full[st]), sb = base + st * S::kStage;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                             :: "r"(bar), "r"(S::kTxBytes) : "memory");
+            for (int l = 0; l < layers && ok; l++) {
+                const uint64_t mapX = reinterpret_cast<uint64_t>(&maps.x[l]),
+                               mapD = reinterpret_cast<uint64_t>(&maps.d[l]);
+                for (int c = blockIdx.x; c < chunks; c += gridDim.x, i++) {
+                    const uint32_t st = i % kWtStages, use = i / kWtStages;
+                    if (use > 0 && !(ok = tc_wait(smem_u32(&empty[st]), (use - 1u) & 1u, &abortFlag)))
+                        break;
+                    const int seg = c % segs, row = c / segs;
+                    const int b = row / H, y = row % H, x0 = seg * kWtPx;
+                    const uint32_t bar = smem_u32(&full[st]), sb = base + st * S::kStage;
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                                 :: "r"(bar), "r"(S::kTxBytes) : "memory");
+                    // word coordinates: pixel * 4 (a 16-byte multiple)
 #pragma unroll
-                // word coordinates: pixel * 4 (a 16-byte multiple)
-                for (int t = 0; t < 3; t++) {
-                    asm volatile(
-                        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
-                        " [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                        :: "r"(sb + (uint32_t)(t * S::KGI) * S::kBlock),
-                           "l"(reinterpret_cast<uint64_t>(&tmX)), "r"(4 * x0), "r"(0),
-                           "r"(y + t - 1), "r"(b), "r"(bar)
-                        : "memory");
-                    asm volatile(
-                        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
-                        " [%0], [%1, {%2, %3, %4, %5}], [%6];"
-                        :: "r"(sb + S::kBOff + (uint32_t)(t * S::KGO) * S::kBlock),
-                           "l"(reinterpret_cast<uint64_t>(&tmD)), "r"(4 * (x0 + 1 - t)), "r"(0),
-                           "r"(y), "r"(b), "r"(bar)
-                        : "memory");
+                    for (int t = 0; t < 3; t++) {
+                        asm volatile(
+                            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+                            " [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                            :: "r"(sb + (uint32_t)(t * S::KGI) * S::kBlock), "l"(mapX), "r"(4 * x0), "r"(0),
+                               "r"(y + t - 1), "r"(b), "r"(bar)
+                            : "memory");
+                        asm volatile(
+                            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+                            " [%0], [%1, {%2, %3, %4, %5}], [%6];"
+                            :: "r"(sb + S::kBOff + (uint32_t)(t * S::KGO) * S::kBlock), "l"(mapD),
+                               "r"(4 * (x0 + 1 - t)), "r"(0), "r"(y), "r"(b), "r"(bar)
+                            : "memory");
+                    }
                 }
             }
             // every box issued has landed before the CTA's shared memory is released
@@ -1253,72 +1286,81 @@ __global__ void __launch_bounds__(kWtThreads, 1) k_conv3x3_wgrad_tma(
             if (!ok) abortFlag = 1u;
         }
         __syncwarp();
-    } else if (warp == 1) {
+    } else if (warp == 9) {
         if (lane == 0) {
             // A and B MN-major (instruction descriptor bits 15 and 16)
             const uint32_t idesc = instr_desc_bf16<128, N>() | (1u << 15) | (1u << 16);
             uint32_t i = 0;
             bool ok = true;
-            for (int c = blockIdx.x; c < chunks && ok; c += gridDim.x, i++) {
-                const uint32_t st = i % kWtStages, use = i / kWtStages;
-                if (!(ok = tc_wait(smem_u32(&full[st]), use & 1u, &abortFlag))) break;
-                asm volatile("tcgen05.fence::after_thread_sync;");
-                const uint32_t aAddr = base + st * S::kStage, bAddr = aAddr + S::kBOff;
-#pragma unroll
-                for (int kk = 0; kk < kWtPx / 16; kk++) {
-                    // K-adjacent core matrices (8 pixels) 128 B apart, M- or N-adjacent
-                    // ones (8 channels) one block apart
-                    const uint64_t bDesc = smem_desc(bAddr + (uint32_t)kk * 256u, 128, S::kBlock);
-#pragma unroll
-                    for (int mb = 0; mb < MB; mb++) {
-                        const uint64_t aDesc = smem_desc(aAddr + (uint32_t)(mb * 16) * S::kBlock +
-                            (uint32_t)kk * 256u, 128, S::kBlock);
-                        tc_mma(tmem + (uint32_t)(mb * N), aDesc, bDesc, idesc,
-                            (i > 0 || kk > 0) ? 1u : 0u);
-                    }
+            for (int l = 0; l < layers && ok; l++) {
+                if (l > 0) {
+                    if (!(ok = tc_wait(smem_u32(&drained), (uint32_t)(l - 1) & 1u, &abortFlag))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;");
                 }
-                tc_commit(smem_u32(&empty[st]));
+                bool first = true;
+                for (int c = blockIdx.x; c < chunks; c += gridDim.x, i++) {
+                    const uint32_t st = i % kWtStages, use = i / kWtStages;
+                    if (!(ok = tc_wait(smem_u32(&full[st]), use & 1u, &abortFlag))) break;
+                    asm volatile("tcgen05.fence::after_thread_sync;");
+                    const uint32_t aAddr = base + st * S::kStage, bAddr = aAddr + S::kBOff;
+#pragma unroll
+                    for (int kk = 0; kk < kWtPx / 16; kk++) {
+                        // K-adjacent core matrices (8 pixels) 128 B apart, M- or N-adjacent
+                        // ones (8 channels) one block apart
+                        const uint64_t bDesc = smem_desc(bAddr + (uint32_t)kk * 256u, 128, S::kBlock);
+#pragma unroll
+                        for (int mb = 0; mb < MB; mb++) {
+                            const uint64_t aDesc = smem_desc(aAddr + (uint32_t)(mb * 16) * S::kBlock +
+                                (uint32_t)kk * 256u, 128, S::kBlock);
+                            tc_mma(tmem + (uint32_t)(mb * N), aDesc, bDesc, idesc,
+                                (!first || kk > 0) ? 1u : 0u);
+                        }
+                    }
+                    first = false;
+                    tc_commit(smem_u32(&empty[st]));
+                }
+                // every MMA issued has finished before the accumulators are read
+                // or freed (waited for even after an abort)
+                tc_commit(smem_u32(&done));
+                volatile uint32_t never = 0u;
+                if (!tc_wait(smem_u32(&done), (uint32_t)l & 1u, &never)) abortFlag = 1u;
             }
-            // every MMA issued has finished before the accumulators are read
-            // or freed (waited for even after an abort)
-            tc_commit(smem_u32(&done));
-            volatile uint32_t never = 0u;
-            if (!tc_wait(smem_u32(&done), 0u, &never)) abortFlag = 1u;
             if (!ok) abortFlag = 1u;
         }
         __syncwarp();
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;");
-    // ---- epilogue: warp w < 4 MB reads TMEM lanes 32 (w % 4) .. + 31 of M block w / 4:
-    // accumulator row R = (ty, ci), or MROWS for the bias; column n = (tx, co)
-    float *out = partial + (size_t)blockIdx.x * (9 * COUT * CIN + COUT);
-    if (blockIdx.x >= chunks) {
-        // no chunk: nothing accumulated (the launch sizes the grid to avoid this)
-        for (int k = tid; k < 9 * COUT * CIN + COUT; k += kWtThreads) out[k] = 0.0f;
-    } else if (!abortFlag && warp < 4 * MB) {
+    } else if (warp < 4 * MB) {
+        // ---- epilogue: warp w reads TMEM lanes 32 (w % 4) .. + 31 of M block w / 4:
+        // accumulator row R = (ty, ci), or MROWS for the bias; column n = (tx, co)
         const int mb = warp >> 2, quarter = warp & 3;
         const int R = mb * 128 + quarter * 32 + lane;
         const int ty = R / CIN, ci = R % CIN;
+        for (int l = 0; l < layers; l++) {
+            uint32_t ok = lane == 0 ? (uint32_t)tc_wait(smem_u32(&done), (uint32_t)l & 1u, &abortFlag) : 0u;
+            if (!__shfl_sync(0xFFFFFFFFu, ok, 0)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+            float *out = partial + ((size_t)l * gridDim.x + blockIdx.x) * (9 * COUT * CIN + COUT);
 #pragma unroll 1
-        for (int c0 = 0; c0 < N; c0 += 16) {
-            uint32_t v[16];
-            tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mb * N + c0), v);
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            if (R < MROWS) {
+            for (int c0 = 0; c0 < N; c0 += 16) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(mb * N + c0), v);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (R < MROWS) {
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int n = c0 + k, tx = n / COUT, co = n % COUT;
-                    out[((size_t)(3 * ty + tx) * COUT + co) * CIN + ci] = __uint_as_float(v[k]);
-                }
-            } else if (R == MROWS) {
+                    for (int k = 0; k < 16; k++) {
+                        const int n = c0 + k, tx = n / COUT, co = n % COUT;
+                        out[((size_t)(3 * ty + tx) * COUT + co) * CIN + ci] = __uint_as_float(v[k]);
+                    }
+                } else if (R == MROWS) {
 #pragma unroll
-                for (int k = 0; k < 16; k++) {
-                    const int n = c0 + k;
-                    if (n / COUT == 1) out[9 * COUT * CIN + n % COUT] = __uint_as_float(v[k]);
+                    for (int k = 0; k < 16; k++) {
+                        const int n = c0 + k;
+                        if (n / COUT == 1) out[9 * COUT * CIN + n % COUT] = __uint_as_float(v[k]);
+                    }
                 }
             }
+            asm volatile("tcgen05.fence::before_thread_sync;");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&drained));
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;");
@@ -1671,6 +1713,21 @@ int sm_count()
 using namespace gbsp;
 using namespace gbsp::dn;
 
+// Appends a layer's slices to a reduction; returns its blocks so far.
+static uint32_t add_reduce(ReduceJobs &jobs, uint32_t blocks, const float *partial, int cout, int cin,
+    float *dW, float *dBias)
+{
+    const int wCount = 9 * cout * cin, perSlice = wCount + cout;
+    jobs.l[jobs.count++] = {partial, dW, dBias, perSlice, wCount, blocks};
+    return blocks + (uint32_t)((perSlice + kReduceEntries - 1) / kReduceEntries);
+}
+
+static cudaError_t launch_reduce(cudaStream_t s, const ReduceJobs &jobs, uint32_t blocks)
+{
+    k_wgrad_reduce<<<blocks, kReduceGroups * kReduceEntries, 0, s>>>(jobs);
+    return cudaGetLastError();
+}
+
 template <int CIN, int COUT>
 static int launch_wgrad_tc(cudaStream_t s, const __nv_bfloat16 *in, const __nv_bfloat16 *d, int B,
     int H, int W, float *dW, float *dBias)
@@ -1687,47 +1744,81 @@ static int launch_wgrad_tc(cudaStream_t s, const __nv_bfloat16 *in, const __nv_b
     k_conv3x3_wgrad_tc<CIN, COUT><<<grid, 288, 0, s>>>(in, d, B, H, W, partial);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        k_wgrad_reduce<<<(perSlice + kReduceEntries - 1) / kReduceEntries,
-            kReduceGroups * kReduceEntries, 0, s>>>(partial, grid, perSlice,
-            9 * COUT * CIN, dW, dBias);
-        e = cudaGetLastError();
+        ReduceJobs jobs = {};
+        jobs.slices = grid;
+        e = launch_reduce(s, jobs, add_reduce(jobs, 0, partial, COUT, CIN, dW, dBias));
     }
     cudaFreeAsync(partial, s);
     if (e != cudaSuccess) return cuda_error(e, "weight gradient");
     return GBSP_OK;
 }
 
+// The layers of shape CIN x COUT among `layers`: one launch, partial sums of the
+// k-th of them at partial + k * grid * perSlice; the reduction jobs are added.
 template <int CIN, int COUT>
-static int launch_wgrad_tma(cudaStream_t s, const __nv_bfloat16 *in, const __nv_bfloat16 *d, int B,
-    int H, int W, float *dW, float *dBias)
+static int launch_wgrad_tma(cudaStream_t s, const gbsp_dn_weight_grad_layer *layers, uint32_t count, int B,
+    int H, int W, int grid, float *&partial, ReduceJobs &jobs, uint32_t &blocks)
 {
     using S = WtShape<CIN, COUT>;
-    const int chunks = ((W + kWtPx - 1) / kWtPx) * B * H;
-    int grid = sm_count();
-    if (grid > chunks) grid = chunks;
     const size_t smem = 1024 + (size_t)kWtStages * S::kStage;
     auto kern = k_conv3x3_wgrad_tma<CIN, COUT>;
-    static SmemLimit limit;
-    int rc = limit((const void *)kern, smem);
-    if (rc) return rc;
-    CUtensorMap mapX, mapD;
-    if ((rc = planar_words_tensor_map(&mapX, in, B, H, W, CIN, kWtPx)) ||
-        (rc = planar_words_tensor_map(&mapD, d, B, H, W, COUT, kWtPx)))
-        return rc;
-    const int perSlice = 9 * COUT * CIN + COUT;
-    float *partial = nullptr;
-    GBSP_CUDA_TRY(cudaMallocAsync((void **)&partial, sizeof(float) * (size_t)grid * perSlice, s));
-    kern<<<grid, kWtThreads, smem, s>>>(mapX, mapD, B, H, W, partial);
-    cudaError_t e = cudaGetLastError();
-    if (e == cudaSuccess) {
-        k_wgrad_reduce<<<(perSlice + kReduceEntries - 1) / kReduceEntries,
-            kReduceGroups * kReduceEntries, 0, s>>>(partial, grid, perSlice,
-            9 * COUT * CIN, dW, dBias);
-        e = cudaGetLastError();
+    WtMaps maps;
+    int n = 0, rc;
+    float *const first = partial;
+    for (uint32_t k = 0; k < count; k++) {
+        const gbsp_dn_weight_grad_layer &l = layers[k];
+        if (l.cin != CIN || l.cout != COUT) continue;
+        if ((rc = planar_words_tensor_map(&maps.x[n], l.in, B, H, W, CIN, kWtPx)) ||
+            (rc = planar_words_tensor_map(&maps.d[n], l.dOut, B, H, W, COUT, kWtPx)))
+            return rc;
+        blocks = add_reduce(jobs, blocks, partial, COUT, CIN, l.dW, l.dBias);
+        partial += (size_t)grid * (9 * COUT * CIN + COUT);
+        n++;
     }
-    cudaFreeAsync(partial, s);
-    if (e != cudaSuccess) return cuda_error(e, "TMA-fed weight gradient");
+    if (!n) return GBSP_OK;
+    static SmemLimit limit;
+    if ((rc = limit((const void *)kern, smem))) return rc;
+    kern<<<grid, kWtThreads, smem, s>>>(maps, n, B, H, W, first);
+    GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
+}
+
+static int wgrad_grid(int B, int H, int W)
+{
+    const int64_t chunks = (int64_t)((W + kWtPx - 1) / kWtPx) * B * H;
+    return (int)std::min<int64_t>(sm_count(), chunks);
+}
+
+static size_t wgrad_scratch_floats(const gbsp_dn_weight_grad_layer *layers, uint32_t count, int grid)
+{
+    size_t floats = 0;
+    for (uint32_t k = 0; k < count; k++)
+        floats += (size_t)grid * (9 * layers[k].cout * layers[k].cin + layers[k].cout);
+    return floats;
+}
+
+static int weight_grads(cudaStream_t s, const gbsp_dn_weight_grad_layer *layers, uint32_t count, int B, int H,
+    int W, float *scratch)
+{
+    const int grid = wgrad_grid(B, H, W);
+    float *own = nullptr;
+    if (!scratch) {
+        GBSP_CUDA_TRY(cudaMallocAsync((void **)&own, sizeof(float) * wgrad_scratch_floats(layers, count, grid), s));
+        scratch = own;
+    }
+    float *partial = scratch;
+    ReduceJobs jobs = {};
+    jobs.slices = grid;
+    uint32_t blocks = 0;
+    int rc = launch_wgrad_tma<16, 48>(s, layers, count, B, H, W, grid, partial, jobs, blocks);
+    if (!rc) rc = launch_wgrad_tma<48, 48>(s, layers, count, B, H, W, grid, partial, jobs, blocks);
+    if (!rc) rc = launch_wgrad_tma<48, 32>(s, layers, count, B, H, W, grid, partial, jobs, blocks);
+    if (!rc) {
+        const cudaError_t e = launch_reduce(s, jobs, blocks);
+        if (e != cudaSuccess) rc = cuda_error(e, "TMA-fed weight gradient");
+    }
+    if (own) cudaFreeAsync(own, s);
+    return rc;
 }
 
 extern "C" {
@@ -1902,20 +1993,34 @@ int gbsp_dn_conv3x3_weight_grad_tc(void *stream, const uint16_t *in, const uint1
     return set_error(GBSP_ERR_INVALID_ARGUMENT, "weight grad %u->%u not instantiated", cin, cout);
 }
 
+uint64_t gbsp_dn_weight_grads_scratch(const gbsp_dn_weight_grad_layer *layers, uint32_t count, uint32_t B,
+    uint32_t H, uint32_t W)
+{
+    return layers ? sizeof(float) * wgrad_scratch_floats(layers, count, wgrad_grid((int)B, (int)H, (int)W)) : 0;
+}
+
+int gbsp_dn_weight_grads_tcgen05(void *stream, const gbsp_dn_weight_grad_layer *layers, uint32_t count,
+    uint32_t B, uint32_t H, uint32_t W, float *scratch)
+{
+    if (!layers || !count || count > (uint32_t)kWgLayers || !B || !H || !W)
+        return set_error(GBSP_ERR_INVALID_ARGUMENT, "bad weight-gradient args");
+    for (uint32_t k = 0; k < count; k++) {
+        const gbsp_dn_weight_grad_layer &l = layers[k];
+        if (!l.in || !l.dOut || !l.dW || !l.dBias)
+            return set_error(GBSP_ERR_INVALID_ARGUMENT, "bad weight-gradient args");
+        if (((uintptr_t)l.in | (uintptr_t)l.dOut) & 15u)
+            return set_error(GBSP_ERR_INVALID_ARGUMENT, "weight-gradient tensors must be 16-byte aligned");
+        if (!((l.cin == 16 && l.cout == 48) || (l.cin == 48 && (l.cout == 48 || l.cout == 32))))
+            return set_error(GBSP_ERR_INVALID_ARGUMENT, "weight grad %u->%u not instantiated", l.cin, l.cout);
+    }
+    return weight_grads((cudaStream_t)stream, layers, count, (int)B, (int)H, (int)W, scratch);
+}
+
 int gbsp_dn_conv3x3_weight_grad_tcgen05(void *stream, const uint16_t *in, const uint16_t *dOut,
     uint32_t B, uint32_t H, uint32_t W, uint32_t cin, uint32_t cout, float *dW, float *dBias)
 {
-    cudaStream_t s = (cudaStream_t)stream;
-    if (!in || !dOut || !dW || !dBias || !B || !H || !W)
-        return set_error(GBSP_ERR_INVALID_ARGUMENT, "bad weight-gradient args");
-    if (((uintptr_t)in | (uintptr_t)dOut) & 15u)
-        return set_error(GBSP_ERR_INVALID_ARGUMENT, "weight-gradient tensors must be 16-byte aligned");
-    const __nv_bfloat16 *i16 = reinterpret_cast<const __nv_bfloat16 *>(in);
-    const __nv_bfloat16 *d16 = reinterpret_cast<const __nv_bfloat16 *>(dOut);
-    if (cin == 16 && cout == 48) return launch_wgrad_tma<16, 48>(s, i16, d16, B, H, W, dW, dBias);
-    if (cin == 48 && cout == 48) return launch_wgrad_tma<48, 48>(s, i16, d16, B, H, W, dW, dBias);
-    if (cin == 48 && cout == 32) return launch_wgrad_tma<48, 32>(s, i16, d16, B, H, W, dW, dBias);
-    return set_error(GBSP_ERR_INVALID_ARGUMENT, "weight grad %u->%u not instantiated", cin, cout);
+    const gbsp_dn_weight_grad_layer l = {in, dOut, dW, dBias, cin, cout};
+    return gbsp_dn_weight_grads_tcgen05(stream, &l, 1, B, H, W, nullptr);
 }
 
 int gbsp_dn_conv3x3_weight_grad(void *stream, const uint16_t *in, const uint16_t *dOut,

@@ -35,10 +35,21 @@ def _stream():
     return _vp(torch.cuda.current_stream().cuda_stream)
 
 
+# gbsp_dn_weight_grad_layer
+_WGRAD_LAYER = np.dtype([("in", "u8"), ("dOut", "u8"), ("dW", "u8"), ("dBias", "u8"), ("cin", "u4"),
+                         ("cout", "u4")])
+# output gradients kept for one weight-gradient call (a batch of 16 crops of 128 x 128 keeps 0.17 GB)
+WGRAD_KEEP = 4 << 30
+
+
 def _stream_handle() -> int:
     import torch
 
-    return torch.cuda.current_stream().cuda_stream
+    # the handle alone: a Stream object around it costs as much as a launch
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    if raw is None:
+        return torch.cuda.current_stream().cuda_stream
+    return raw(torch.cuda.current_device())
 
 
 def _ptr(t) -> _vp:
@@ -347,6 +358,26 @@ class KPCNN:
         _check(self._wgrad(_stream_handle(), x.data_ptr(), d.data_ptr(), B, H, W, cin, cout,
                            dw.data_ptr(), db.data_ptr()))
 
+    def weight_grads(self, todo, inputs, dws, dbs):
+        """weight_grad for several (layer, output gradient) pairs of one batch;
+        on the tcgen05 path a launch per layer shape and one reduction."""
+        import torch
+
+        if self.wgrad_impl != "tcgen05":
+            for li, d in todo:
+                self.weight_grad(li, inputs[li], d, dws[li], dbs[li])
+            return
+        rows = np.array([(inputs[li].data_ptr(), d.data_ptr(), dws[li].data_ptr(), dbs[li].data_ptr(),
+                          _dims(inputs[li])[3], _dims(d)[3]) for li, d in todo], _WGRAD_LAYER)
+        B, H, W, _ = _dims(todo[0][1])
+        # from the tensors' allocator: the driver's pool gives its memory back at
+        # every wait, and mapping 88 MB again costs more than the reduction
+        table = rows.ctypes.data
+        scratch = torch.empty(self.L.gbsp_dn_weight_grads_scratch(table, len(rows), B, H, W) // 4,
+                              dtype=torch.float32, device="cuda")
+        _check(self.L.gbsp_dn_weight_grads_tcgen05(_stream_handle(), table, len(rows), B, H, W,
+                                                   scratch.data_ptr()))
+
     def gradients(self, feats, noisy, target):
         """Loss and parameter gradients for one batch."""
         import torch
@@ -365,11 +396,18 @@ class KPCNN:
         dbs = list(flat[len(self.w):])
         last = len(LAYERS) - 1
         inputs = [feats] + acts
-        self.weight_grad(last, inputs[last], dlog, dws[last], dbs[last])
+        # weight gradients are taken together, in the order of the backward pass,
+        # at the latest when the kept output gradients reach WGRAD_KEEP bytes
+        todo, kept = [(last, dlog)], 0
         d = dlog
         for li in range(last - 1, -1, -1):
+            if kept + d.numel() * 2 > WGRAD_KEEP:
+                self.weight_grads(todo, inputs, dws, dbs)
+                todo, kept = [], 0
+            kept += d.numel() * 2
             d = self.data_grad_relu(li + 1, d, acts[li])
-            self.weight_grad(li, inputs[li], d, dws[li], dbs[li])
+            todo.append((li, d))
+        self.weight_grads(todo, inputs, dws, dbs)
         return loss, dws, dbs
 
     def train_step(self, feats, noisy, target, lr=1e-4):

@@ -59,6 +59,7 @@ EXPORTS = [
     "gbsp_dn_tile_fallback", "gbsp_scene_set_node_width", "gbsp_scene_node_width",
     "gbsp_batch_set_node_widths", "gbsp_batch_get_node_widths", "gbsp_path_trace_tile_list",
     "gbsp_dn_tile_check", "gbsp_dn_tile_merge", "gbsp_dn_conv3x3_weight_grad_tcgen05",
+    "gbsp_dn_weight_grads_tcgen05", "gbsp_dn_weight_grads_scratch",
     "gbsp_path_trace_tile_list_spp", "gbsp_path_trace_tile_split",
     "gbsp_dn_conv3x3_data_grad_relu_tc", "gbsp_dn_adam_all",
 ]
@@ -120,6 +121,8 @@ _ARGTYPES = {
     "gbsp_dn_conv3x3_forward_tc": [_vp, _vp, _u32, _u32, _u32, _u32, _vp, _vp, _u32, _i32, _vp, _vp],
     "gbsp_dn_conv3x3_forward": [_vp, _vp, _u32, _u32, _u32, _u32, _vp, _vp, _u32, _i32, _vp, _vp],
     "gbsp_dn_conv3x3_data_grad_relu_tc": [_vp, _vp, _u32, _u32, _u32, _u32, _vp, _u32, _vp, _vp],
+    "gbsp_dn_weight_grads_tcgen05": [_vp, _vp, _u32, _u32, _u32, _u32, _vp],
+    "gbsp_dn_weight_grads_scratch": [_vp, _u32, _u32, _u32, _u32],
     "gbsp_dn_conv3x3_weight_grad_tcgen05": [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp],
     "gbsp_dn_conv3x3_weight_grad_tc": [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp],
     "gbsp_dn_conv3x3_weight_grad": [_vp, _vp, _vp, _u32, _u32, _u32, _u32, _u32, _vp, _vp],
@@ -153,6 +156,7 @@ def load(build_if_missing: bool = True):
     lib.gbsp_frame_device_pointer.restype = _vp
     lib.gbsp_frame_aov_device_pointer.restype = _vp
     lib.gbsp_sample_seed.restype = _u32
+    lib.gbsp_dn_weight_grads_scratch.restype = _u64
     lib.gbsp_calculate_film_positions.restype = _u32
     lib.gbsp_xorshift32_jump.restype = _u32
     lib.gbsp_xorshift32_jump.argtypes = [_u32, ctypes.c_uint64]
