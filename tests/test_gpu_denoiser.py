@@ -652,3 +652,31 @@ def test_kept_output_gradients_are_bounded(gpu_lib, monkeypatch):
     torch.cuda.synchronize()
     for other in out[1:]:
         assert all(torch.equal(a, b) for a, b in zip(out[0], other))
+
+
+def test_chained_layers_capture_into_a_graph(gpu_lib):
+    # the layers start while their predecessors drain; captured behind a memset
+    # and a kernel of another library, and replayed, they give the same image
+    import torch
+
+    from vk_cinematic_gb300 import denoiser
+
+    torch.manual_seed(4)
+    net = denoiser.KPCNN(seed=5)
+    rad = torch.rand((1, 70, 150, 4), device="cuda")
+    aov = torch.rand((1, 70, 150, 8), device="cuda")
+    ref = net.denoise(rad, aov)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        net.denoise(rad, aov)
+        stream.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            other = torch.zeros_like(rad)
+            out = net.denoise(rad + other, aov)
+        for _ in range(3):
+            out.zero_()
+            graph.replay()
+            stream.synchronize()
+            assert torch.equal(out, ref)

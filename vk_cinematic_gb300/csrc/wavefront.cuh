@@ -5,6 +5,7 @@
 #pragma once
 
 #include "gbsp_internal.h"
+#include "launch.cuh"
 #include "traverse.cuh"
 #include "shading.cuh"
 
@@ -29,37 +30,6 @@ __device__ __forceinline__ void reset_wave_ctl(unsigned int *ctl, uint32_t paths
     ctl[kCtlTraceWork] = 0;
     ctl[queue_word(0)] = paths;
     ctl[queue_word(1)] = ctl[queue_word(2)] = 0;
-}
-
-// Kernels of a wave follow one another through memory.  Launched with
-// launch_next, a kernel may become resident while the one before it drains;
-// stage_begin, its first statement, holds it until that one has completed and
-// its writes are visible, and only then lets the next one in.  The chain is
-// transitive: a kernel completes after its predecessor did.  What one of them
-// writes, the next reads by plain loads: no __ldg and no const __restrict__,
-// which promise data that is constant for the whole life of a kernel.
-// 128 x 128 x 8 frame 227 -> 214 us, 641 x 359 x 7 watertight 929 -> 899 us, a
-// 128 x 128 x 4 crop 248 -> 232 us; long kernels are the same either way.
-__device__ __forceinline__ void stage_begin()
-{
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
-
-// For kernels that start with stage_begin only.
-template <class... P, class... A>
-void launch_next(void (*kernel)(P...), int grid, int block, cudaStream_t s, A... args)
-{
-    cudaLaunchAttribute attr = {};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.stream = s;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, P(args)...);  // the caller reads cudaGetLastError
 }
 
 struct WaveBuffers {
