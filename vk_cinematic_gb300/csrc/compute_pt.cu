@@ -29,9 +29,13 @@
 // longest tile has 768 rays).  A ray among 18 spheres of 1,280 triangles costs
 // 1,440 cluster tests and the tests of about 55 listed clusters instead of
 // 23,042 triangle tests.  512 x 384 pixels of that scene: 107.5 ms with a warp
-// per tile and every triangle staged through shared memory, 5.9 ms now.
-// 4 blocks of 8 warps per SM (64 registers) 5.9 ms, unbounded (2 blocks) 7.4,
-// 4 warps 6.6 and 2 warps per tile 9.8 ms.
+// per tile and every triangle staged through shared memory, 5.45 ms now (5.88
+// before the cluster test's sums were fused multiply-adds and the winner a
+// minimum reduction).  Before those two: 4 blocks of 8 warps per SM (64
+// registers) 5.88 ms, unbounded (2 blocks) 7.4, 4 warps 6.6 and 2 warps per
+// tile 9.8 ms.  Worse since: clusters of 8 or 32 triangles 6.4 and 7.7 ms, one
+// list for all warps of a tile (a barrier more) 6.1, the next clusters loaded
+// ahead (registers) 7.0, 5 blocks per SM 5.7.
 //
 // Built-ins are fixed to one IEEE definition shared with the oracle (dot in
 // x, y, z order; normalize = v * (1 / sqrt(dot)); mat4 * vec4 summed over
@@ -383,17 +387,10 @@ __global__ void __launch_bounds__(32 * kWarps, kWarps == 8 ? 4 : 1) k_compute_pt
                     normal = cnormalize(mat_mul(ent.model, localNormal, 0.0f));
                     cand = t >= 0.0f && t < res.t;
                 }
-                float best = cand ? t : kF32Max;
-                int who = cand ? lane : 32;
-#pragma unroll
-                for (int off = 16; off; off >>= 1) {
-                    const float ot = __shfl_xor_sync(0xFFFFFFFFu, best, off);
-                    const int ow = __shfl_xor_sync(0xFFFFFFFFu, who, off);
-                    if (ow < 32 && (who == 32 || ot < best || (ot == best && ow < who))) {
-                        best = ot;
-                        who = ow;
-                    }
-                }
+                // t >= 0 orders as its bits (+ 0 makes a zero positive)
+                const uint32_t key = cand ? __float_as_uint(t + 0.0f) : 0xFFFFFFFFu;
+                const uint32_t best = __reduce_min_sync(0xFFFFFFFFu, key);
+                const int who = best == 0xFFFFFFFFu ? 32 : __ffs(__ballot_sync(0xFFFFFFFFu, key == best)) - 1;
                 if (who < 32) {
                     res.t = __shfl_sync(0xFFFFFFFFu, t, who);
                     res.normal.x = __shfl_sync(0xFFFFFFFFu, normal.x, who);

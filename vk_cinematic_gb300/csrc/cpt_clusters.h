@@ -76,6 +76,10 @@ GBSP_HD MtHit mt_test(V3 lo, V3 ld, V3 a, V3 e1, V3 e2, float tMax)
     return r;
 }
 
+// Products added without a rounding in between: for the bounds below, not for
+// the shader's own arithmetic.
+GBSP_HD float fdot(V3 a, V3 b) { return fmaf(a.z, b.z, fmaf(a.y, b.y, a.x * b.x)); }
+
 GBSP_HD float inverse_sqrt(float x)
 {
 #ifdef __CUDA_ARCH__
@@ -90,16 +94,17 @@ GBSP_HD float inverse_sqrt(float x)
 GBSP_HD bool cluster_may_hit(float4 sphere, float4 cone, float4 edge, V3 lo, V3 ld)
 {
     const V3 w = v3(sphere.x - lo.x, sphere.y - lo.y, sphere.z - lo.z);
-    const float s = cdot(w, ld);
-    const V3 q = v3(w.x - ld.x * s, w.y - ld.y * s, w.z - ld.z * s);  // from the line to the centre
-    const float q2 = cdot(q, q), iq = inverse_sqrt(q2), ql = q2 * iq;
+    const float s = fdot(w, ld);
+    // from the line to the centre
+    const V3 q = v3(fmaf(-ld.x, s, w.x), fmaf(-ld.y, s, w.y), fmaf(-ld.z, s, w.z));
+    const float q2 = fdot(q, q), iq = inverse_sqrt(q2), ql = q2 * iq;
     // >= |T| + L: |w| is at most |s| + |q|
-    const float far = (fabsf(s) + ql) * 1.0001f + (sphere.w + edge.z);
-    const float c = cdot(ld, v3(cone.x, cone.y, cone.z));
-    const float e = cdot(q, v3(cone.x, cone.y, cone.z)) * iq;
-    const float reach = cone.w + (edge.x + edge.y * far) * iq;  // sin y + x
-    const bool outside = ql > sphere.w + 1.01e-3f * far;
-    const bool away = c * c + e * e > reach * reach * 1.0001f + 1e-5f;
+    const float far = fmaf(fabsf(s) + ql, 1.0001f, sphere.w + edge.z);
+    const float c = fdot(ld, v3(cone.x, cone.y, cone.z));
+    const float e = fdot(q, v3(cone.x, cone.y, cone.z)) * iq;
+    const float reach = fmaf(fmaf(edge.y, far, edge.x), iq, cone.w);  // sin y + x
+    const bool outside = ql > fmaf(1.01e-3f, far, sphere.w);
+    const bool away = fmaf(c, c, e * e) > fmaf(reach * reach, 1.0001f, 1e-5f);
     return !(outside && away);
 }
 
