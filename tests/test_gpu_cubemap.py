@@ -80,6 +80,18 @@ def test_irradiance_random_stream_is_the_references(gpu_lib):
     assert np.abs(got - ref).max() <= 1e-6
 
 
+@pytest.mark.parametrize("width,height,spp", [(5, 3, 1), (7, 2, 31), (6, 6, 33), (9, 4, 65), (33, 1, 64)])
+def test_irradiance_random_splits_the_stream(gpu_lib, hdri, width, height, spp):
+    # a warp per texel, a run of samples per lane: one sample, a lane short, a run
+    # of two with idle lanes, a ragged last run, full runs
+    import torch
+
+    got = gbsp.create_irradiance_cube_map(torch.from_numpy(hdri).cuda(), width, height, spp,
+                                          gbsp.IRRADIANCE_RANDOM).cpu().numpy()
+    ref = pyoracle.create_irradiance_cube_map(hdri, width, height, spp, gbsp.IRRADIANCE_RANDOM)
+    assert rel_err(got, ref).mean() <= 1e-4
+
+
 def test_rejects_bad_arguments(gpu_lib):
     import torch
 

@@ -15,11 +15,13 @@
 //
 // Random mode: the reference draws 3 numbers per sample from ONE XorShift32
 // stream for the whole cube (face, row, column, sample order).  Every texel
-// draws exactly 3 * samplesPerPixel numbers, so texel i starts at state
-// J^i * s0 with J = M^(3 * samplesPerPixel), M the 32 x 32 GF(2) matrix of one
-// XorShift32 step; the host tabulates J^(2^k) and each thread jumps to its
-// texel's state with at most 32 GF(2) matrix-vector products, then runs its
-// samples sequentially.
+// draws exactly 3 * samplesPerPixel numbers, so sample k of texel i starts at
+// state M^(3 (i samplesPerPixel + k)) * s0, M the 32 x 32 GF(2) matrix of one
+// XorShift32 step.  One warp integrates one texel: it jumps to the texel's
+// state with the matrices J^(2^b), J = M^(3 samplesPerPixel), of the set bits b
+// of i (lane c holds column c, one xor reduction per product), and lane l to
+// its run of samples with a matrix of its own.  The host makes both tables and
+// passes them with the launch.
 //
 // Transcendentals are CUDA's sinf/cosf/atan2f (their last bits differ from
 // glibc's), so results match the reference to within those differences;
@@ -194,34 +196,42 @@ __global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_uniform(Image im,
     }
 }
 
-struct JumpTable {
-    uint32_t col[32][32];  // col[k][c]: column c of J^(2^k)
+struct JumpTables {
+    uint32_t texel[32][32];  // texel[b][c]: column c of J^(2^b)
+    uint32_t lane[32][32];   // lane[l][c]: column c of M^(3 run l), lane l's first sample
 };
 
-__device__ __forceinline__ uint32_t gf2_apply(const uint32_t *cols, uint32_t s)
+// Bound: latency of the samples' dependent chains (random numbers, direction,
+// lookup).  A thread per texel walked all of its samples one after another,
+// with at most 24,576 threads for a 6 x 64^2 map, and the call waited for its
+// table's upload.  6 x 8^2 texels of 128 samples 394 -> 47 us for the call, 6 x
+// 64^2 of 8 300 -> 96, of 128 401 -> 122; the host's tables take 25 us of it.
+__global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_random(Image im, uint32_t width,
+    uint32_t height, uint32_t spp, uint32_t run, const __grid_constant__ JumpTables jumps, uint32_t seed,
+    float4 *__restrict__ out)
 {
-    uint32_t r = 0;
-#pragma unroll
-    for (int c = 0; c < 32; c++) r ^= (s >> c & 1u) ? cols[c] : 0u;
-    return r;
-}
-
-__global__ void k_irradiance_random(Image im, uint32_t width, uint32_t height, uint32_t spp,
-    const JumpTable *__restrict__ jumps, uint32_t seed, float4 *__restrict__ out)
-{
-    uint64_t total = 6ull * width * height;
-    float contribution = 1.0f / (float)spp;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < total;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t x = (uint32_t)(i % width);
-        uint32_t y = (uint32_t)((i / width) % height);
-        uint32_t layer = (uint32_t)(i / ((uint64_t)width * height));
-        uint32_t rng = seed;
-        for (int k = 0; k < 32 && (i >> k); k++)
-            if ((i >> k) & 1u) rng = gf2_apply(jumps->col[k], rng);
+    __shared__ uint32_t texelCols[32][32], laneCols[32][33];  // laneCols[c][l]
+    for (uint32_t k = threadIdx.x; k < 1024; k += blockDim.x) {
+        texelCols[k >> 5][k & 31] = jumps.texel[k >> 5][k & 31];
+        laneCols[k & 31][k >> 5] = jumps.lane[k >> 5][k & 31];
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t total = 6u * width * height;  // checked to fit
+    const uint32_t warps = gridDim.x * kIrrWarps;
+    const float contribution = 1.0f / (float)spp;
+    // 64 bits: run * lane may pass 2^32
+    const uint64_t first = (uint64_t)run * lane, last = min((uint64_t)spp, first + run);
+    for (uint64_t i64 = blockIdx.x * kIrrWarps + (threadIdx.x >> 5); i64 < total; i64 += warps) {
+        const uint32_t i = (uint32_t)i64, x = i % width, y = i / width % height, layer = i / width / height;
+        uint32_t state = seed;
+        for (uint32_t bits = i; bits; bits &= bits - 1)
+            state = __reduce_xor_sync(0xFFFFFFFFu, state >> lane & 1u ? texelCols[__ffs(bits) - 1][lane] : 0u);
+        uint32_t rng = 0;
+        for (uint32_t bits = state; bits; bits &= bits - 1) rng ^= laneCols[__ffs(bits) - 1][lane];
         V3 dir = face_direction(face_basis(layer), x, y, width, height);
         V3 irr = v3(0.0f, 0.0f, 0.0f);
-        for (uint32_t k = 0; k < spp; k++) {
+        for (uint64_t k = first; k < last; k++) {
             // Vec3(RandomBilateral() x3) with GCC's right-to-left argument order
             float oz = random_bilateral(rng);
             float oy = random_bilateral(rng);
@@ -236,7 +246,13 @@ __global__ void k_irradiance_random(Image im, uint32_t width, uint32_t height, u
                 rclamp(s.y * cosine, 0.0f, kRadianceClamp), rclamp(s.z * cosine, 0.0f, kRadianceClamp));
             irr = add(irr, mul(rad, contribution));
         }
-        out[i] = make_float4(irr.x, irr.y, irr.z, 1.0f);
+#pragma unroll
+        for (int off = 16; off; off >>= 1) {
+            irr.x += __shfl_xor_sync(0xFFFFFFFFu, irr.x, off);
+            irr.y += __shfl_xor_sync(0xFFFFFFFFu, irr.y, off);
+            irr.z += __shfl_xor_sync(0xFFFFFFFFu, irr.z, off);
+        }
+        if (lane == 0) out[i] = make_float4(irr.x, irr.y, irr.z, 1.0f);
     }
 }
 
@@ -246,8 +262,7 @@ using Mat = std::vector<uint32_t>;  // 32 columns
 static uint32_t apply(const Mat &m, uint32_t s)
 {
     uint32_t r = 0;
-    for (int c = 0; c < 32; c++)
-        if (s >> c & 1u) r ^= m[c];
+    for (; s; s &= s - 1) r ^= m[__builtin_ctz(s)];
     return r;
 }
 
@@ -354,24 +369,26 @@ int gbsp_create_irradiance_cube_map(void *stream, const float *equirect, uint32_
         GBSP_CUDA_TRY(cudaGetLastError());
         return GBSP_OK;
     }
-    // random mode: jump table J^(2^k), J = M^(3 spp); host copy waits for the upload
-    cube::JumpTable table;
+    // random mode: lane l of a texel's warp takes samples run l, run l + 1, ...
+    const uint32_t run = (uint32_t)(((uint64_t)samplesPerPixel + 31) / 32);
+    cube::JumpTables jumps = {};
+    const auto copy = [](uint32_t *dst, const cube::Mat &m) { std::copy(m.begin(), m.end(), dst); };
     cube::Mat j = cube::power(cube::step_matrix(), 3ull * samplesPerPixel);
-    for (int k = 0; k < 32; k++) {
-        for (int c = 0; c < 32; c++) table.col[k][c] = j[c];
+    for (int b = 0; b < 32 && total >> b; b++) {
+        copy(jumps.texel[b], j);
         j = cube::multiply(j, j);
     }
-    cube::JumpTable *dTable = nullptr;
-    GBSP_CUDA_TRY(cudaMallocAsync((void **)&dTable, sizeof(table), s));
-    cudaError_t e = cudaMemcpyAsync(dTable, &table, sizeof(table), cudaMemcpyHostToDevice, s);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // `table` lives on this stack frame
-    if (e == cudaSuccess) {
-        cube::k_irradiance_random<<<grid_for(total, 128), 128, 0, s>>>(im, width, height,
-            samplesPerPixel, dTable, 0x45BA12F3u, reinterpret_cast<float4 *>(faces));
-        e = cudaGetLastError();
+    const cube::Mat step = cube::power(cube::step_matrix(), 3ull * run);
+    j = cube::power(step, 0);
+    for (uint64_t l = 0; l < 32 && l * run < samplesPerPixel; l++) {
+        copy(jumps.lane[l], j);
+        j = cube::multiply(j, step);
     }
-    cudaFreeAsync(dTable, s);
-    if (e != cudaSuccess) return cuda_error(e, "irradiance (random)");
+    const uint64_t blocks = (total + cube::kIrrWarps - 1) / cube::kIrrWarps;
+    const int block = 32 * cube::kIrrWarps;
+    cube::k_irradiance_random<<<grid_for(blocks * block, block), block, 0, s>>>(im, width, height,
+        samplesPerPixel, run, jumps, 0x45BA12F3u, reinterpret_cast<float4 *>(faces));
+    GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
 }
 
