@@ -859,6 +859,33 @@ static int planar_words_tensor_map(CUtensorMap *map, const void *in, int B, int 
     return GBSP_OK;
 }
 
+// Rows per strip for `cols` columns of H rows on `ctas` CTAs: strips go
+// round-robin, so a launch takes as long as the CTA with the most rows, `rounds`
+// strips of `rows` and about one row's time per strip for its halo.  Eight
+// layers at 1080p (15 columns): strips of 20 rows, "about six per CTA", which
+// left the last of six rounds a third full, 626 us; 12, 16, 28, 36 and 56 rows
+// 583, 591, 591, 571 and 580; 108, one strip for each of 150 CTAs, 555.
+inline int strip_rows(int cols, int H, int ctas)
+{
+    const auto whole = [](int64_t rows) {
+        return (int)((rows + kTcGroupRows - 1) / kTcGroupRows * kTcGroupRows);  // whole row groups
+    };
+    const int first = (cols + ctas - 1) / ctas;
+    int best = whole(H);
+    int64_t bestCost = (int64_t)first * (best + 1);
+    for (int r = first; r < first + 8; r++) {
+        const int64_t perCol = (int64_t)r * ctas / cols;  // strips a column may have in r rounds
+        const int rows = whole((H + perCol - 1) / perCol);
+        const int64_t strips = (int64_t)cols * ((H + rows - 1) / rows);
+        const int64_t cost = (strips + ctas - 1) / ctas * (rows + 1);
+        if (cost < bestCost) {
+            bestCost = cost;
+            best = rows;
+        }
+    }
+    return best;
+}
+
 template <int CIN, int COUT, int EPI>
 int launch_conv_tc(cudaStream_t s, int smCount, const void *in, int B, int H, int W, const void *w,
     const float *bias, void *outB, float *outF, const float4 *noisy = nullptr,
@@ -872,12 +899,8 @@ int launch_conv_tc(cudaStream_t s, int smCount, const void *in, int B, int H, in
     if (int rc = limit((const void *)kern, smem)) return rc;
     const int ctas = smCount;  // one CTA per SM (the row ring takes most of shared memory)
     const int cols = B * ((W + kTcTileP - 1) / kTcTileP);
-    // rows per strip: about six strips per CTA (strips go round-robin, so
-    // the last round is nearly full), at least 4 rows
-    int rows = (int)(((int64_t)cols * H + 6 * ctas - 1) / (6 * ctas));
-    rows = rows < 4 ? 4 : (rows > H ? H : rows);
-    rows = (rows + kTcGroupRows - 1) / kTcGroupRows * kTcGroupRows;  // whole row groups
-    int strips = cols * ((H + rows - 1) / rows);
+    const int rows = strip_rows(cols, H, ctas);
+    const int strips = cols * ((H + rows - 1) / rows);
     int grid = strips < ctas ? strips : ctas;
     // consecutive convolutions walk the strips in opposite orders, so a layer
     // starts on the rows its predecessor wrote last (still in L2)
