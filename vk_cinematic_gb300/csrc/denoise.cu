@@ -420,7 +420,7 @@ __device__ __forceinline__ void conv_filter_store(const uint32_t (&r)[COUT], siz
 
 template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat16 *__restrict__ in,
-    int B, int H, int W, int rowsPerStrip, int reverseStrips, const __nv_bfloat16 *__restrict__ w,
+    int B, int H, int W, int rowsPerStrip, int reverse, const __nv_bfloat16 *__restrict__ w,
     const float *__restrict__ bias, __nv_bfloat16 *__restrict__ outB, float *__restrict__ outF,
     const float4 *__restrict__ noisy, float4 *__restrict__ outFilt, const __nv_bfloat16 *__restrict__ act)
 {
@@ -506,7 +506,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
     // strip geometry: segment origin x0, output rows [y0, y1) in P groups of G rows
     // (the last group may reach past the image); staged input rows y0 - 1 .. y0 + G P
 #define GBSP_STRIP_GEOMETRY(strip)                                                       \
-    const int st = reverseStrips ? numStrips - 1 - (strip) : (strip);                     \
+    const int st = reverse ? numStrips - 1 - (strip) : (strip);                     \
     const int sy = st % stripsPerCol, seg = (st / stripsPerCol) % segs;                  \
     const int b = st / (stripsPerCol * segs);                                             \
     const int x0 = seg * kTcTileP, y0 = sy * rowsPerStrip;                                \
@@ -548,6 +548,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
                 ok = wait_pair(pos);
                 for (int p = 0; p < P && ok; p++) {
                     // input rows y - 1 .. y + G: the pairs in slots pos, pos + 1 and pos + 2
+                    // (from the bottom up when reversed)
                     const uint32_t slot1 = next_slot(pos), slot2 = next_slot(slot1);
                     ok = wait_pair(slot1);
                     ok = ok && wait_pair(slot2);
@@ -562,9 +563,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
                     const uint32_t dAcc = tmem + acc * (uint32_t)ACC_COLS;
                     // A descriptors of the three pairs: only the low word's address field differs
                     const uint32_t aHi = (uint32_t)(aDesc0 >> 32);
-                    const uint32_t aLo[3] = {(uint32_t)aDesc0 + pos * (kSlotBytes / 16),
+                    const uint32_t top = reverse ? slot2 : pos, bottom = reverse ? pos : slot2;
+                    const uint32_t aLo[3] = {(uint32_t)aDesc0 + top * (kSlotBytes / 16),
                         (uint32_t)aDesc0 + slot1 * (kSlotBytes / 16),
-                        (uint32_t)aDesc0 + slot2 * (kSlotBytes / 16)};
+                        (uint32_t)aDesc0 + bottom * (kSlotBytes / 16)};
 #pragma unroll
                     for (int tx = 0; tx < 3; tx++) {
 #pragma unroll
@@ -586,7 +588,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
                         }
                     }
                     tc_commit(smem_u32(&accFull[acc]));
-                    // input rows y - 1 .. y + G - 2 have no later reader
+                    // the group's first two pairs have no later reader
                     tc_commit(smem_u32(&rowEmpty[pos]));
                     tc_commit(smem_u32(&rowEmpty[slot1]));
                     pos = slot2;
@@ -621,7 +623,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
                 // pixels [first, last) of the 130 lie inside the image
                 const int first = x0 == 0 ? 1 : 0;
                 const int last = min(kTcSpx, W - x0 + 1);
-                for (int gy = y0 - 1; gy <= y0 + G * P; gy += 2, q++) {
+                for (int k = 0; k <= G / 2 * P; k++, q++) {
+                    const int gy = y0 - 1 + 2 * (reverse ? G / 2 * P - k : k);
                     if (use > 0)
                         ok = tc_wait(smem_u32(&rowEmpty[slot]), (use - 1u) & 1u, &abortFlag);
                     if (!__all_sync(0xFFFFFFFFu, ok)) {
@@ -702,7 +705,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
                 const int x = x0 + quarter * 32 + lane;
 #pragma unroll 1
                 for (int j = 0; j < G; j++) {
-                    const int y = y0 + G * p + j;
+                    const int y = y0 + G * (reverse ? P - 1 - p : p) + j;
                     // the ReLU mask is asked for before the accumulators
                     uint4 mask[COUT / 8] = {};
                     if (EPI == kEpiReluGrad && x < W && y < y1) {
@@ -902,8 +905,9 @@ int launch_conv_tc(cudaStream_t s, int smCount, const void *in, int B, int H, in
     const int rows = strip_rows(cols, H, ctas);
     const int strips = cols * ((H + rows - 1) / rows);
     int grid = strips < ctas ? strips : ctas;
-    // consecutive convolutions walk the strips in opposite orders, so a layer
-    // starts on the rows its predecessor wrote last (still in L2)
+    // consecutive convolutions walk the strips, and the rows of a strip, in
+    // opposite orders, so a layer starts on the rows its predecessor wrote last
+    // (still in L2): eight layers at 1080p 548 us, with the strips alone 555
     const int reverse = (int)(g_convLaunches.fetch_add(1, std::memory_order_relaxed) & 1u);
     launch_next_smem(kern, grid, kTcThreads, smem, s, reinterpret_cast<const __nv_bfloat16 *>(in), B, H, W, rows,
         reverse, reinterpret_cast<const __nv_bfloat16 *>(w), bias, reinterpret_cast<__nv_bfloat16 *>(outB),
