@@ -384,8 +384,9 @@ int gbsp_batch_destroy(gbsp_batch *batch);
 int gbsp_batch_set_config(gbsp_batch *batch, const gbsp_batch_config *config);
 int gbsp_batch_get_config(const gbsp_batch *batch, gbsp_batch_config *config);
 /* First picks each item's BVH node width (8 or 4): the item's frame is
- * timed alone at both widths (spp capped at 8) and the faster is kept; then
- * times every candidate configuration (36: thread-per-pixel block x chunk x
+ * timed alone at both widths (spp capped at 8) and the faster is kept, unless
+ * the batch is faster with 8 for all (items of one width share kernels made
+ * for it); then times every candidate configuration (36: thread-per-pixel block x chunk x
  * blocks per SM, path-state block x blocks per SM, wavefront blocks per SM x
  * wave size 2^22..2^25) over `trials` launches each and keeps the fastest;
  * *best receives it.  Items start at their scene's gbsp_scene_set_node_width. */
