@@ -309,7 +309,7 @@ int gbsp_path_trace_tile_list_spp(const gbsp_context *ctx, const gbsp_tile *tile
  * deviceImage (device memory, imagePlane->width * imagePlane->height
  * RGBA32F, 16-byte aligned; only the tile is written).  The working memory is
  * one fixed array inside libgbsp that every GPU loading the library holds
- * until exit (about 5.8 MB): at most 16384 paths in flight, 8 bounces and
+ * until exit (about 5.3 MB): at most 16384 paths in flight, 8 bounces and
  * 4096 objects; larger requests fail with GBSP_ERR_CAPACITY.  The scene's
  * broadphase must be built and the material system uploaded by an earlier
  * render (else GBSP_ERR_NOT_READY).  The first call on a device looks up the

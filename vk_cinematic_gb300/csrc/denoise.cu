@@ -219,9 +219,9 @@ int launch_conv(cudaStream_t s, int smCount, const void *in, int B, int H, int W
 // Every wait is bounded; a timeout raises a shared abort flag that ends the
 // other roles' waits, and sets g_dnStatus.
 //
-// What bounds it (48 -> 48 at 1080p, 85.9 GFLOP, 398 MB in and out): memory, 79
-// us = 5.0 TB/s, with the MMAs behind it (54 of about 70 cycles per row group,
-// 49 us).  Before, 99 us: the issuing thread waited on six row barriers per
+// What bounds it (48 -> 48 at 1080p, 85.9 GFLOP, 398 MB in and out): memory, 69
+// us by itself = 5.8 TB/s (79 before strip_rows), with the MMAs behind it (54 of
+// about 70 cycles per row group, 49 us).  Before, 99 us: the issuing thread waited on six row barriers per
 // group at about 340 cycles each, none of it hidden (without loads, stores and
 // eight ninths of the MMAs 47 us; with one wait per group 29); and TMA boxes of
 // [group][130 pixels][8 channels] move 16 bytes per request (loads alone 60
@@ -235,8 +235,9 @@ constexpr int kTcEpiGroups = 2;
 constexpr int kTcAccSlots = 4;  // at most; accumulator a is drained by epilogue group a % 2
 constexpr int kTcSpx = kTcTileP + 2;     // staged pixels per row: x0 - 1 .. x0 + 128
 constexpr int kTcGroupRows = 4;  // output rows per accumulator
-// Input rows travel in pairs: one full and one empty barrier per two rows.  A row group reads three pairs, two of them new, so its issuing
-// thread waits twice for rows and releases two slots.
+// Input rows travel in pairs: one full and one empty barrier per two rows.  A row
+// group reads three pairs, two of them new, so its issuing thread waits twice for
+// rows and releases two slots.
 constexpr int kTcRing = 7;  // row pairs in shared memory: 3 read by a group's MMAs, the rest in flight
 constexpr uint32_t kTcWaitLimit = 1u << 26;
 
@@ -388,7 +389,9 @@ __device__ __forceinline__ void conv_store(const uint32_t (&r)[COUT], size_t row
 // clamped columns and rows are computed once each (25 clamped tap indices had
 // cost more than the filter: 160 -> 117 us at 1080p).  Loading the 25 taps
 // ahead of the accumulators spills and was slower (129 us), as were twice the
-// epilogue warps (129 us).
+// epilogue warps (129 us).  All of the filter's arithmetic and loads now cost 22
+// of a whole inference's 548 us; four rows of a group sharing their taps 562
+// (168 registers, spills), two rows 548.
 template <int COUT>
 __device__ __forceinline__ void conv_filter_store(const uint32_t (&r)[COUT], size_t p, int x, int y,
     int W, int H, const float *__restrict__ bias, const float4 *__restrict__ noisy,
@@ -435,7 +438,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
     constexpr int TMEM_COLS = 512;
     extern __shared__ __align__(128) unsigned char smemRaw[];
     uint4 *sW = reinterpret_cast<uint4 *>(smemRaw);  // [3][KG][3 COUT]
-    // ring slots of [2 rows][KG][kTcSpx] 16-byte pixels, each slot 128-byte aligned for TMA
+    // ring slots of [2 rows][KG][kTcSpx] 16-byte pixels, each slot 128-byte aligned
     constexpr uint32_t kRowUnits = (uint32_t)(KG * kTcSpx);  // 16-byte units
     constexpr uint32_t kSlotBytes = (2 * kRowUnits * 16 + 127) / 128 * 128;
     const uint32_t ringAddr = (smem_u32(sW + 9 * KG * COUT) + 127u) & ~127u;
