@@ -697,6 +697,19 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
             for (int p = 0; p < P; p++, groupCount++) {
                 if ((int)(groupCount % kTcEpiGroups) != group) continue;
                 const uint32_t acc = groupCount % SLOTS, use = groupCount / SLOTS;
+                if (EPI == kEpiReluGrad) {
+                    // the group's mask rows are on their way from memory while its MMAs run: G
+                    // rows of COUT / 8 planes, four 128-byte lines of eight pixels each (a
+                    // training step of 16 crops of 128 x 128 489 -> 469 us; one or two groups
+                    // further ahead they hold up the input rows, 481)
+                    const int yg = y0 + G * (reverse ? P - 1 - p : p);
+                    for (int i = lane; i < G * (COUT / 8) * 4; i += 32) {
+                        const int y = yg + i / (COUT / 2), px = x0 + quarter * 32 + 8 * (i & 3);
+                        if (y < y1 && px < W)
+                            asm volatile("prefetch.global.L2 [%0];"
+                                         :: "l"(act + cg_index((size_t)(b * H + y), px, 8 * (i / 4 % (COUT / 8)), W, COUT)));
+                    }
+                }
                 ok = tc_wait(smem_u32(&accFull[acc]), use & 1u, &abortFlag);
                 __syncwarp();
                 if (!__all_sync(0xFFFFFFFFu, ok)) {
