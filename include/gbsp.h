@@ -609,6 +609,12 @@ int gbsp_dn_filter(void *stream, const float *logits, const float *noisy, uint32
  * to the logits (BF16, 32 channels); adds the unnormalised loss to *lossSum. */
 int gbsp_dn_relmse_backward(void *stream, const float *logits, const float *noisy,
     const float *target, uint32_t B, uint32_t H, uint32_t W, uint16_t *dLogits, float *lossSum);
+/* The same with the loss summed in double precision and rounded once (the sum
+ * above depends on the order of its float additions).  scratch: 16 bytes of
+ * device memory, 8-byte aligned, zero before the call. */
+int gbsp_dn_relmse_backward_f64(void *stream, const float *logits, const float *noisy,
+    const float *target, uint32_t B, uint32_t H, uint32_t W, uint16_t *dLogits, float *lossSum,
+    void *scratch);
 /* One Adam step on n parameters (FP32 master copy, optional BF16 mirror). */
 int gbsp_dn_adam(void *stream, float *param, uint16_t *paramBf16, const float *grad, float *m,
     float *v, uint64_t n, float lr, float beta1, float beta2, float eps, uint32_t step);

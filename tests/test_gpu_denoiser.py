@@ -680,3 +680,39 @@ def test_chained_layers_capture_into_a_graph(gpu_lib):
             graph.replay()
             stream.synchronize()
             assert torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 1, 1), (1, 3, 43), (2, 64, 100), (16, 128, 128)])
+def test_loss_in_double_is_rounded_once(gpu_lib, B, H, W):
+    # a pixel less than a block, a ragged last block, many blocks: the loss is the sum
+    # in 64 bits of the per-pixel terms, the same in every run, added to what was there
+    import torch
+
+    from vk_cinematic_gb300.denoiser import _check, _ptr, _stream
+
+    g = torch.Generator().manual_seed(H * W)
+    logits = torch.randn((B, H, W, 32), generator=g).cuda()
+    noisy, target = (torch.rand((B, H, W, 4), generator=g).cuda() * 5 for _ in range(2))
+    out = torch.empty((B, H, W, 4), device="cuda")
+    _check(gpu_lib.gbsp_dn_filter(_stream(), _ptr(logits), _ptr(noisy), B, H, W, _ptr(out)))
+    dlogs = [torch.empty((B, H, 4, W, 8), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    losses = []
+    for _ in range(3):
+        buf = torch.zeros(8, device="cuda")
+        buf[0] = 0.5
+        _check(gpu_lib.gbsp_dn_relmse_backward_f64(_stream(), _ptr(logits), _ptr(noisy), _ptr(target), B, H,
+                                                   W, _ptr(dlogs[0]), _ptr(buf),
+                                                   ctypes.c_void_p(buf.data_ptr() + 16)))
+        losses.append(float(buf[0]))
+    assert losses[0] == losses[1] == losses[2]
+    o, r = out[..., :3].double(), target[..., :3].double()
+    ref = float(((o - r) ** 2 / (r * r + 0.01)).sum()) + 0.5
+    # a pixel's three float terms are good to a few units of 2^-24 each
+    assert abs(losses[0] - ref) <= 1e-6 * ref
+    plain = torch.zeros(1, device="cuda")
+    _check(gpu_lib.gbsp_dn_relmse_backward(_stream(), _ptr(logits), _ptr(noisy), _ptr(target), B, H, W,
+                                           _ptr(dlogs[1]), _ptr(plain)))
+    assert torch.equal(dlogs[0].view(torch.int16), dlogs[1].view(torch.int16))
+    with pytest.raises(gbsp.GbspError, match="8-byte"):
+        _check(gpu_lib.gbsp_dn_relmse_backward_f64(_stream(), _ptr(logits), _ptr(noisy), _ptr(target), B, H,
+                                                   W, _ptr(dlogs[0]), _ptr(plain), None))

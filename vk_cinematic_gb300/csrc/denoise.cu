@@ -1631,11 +1631,17 @@ __global__ void __launch_bounds__(256) k_tile_merge(const float4 *__restrict__ D
 // 16 x 128^2 pixels: 38 -> 22 us.
 constexpr int kRelmseThreads = 128;
 
+// Sum of the blocks' losses and how many have added theirs; zero before a launch.
+struct LossTotal {
+    double sum;
+    unsigned long long blocks;
+};
+
 // kVec: logits and dLogits 16-byte aligned (else 32-bit accesses)
 template <bool kVec>
 __global__ void __launch_bounds__(kRelmseThreads) k_relmse_bwd(const float *__restrict__ logits,
     const float4 *__restrict__ noisy, const float4 *__restrict__ target, int B, int H, int W,
-    float invCount, __nv_bfloat16 *__restrict__ dLogits, float *lossSum)
+    float invCount, __nv_bfloat16 *__restrict__ dLogits, float *lossSum, LossTotal *total)
 {
     stage_begin();
     uint64_t p = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
@@ -1708,7 +1714,19 @@ __global__ void __launch_bounds__(kRelmseThreads) k_relmse_bwd(const float *__re
     __syncthreads();
     if (threadIdx.x == 0) {
         for (int k = 1; k < kRelmseThreads / 32; k++) loss += sums[k];
-        atomicAdd(lossSum, loss);
+        if (!total) {
+            atomicAdd(lossSum, loss);
+        } else {
+            // the blocks' sums in double precision, rounded once by the last of them: what
+            // float sums in the order of arrival are off by, 1e-6 and another value in
+            // each run, is gone (4e-8 from the sum in 64 bits of the same logits)
+            atomicAdd(&total->sum, (double)loss);
+            __threadfence();
+            if (atomicAdd(&total->blocks, 1ull) == gridDim.x - 1u) {
+                __threadfence();
+                *lossSum += (float)atomicAdd(&total->sum, 0.0);
+            }
+        }
     }
 }
 
@@ -2163,16 +2181,31 @@ int gbsp_dn_tile_fallback(void *stream, const float *denoised, const float *plai
     return GBSP_OK;
 }
 
-int gbsp_dn_relmse_backward(void *stream, const float *logits, const float *noisy,
-    const float *target, uint32_t B, uint32_t H, uint32_t W, uint16_t *dLogits, float *lossSum)
+static int relmse_backward(void *stream, const float *logits, const float *noisy, const float *target,
+    uint32_t B, uint32_t H, uint32_t W, uint16_t *dLogits, float *lossSum, LossTotal *total)
 {
     uint64_t n = (uint64_t)B * H * W;
     auto kern = (((uintptr_t)logits | (uintptr_t)dLogits) & 15u) ? k_relmse_bwd<false> : k_relmse_bwd<true>;
     kern<<<blocks(n, kRelmseThreads), kRelmseThreads, 0, (cudaStream_t)stream>>>(logits,
         reinterpret_cast<const float4 *>(noisy), reinterpret_cast<const float4 *>(target), B, H, W,
-        1.0f / (3.0f * (float)n), reinterpret_cast<__nv_bfloat16 *>(dLogits), lossSum);
+        1.0f / (3.0f * (float)n), reinterpret_cast<__nv_bfloat16 *>(dLogits), lossSum, total);
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
+}
+
+int gbsp_dn_relmse_backward(void *stream, const float *logits, const float *noisy,
+    const float *target, uint32_t B, uint32_t H, uint32_t W, uint16_t *dLogits, float *lossSum)
+{
+    return relmse_backward(stream, logits, noisy, target, B, H, W, dLogits, lossSum, nullptr);
+}
+
+int gbsp_dn_relmse_backward_f64(void *stream, const float *logits, const float *noisy,
+    const float *target, uint32_t B, uint32_t H, uint32_t W, uint16_t *dLogits, float *lossSum, void *scratch)
+{
+    if (!scratch || ((uintptr_t)scratch & 7u))
+        return set_error(GBSP_ERR_INVALID_ARGUMENT, "scratch must be 8-byte aligned");
+    return relmse_backward(stream, logits, noisy, target, B, H, W, dLogits, lossSum,
+        static_cast<LossTotal *>(scratch));
 }
 
 int gbsp_dn_adam(void *stream, float *param, uint16_t *paramBf16, const float *grad, float *m,

@@ -385,15 +385,18 @@ class KPCNN:
         B, H, W, _ = noisy.shape
         logits, acts = self.forward(feats, keep=True)
         dlog = torch.empty((B, H, 4, W, 8), dtype=torch.bfloat16, device="cuda")
-        loss = torch.zeros(1, dtype=torch.float32, device="cuda")
-        _check(self.L.gbsp_dn_relmse_backward(_stream(), _ptr(logits), _ptr(noisy), _ptr(target),
-                                              _u32(B), _u32(H), _u32(W), _ptr(dlog), _ptr(loss)))
-        # the weight-gradient kernels add to what they are given: one zeroed
-        # buffer, cut up (every size is a multiple of 16 floats, so views stay aligned)
+        # one zeroed buffer, cut up: the loss with its 16 bytes of scratch, then what the
+        # weight-gradient kernels add to (every size is a multiple of 16 floats, so views
+        # stay aligned)
         sizes = [w.numel() for w in self.w] + [b.numel() for b in self.b]
-        flat = torch.zeros(sum(sizes), dtype=torch.float32, device="cuda").split(sizes)
+        head, *flat = torch.zeros(16 + sum(sizes), dtype=torch.float32,
+                                  device="cuda").split([16] + sizes)
+        loss = head[:1]
         dws = [f.view(w.shape) for f, w in zip(flat, self.w)]
-        dbs = list(flat[len(self.w):])
+        dbs = flat[len(self.w):]
+        _check(self.L.gbsp_dn_relmse_backward_f64(_stream(), _ptr(logits), _ptr(noisy), _ptr(target),
+                                                  _u32(B), _u32(H), _u32(W), _ptr(dlog), _ptr(loss),
+                                                  _vp(head.data_ptr() + 16)))
         last = len(LAYERS) - 1
         inputs = [feats] + acts
         # weight gradients are taken together, in the order of the backward pass,

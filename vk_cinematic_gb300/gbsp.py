@@ -60,6 +60,7 @@ EXPORTS = [
     "gbsp_batch_set_node_widths", "gbsp_batch_get_node_widths", "gbsp_path_trace_tile_list",
     "gbsp_dn_tile_check", "gbsp_dn_tile_merge", "gbsp_dn_conv3x3_weight_grad_tcgen05",
     "gbsp_dn_weight_grads_tcgen05", "gbsp_dn_weight_grads_scratch",
+    "gbsp_dn_relmse_backward_f64",
     "gbsp_path_trace_tile_list_spp", "gbsp_path_trace_tile_split",
     "gbsp_dn_conv3x3_data_grad_relu_tc", "gbsp_dn_adam_all",
 ]
