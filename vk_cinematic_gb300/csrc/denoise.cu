@@ -1141,15 +1141,15 @@ __global__ void __launch_bounds__(288) k_conv3x3_wgrad_tc(const __nv_bfloat16 *_
     if (tid < COUT) out[9 * COUT * CIN + tid] = bacc;
 }
 
-// dW[i] += sum over CTA slices of partial[slice][i] in a fixed order, for one
-// or several layers: thread group g of kReduceGroups adds slices g, g + 8, ...
-// and the groups' sums are added in pairs; the last COUT entries of a slice are
-// the bias gradient.
-// Bound: the latency of the loads (12.6 MB at 152 slices of 48 x 48 weights).
-// One thread per entry walking all slices took 13 us a layer, 8 groups of
-// threads with 8 loads in flight each 7 us (4 groups 9.6); the eight layers of
-// the network in one launch 27 us instead of 54.
-constexpr int kReduceGroups = 8, kReduceEntries = 32;
+// dW[i] += sum over CTA slices of partial[slice][i], added from the first slice
+// to the last, for one or several layers, a thread per entry; the last COUT
+// entries of a slice are the bias gradient.  A bias gradient is a small sum of
+// large terms, so the order of its additions shows (1e-5 for a sum in eight
+// groups).
+// Bound: the loads (12.6 MB at 152 slices of 48 x 48 weights), latency for a layer
+// by itself (13 us), memory for the eight layers of the network in one launch (88
+// MB, 19 us; 27 with eight groups of threads, 37 through shared memory).
+constexpr int kReduceThreads = 128;
 constexpr int kWgLayers = 8;  // layers per launch
 
 struct ReduceJobs {
@@ -1162,27 +1162,18 @@ struct ReduceJobs {
     int count, slices;
 };
 
-__global__ void __launch_bounds__(kReduceGroups * kReduceEntries) k_wgrad_reduce(
-    const __grid_constant__ ReduceJobs jobs)
+__global__ void __launch_bounds__(kReduceThreads) k_wgrad_reduce(const __grid_constant__ ReduceJobs jobs)
 {
     stage_begin();
-    __shared__ float sums[kReduceGroups][kReduceEntries];
     int layer = 0;
     while (layer + 1 < jobs.count && blockIdx.x >= jobs.l[layer + 1].firstBlock) layer++;
     const ReduceJobs::Layer &l = jobs.l[layer];
-    const int e = threadIdx.x % kReduceEntries, g = threadIdx.x / kReduceEntries;
-    const int i = (int)(blockIdx.x - l.firstBlock) * kReduceEntries + e;
+    const int i = (int)(blockIdx.x - l.firstBlock) * kReduceThreads + threadIdx.x;
+    if (i >= l.perSlice) return;
+    const float *partial = l.partial + i;  // plain loads: the kernel before this one writes it
     float sum = 0.0f;
-    if (i < l.perSlice) {
-        const float *partial = l.partial;  // plain loads: the kernel before this one writes it
 #pragma unroll 8
-        for (int k = g; k < jobs.slices; k += kReduceGroups) sum += partial[(size_t)k * l.perSlice + i];
-    }
-    sums[g][e] = sum;
-    __syncthreads();
-    if (g != 0 || i >= l.perSlice) return;
-    sum = ((sums[0][e] + sums[1][e]) + (sums[2][e] + sums[3][e])) +
-        ((sums[4][e] + sums[5][e]) + (sums[6][e] + sums[7][e]));
+    for (int k = 0; k < jobs.slices; k++) sum += partial[(size_t)k * l.perSlice];
     if (i < l.wCount)
         l.dW[i] += sum;
     else
@@ -1794,12 +1785,12 @@ static uint32_t add_reduce(ReduceJobs &jobs, uint32_t blocks, const float *parti
 {
     const int wCount = 9 * cout * cin, perSlice = wCount + cout;
     jobs.l[jobs.count++] = {partial, dW, dBias, perSlice, wCount, blocks};
-    return blocks + (uint32_t)((perSlice + kReduceEntries - 1) / kReduceEntries);
+    return blocks + (uint32_t)((perSlice + kReduceThreads - 1) / kReduceThreads);
 }
 
 static cudaError_t launch_reduce(cudaStream_t s, const ReduceJobs &jobs, uint32_t blocks)
 {
-    launch_next(k_wgrad_reduce, (int)blocks, kReduceGroups * kReduceEntries, s, jobs);
+    launch_next(k_wgrad_reduce, (int)blocks, kReduceThreads, s, jobs);
     return cudaGetLastError();
 }
 
