@@ -80,6 +80,20 @@ def test_irradiance_random_stream_is_the_references(gpu_lib):
     assert np.abs(got - ref).max() <= 1e-6
 
 
+@pytest.mark.parametrize("width,height", [(700, 333), (1030, 517)])
+def test_cube_map_rows_per_thread(gpu_lib, hdri, width, height):
+    # sizes at which a thread takes two and four rows, the last ones past the map
+    import torch
+
+    src = np.ascontiguousarray(hdri[::4, ::4])
+    got = gbsp.create_cube_map(torch.from_numpy(src).cuda(), width, height).cpu().numpy()
+    ref = pyoracle.create_cube_map(src, width, height)
+    e = rel_err(got, ref)
+    assert e.mean() <= 1e-5
+    assert np.mean(e > 1e-3) < 1e-3
+    assert np.array_equal(got[..., 3], ref[..., 3])
+
+
 @pytest.mark.parametrize("width,height,spp", [(5, 3, 1), (7, 2, 31), (6, 6, 33), (9, 4, 65), (33, 1, 64)])
 def test_irradiance_random_splits_the_stream(gpu_lib, hdri, width, height, spp):
     # a warp per texel, a run of samples per lane: one sample, a lane short, a run

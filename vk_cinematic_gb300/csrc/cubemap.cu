@@ -116,7 +116,10 @@ __device__ __forceinline__ V3 face_direction(const Basis &b, uint32_t x, uint32_
 // four divisions per texel), about 40 us of them at 6 x 1024^2 texels; 134 MB
 // of traffic would take 20.  Texel coordinates come from a 3-d grid: three
 // 64-bit divisions of a flat index had cost a fifth of the kernel.  6 x 1024^2
-// from 2048 x 1024: 78 -> 64 us, 90 % of the issue slots busy.
+// from 2048 x 1024: 78 -> 64 us, 90 % of the issue slots busy.  A thread takes
+// up to four rows of a column (the column's division and products once) while
+// that leaves two waves of blocks: with the irradiance map 162.4 -> 156.3 us (two
+// rows 158.9, eight 158.6).
 constexpr int kCubeX = 32, kCubeY = 8;
 
 __global__ void __launch_bounds__(kCubeX * kCubeY) k_cube_map(Image im, uint32_t width, uint32_t height,
@@ -310,13 +313,18 @@ static int check_image(const float *equirect, uint32_t eqW, uint32_t eqH, uint32
     return GBSP_OK;
 }
 
-static int grid_for(uint64_t work, int block)
+static int sm_count()
 {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    return sms > 0 ? sms : 1;
+}
+
+static int grid_for(uint64_t work, int block)
+{
     uint64_t want = (work + block - 1) / block;
-    uint64_t cap = (uint64_t)(sms > 0 ? sms : 1) * 16;
+    uint64_t cap = (uint64_t)sm_count() * 16;
     return (int)(want < cap ? (want ? want : 1) : cap);
 }
 
@@ -333,8 +341,11 @@ int gbsp_create_cube_map(void *stream, const float *equirect, uint32_t eqWidth, 
     int rc = check_image(equirect, eqWidth, eqHeight, width, height, faces);
     if (rc) return rc;
     cube::Image im{reinterpret_cast<const float4 *>(equirect), eqWidth, eqHeight};
-    const dim3 grid((width + cube::kCubeX - 1) / cube::kCubeX,
-        std::min((height + cube::kCubeY - 1) / cube::kCubeY, 65535u), 6);
+    const uint32_t cols = (width + cube::kCubeX - 1) / cube::kCubeX,
+                   bands = (height + cube::kCubeY - 1) / cube::kCubeY;
+    // two waves of 8 blocks per SM
+    const uint64_t rows = std::min<uint64_t>(4, std::max<uint64_t>(1, 6ull * cols * bands / (16ull * sm_count())));
+    const dim3 grid(cols, (uint32_t)std::min<uint64_t>((bands + rows - 1) / rows, 65535u), 6);
     cube::k_cube_map<<<grid, dim3(cube::kCubeX, cube::kCubeY), 0, (cudaStream_t)stream>>>(im, width, height,
         reinterpret_cast<float4 *>(faces));
     GBSP_CUDA_TRY(cudaGetLastError());
