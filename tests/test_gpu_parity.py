@@ -748,6 +748,45 @@ def test_query_sizes_match_the_large_batch(rt, wt, width):
         assert m["rays_traced"] == k == m["ray_hit_count"] + m["ray_miss_count"]
 
 
+@pytest.mark.parametrize("n", [700, 65536 + 300])
+@pytest.mark.parametrize("wt", [False, True])
+@pytest.mark.parametrize("width", [8, 4])
+def test_rays_without_a_finite_origin_miss_at_the_root(rt, width, wt, n):
+    """Rays whose origin is NaN in some or all components, or infinite, mixed
+    into a batch of either size class: they miss, no status is raised and the
+    other rays' results stay the same bits.  A batch whose origins are NaN
+    throughout (in watertight mode: in z) meets no object at all."""
+    s = scenes.config3_scene(width=64, height=64, spp=1, n_spheres=12, level=2, seed=3)
+    scene, ms, _ = gbsp.upload_scene(rt, s)
+    scene.set_intersection(gbsp.ISECT_WATERTIGHT if wt else gbsp.ISECT_REFERENCE_MT)
+    scene.set_node_width(width)
+    rng = np.random.default_rng(8)
+    rays = np.concatenate([rng.uniform(-8, 8, (n, 3)), rng.normal(size=(n, 3))], 1).astype(np.float32)
+    clean, mats, _ = scene.intersect(rays)
+    nan, inf = np.float32(np.nan), np.float32(np.inf)
+    bad = [(nan, nan, nan), (nan, 0, 0), (0, nan, 0), (0, 0, nan), (nan, nan, 0), (nan, 0, nan),
+           (0, nan, nan), (inf, 0, 0), (0, -inf, 0), (inf, inf, -inf), (nan, inf, 0)]
+    mixed = rays.copy()
+    at = np.arange(0, n, 13)
+    for j, k in enumerate(at):
+        o = np.array(bad[j % len(bad)], np.float32)
+        mixed[k, :3] = np.where(np.isfinite(o), mixed[k, :3], o)
+    got, gmats, m = scene.intersect(mixed)
+    assert m.as_dict()["rays_traced"] == n
+    assert (got[at, 0] == -1).all() and (gmats[at] == 0).all()
+    rest = np.ones(n, bool)
+    rest[at] = False
+    assert np.array_equal(got[rest].view(np.uint32), clean[rest].view(np.uint32))
+    assert np.array_equal(gmats[rest], mats[rest])
+    for o in [(nan, nan, nan)] + ([(0, 0, nan)] if wt else []):
+        none = rays.copy()
+        none[:, :3] = np.where(np.isnan(o), nan, rays[:, :3])
+        got, _, m = scene.intersect(none)
+        m = m.as_dict()
+        assert (got[:, 0] == -1).all()
+        assert m["mesh_tests_performed"] == 0 and m["broadphase_node_visits"] == n
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

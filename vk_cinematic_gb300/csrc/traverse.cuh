@@ -188,7 +188,8 @@ __device__ __forceinline__ float min3(float a, float b, float c)
 // after rounding (subtraction and multiplication round monotonically), and
 // the other way round for invd < 0.  Two children share one f32x2 operation,
 // each half rounded like the scalar one: entry distances and decisions are
-// those of slab_entry_node.  1080p benchmark frame: 85.3 -> 79.1 ms, 2^20
+// those of slab_entry_node, also for an origin that is NaN in some or all
+// components, and those of slab_entry_robust unless o.z is NaN.  1080p benchmark frame: 85.3 -> 79.1 ms, 2^20
 // rays against 2^18 triangles 2,366 -> 1,905 us (both at 6 blocks per SM).
 template <bool kWT>
 __device__ __forceinline__ uint32_t visit_node8(const float4 *__restrict__ pool, uint32_t ref,
@@ -227,7 +228,9 @@ __device__ __forceinline__ uint32_t visit_node8(const float4 *__restrict__ pool,
             if (kWT) tf = tf * 1.0000004f;
             const bool present = cc[j] != kEmptyChild;
             boxes += present ? 1u : 0u;
-            const bool hit = present && tn <= fminf(tf, bound);
+            // tf is NaN (a miss) when the origin is NaN in every component; fminf(tf,
+            // bound) would drop it and take every box
+            const bool hit = present && tn <= tf && !(tn > bound);
             const bool closer = tn < nearT;
             const StackEntry push{closer ? nearRef : cc[j], closer ? nearT : tn};
             if (hit && push.ref != kEmptyChild) {
@@ -306,7 +309,9 @@ __device__ __forceinline__ uint32_t visit_nearest(const float4 *__restrict__ poo
     uint32_t &boxes)
 {
     if constexpr (kQ == 2) {
-        if (isfinite(invd.x) && isfinite(invd.y) && isfinite(invd.z))
+        // slab_entry_robust misses every box from an origin with a NaN in z and has no
+        // constraint from one in x or y, as the instructions of visit_node8 have for all three
+        if (isfinite(invd.x) && isfinite(invd.y) && isfinite(invd.z) && (!kWT || o.z == o.z))
             return visit_node8<kWT>(pool, ref, o, invd, bound, stack, sp, status, boxes);
         return visit_node8_any<kWT>(pool, ref, o, invd, bound, stack, sp, status, boxes);
     } else {
