@@ -787,6 +787,54 @@ def test_rays_without_a_finite_origin_miss_at_the_root(rt, width, wt, n):
         assert m["mesh_tests_performed"] == 0 and m["broadphase_node_visits"] == n
 
 
+def test_captured_query_keeps_apart_from_renders(gpu_lib):
+    """A large device query captured into a graph has its queue, hits and
+    control words to itself: replayed on another stream while the runtime it
+    was captured on renders frames and answers queries of its own, the
+    replays, the frames and the queries all give the values they give alone."""
+    import torch
+
+    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
+    r = gbsp.Runtime(0, stream=stream.cuda_stream)
+    s = scenes.config3_scene(width=96, height=64, spp=4, n_spheres=24, level=2, seed=3)
+    scene, ms, rend = gbsp.upload_scene(r, s)
+    n = 65536 + 77
+    rng = np.random.default_rng(4)
+    rays = np.zeros((2, n, 8), np.float32)
+    rays[..., 0:3], rays[..., 4:7] = rng.uniform(-8, 8, (2, n, 3)), rng.normal(size=(2, n, 3))
+    dr = torch.from_numpy(rays).cuda()
+    t = torch.empty((2, n), device="cuda")
+    tri, obj = (torch.empty((2, n), dtype=torch.int32, device="cuda") for _ in range(2))
+
+    def query(k):
+        scene.intersect_closest_device(n, dr[k].data_ptr(), t[k].data_ptr(), tri[k].data_ptr(),
+                                       obj[k].data_ptr())
+
+    torch.cuda.synchronize()
+    for k in range(2):
+        query(k)
+    r.synchronize()
+    alone = [x.cpu().numpy() for x in (t, tri, obj)]
+    image = rend.frame()[0].copy()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        query(0)
+    for x in (t, tri, obj):
+        x.zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(other):
+            graph.replay()
+        query(1)
+        img = rend.frame()[0]
+        assert np.array_equal(img.view(np.uint32), image.view(np.uint32))
+    torch.cuda.synchronize()
+    for x, want in zip((t, tri, obj), alone):
+        assert np.array_equal(x.cpu().numpy().view(np.uint32), want.view(np.uint32))
+    del graph
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

@@ -305,6 +305,7 @@ static void runtime_teardown(gbsp_runtime *rt)
     rt->vert.release();
     rt->pathRad.release();
     rt->query.release();
+    rt->queryQueue.release();
     rt->slots.release();
     rt->frame.release();
     rt->aov.release();

@@ -118,6 +118,7 @@ struct gbsp_runtime {
     gbsp::DeviceBuffer<int32_t> slots;   // material slot per instance of the current render
     gbsp::DeviceBuffer<float> query;     // rays and results of a host query
     unsigned char *stage = nullptr;      // pinned results of a host query, kStageBytes
+    gbsp::DeviceBuffer<float4> queryQueue;  // queue, hits and control words of a large query
     cudaEvent_t ev[8] = {};
     // wavefront state, grown on demand
     gbsp::DeviceBuffer<float4> rayO, rayD;         // two queues back to back

@@ -174,32 +174,28 @@ int launch_intersect(gbsp_runtime *rt, const SceneView &sv, uint32_t count, cons
         return launch(s, sv, count, rays, out, rt->smCount, rt->dCounters, rt->dStatus);
     }
     const size_t n = count;
-    // The runtime's wave buffers hold the queue.  A call that is being captured
-    // brings its own memory: a graph must not refer to buffers that a later
-    // call may replace.
+    // One block holds the batch: origins, directions, hits (16 bytes each), object
+    // ids, and the queue's control words, so that a call shares nothing with a
+    // render but the metrics.  A call that is being captured brings its own block:
+    // a graph must not refer to one that a later call may replace.
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     GBSP_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
-    DeviceBuffer<float4> ownRays;
-    DeviceBuffer<int4> ownHits;
-    DeviceBuffer<int> ownInst;
-    const bool own = capture != cudaStreamCaptureStatusNone;
-    DeviceBuffer<int4> &hits = own ? ownHits : rt->hitA;
-    DeviceBuffer<int> &inst = own ? ownInst : rt->hitInst;
-    int rc;
-    if ((own && (rc = ownRays.reserve(2 * n, s))) ||
-        (!own && ((rc = rt->rayO.reserve(n, s)) || (rc = rt->rayD.reserve(n, s)))) ||
-        (rc = hits.reserve(n, s)) || (rc = inst.reserve(n, s)))
-        return rc;
-    float4 *o = own ? ownRays.ptr : rt->rayO.ptr, *d = own ? ownRays.ptr + n : rt->rayD.ptr;
-    unsigned int *ctl = reinterpret_cast<unsigned int *>(rt->dCounters + GBSP_METRIC_COUNT);
+    DeviceBuffer<float4> ownQueue;
+    DeviceBuffer<float4> &queue = capture != cudaStreamCaptureStatusNone ? ownQueue : rt->queryQueue;
+    const size_t instQuads = (n + 3) / 4, ctlQuads = kCtlCount * sizeof(unsigned int) / sizeof(float4);
+    if (int rc = queue.reserve(3 * n + instQuads + ctlQuads, s)) return rc;
+    float4 *o = queue.ptr, *d = o + n;
+    int4 *hits = reinterpret_cast<int4 *>(d + n);
+    int *inst = reinterpret_cast<int *>(hits + n);
+    unsigned int *ctl = reinterpret_cast<unsigned int *>(hits + n + instQuads);
     OneScene one = {};
     one.sv = sv;
     const int blocks = (int)((n + 255) / 256);
     (packed ? k_split_rays<true> : k_split_rays<false>)<<<blocks, 256, 0, s>>>(rays, count, o, d, ctl);
     launch_trace_stage(true, watertight, sv.nodeQuads,
         trace_grid<OneScene>(true, watertight, sv.nodeQuads, rt->smCount), s, one, o, d,
-        ctl + queue_word(0), hits.ptr, inst.ptr, ctl, rt->dCounters, rt->dStatus);
-    launch_next(k_intersect_outputs, blocks, 256, s, sv, hits.ptr, inst.ptr, count, out);
+        ctl + queue_word(0), hits, inst, ctl, rt->dCounters, rt->dStatus);
+    launch_next(k_intersect_outputs, blocks, 256, s, sv, hits, inst, count, out);
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
 }
