@@ -835,6 +835,41 @@ def test_captured_query_keeps_apart_from_renders(gpu_lib):
     del graph
 
 
+def test_huge_query_gives_its_memory_back(rt):
+    """A device query past the size of the queue that a runtime keeps (512 MB,
+    52 bytes per ray) goes through it in pieces: no more memory than that is
+    held once it is done, and every part of it is answered as by itself."""
+    import torch
+
+    s = scenes.config3_scene(width=64, height=64, spp=1, n_spheres=2, level=1, seed=3)
+    scene, ms, _ = gbsp.upload_scene(rt, s)
+    n, part = (1 << 24) + 5, 1 << 17  # 872 MB: two pieces
+    g = torch.Generator(device="cuda").manual_seed(2)
+    rays = torch.randn((n, 8), generator=g, device="cuda")
+    rays[n - part:] = rays[:part]
+    rays[n // 2 - part:n // 2 + part] = torch.cat([rays[:part], rays[:part]])  # around the cut
+    t = torch.empty(n, device="cuda")
+    tri, obj = (torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2))
+
+    def query(k):
+        torch.cuda.synchronize()
+        scene.intersect_closest_device(k, rays.data_ptr(), t.data_ptr(), tri.data_ptr(), obj.data_ptr())
+        rt.synchronize()
+        torch.cuda.synchronize()
+
+    query(part)
+    want = [x[:part].clone() for x in (t, tri, obj)]
+    assert 0.02 < (want[1] >= 0).float().mean() < 0.98
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    query(n)
+    kept = before - torch.cuda.mem_get_info()[0]
+    assert kept <= 576 << 20, kept
+    for x, w in zip((t, tri, obj), want):
+        for first in (0, n // 2 - part, n // 2, n - part):
+            assert torch.equal(x[first:first + part], w), first
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

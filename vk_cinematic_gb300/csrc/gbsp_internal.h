@@ -67,6 +67,11 @@ struct DeviceBuffer {
 
 // Memory of host queries that a runtime keeps: device block, pinned results.
 constexpr size_t kQueryKeep = 64u << 20, kStageBytes = 1u << 20;
+// Queue memory of large queries that a runtime keeps, at most (52 bytes per ray):
+// longer batches go through it in pieces.  A piece more costs its tail: 2^24 rays
+// 23.55 ms with 872 MB for all of them, 23.9 in two pieces, 25.45 with a block of
+// the call's own (its memory is mapped anew on every call).
+constexpr size_t kQueueKeep = 512u << 20;
 
 // The block of counters, queue words and status as the host reads it.
 constexpr int kStatusSlot = GBSP_METRIC_COUNT + 8;  // u64 index of the status word

@@ -168,34 +168,43 @@ int launch_intersect(gbsp_runtime *rt, const SceneView &sv, uint32_t count, cons
     if (!count) return GBSP_OK;
     cudaStream_t s = rt->stream;
     const bool watertight = sv.watertight != 0;
-    const QueryOutputs out = {tOut, triOut, objOut, attrOut, matOut};
     if (count < kPerLaneBatch) {
+        const QueryOutputs out = {tOut, triOut, objOut, attrOut, matOut};
         auto launch = packed ? launch_small<true> : launch_small<false>;
         return launch(s, sv, count, rays, out, rt->smCount, rt->dCounters, rt->dStatus);
     }
-    const size_t n = count;
-    // One block holds the batch: origins, directions, hits (16 bytes each), object
-    // ids, and the queue's control words, so that a call shares nothing with a
-    // render but the metrics.  A call that is being captured brings its own block:
-    // a graph must not refer to one that a later call may replace.
+    // One block holds a piece of the batch: origins, directions, hits (16 bytes each),
+    // object ids, and the queue's control words, so that a call shares nothing with a
+    // render but the metrics.  A call that is being captured brings its own block: a
+    // graph must not refer to one that a later call may replace.
+    const size_t ctlQuads = kCtlCount * sizeof(unsigned int) / sizeof(float4);
+    const auto quads_for = [&](size_t n) { return 3 * n + (n + 3) / 4 + ctlQuads; };
+    const size_t most = (kQueueKeep / sizeof(float4) - ctlQuads - 1) * 4 / 13;
+    const size_t pieces = (count + most - 1) / most, piece = (count + pieces - 1) / pieces;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     GBSP_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
     DeviceBuffer<float4> ownQueue;
     DeviceBuffer<float4> &queue = capture != cudaStreamCaptureStatusNone ? ownQueue : rt->queryQueue;
-    const size_t instQuads = (n + 3) / 4, ctlQuads = kCtlCount * sizeof(unsigned int) / sizeof(float4);
-    if (int rc = queue.reserve(3 * n + instQuads + ctlQuads, s)) return rc;
-    float4 *o = queue.ptr, *d = o + n;
-    int4 *hits = reinterpret_cast<int4 *>(d + n);
-    int *inst = reinterpret_cast<int *>(hits + n);
-    unsigned int *ctl = reinterpret_cast<unsigned int *>(hits + n + instQuads);
+    if (int rc = queue.reserve(quads_for(piece), s)) return rc;
     OneScene one = {};
     one.sv = sv;
-    const int blocks = (int)((n + 255) / 256);
-    (packed ? k_split_rays<true> : k_split_rays<false>)<<<blocks, 256, 0, s>>>(rays, count, o, d, ctl);
-    launch_trace_stage(true, watertight, sv.nodeQuads,
-        trace_grid<OneScene>(true, watertight, sv.nodeQuads, rt->smCount), s, one, o, d,
-        ctl + queue_word(0), hits, inst, ctl, rt->dCounters, rt->dStatus);
-    launch_next(k_intersect_outputs, blocks, 256, s, sv, hits, inst, count, out);
+    for (size_t first = 0; first < count; first += piece) {
+        const uint32_t n = (uint32_t)std::min<size_t>(piece, count - first);
+        float4 *o = queue.ptr, *d = o + n;
+        int4 *hits = reinterpret_cast<int4 *>(d + n);
+        int *inst = reinterpret_cast<int *>(hits + n);
+        unsigned int *ctl = reinterpret_cast<unsigned int *>(queue.ptr + quads_for(n) - ctlQuads);
+        const QueryOutputs at = {tOut ? tOut + first : nullptr, triOut ? triOut + first : nullptr,
+            objOut ? objOut + first : nullptr, attrOut ? attrOut + 6 * first : nullptr,
+            matOut ? matOut + first : nullptr};
+        const int blocks = (int)((n + 255) / 256);
+        (packed ? k_split_rays<true> : k_split_rays<false>)<<<blocks, 256, 0, s>>>(
+            rays + (packed ? 6 : 8) * first, n, o, d, ctl);
+        launch_trace_stage(true, watertight, sv.nodeQuads,
+            trace_grid<OneScene>(true, watertight, sv.nodeQuads, rt->smCount), s, one, o, d,
+            ctl + queue_word(0), hits, inst, ctl, rt->dCounters, rt->dStatus);
+        launch_next(k_intersect_outputs, blocks, 256, s, sv, hits, inst, n, at);
+    }
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
 }
