@@ -232,7 +232,8 @@ int gbsp_scene_info(const gbsp_scene *scene, uint32_t *objects,
 /* replaces sp_RayIntersectScene (src/sp_scene.cpp:229-339) for a batch of
  * rays in host memory: rays = count * (origin xyz, direction xyz).
  * resultOut = count * (t, normal xyz, u, v), t = -1 on a miss;
- * materialOut = count material ids. */
+ * materialOut = count material ids.  Scenes of one runtime may be queried from
+ * a thread each; only their metrics then mix. */
 int gbsp_ray_intersect_scene(gbsp_scene *scene, uint32_t count,
     const float *rays, float *resultOut, uint32_t *materialOut,
     gbsp_metrics *metrics);

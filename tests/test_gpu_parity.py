@@ -870,6 +870,50 @@ def test_huge_query_gives_its_memory_back(rt):
             assert torch.equal(x[first:first + part], w), first
 
 
+@pytest.mark.parametrize("n", [3001, 65536 + 900])
+def test_queries_from_two_threads(gpu_lib, n):
+    """Two scenes on one runtime, each queried from a thread of its own (small
+    and growing host batches and device batches of either size class): every
+    answer is the one the scene gives alone."""
+    import threading
+
+    import torch
+
+    r = gbsp.Runtime()
+    work = []
+    for k in range(2):
+        s = scenes.config3_scene(width=64, height=64, spp=1, n_spheres=8 + 9 * k, level=1 + k, seed=3 + k)
+        scene, ms, _ = gbsp.upload_scene(r, s)
+        rng = np.random.default_rng(4 + k)
+        rays = np.concatenate([rng.uniform(-8, 8, (n, 3)), rng.normal(size=(n, 3))], 1).astype(np.float32)
+        packed = np.zeros((n, 8), np.float32)
+        packed[:, 0:3], packed[:, 4:7] = rays[:, :3], rays[:, 3:]
+        out = [torch.empty(n, device="cuda")] + [torch.empty(n, dtype=torch.int32, device="cuda") for _ in range(2)]
+        work.append((scene, ms, rays, torch.from_numpy(packed).cuda(), out, scene.intersect(rays)))
+    torch.cuda.synchronize()
+    wrong = []
+
+    def queries(k):
+        scene, _, rays, dr, out, (attr, mat, _) = work[k]
+        for i in range(60):
+            m = n - 7 * (60 - i) if i % 3 else n
+            got, mats, _ = scene.intersect(rays[:m])
+            if not (np.array_equal(got.view(np.uint32), attr[:m].view(np.uint32)) and
+                    np.array_equal(mats, mat[:m])):
+                wrong.append((k, i, "host"))
+            scene.intersect_closest_device(n, dr.data_ptr(), *(x.data_ptr() for x in out))
+        r.synchronize()
+        if not np.array_equal(out[0].cpu().numpy().view(np.uint32), attr[:, 0].copy().view(np.uint32)):
+            wrong.append((k, "device"))
+
+    threads = [threading.Thread(target=queries, args=(k,)) for k in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong, wrong[:5]
+
+
 def test_watertight_mode_closes_shared_edges(rt):
     """GBSP_ISECT_WATERTIGHT: rays aimed at the shared edges and vertices of
     a closed icosphere never miss, and every query agrees bit for bit with the

@@ -756,6 +756,7 @@ int gbsp_ray_intersect_scene(gbsp_scene *scene, uint32_t count, const float *ray
     // blocks past kQueryKeep are not kept.  The rays go up as they are: packing
     // them into float4 pairs first, a buffer each and a wait per result took
     // 198 us for 20,011 rays that the device walks in 35; 138 us so.
+    std::lock_guard<std::mutex> lock(rt->hostQueries);
     DeviceBuffer<float> big;
     DeviceBuffer<float> &buf = 13 * (size_t)count * sizeof(float) > kQueryKeep ? big : rt->query;
     if ((rc = buf.reserve(13 * (size_t)count, s))) return rc;

@@ -3,6 +3,7 @@
 
 #include <cstdint>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -121,6 +122,10 @@ struct gbsp_runtime {
     uint32_t *dStatus = nullptr;        // kernel status word, in that block
     gbsp::Readback *readback = nullptr;  // pinned copy of the block
     gbsp::DeviceBuffer<int32_t> slots;   // material slot per instance of the current render
+    // Queries of several scenes may come from several threads: a host query holds
+    // hostQueries until its results are out of `stage`, and a large one holds
+    // queryLaunch while it enqueues (the stream then keeps the calls apart).
+    std::mutex hostQueries, queryLaunch;
     gbsp::DeviceBuffer<float> query;     // rays and results of a host query
     unsigned char *stage = nullptr;      // pinned results of a host query, kStageBytes
     gbsp::DeviceBuffer<float4> queryQueue;  // queue, hits and control words of a large query

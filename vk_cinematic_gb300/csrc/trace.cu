@@ -183,6 +183,7 @@ int launch_intersect(gbsp_runtime *rt, const SceneView &sv, uint32_t count, cons
     const size_t pieces = (count + most - 1) / most, piece = (count + pieces - 1) / pieces;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     GBSP_CUDA_TRY(cudaStreamIsCapturing(s, &capture));
+    std::lock_guard<std::mutex> lock(rt->queryLaunch);
     DeviceBuffer<float4> ownQueue;
     DeviceBuffer<float4> &queue = capture != cudaStreamCaptureStatusNone ? ownQueue : rt->queryQueue;
     if (int rc = queue.reserve(quads_for(piece), s)) return rc;
