@@ -716,3 +716,35 @@ def test_loss_in_double_is_rounded_once(gpu_lib, B, H, W):
     with pytest.raises(gbsp.GbspError, match="8-byte"):
         _check(gpu_lib.gbsp_dn_relmse_backward_f64(_stream(), _ptr(logits), _ptr(noisy), _ptr(target), B, H,
                                                    W, _ptr(dlogs[0]), _ptr(plain), None))
+
+
+@pytest.mark.parametrize("B,H,W", [(1, 5, 130), (4, 64, 128)])
+def test_mask_from_the_launch_before(gpu_lib, B, H, W):
+    """The data gradient reads its mask from activations that the chained launch
+    right before it writes, into a buffer that held other values: the same bits
+    as with a wait in between."""
+    import torch
+
+    from vk_cinematic_gb300.denoiser import KPCNN, _check, _stream_handle
+
+    torch.manual_seed(H)
+    net = KPCNN(seed=2)
+    d = torch.randn((B, H, 6, W, 8), device="cuda").to(torch.bfloat16)
+    xs = [torch.randn((B, H, 6, W, 8), device="cuda").to(torch.bfloat16) for _ in range(4)]
+    act = torch.empty_like(d)
+    torch.cuda.synchronize()
+
+    def step(x, wait):
+        _check(net.L.gbsp_dn_conv3x3_forward_tc(_stream_handle(), x.data_ptr(), B, H, W, 48,
+                                                net.wb[2].data_ptr(), net.b[2].data_ptr(), 48, 0,
+                                                act.data_ptr(), None))
+        if wait:
+            torch.cuda.synchronize()
+        return net.data_grad_relu(1, d, act)
+
+    want = [step(x, True) for x in xs]
+    for _ in range(10):
+        got = [step(x, False) for x in xs]
+        torch.cuda.synchronize()
+        for a, b in zip(got, want):
+            assert torch.equal(a.view(torch.int16), b.view(torch.int16))

@@ -394,8 +394,7 @@ __device__ __forceinline__ void conv_store(const uint32_t (&r)[COUT], size_t row
 // (168 registers, spills), two rows 548.
 template <int COUT>
 __device__ __forceinline__ void conv_filter_store(const uint32_t (&r)[COUT], size_t p, int x, int y,
-    int W, int H, const float *__restrict__ bias, const float4 *__restrict__ noisy,
-    float4 *__restrict__ out)
+    int W, int H, const float *__restrict__ bias, const float4 *noisy, float4 *out)
 {
     static_assert(COUT >= 25, "kernel logits");
     float wk[25];
@@ -412,7 +411,7 @@ __device__ __forceinline__ void conv_filter_store(const uint32_t (&r)[COUT], siz
         const float4 *line = image + (size_t)min(max(y + j - 2, 0), H - 1) * W;
 #pragma unroll
         for (int i = 0; i < 5; i++) {
-            const float4 c = __ldg(line + dx[i]);
+            const float4 c = line[dx[i]];
             o.x += wk[5 * j + i] * c.x;
             o.y += wk[5 * j + i] * c.y;
             o.z += wk[5 * j + i] * c.z;
@@ -421,11 +420,12 @@ __device__ __forceinline__ void conv_filter_store(const uint32_t (&r)[COUT], siz
     out[p] = make_float4(o.x, o.y, o.z, 1.0f);
 }
 
+// A chained kernel: what it reads may be what the launch before it writes, so
+// no operand is __restrict__ or read with __ldg (launch.cuh).
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat16 *__restrict__ in,
-    int B, int H, int W, int rowsPerStrip, int reverse, const __nv_bfloat16 *__restrict__ w,
-    const float *__restrict__ bias, __nv_bfloat16 *__restrict__ outB, float *__restrict__ outF,
-    const float4 *__restrict__ noisy, float4 *__restrict__ outFilt, const __nv_bfloat16 *__restrict__ act)
+__global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat16 *in, int B, int H, int W,
+    int rowsPerStrip, int reverse, const __nv_bfloat16 *w, const float *bias, __nv_bfloat16 *outB,
+    float *outF, const float4 *noisy, float4 *outFilt, const __nv_bfloat16 *act)
 {
     constexpr int G = kTcGroupRows;
     static_assert(CIN % 16 == 0 && COUT % 16 == 0 && 3 * COUT <= 256, "tcgen05 tile shape");
@@ -727,8 +727,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) k_conv3x3_tc(const __nv_bfloat1
                     if (EPI == kEpiReluGrad && x < W && y < y1) {
 #pragma unroll
                         for (int c = 0; c < COUT; c += 8)
-                            mask[c / 8] = __ldg(reinterpret_cast<const uint4 *>(
-                                act + cg_index((size_t)(b * H + y), x, c, W, COUT)));
+                            mask[c / 8] = *reinterpret_cast<const uint4 *>(
+                                act + cg_index((size_t)(b * H + y), x, c, W, COUT));
                     }
                     uint32_t r[COUT];
 #pragma unroll
