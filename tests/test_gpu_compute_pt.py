@@ -118,3 +118,36 @@ def test_clusters_lose_no_hit(gpu_lib, entities, tris, sliver):
     same = (got.view(np.uint32) == ref.view(np.uint32)) | (np.isnan(got) & np.isnan(ref))
     assert same.all(), f"{(~same).sum()} words differ"
     assert (m["rays_traced"], m["ray_hit_count"], m["triangle_tests"]) == tuple(int(v) for v in c[:3])
+
+
+@pytest.mark.parametrize("scale", [1e19, 1e22, 2e22])
+def test_huge_entities_lose_no_hit(gpu_lib, scale):
+    """Entities scaled until the squares of an object-space direction are
+    denormal, so that its normalisation no longer gives unit length: the image
+    is the brute-force oracle's, bit for bit."""
+    pyoracle.build_port()
+    s = scenes.compute_pt_scene(n_spheres=1, level=0)
+    v, i = gbsp.icosphere(3)[:2]
+    s["vertices"], s["indices"] = np.ascontiguousarray(v, np.float32), np.ascontiguousarray(i, np.uint32)
+    s["meshes"] = np.array([[len(i), 0, 0]], np.uint32)
+    model, inv, ents = [], [], []
+    for x in (-1, 0, 1):
+        for y in (-1, 0, 1):
+            for z in (-1, 0, 1):
+                if (x, y, z) == (0, 0, 0):
+                    continue
+                m, n = scenes._trs(np.array([x, y, z]) * 3.0 * scale, 1.0, np.full(3, scale))
+                ents.append((0, [5, 0][len(ents) % 2], len(ents)))
+                model.append(m)
+                inv.append(n)
+    s["model"] = np.array(model, np.float32).reshape(-1, 16)
+    s["inv_model"] = np.array(inv, np.float32).reshape(-1, 16)
+    s["entities"] = np.array(ents, np.uint32)
+    w, h = 48, 32
+    tiles = np.arange(6)
+    ref, c = pyoracle.compute_pt_tiles(s, w, h, 16, 0.8, tiles)
+    got, m = render_gpu(s, w, h, tiles)
+    same = (got.view(np.uint32) == ref.view(np.uint32)) | (np.isnan(got) & np.isnan(ref))
+    assert same.all(), f"{(~same).sum()} words differ"
+    assert (m["rays_traced"], m["ray_hit_count"]) == (int(c[0]), int(c[1]))
+    assert m["ray_hit_count"] > 0

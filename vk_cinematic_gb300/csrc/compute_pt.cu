@@ -557,9 +557,26 @@ int gbsp_cpt_scene_create(gbsp_runtime *rt, const gbsp_vertex *vertices, uint32_
         }
     }
     uint64_t triangleTests = 0, units = 0;
+    std::vector<uint32_t> openBegin(meshCount, 0xFFFFFFFFu);  // a mesh's clusters without a bound
     for (uint32_t e = 0; e < entityCount; e++) {
         const uint32_t m = entities[e].meshIndex;
         ents[e].clusterBegin = clusterBegin[m];
+        if (!cpt::unit_directions(ents[e].inv)) {
+            if (openBegin[m] == 0xFFFFFFFFu) {
+                openBegin[m] = (uint32_t)clusters.size();
+                const size_t b = clusterBegin[m], n = clusterCount[m];
+                cpt::Cluster open = {};
+                open.sphere.w = INFINITY;
+                clusters.resize(clusters.size() + n, open);
+                index.resize(index.size() + n * cpt::kClusterTris);
+                std::copy_n(index.begin() + b * cpt::kClusterTris, n * cpt::kClusterTris,
+                    index.end() - n * cpt::kClusterTris);
+                clustered.resize(clustered.size() + n * 9 * cpt::kClusterTris);
+                std::copy_n(clustered.begin() + b * 9 * cpt::kClusterTris, n * 9 * cpt::kClusterTris,
+                    clustered.end() - n * 9 * cpt::kClusterTris);
+            }
+            ents[e].clusterBegin = openBegin[m];
+        }
         ents[e].clusterCount = clusterCount[m];
         triangleTests += meshTris[m];
         units += (clusterCount[m] + 31) / 32;

@@ -7,7 +7,8 @@
 // although it passes far beside the triangle.  cluster_may_hit therefore
 // rejects a cluster only where no such rounding is possible.
 //
-// Bound.  With T = o - a, unit roundoff u = 2^-24 and |d| = 1, the computed
+// Bound.  With T = o - a, unit roundoff u = 2^-24 and |d| = 1 (unit_directions
+// says for which entities that holds; the others test all clusters), the computed
 // numerators and determinant of the test are off by at most 8 u times the
 // product of the vectors in them (7 u counted, no contraction).  Let the test
 // accept with barycentrics (x, y), p = a + x e1 + y e2 (within a few u of the
@@ -106,6 +107,30 @@ GBSP_HD bool cluster_may_hit(float4 sphere, float4 cone, float4 edge, V3 lo, V3 
     const bool outside = ql > fmaf(1.01e-3f, far, sphere.w);
     const bool away = fmaf(c, c, e * e) > fmaf(reach * reach, 1.0001f, 1e-5f);
     return !(outside && away);
+}
+
+// Whether every unit direction d comes out of an entity's space with unit length:
+// v / |v| in floats, v = R d with R the upper 3 x 3 of inv (column-major 4 x 4), has
+// unit length up to 12 u unless the squares in |v| are denormal, |v| below 1e-18.
+// |v| is at least the smallest singular value of R, itself at least 1 / |R^-1|, less
+// the rounding of the product, 3 u |R|.
+inline bool unit_directions(const float *inv)
+{
+    double r[9], norm = 0.0, adj = 0.0;
+    for (int k = 0; k < 9; k++) {
+        r[k] = inv[4 * (k / 3) + k % 3];
+        norm += r[k] * r[k];
+    }
+    double det = 0.0;
+    for (int i = 0; i < 3; i++)
+        for (int j = 0; j < 3; j++) {
+            const double c = r[3 * ((i + 1) % 3) + (j + 1) % 3] * r[3 * ((i + 2) % 3) + (j + 2) % 3] -
+                r[3 * ((i + 1) % 3) + (j + 2) % 3] * r[3 * ((i + 2) % 3) + (j + 1) % 3];
+            adj += c * c;
+            if (i == 0) det += r[j] * c;
+        }
+    const double smallest = std::fabs(det) / std::sqrt(adj);
+    return smallest >= 1e-16 && smallest >= 1e-6 * std::sqrt(norm) && std::isfinite(norm);
 }
 
 // Builds the clusters of one mesh: triangle k has vertex a[k] and edges e1[k],
