@@ -1,6 +1,8 @@
 // CPU check of the compute path tracer's cluster rejection where floats run out
-// of exponent: rays whose direction comes out of a normalisation that underflows.
-// No triangle of a rejected cluster is accepted by the triangle test.
+// of exponent: rays whose direction comes out of a normalisation that underflows,
+// meshes so small or large that products of their edges under- or overflow.  No
+// triangle of a rejected cluster is accepted by the triangle test, and what the
+// bound does not cover has no finite sphere.
 #include <cstdio>
 #include <random>
 
@@ -141,5 +143,21 @@ int main(int, char **)
             if (e <= 15 && rejected == 0) all++;
         }
     }
+    for (float size : {1.0f, -0.3f, -0.02f})
+        for (int e = -22; e <= 20; e++) {
+            long long accepted = 0, rejected = 0;
+            const float scale = powf(10.0f, (float)e);
+            const Mesh m = mesh(scale, size);
+            const long long wrong = run(m, scale, 1.0f, 600, accepted, rejected);
+            int open = 0;
+            for (const Cluster &c : m.clusters) open += std::isinf(c.sphere.w);
+            printf("size %5.2f scale %g: %lld accepted, %lld clusters rejected, %d of %zu open, %lld wrong\n", size,
+                scale, accepted, rejected, open, m.clusters.size(), wrong);
+            all += wrong;
+            // the longest edge is below 0.6 of the scale, the shortest above 1e-6 of it
+            // (without area: pole triangles, always tested)
+            if (e <= -15 || e >= 17) all += open != (int)m.clusters.size();
+            if (e >= -12 && e <= 14 && size < 0.0f) all += open != 0 || rejected == 0;
+        }
     return all ? 1 : 0;
 }

@@ -10,7 +10,10 @@
 // Bound.  With T = o - a, unit roundoff u = 2^-24 and |d| = 1 (unit_directions
 // says for which entities that holds; the others test all clusters), the computed
 // numerators and determinant of the test are off by at most 8 u times the
-// product of the vectors in them (7 u counted, no contraction).  Let the test
+// product of the vectors in them (7 u counted, no contraction; with edges of
+// 1e-15 to 1e15 what underflow adds, 2^-147 at most, is below u |e| (|T| + L), and
+// no determinant is so large that its reciprocal is denormal; a cluster with any
+// other edge is always tested).  Let the test
 // accept with barycentrics (x, y), p = a + x e1 + y e2 (within a few u of the
 // triangle), r = o - p, and r' its part perpendicular to d.  Then
 //     |r' . (d x e_i)| <= h |e_i|,   h = 8 u (|T| + L),  L = max |e_i|,
@@ -221,7 +224,7 @@ inline void build_clusters(const ClusterTriangles &t, std::vector<Cluster> &clus
             }
             const D3 m = cross3(e1, e2);
             const double len = std::sqrt(dot3(m, m)), l1 = std::sqrt(dot3(e1, e1)), l2 = std::sqrt(dot3(e2, e2));
-            if (!(len > 1e-9 * l1 * l2) || !std::isfinite(len)) {
+            if (!(len > 1e-9 * l1 * l2) || !(std::min(l1, l2) >= 1e-15 && std::max(l1, l2) <= 1e15)) {
                 bad = true;
                 continue;
             }
