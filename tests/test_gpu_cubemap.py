@@ -106,6 +106,27 @@ def test_irradiance_random_splits_the_stream(gpu_lib, hdri, width, height, spp):
     assert rel_err(got, ref).mean() <= 1e-4
 
 
+@pytest.mark.parametrize("width,height,spp", [(65, 67, 1), (65, 67, 8), (65, 67, 33), (33, 31, 1), (131, 1, 1),
+                                              (160, 90, 100), (64, 64, 34), (64, 64, 35)])
+def test_irradiance_random_lane_per_texel(gpu_lib, hdri, width, height, spp):
+    """Maps around the size from which a lane takes a whole texel, with a last
+    warp that is partly past the map, at sample counts of one run and of
+    several: the oracle's values.  With a constant image a texel is a sum of
+    spp cosines over spp, whose float sums are off by at most spp 2^-24 on
+    either side, besides the samples' own rounding (1e-6)."""
+    import torch
+
+    flat = np.ones((32, 64, 4), np.float32)
+    got = gbsp.create_irradiance_cube_map(torch.from_numpy(flat).cuda(), width, height, spp,
+                                          gbsp.IRRADIANCE_RANDOM).cpu().numpy()
+    ref = pyoracle.create_irradiance_cube_map(flat, width, height, spp, gbsp.IRRADIANCE_RANDOM)
+    assert np.abs(got - ref).max() <= 1e-6 + 2 * spp * 2.0 ** -24
+    got = gbsp.create_irradiance_cube_map(torch.from_numpy(hdri).cuda(), width, height, spp,
+                                          gbsp.IRRADIANCE_RANDOM).cpu().numpy()
+    ref = pyoracle.create_irradiance_cube_map(hdri, width, height, spp, gbsp.IRRADIANCE_RANDOM)
+    assert rel_err(got, ref).mean() <= 1e-4
+
+
 def test_rejects_bad_arguments(gpu_lib):
     import torch
 

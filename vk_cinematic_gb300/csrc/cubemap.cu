@@ -201,8 +201,54 @@ __global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_uniform(Image im,
 
 struct JumpTables {
     uint32_t texel[32][32];  // texel[b][c]: column c of J^(2^b)
-    uint32_t lane[32][32];   // lane[l][c]: column c of M^(3 run l), lane l's first sample
+    uint32_t lane[32][32];   // lane[l][c]: column c of M^(3 step l), lane l's first sample
+    uint32_t step;           // samples between the lanes' first ones
 };
+
+// The tables in shared memory, and the state of lane l of a warp whose first
+// sample is that of texel i.
+struct SharedJumps {
+    uint32_t texelCols[32][32], laneCols[32][33];  // laneCols[c][l]
+    __device__ __forceinline__ void load(const JumpTables &jumps)
+    {
+        for (uint32_t k = threadIdx.x; k < 1024; k += blockDim.x) {
+            texelCols[k >> 5][k & 31] = jumps.texel[k >> 5][k & 31];
+            laneCols[k & 31][k >> 5] = jumps.lane[k >> 5][k & 31];
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ uint32_t state(uint32_t seed, uint32_t i, uint32_t lane) const
+    {
+        uint32_t state = seed;
+        for (uint32_t bits = i; bits; bits &= bits - 1)
+            state = __reduce_xor_sync(0xFFFFFFFFu, state >> lane & 1u ? texelCols[__ffs(bits) - 1][lane] : 0u);
+        uint32_t rng = 0;
+        for (uint32_t bits = state; bits; bits &= bits - 1) rng ^= laneCols[__ffs(bits) - 1][lane];
+        return rng;
+    }
+};
+
+// irr plus `count` samples around dir, one after another.
+__device__ __forceinline__ V3 add_samples(V3 irr, const Image &im, V3 dir, uint64_t count, float contribution,
+    uint32_t &rng)
+{
+    for (uint64_t k = 0; k < count; k++) {
+        // Vec3(RandomBilateral() x3) with GCC's right-to-left argument order
+        float oz = random_bilateral(rng);
+        float oy = random_bilateral(rng);
+        float ox = random_bilateral(rng);
+        V3 sd = normalize(add(dir, v3(ox, oy, oz)));
+        if (dot(sd, dir) < 0.0f) sd = neg(sd);
+        float cosine = rmax(dot(dir, sd), 0.0f);
+        float u, v;
+        direction_uv(sd, u, v);
+        float4 s = sample_bilinear(im, u, v);
+        V3 rad = v3(rclamp(s.x * cosine, 0.0f, kRadianceClamp),
+            rclamp(s.y * cosine, 0.0f, kRadianceClamp), rclamp(s.z * cosine, 0.0f, kRadianceClamp));
+        irr = add(irr, mul(rad, contribution));
+    }
+    return irr;
+}
 
 // Bound: latency of the samples' dependent chains (random numbers, direction,
 // lookup).  A thread per texel walked all of its samples one after another,
@@ -210,45 +256,23 @@ struct JumpTables {
 // table's upload.  6 x 8^2 texels of 128 samples 394 -> 47 us for the call, 6 x
 // 64^2 of 8 300 -> 96, of 128 401 -> 122; the host's tables take 25 us of it.
 __global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_random(Image im, uint32_t width,
-    uint32_t height, uint32_t spp, uint32_t run, const __grid_constant__ JumpTables jumps, uint32_t seed,
+    uint32_t height, uint32_t spp, const __grid_constant__ JumpTables jumps, uint32_t seed,
     float4 *__restrict__ out)
 {
-    __shared__ uint32_t texelCols[32][32], laneCols[32][33];  // laneCols[c][l]
-    for (uint32_t k = threadIdx.x; k < 1024; k += blockDim.x) {
-        texelCols[k >> 5][k & 31] = jumps.texel[k >> 5][k & 31];
-        laneCols[k & 31][k >> 5] = jumps.lane[k >> 5][k & 31];
-    }
-    __syncthreads();
+    __shared__ SharedJumps shared;
+    shared.load(jumps);
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t total = 6u * width * height;  // checked to fit
     const uint32_t warps = gridDim.x * kIrrWarps;
     const float contribution = 1.0f / (float)spp;
-    // 64 bits: run * lane may pass 2^32
-    const uint64_t first = (uint64_t)run * lane, last = min((uint64_t)spp, first + run);
+    // 64 bits: step * lane may pass 2^32
+    const uint64_t first = min((uint64_t)spp, (uint64_t)jumps.step * lane),
+                   count = min((uint64_t)spp - first, (uint64_t)jumps.step);
     for (uint64_t i64 = blockIdx.x * kIrrWarps + (threadIdx.x >> 5); i64 < total; i64 += warps) {
         const uint32_t i = (uint32_t)i64, x = i % width, y = i / width % height, layer = i / width / height;
-        uint32_t state = seed;
-        for (uint32_t bits = i; bits; bits &= bits - 1)
-            state = __reduce_xor_sync(0xFFFFFFFFu, state >> lane & 1u ? texelCols[__ffs(bits) - 1][lane] : 0u);
-        uint32_t rng = 0;
-        for (uint32_t bits = state; bits; bits &= bits - 1) rng ^= laneCols[__ffs(bits) - 1][lane];
-        V3 dir = face_direction(face_basis(layer), x, y, width, height);
-        V3 irr = v3(0.0f, 0.0f, 0.0f);
-        for (uint64_t k = first; k < last; k++) {
-            // Vec3(RandomBilateral() x3) with GCC's right-to-left argument order
-            float oz = random_bilateral(rng);
-            float oy = random_bilateral(rng);
-            float ox = random_bilateral(rng);
-            V3 sd = normalize(add(dir, v3(ox, oy, oz)));
-            if (dot(sd, dir) < 0.0f) sd = neg(sd);
-            float cosine = rmax(dot(dir, sd), 0.0f);
-            float u, v;
-            direction_uv(sd, u, v);
-            float4 s = sample_bilinear(im, u, v);
-            V3 rad = v3(rclamp(s.x * cosine, 0.0f, kRadianceClamp),
-                rclamp(s.y * cosine, 0.0f, kRadianceClamp), rclamp(s.z * cosine, 0.0f, kRadianceClamp));
-            irr = add(irr, mul(rad, contribution));
-        }
+        uint32_t rng = shared.state(seed, i, lane);
+        const V3 dir = face_direction(face_basis(layer), x, y, width, height);
+        V3 irr = add_samples(v3(0.0f, 0.0f, 0.0f), im, dir, count, contribution, rng);
 #pragma unroll
         for (int off = 16; off; off >>= 1) {
             irr.x += __shfl_xor_sync(0xFFFFFFFFu, irr.x, off);
@@ -256,6 +280,55 @@ __global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_random(Image im, 
             irr.z += __shfl_xor_sync(0xFFFFFFFFu, irr.z, off);
         }
         if (lane == 0) out[i] = make_float4(irr.x, irr.y, irr.z, 1.0f);
+    }
+}
+
+// Whether a lane takes a whole texel.  A warp per texel jumps for each of them and
+// leaves lanes idle below 32 samples and behind 33 (0.67 + 0.28 run ns a texel); a
+// lane per texel takes 0.035 + 0.011 spp ns but at least 0.73 us a sample, its chain.
+// The line is where the chain is 1.2 times shorter than the warps' work; from 257
+// samples on the jump no longer shows and the warps' finer grain wins (256^2 of 512:
+// 2,217 us, 2,345 with lanes).  Calls in us, warp and lane per texel, maps of 6 x:
+//   32^2   1 sample  46  40;    8  49  51;  128  67  143
+//   64^2   8 samples 90  51;   33  99  74;  128 116  145
+//   128^2  8 samples 150 65;   33 183 102;  128 243  221
+//   512^2  8 samples 1,509 254;  33 1,904 710;  128 2,800 2,291
+// (a thread per texel that jumped by itself, with an upload per call: 512^2 543, 956
+// and 2,562).
+static bool lane_per_texel(uint64_t texels, uint32_t spp, uint32_t run)
+{
+    return run <= 8 && texels * (12 + 5 * run) >= 16000ull * spp;
+}
+
+// The same values with a lane per texel: a warp jumps once for 32 texels, and a
+// lane adds the sums of the runs in the order of the warp's reduction above.
+__global__ void __launch_bounds__(32 * kIrrWarps) k_irradiance_random_wide(Image im, uint32_t width,
+    uint32_t height, uint32_t spp, uint32_t run, const __grid_constant__ JumpTables jumps, uint32_t seed,
+    float4 *__restrict__ out)
+{
+    __shared__ SharedJumps shared;
+    shared.load(jumps);
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t total = 6u * width * height;  // checked to fit
+    const uint64_t texels = 32ull * kIrrWarps * gridDim.x;
+    const float contribution = 1.0f / (float)spp;
+    const int runs = (int)((spp + (uint64_t)run - 1) / run);  // at most 32
+    for (uint64_t base = 32ull * (blockIdx.x * kIrrWarps + (threadIdx.x >> 5)); base < total; base += texels) {
+        uint32_t rng = shared.state(seed, (uint32_t)base, lane);
+        const uint64_t i64 = base + lane;
+        if (i64 >= total) continue;
+        const uint32_t i = (uint32_t)i64, x = i % width, y = i / width % height, layer = i / width / height;
+        const V3 dir = face_direction(face_basis(layer), x, y, width, height);
+        V3 sums[16];
+        for (int r = 0; r < runs; r++) {
+            const uint64_t first = (uint64_t)run * r;
+            const V3 sum = add_samples(v3(0.0f, 0.0f, 0.0f), im, dir, min((uint64_t)run, spp - first),
+                contribution, rng);
+            sums[r & 15] = r < 16 ? sum : add(sums[r & 15], sum);
+        }
+        for (int off = 8; off; off >>= 1)
+            for (int r = 0; r < off && r + off < runs; r++) sums[r] = add(sums[r], sums[r + off]);
+        out[i] = make_float4(sums[0].x, sums[0].y, sums[0].z, 1.0f);
     }
 }
 
@@ -380,25 +453,32 @@ int gbsp_create_irradiance_cube_map(void *stream, const float *equirect, uint32_
         GBSP_CUDA_TRY(cudaGetLastError());
         return GBSP_OK;
     }
-    // random mode: lane l of a texel's warp takes samples run l, run l + 1, ...
+    // random mode: a texel's sum is that of up to 32 runs of `run` samples each
     const uint32_t run = (uint32_t)(((uint64_t)samplesPerPixel + 31) / 32);
+    const bool wide = cube::lane_per_texel(total, samplesPerPixel, run);
     cube::JumpTables jumps = {};
+    jumps.step = wide ? samplesPerPixel : run;
     const auto copy = [](uint32_t *dst, const cube::Mat &m) { std::copy(m.begin(), m.end(), dst); };
     cube::Mat j = cube::power(cube::step_matrix(), 3ull * samplesPerPixel);
     for (int b = 0; b < 32 && total >> b; b++) {
         copy(jumps.texel[b], j);
         j = cube::multiply(j, j);
     }
-    const cube::Mat step = cube::power(cube::step_matrix(), 3ull * run);
+    const cube::Mat step = cube::power(cube::step_matrix(), 3ull * jumps.step);
     j = cube::power(step, 0);
-    for (uint64_t l = 0; l < 32 && l * run < samplesPerPixel; l++) {
+    for (uint64_t l = 0; l < 32 && (wide || l * run < samplesPerPixel); l++) {
         copy(jumps.lane[l], j);
         j = cube::multiply(j, step);
     }
-    const uint64_t blocks = (total + cube::kIrrWarps - 1) / cube::kIrrWarps;
-    const int block = 32 * cube::kIrrWarps;
-    cube::k_irradiance_random<<<grid_for(blocks * block, block), block, 0, s>>>(im, width, height,
-        samplesPerPixel, run, jumps, 0x45BA12F3u, reinterpret_cast<float4 *>(faces));
+    const uint64_t warps = wide ? (total + 31) / 32 : total;
+    const uint64_t blocks = (warps + cube::kIrrWarps - 1) / cube::kIrrWarps;
+    const int block = 32 * cube::kIrrWarps, grid = grid_for(blocks * block, block);
+    if (wide)
+        cube::k_irradiance_random_wide<<<grid, block, 0, s>>>(im, width, height, samplesPerPixel, run, jumps,
+            0x45BA12F3u, reinterpret_cast<float4 *>(faces));
+    else
+        cube::k_irradiance_random<<<grid, block, 0, s>>>(im, width, height, samplesPerPixel, jumps,
+            0x45BA12F3u, reinterpret_cast<float4 *>(faces));
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;
 }
