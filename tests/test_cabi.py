@@ -187,3 +187,26 @@ def test_header_is_plain_c_and_links(tmp_path):
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=60)
     assert r.returncode == 0, r.stderr
     assert int(r.stdout.strip()) == len(names)
+
+
+@pytest.mark.parametrize("bad", [0, 31, 32, 70])
+def test_adam_refuses_before_it_updates_anything(bad):
+    """A NULL pointer anywhere among the tensors is refused before the first
+    launch (32 tensors each), so a refused step has changed nothing.  (A launch
+    would fail here, without a device, with another error.)"""
+    import ctypes
+
+    import torch
+
+    if torch.cuda.is_available():
+        pytest.skip("for a host without a device")
+    lib = gbsp.load()
+    rows = np.full((71, 6), 256, np.uint64)  # never dereferenced
+    rows[:, 1] = 0
+    rows[bad, 2] = 0
+    f = ctypes.c_float
+    rc = lib.gbsp_dn_adam_all(None, rows.ctypes.data_as(ctypes.c_void_p), ctypes.c_uint32(71), f(1e-3), f(0.9),
+                              f(0.999), f(1e-8), ctypes.c_uint32(1))
+    lib.gbsp_last_error_string.restype = ctypes.c_char_p
+    assert rc != 0
+    assert f"tensor {bad} has a NULL pointer" in lib.gbsp_last_error_string().decode()

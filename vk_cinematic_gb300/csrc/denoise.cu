@@ -2213,6 +2213,12 @@ int gbsp_dn_adam_all(void *stream, const gbsp_dn_adam_tensor *tensors, uint32_t 
     float beta1, float beta2, float eps, uint32_t step)
 {
     if (count && !tensors) return set_error(GBSP_ERR_INVALID_ARGUMENT, "tensors is NULL");
+    for (uint32_t k = 0; k < count; k++) {  // all of them before the first is updated
+        const gbsp_dn_adam_tensor &t = tensors[k];
+        if (t.n && (!t.param || !t.grad || !t.m || !t.v))
+            return set_error(GBSP_ERR_INVALID_ARGUMENT, "Adam tensor %u has a NULL pointer", k);
+        if ((t.n + 255) / 256 > 0x7FFFFFFFull) return set_error(GBSP_ERR_CAPACITY, "too many parameters");
+    }
     float c1 = 1.0f - powf(beta1, (float)step), c2 = 1.0f - powf(beta2, (float)step);
     for (uint32_t k0 = 0; k0 < count;) {
         AdamTensors a = {};
@@ -2221,12 +2227,10 @@ int gbsp_dn_adam_all(void *stream, const gbsp_dn_adam_tensor *tensors, uint32_t 
         for (; k0 < count && n < kAdamTensors; k0++) {
             const gbsp_dn_adam_tensor &t = tensors[k0];
             if (!t.n) continue;
-            if (!t.param || !t.grad || !t.m || !t.v)
-                return set_error(GBSP_ERR_INVALID_ARGUMENT, "Adam tensor %u has a NULL pointer", k0);
+            if (block + (t.n + 255) / 256 > 0x7FFFFFFFull) break;  // in a launch of its own
             a.t[n] = t;
             a.firstBlock[n++] = (uint32_t)block;
             block += (t.n + 255) / 256;
-            if (block > 0x7FFFFFFFull) return set_error(GBSP_ERR_CAPACITY, "too many parameters");
         }
         if (!n) break;
         a.firstBlock[n] = (uint32_t)block;
