@@ -93,3 +93,15 @@ def test_cpu_tile_samples_are_whole_waves_spread_over_the_frame():
         assert 1 <= n <= total
         assert n == total or n % threads == 0
         assert n == total or n * per_tile / threads >= target * 0.999 or n == threads
+
+
+def test_reference_arm_says_that_it_is_unavailable():
+    """The reference does not build on the host, and no code of this repository
+    may stand in for it: one line with the reason, and no value."""
+    import json
+
+    r = subprocess.run([sys.executable, os.path.join(ROOT, "bench.py"), "--impl", "reference", "--steps", "1",
+                        "--warmup", "0"], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stderr
+    line = json.loads(r.stdout)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line
