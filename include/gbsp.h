@@ -404,9 +404,11 @@ int gbsp_batch_launch(gbsp_batch *batch, gbsp_metrics *metrics);
  * as CUDA: replaces its Vulkan dispatch (src/vulkan_renderer.cpp:1340-1368:
  * up to 64 tile indices in push constants, one invocation per tile) and the
  * descriptor bindings of its scene buffers (test_compute.comp.glsl:60-100).
- * Brute-force closest hit over every entity's triangles, RNG chained through
- * each tile, three bounces, hard-coded material ids (0 red, 2 checkerboard,
- * 5 white light, others black). */
+ * The closest hit is that of a brute-force test of every entity's triangles
+ * (clusters of triangles that provably hold no hit are skipped), RNG chained
+ * through each tile, three bounces, hard-coded material ids (0 red,
+ * 2 checkerboard, 5 white light, others black).  TRIANGLE_TESTS counts what
+ * brute force tests, rays times triangles, not the tests carried out. */
 typedef struct gbsp_cpt_scene gbsp_cpt_scene;
 
 typedef struct {                 /* Mesh, test_compute.comp.glsl:46-51 */

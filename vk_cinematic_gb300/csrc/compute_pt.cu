@@ -29,9 +29,9 @@
 // longest tile has 768 rays).  A ray among 18 spheres of 1,280 triangles costs
 // 1,440 cluster tests and the tests of about 55 listed clusters instead of
 // 23,042 triangle tests.  512 x 384 pixels of that scene: 107.5 ms with a warp
-// per tile and every triangle staged through shared memory, 5.45 ms now (5.88
-// before the cluster test's sums were fused multiply-adds and the winner a
-// minimum reduction).  Before those two: 4 blocks of 8 warps per SM (64
+// per tile and every triangle staged through shared memory, 5.6 to 5.8 ms now
+// (three machines; 0.4 more before the cluster test's sums were fused multiply-adds
+// and the winner a minimum reduction).  Before those two: 4 blocks of 8 warps per SM (64
 // registers) 5.88 ms, unbounded (2 blocks) 7.4, 4 warps 6.6 and 2 warps per
 // tile 9.8 ms.  Worse since: clusters of 8 or 32 triangles 6.4 and 7.7 ms, one
 // list for all warps of a tile (a barrier more) 6.1, the next clusters loaded

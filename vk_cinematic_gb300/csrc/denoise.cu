@@ -220,16 +220,17 @@ int launch_conv(cudaStream_t s, int smCount, const void *in, int B, int H, int W
 // other roles' waits, and sets g_dnStatus.
 //
 // What bounds it (48 -> 48 at 1080p, 85.9 GFLOP, 398 MB in and out): memory, 69
-// us by itself = 5.8 TB/s (79 before strip_rows), with the MMAs behind it (54 of
-// about 70 cycles per row group, 49 us).  Before, 99 us: the issuing thread waited on six row barriers per
-// group at about 340 cycles each, none of it hidden (without loads, stores and
+// us by itself = 5.8 TB/s (79 before strip_rows), with the MMAs behind it (54 per
+// row group, of about 70 cycles each: 49 us).  Before, 99 us: the issuing thread
+// waited on six row barriers per group at about 340 cycles each, none of it hidden
+// (without loads, stores and
 // eight ninths of the MMAs 47 us; with one wait per group 29); and TMA boxes of
 // [group][130 pixels][8 channels] move 16 bytes per request (loads alone 60
 // us, 49 as runs).  Two epilogue groups per accumulator: 79 us, the same.
 // ---------------------------------------------------------------------------
 constexpr int kTcTileP = 128;
-// One CTA per SM: warp 0 issues the MMAs, lane 0 of warp 1 loads rows, warps 4-11 are
-// two epilogue groups that take alternate row groups.
+// One CTA per SM: warp 0 issues the MMAs, warp 1 loads rows (a lane per channel plane
+// of a row pair), warps 4-11 are two epilogue groups that take alternate row groups.
 constexpr int kTcThreads = 384;
 constexpr int kTcEpiGroups = 2;
 constexpr int kTcAccSlots = 4;  // at most; accumulator a is drained by epilogue group a % 2

@@ -229,7 +229,8 @@ __device__ __forceinline__ uint32_t visit_node8(const float4 *__restrict__ pool,
             const bool present = cc[j] != kEmptyChild;
             boxes += present ? 1u : 0u;
             // tf is NaN (a miss) when the origin is NaN in every component; fminf(tf,
-            // bound) would drop it and take every box
+            // bound) would drop it and take every box.  In time the same as fminf was;
+            // min.NaN cost frames and rays 2% and a batch 4%, `&& tn <= bound` rays 3%
             const bool hit = present && tn <= tf && !(tn > bound);
             const bool closer = tn < nearT;
             const StackEntry push{closer ? nearRef : cc[j], closer ? nearT : tn};

@@ -360,7 +360,8 @@ class KPCNN:
 
     def weight_grads(self, todo, inputs, dws, dbs):
         """weight_grad for several (layer, output gradient) pairs of one batch;
-        on the tcgen05 path a launch per layer shape and one reduction."""
+        on the tcgen05 path a launch per layer shape and one reduction.  The
+        gradients are kept until then: at most WGRAD_KEEP bytes of them."""
         import torch
 
         if self.wgrad_impl != "tcgen05":
@@ -379,7 +380,8 @@ class KPCNN:
                                                    scratch.data_ptr()))
 
     def gradients(self, feats, noisy, target):
-        """Loss and parameter gradients for one batch."""
+        """Loss and parameter gradients for one batch.  Beside the activations
+        it holds up to WGRAD_KEEP (4 GiB) bytes of the layers' output gradients."""
         import torch
 
         B, H, W, _ = noisy.shape
