@@ -79,8 +79,11 @@ __device__ __forceinline__ void load_ray(const float *rays, size_t i, V3 &o, V3 
 // general node visits); at 4 warps per SM 30.0, 40.4 and 41.3, at 14 27.1, 35.8
 // and 40.2, at 28 37.4, 44.6 and 45.6 us.  The per-lane path's three launches
 // cost 35 us for one ray where this takes 8.
+// 7 blocks per SM (72 registers) are for 8-wide nodes; walks of a width read from the
+// scene spill at that: 40,000 watertight rays over 4-wide nodes 50.2 us so, 48.5
+// without the bound.
 template <bool kWT, int kQ, bool kPacked>
-__global__ void __launch_bounds__(128, 7) k_intersect(SceneView sv, const float *__restrict__ rays,
+__global__ void __launch_bounds__(128, kQ == 2 ? 7 : 1) k_intersect(SceneView sv, const float *__restrict__ rays,
     uint32_t count, uint32_t lanes, QueryOutputs out, unsigned long long *counters, uint32_t *status)
 {
     const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
