@@ -127,6 +127,18 @@ def test_irradiance_random_lane_per_texel(gpu_lib, hdri, width, height, spp):
     assert rel_err(got, ref).mean() <= 1e-4
 
 
+@pytest.mark.parametrize("width,height", [(1, 700), (2, 257), (3, 129), (7, 64), (9, 33), (17, 40), (41, 300)])
+def test_cube_map_narrow_blocks(gpu_lib, hdri, width, height):
+    # widths for which a block is 1, 2, 8 and 16 texels wide, partly past the map's rows
+    import torch
+
+    got = gbsp.create_cube_map(torch.from_numpy(hdri).cuda(), width, height).cpu().numpy()
+    ref = pyoracle.create_cube_map(hdri, width, height)
+    e = rel_err(got, ref)
+    assert np.median(e) <= 1e-5
+    assert np.mean(e > 1e-3) <= max(1e-3, 3 / e.size)
+
+
 def test_rejects_bad_arguments(gpu_lib):
     import torch
 

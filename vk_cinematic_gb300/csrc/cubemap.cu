@@ -120,15 +120,32 @@ __device__ __forceinline__ V3 face_direction(const Basis &b, uint32_t x, uint32_
 // up to four rows of a column (the column's division and products once) while
 // that leaves two waves of blocks: with the irradiance map 162.4 -> 156.3 us (two
 // rows 158.9, eight 158.6).
-constexpr int kCubeX = 32, kCubeY = 8;
+//
+// Blocks are kX = 32 texels wide, or where that pads the rows by more than a quarter
+// as wide as pads them least (below 16 texels down to one; from there on blocks of 4
+// lose 0.3 us on small maps).  6 x 1 x 4096 texels 9.7 -> 2.2 us, 6 x 33 x 4000 16.1
+// -> 11.2; a flat index took 2.6 and 11.9.
+constexpr uint32_t kCubeThreads = 256;
 
-__global__ void __launch_bounds__(kCubeX * kCubeY) k_cube_map(Image im, uint32_t width, uint32_t height,
+static uint32_t cube_block_width(uint32_t width)
+{
+    uint32_t best = 32;
+    const auto padded = [&](uint32_t x) { return ((uint64_t)width + x - 1) / x * x; };
+    if (4 * padded(32) <= 5 * (uint64_t)width) return 32;
+    for (uint32_t x = 16; x; x >>= 1)
+        if ((x >= 8 || width < 16) && padded(x) < padded(best)) best = x;
+    return best;
+}
+
+template <int kX>
+__global__ void __launch_bounds__(kCubeThreads) k_cube_map(Image im, uint32_t width, uint32_t height,
     float4 *__restrict__ out)
 {
-    const uint32_t x = blockIdx.x * kCubeX + threadIdx.x, layer = blockIdx.z;
+    constexpr uint32_t kY = kCubeThreads / kX;
+    const uint32_t x = blockIdx.x * kX + threadIdx.x, layer = blockIdx.z;
     if (x >= width) return;
     const Basis b = face_basis(layer);
-    for (uint32_t y = blockIdx.y * kCubeY + threadIdx.y; y < height; y += gridDim.y * kCubeY) {
+    for (uint32_t y = blockIdx.y * kY + threadIdx.y; y < height; y += gridDim.y * kY) {
         V3 dir = face_direction(b, x, y, width, height);
         float u, v;
         direction_uv(dir, u, v);
@@ -414,12 +431,18 @@ int gbsp_create_cube_map(void *stream, const float *equirect, uint32_t eqWidth, 
     int rc = check_image(equirect, eqWidth, eqHeight, width, height, faces);
     if (rc) return rc;
     cube::Image im{reinterpret_cast<const float4 *>(equirect), eqWidth, eqHeight};
-    const uint32_t cols = (width + cube::kCubeX - 1) / cube::kCubeX,
-                   bands = (height + cube::kCubeY - 1) / cube::kCubeY;
+    const dim3 block(cube::cube_block_width(width), cube::kCubeThreads / cube::cube_block_width(width));
+    const uint32_t cols = (width + block.x - 1) / block.x, bands = (height + block.y - 1) / block.y;
     // two waves of 8 blocks per SM
     const uint64_t rows = std::min<uint64_t>(4, std::max<uint64_t>(1, 6ull * cols * bands / (16ull * sm_count())));
     const dim3 grid(cols, (uint32_t)std::min<uint64_t>((bands + rows - 1) / rows, 65535u), 6);
-    cube::k_cube_map<<<grid, dim3(cube::kCubeX, cube::kCubeY), 0, (cudaStream_t)stream>>>(im, width, height,
+    auto kern = block.x == 32 ? cube::k_cube_map<32>
+        : block.x == 16       ? cube::k_cube_map<16>
+        : block.x == 8        ? cube::k_cube_map<8>
+        : block.x == 4        ? cube::k_cube_map<4>
+        : block.x == 2        ? cube::k_cube_map<2>
+                              : cube::k_cube_map<1>;
+    kern<<<grid, block, 0, (cudaStream_t)stream>>>(im, width, height,
         reinterpret_cast<float4 *>(faces));
     GBSP_CUDA_TRY(cudaGetLastError());
     return GBSP_OK;

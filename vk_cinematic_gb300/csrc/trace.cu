@@ -80,8 +80,8 @@ __device__ __forceinline__ void load_ray(const float *rays, size_t i, V3 &o, V3 
 // and 40.2, at 28 37.4, 44.6 and 45.6 us.  The per-lane path's three launches
 // cost 35 us for one ray where this takes 8.
 // 7 blocks per SM (72 registers) are for 8-wide nodes; walks of a width read from the
-// scene spill at that: 40,000 watertight rays over 4-wide nodes 50.2 us so, 48.5
-// without the bound.
+// scene take 88 to 92 without a bound: 40,000 watertight rays over 4-wide nodes
+// 50.2 us with it, 48.5 without.
 template <bool kWT, int kQ, bool kPacked>
 __global__ void __launch_bounds__(128, kQ == 2 ? 7 : 1) k_intersect(SceneView sv, const float *__restrict__ rays,
     uint32_t count, uint32_t lanes, QueryOutputs out, unsigned long long *counters, uint32_t *status)
